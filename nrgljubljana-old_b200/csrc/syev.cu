@@ -15,18 +15,17 @@
 //    keeps them orthogonal without extra precision.
 #include <map>
 #include <mutex>
-#include <cooperative_groups.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
 #include <numeric>
-#include <type_traits>
 
 #include "gemm_f64.cuh"
 #include "syev.cuh"
 #include "schedule.cuh"
+#include "trd_regs.cuh"
 
 namespace nrgb {
 
@@ -37,9 +36,6 @@ constexpr int LEAF = 16;        // D&C leaf size
 constexpr int NB = 32;          // tridiagonalisation panel width
 constexpr int NBB = 64;         // back-transformation block of reflectors
 constexpr int TRD_NT = 256;     // threads of the panel kernel
-constexpr int TRDC_NT = 256;    // threads of a CTA of the cluster kernel
-constexpr size_t TRDC_SMEM = 227 * 1024;  // shared memory one CTA of the cluster kernel may use
-constexpr int TRDC_CL_MAX = 16;           // largest cluster (non-portable above 8)
 constexpr double EPS = 2.220446049250313e-16;
 
 // --------------------------------------------------------------------------
@@ -475,837 +471,6 @@ __global__ void __launch_bounds__(TRD_NT) trd_panel_kernel(const TrdProb* __rest
   }
   // a barrier that gave up is reported to the host (the barriers are reset per launch)
   if (tid == 0 && *reinterpret_cast<volatile int*>(&bar->error)) atomicExch(fail, 1);
-}
-
-// --------------------------------------------------------------------------
-// Tridiagonalisation of a medium block inside one thread-block cluster.
-// --------------------------------------------------------------------------
-struct TrdClProb {
-  double* A;    // n x n, leading dimension ld: input; on return the reflectors below the subdiagonal
-  double* d;    // n
-  double* e;    // n-1
-  double* tau;  // n-1
-  int n;
-  int ld;       // n for a whole block; the block's size for its trailing part
-};
-
-// Leading dimension of a column held in shared memory: odd, so that 32 lanes
-// reading the same row of 32 different columns hit 32 different banks.
-__host__ __device__ inline int trdc_ld(int n) { return n | 1; }
-
-// Doubles of dynamic shared memory one CTA needs for a block of size n on
-// a cluster of cl CTAs: its columns (j = rank, rank + cl, ...) in full, then
-// v and y (n each), one partial column dot per thread, one partial sum of
-// y^T v per warp of every CTA, 2 x 4 scalars.
-__host__ __device__ inline size_t trdc_smem_doubles(int n, int cl) {
-  return (size_t)((n + cl - 1) / cl) * trdc_ld(n) + 2 * (size_t)n + TRDC_NT + (size_t)cl * (TRDC_NT / 32) + 8;
-}
-
-// Active held columns up to this count take the warp-per-column-group
-// product (lanes across rows, shuffle reductions, no CTA barrier); more take
-// lanes across columns (no shuffles) with a CTA barrier before the sums.
-constexpr int TRDC_WARPCOL_MAX = 32;
-
-// Barrier over the CTAs of the cluster (a plain CTA barrier for CL = 1).
-template <int CL>
-__device__ __forceinline__ void trdc_sync() {
-  if constexpr (CL == 1) {
-    __syncthreads();
-  } else {
-    cooperative_groups::this_cluster().sync();
-  }
-}
-
-// Address of `p` in the shared memory of CTA `rank` of the cluster.
-template <int CL, class T>
-__device__ __forceinline__ T* trdc_at(T* p, int rank) {
-  if constexpr (CL == 1) {
-    return p;
-  } else {
-    return cooperative_groups::this_cluster().map_shared_rank(p, rank);
-  }
-}
-
-// Reflector of column cc, held in shared memory (`col`), by one warp of its
-// owner: beta, tau and the scale of v, written into every CTA's scalars
-// `mc`; d, e, tau to global memory.
-template <int CL>
-__device__ __forceinline__ void trdc_reflector(const TrdClProb& P, const double* col, int cc, int n, double* mc,
-                                               int lane) {
-  double ss = 0.0;
-  for (int i = cc + 2 + lane; i < n; i += 32) ss += col[i] * col[i];
-  ss = warp_sum(ss);
-  const double alpha = col[cc + 1];
-  double beta = alpha, tc = 0.0, scal = 0.0;
-  if (ss != 0.0) {
-    beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-    tc = (beta - alpha) / beta;
-    scal = 1.0 / (alpha - beta);
-  }
-  if (lane < CL) {
-    double* rm = trdc_at<CL>(mc, lane);
-    rm[0] = tc;
-    rm[1] = scal;
-  }
-  if (lane == 0) {
-    P.d[cc] = col[cc];
-    P.e[cc] = beta;
-    P.tau[cc] = tc;
-  }
-}
-
-// Unblocked Householder tridiagonalisation (the dsytd2 recurrence, lower)
-// of one block per cluster of CL CTAs.  The matrix lives in the CTAs'
-// shared memory, distributed by columns (CTA r holds the columns j with
-// j % CL == r, each in full), so the symmetric product y = A v needs no
-// reduction across CTAs: y_j is the dot product of the held column j with v.
-// Per column c, two cluster barriers:
-//   a. every CTA reads the owner's column c through distributed shared
-//      memory to form v (CTA barrier) and computes y_j for its columns:
-//      with few active columns each warp takes four columns at a time
-//      (lanes across rows, shuffle reductions); with many, lanes take
-//      columns and warps row segments, summed after a CTA barrier.  Each
-//      y_j goes into every CTA, and each warp's part of y^T v into its own
-//      slot of every CTA; cluster barrier;
-//   b. every warp sums the slots (all in the same order, so every CTA
-//      holds the same y^T v) and applies A -= v w^T + w v^T to its columns
-//      with w = tau y - tau^2/2 (y^T v) v formed on the fly (loads of four
-//      columns and two rows issued before their stores).  Meanwhile warp 0
-//      of the owner of column c+1 updates that column first and forms its
-//      reflector (norm, beta, tau), writing the scalars into every CTA;
-//      cluster barrier.
-// Output as the panel kernel: d, e, tau, and v below the subdiagonal of A.
-template <int CL>
-__global__ void __launch_bounds__(TRDC_NT) trd_cluster_kernel(const TrdClProb* __restrict__ probs) {
-  int r = 0;
-  if constexpr (CL > 1) r = (int)cooperative_groups::this_cluster().block_rank();
-  const TrdClProb P = probs[blockIdx.x / CL];
-  const int n = P.n;
-  const size_t ld = (size_t)P.ld;
-  const int lds = trdc_ld(n);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int nwarps = TRDC_NT / 32;
-  const int ncol = r < n ? (n - r + CL - 1) / CL : 0;
-  extern __shared__ double sm[];
-  double* Acol = sm;                                     // ncol columns, ld lds
-  double* v = Acol + (size_t)((n + CL - 1) / CL) * lds;  // n
-  double* y = v + n;                                     // n (written by every CTA)
-  double* ypart = y + n;                                 // TRDC_NT partial column dots
-  double* part = ypart + TRDC_NT;                        // CL x nwarps parts of y^T v
-  double* misc = part + CL * nwarps;                     // 2 x 4 reflector scalars
-
-  for (int l = 0; l < ncol; ++l) {
-    const double* src = P.A + (size_t)(r + l * CL) * ld;
-    for (int i = tid; i < n; i += TRDC_NT) Acol[(size_t)l * lds + i] = src[i];
-  }
-  // every CTA of the cluster has started (and loaded) before any of them
-  // touches another's shared memory
-  trdc_sync<CL>();
-  if (n > 1 && r == 0 && warp == 0) trdc_reflector<CL>(P, Acol, 0, n, misc, lane);
-  trdc_sync<CL>();
-
-  for (int c = 0; c < n - 1; ++c) {
-    const int o = c % CL;
-    const double* mc = misc + (c & 1) * 4;
-    // ---- a: v, y_j for the columns held here, parts of y^T v ----
-    const double tc = mc[0], scal = mc[1];
-    {
-      const double* ocol = trdc_at<CL>(Acol, o) + (size_t)(c / CL) * lds;
-      for (int i = c + 1 + tid; i < n; i += TRDC_NT) v[i] = (i == c + 1) ? 1.0 : ocol[i] * scal;
-    }
-    __syncthreads();
-    // held columns after c: local indices l0 .. ncol-1
-    const int l0 = (c + 1 - r + CL - 1) / CL > 0 ? (c + 1 - r + CL - 1) / CL : 0;
-    const int nact = ncol > l0 ? ncol - l0 : 0;
-    double sp = 0.0;
-    if (nact <= TRDC_WARPCOL_MAX) {
-      // warp w: active columns t = w, w + nwarps, ..., four at a time
-      for (int t0 = warp; t0 < nact; t0 += 4 * nwarps) {
-        const double* a[4];
-        bool on[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int t = t0 + k * nwarps;
-          on[k] = t < nact;
-          a[k] = Acol + (size_t)(l0 + (on[k] ? t : t0)) * lds;
-        }
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = c + 1 + lane; i < n; i += 32) {
-          const double vi = v[i];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] += a[k][i] * vi;
-        }
-#pragma unroll
-        for (int o2 = 16; o2 > 0; o2 >>= 1) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o2);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (!on[k]) continue;
-          const int j = r + (l0 + t0 + k * nwarps) * CL;
-          if (lane < CL) trdc_at<CL>(y, lane)[j] = acc[k];
-          sp += acc[k] * v[j];
-        }
-      }
-    } else {
-      // lanes across 32 columns, warps across column groups and row segments
-      const int chunks = (nact + 31) >> 5;
-      const int segs = max(1, nwarps / chunks);
-      if (warp < chunks * segs) {
-        const int ch = warp % chunks, sg = warp / chunks;
-        const int m = n - c - 1;
-        const int per = (m + segs - 1) / segs;
-        const int i0 = c + 1 + sg * per, i1 = min(n, i0 + per);
-        const int t = ch * 32 + lane;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        if (t < nact) {
-          const double* a = Acol + (size_t)(l0 + t) * lds;
-          int i = i0;
-          for (; i + 3 < i1; i += 4) {
-            s0 += a[i] * v[i];
-            s1 += a[i + 1] * v[i + 1];
-            s2 += a[i + 2] * v[i + 2];
-            s3 += a[i + 3] * v[i + 3];
-          }
-          for (; i < i1; ++i) s0 += a[i] * v[i];
-        }
-        ypart[sg * (chunks * 32) + t] = (s0 + s1) + (s2 + s3);
-      }
-      __syncthreads();
-      for (int t = tid; t < nact; t += TRDC_NT) {
-        double yj = 0.0;
-        for (int sg = 0; sg < segs; ++sg) yj += ypart[sg * (chunks * 32) + t];
-        const int j = r + (l0 + t) * CL;
-#pragma unroll
-        for (int q = 0; q < CL; ++q) trdc_at<CL>(y, q)[j] = yj;
-        sp += yj * v[j];
-      }
-      sp = warp_sum(sp);
-    }
-    if (lane < CL) trdc_at<CL>(part, lane)[r * nwarps + warp] = sp;
-    trdc_sync<CL>();
-    // ---- b: the rank-2 update with w on the fly, the next reflector ----
-    double ytv = 0.0;
-    for (int q = lane; q < CL * nwarps; q += 32) ytv += part[q];
-    ytv = warp_sum(ytv);
-    const double a2 = -0.5 * tc * tc * ytv;
-    if (r == o)
-      for (int i = c + 2 + tid; i < n; i += TRDC_NT) P.A[i + (size_t)c * ld] = v[i];
-    const int cn = c + 1;
-    const bool own_next = cn < n - 1 && r == cn % CL;  // column cn is then local column l0
-    const int wfirst = own_next ? 1 : 0;
-    if (tc != 0.0 && warp >= wfirst) {
-      const int nw = nwarps - wfirst;
-      for (int l = l0 + wfirst + 4 * (warp - wfirst); l < ncol; l += 4 * nw) {
-        const int nl = min(4, ncol - l);
-        double vj[4], wj[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int j = r + (l + min(k, nl - 1)) * CL;
-          vj[k] = v[j];
-          wj[k] = tc * y[j] + a2 * v[j];
-        }
-        double* a0 = Acol + (size_t)l * lds;
-        int i = c + 1 + lane;
-        for (; i + 32 < n; i += 64) {
-          const double v0 = v[i], v1 = v[i + 32];
-          const double w0 = tc * y[i] + a2 * v0, w1 = tc * y[i + 32] + a2 * v1;
-          double x[8];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-            x[4 + k] = k < nl ? a0[(size_t)k * lds + i + 32] : 0.0;
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            x[k] -= v0 * wj[k] + w0 * vj[k];
-            x[4 + k] -= v1 * wj[k] + w1 * vj[k];
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) {
-              a0[(size_t)k * lds + i] = x[k];
-              a0[(size_t)k * lds + i + 32] = x[4 + k];
-            }
-        }
-        if (i < n) {
-          const double v0 = v[i];
-          const double w0 = tc * y[i] + a2 * v0;
-          double x[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] -= v0 * wj[k] + w0 * vj[k];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) a0[(size_t)k * lds + i] = x[k];
-        }
-      }
-    }
-    if (own_next && warp == 0) {
-      double* col = Acol + (size_t)l0 * lds;
-      if (tc != 0.0) {
-        const double vj = v[cn], wj = tc * y[cn] + a2 * v[cn];
-        for (int i = c + 1 + lane; i < n; i += 32) col[i] -= v[i] * wj + (tc * y[i] + a2 * v[i]) * vj;
-        __syncwarp();
-      }
-      trdc_reflector<CL>(P, col, cn, n, misc + (cn & 1) * 4, lane);
-    }
-    trdc_sync<CL>();
-  }
-  if (n >= 1 && r == (n - 1) % CL && tid == 0) P.d[n - 1] = Acol[(size_t)((n - 1) / CL) * lds + (n - 1)];
-  // no CTA leaves while another may still read its shared memory
-  trdc_sync<CL>();
-}
-
-// Threads of a CTA of the one-barrier kernel (8 warps; 16 measured slower,
-// and so did splitting the rank-2 update into column x row-segment tasks).
-constexpr int TRDC1_NT = 256;
-// Rows of the next column each thread of the one-barrier kernel reads from
-// its owner before the rank-2 update and finishes after it.
-constexpr int TRDC1_ROWS = 4;
-
-// Doubles of dynamic shared memory of the one-barrier kernel: the held
-// columns, v, the running copy of the next column, y twice (alternating by
-// column parity), one partial column dot per thread, the parts of y^T v
-// twice, one partial norm per warp, scalars.
-__host__ __device__ inline size_t trdc1_smem_doubles(int n, int cl) {
-  return (size_t)((n + cl - 1) / cl) * trdc_ld(n) + 4 * (size_t)n + TRDC1_NT + 2 * (size_t)cl * (TRDC1_NT / 32) +
-         (TRDC1_NT / 32) + 8;
-}
-
-
-
-// The same recurrence with one cluster barrier per column.  Every CTA keeps
-// its own copy of the column being reduced and forms each reflector itself
-// (all CTAs run the same arithmetic on the same values, so they agree to the
-// bit); the owner of a column therefore never broadcasts it, and the second
-// cluster barrier of trd_cluster_kernel is gone.  Per column c:
-//   a. beta, tau and v of column c from the local copy (the norm's partial
-//      sums were left by step c-1); y_j of the held columns j > c into
-//      every CTA's y buffer of this parity, parts of y^T v likewise; cluster
-//      barrier;
-//   b. every CTA reads column c+1 from its owner's shared memory (which the
-//      owner no longer updates from this step on), applies this step's
-//      rank-2 correction to it and leaves the partial norms for step c+1;
-//      the held columns j > c+1 take the rank-2 update; CTA barrier.
-// y and the parts alternate by parity: a CTA writes step c+1's values only
-// after the cluster barrier of step c+1, which every CTA reaches after it has
-// read step c-1's.  Output as trd_cluster_kernel.
-template <int CL>
-__global__ void __launch_bounds__(TRDC1_NT) trd_cluster1_kernel(const TrdClProb* __restrict__ probs) {
-  int r = 0;
-  if constexpr (CL > 1) r = (int)cooperative_groups::this_cluster().block_rank();
-  const TrdClProb P = probs[blockIdx.x / CL];
-  const int n = P.n;
-  const size_t ld = (size_t)P.ld;
-  const int lds = trdc_ld(n);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int nwarps = TRDC1_NT / 32;
-  const int ncol = r < n ? (n - r + CL - 1) / CL : 0;
-  extern __shared__ double sm[];
-  double* Acol = sm;                                     // ncol columns, ld lds
-  double* v = Acol + (size_t)((n + CL - 1) / CL) * lds;  // n
-  double* cur = v + n;                                   // n: column c (rows c .. n-1)
-  double* ybuf = cur + n;                                // 2 x n (written by every CTA)
-  double* ypart = ybuf + 2 * (size_t)n;                  // TRDC1_NT partial column dots
-  double* pbuf = ypart + TRDC1_NT;                        // 2 x CL x nwarps parts of y^T v
-  double* psq = pbuf + 2 * CL * nwarps;                  // nwarps partial norms
-
-  for (int l = 0; l < ncol; ++l) {
-    const double* src = P.A + (size_t)(r + l * CL) * ld;
-    for (int i = tid; i < n; i += TRDC1_NT) Acol[(size_t)l * lds + i] = src[i];
-  }
-  // every CTA of the cluster has loaded before any of them reads another's
-  // shared memory; then column 0 from CTA 0
-  trdc_sync<CL>();
-  {
-    const double* c0 = trdc_at<CL>(Acol, 0);
-    double sq = 0.0;
-    for (int i = tid; i < n; i += TRDC1_NT) {
-      const double x = c0[i];
-      cur[i] = x;
-      if (i >= 2) sq += x * x;
-    }
-    sq = warp_sum(sq);
-    if (lane == 0) psq[warp] = sq;
-  }
-  __syncthreads();
-
-  for (int c = 0; c < n - 1; ++c) {
-    double* y = ybuf + (size_t)(c & 1) * n;
-    double* part = pbuf + (c & 1) * CL * nwarps;
-    // ---- a: reflector of column c, v, y_j for the columns held here ----
-    double ss = 0.0;
-#pragma unroll
-    for (int q = 0; q < nwarps; ++q) ss += psq[q];
-    const double alpha = cur[c + 1];
-    double beta = alpha, tc = 0.0, scal = 0.0;
-    if (ss != 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-      tc = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
-    }
-    if (r == 0 && tid == 0) {
-      P.d[c] = cur[c];
-      P.e[c] = beta;
-      P.tau[c] = tc;
-    }
-    const bool own = r == c % CL;
-    for (int i = c + 1 + tid; i < n; i += TRDC1_NT) {
-      const double vi = (i == c + 1) ? 1.0 : cur[i] * scal;
-      v[i] = vi;
-      if (own && i >= c + 2) P.A[i + (size_t)c * ld] = vi;
-    }
-    __syncthreads();
-    // held columns after c: local indices l0 .. ncol-1
-    const int l0 = (c + 1 - r + CL - 1) / CL > 0 ? (c + 1 - r + CL - 1) / CL : 0;
-    const int nact = ncol > l0 ? ncol - l0 : 0;
-    double sp = 0.0;
-    if (nact <= TRDC_WARPCOL_MAX) {
-      for (int t0 = warp; t0 < nact; t0 += 4 * nwarps) {
-        const double* a[4];
-        bool on[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int t = t0 + k * nwarps;
-          on[k] = t < nact;
-          a[k] = Acol + (size_t)(l0 + (on[k] ? t : t0)) * lds;
-        }
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = c + 1 + lane; i < n; i += 32) {
-          const double vi = v[i];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] += a[k][i] * vi;
-        }
-#pragma unroll
-        for (int o2 = 16; o2 > 0; o2 >>= 1) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o2);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (!on[k]) continue;
-          const int j = r + (l0 + t0 + k * nwarps) * CL;
-          if (lane < CL) trdc_at<CL>(y, lane)[j] = acc[k];
-          sp += acc[k] * v[j];
-        }
-      }
-    } else {
-      const int chunks = (nact + 31) >> 5;
-      const int segs = max(1, nwarps / chunks);
-      if (warp < chunks * segs) {
-        const int ch = warp % chunks, sg = warp / chunks;
-        const int m = n - c - 1;
-        const int per = (m + segs - 1) / segs;
-        const int i0 = c + 1 + sg * per, i1 = min(n, i0 + per);
-        const int t = ch * 32 + lane;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        if (t < nact) {
-          const double* a = Acol + (size_t)(l0 + t) * lds;
-          int i = i0;
-          for (; i + 3 < i1; i += 4) {
-            s0 += a[i] * v[i];
-            s1 += a[i + 1] * v[i + 1];
-            s2 += a[i + 2] * v[i + 2];
-            s3 += a[i + 3] * v[i + 3];
-          }
-          for (; i < i1; ++i) s0 += a[i] * v[i];
-        }
-        ypart[sg * (chunks * 32) + t] = (s0 + s1) + (s2 + s3);
-      }
-      __syncthreads();
-      for (int t = tid; t < nact; t += TRDC1_NT) {
-        double yj = 0.0;
-        for (int sg = 0; sg < segs; ++sg) yj += ypart[sg * (chunks * 32) + t];
-        const int j = r + (l0 + t) * CL;
-#pragma unroll
-        for (int q = 0; q < CL; ++q) trdc_at<CL>(y, q)[j] = yj;
-        sp += yj * v[j];
-      }
-      sp = warp_sum(sp);
-    }
-    if (lane < CL) trdc_at<CL>(part, lane)[r * nwarps + warp] = sp;
-    trdc_sync<CL>();
-    // ---- b: column c+1 from its owner, the rank-2 update ----
-    const int cn = c + 1;
-    double xr[TRDC1_ROWS];
-    {
-      const double* ocol = trdc_at<CL>(Acol, cn % CL) + (size_t)(cn / CL) * lds;
-#pragma unroll
-      for (int k = 0; k < TRDC1_ROWS; ++k) {
-        const int i = cn + tid + k * TRDC1_NT;
-        xr[k] = i < n ? ocol[i] : 0.0;
-      }
-    }
-    double ytv = 0.0;
-    for (int q = lane; q < CL * nwarps; q += 32) ytv += part[q];
-    ytv = warp_sum(ytv);
-    const double a2 = -0.5 * tc * tc * ytv;
-    // held columns after c+1: local indices l1 .. ncol-1
-    const int l1 = (c + 2 - r + CL - 1) / CL > 0 ? (c + 2 - r + CL - 1) / CL : 0;
-    if (tc != 0.0) {
-      for (int l = l1 + 4 * warp; l < ncol; l += 4 * nwarps) {
-        const int nl = min(4, ncol - l);
-        double vj[4], wj[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int j = r + (l + min(k, nl - 1)) * CL;
-          vj[k] = v[j];
-          wj[k] = tc * y[j] + a2 * v[j];
-        }
-        double* a0 = Acol + (size_t)l * lds;
-        int i = c + 1 + lane;
-        for (; i + 32 < n; i += 64) {
-          const double v0 = v[i], v1 = v[i + 32];
-          const double w0 = tc * y[i] + a2 * v0, w1 = tc * y[i + 32] + a2 * v1;
-          double x[8];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-            x[4 + k] = k < nl ? a0[(size_t)k * lds + i + 32] : 0.0;
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            x[k] -= v0 * wj[k] + w0 * vj[k];
-            x[4 + k] -= v1 * wj[k] + w1 * vj[k];
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) {
-              a0[(size_t)k * lds + i] = x[k];
-              a0[(size_t)k * lds + i + 32] = x[4 + k];
-            }
-        }
-        if (i < n) {
-          const double v0 = v[i];
-          const double w0 = tc * y[i] + a2 * v0;
-          double x[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] -= v0 * wj[k] + w0 * vj[k];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) a0[(size_t)k * lds + i] = x[k];
-        }
-      }
-    }
-    {
-      // column c+1 after this step (rows c+1 .. n-1) and its partial norm
-      // over rows c+3 .. n-1 (v[c+1] = 1)
-      const double wn = tc * y[cn] + a2;
-      double sq = 0.0;
-#pragma unroll
-      for (int k = 0; k < TRDC1_ROWS; ++k) {
-        const int i = cn + tid + k * TRDC1_NT;
-        if (i < n) {
-          double x = xr[k];
-          if (tc != 0.0) x -= v[i] * wn + (tc * y[i] + a2 * v[i]);
-          cur[i] = x;
-          if (i >= cn + 2) sq += x * x;
-        }
-      }
-      sq = warp_sum(sq);
-      if (lane == 0) psq[warp] = sq;
-    }
-    __syncthreads();
-  }
-  if (n >= 1 && r == 0 && tid == 0) P.d[n - 1] = cur[n - 1];
-  // no CTA leaves while another may still read its shared memory
-  trdc_sync<CL>();
-}
-
-// Doubles of dynamic shared memory of the fused kernel: the held columns, v
-// twice, the running copy of the next column, y twice, the parts of y^T v
-// twice, one partial norm per warp, scalars.
-__host__ __device__ inline size_t trdc2_smem_doubles(int n, int cl) {
-  return (size_t)((n + cl - 1) / cl) * trdc_ld(n) + 5 * (size_t)n + 2 * (size_t)cl * (TRDC1_NT / 32) +
-         (TRDC1_NT / 32) + 8;
-}
-
-// The one-barrier recurrence with the rank-2 update of step c and the
-// products of step c+1 in one pass over the held columns.  Right after the
-// cluster barrier of step c every CTA holds y_c, v_c and the parts of
-// y_c^T v_c, so it can finish column c+1 (read from its owner) and form
-// v_{c+1} before it touches its own columns; then each held column j > c+1
-// is updated and, while its rows are in registers, dotted with v_{c+1}.
-// Per column: one pass over the held columns, one CTA barrier (after the
-// next column's partial norms) and one cluster barrier (after y_{c+1} and
-// the parts of y_{c+1}^T v_{c+1} reach every CTA).  v, y and the parts
-// alternate between two buffers by column parity.  The loop starts at
-// c = -1 (no update; column 0 read raw), so the first products need no
-// separate pass.  Rows above c+2 of a held column are dead after step c and
-// are not updated.  Output as trd_cluster_kernel.
-template <int CL>
-__global__ void __launch_bounds__(TRDC1_NT) trd_cluster2_kernel(const TrdClProb* __restrict__ probs) {
-  int r = 0;
-  if constexpr (CL > 1) r = (int)cooperative_groups::this_cluster().block_rank();
-  const TrdClProb P = probs[blockIdx.x / CL];
-  const int n = P.n;
-  const size_t ld = (size_t)P.ld;
-  const int lds = trdc_ld(n);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int nwarps = TRDC1_NT / 32;
-  const int ncol = r < n ? (n - r + CL - 1) / CL : 0;
-  extern __shared__ double sm[];
-  double* Acol = sm;                                        // ncol columns, ld lds
-  double* vbuf = Acol + (size_t)((n + CL - 1) / CL) * lds;  // 2 x n
-  double* cur = vbuf + 2 * (size_t)n;                       // n: column c+1 (rows c+1 .. n-1)
-  double* ybuf = cur + n;                                   // 2 x n (written by every CTA)
-  double* pbuf = ybuf + 2 * (size_t)n;                      // 2 x CL x nwarps parts of y^T v
-  double* psq = pbuf + 2 * CL * nwarps;                     // nwarps partial norms
-
-  for (int l = 0; l < ncol; ++l) {
-    const double* src = P.A + (size_t)(r + l * CL) * ld;
-    for (int i = tid; i < n; i += TRDC1_NT) Acol[(size_t)l * lds + i] = src[i];
-  }
-  // every CTA of the cluster has loaded before any of them reads another's
-  trdc_sync<CL>();
-
-  double tc = 0.0;  // tau of column c (0 for c = -1)
-  for (int c = -1; c < n - 1; ++c) {
-    const int cn = c + 1;
-    const double* v = vbuf + (size_t)((c + 2) & 1) * n;  // v_c (parity of c, kept non-negative)
-    double* vn = vbuf + (size_t)((c + 1) & 1) * n;        // v_{c+1}
-    const double* y = ybuf + (size_t)((c + 2) & 1) * n;
-    double* yn = ybuf + (size_t)((c + 1) & 1) * n;
-    const double* part = pbuf + ((c + 2) & 1) * CL * nwarps;
-    double* partn = pbuf + ((c + 1) & 1) * CL * nwarps;
-    // ---- column c+1 from its owner, corrected by step c; its partial norm ----
-    double xr[TRDC1_ROWS];
-    {
-      const double* ocol = trdc_at<CL>(Acol, cn % CL) + (size_t)(cn / CL) * lds;
-#pragma unroll
-      for (int k = 0; k < TRDC1_ROWS; ++k) {
-        const int i = cn + tid + k * TRDC1_NT;
-        xr[k] = i < n ? ocol[i] : 0.0;
-      }
-    }
-    double a2 = 0.0;
-    if (c >= 0 && tc != 0.0) {
-      double ytv = 0.0;
-      for (int q = lane; q < CL * nwarps; q += 32) ytv += part[q];
-      ytv = warp_sum(ytv);
-      a2 = -0.5 * tc * tc * ytv;
-    }
-    {
-      const double wn = (c >= 0 && tc != 0.0) ? tc * y[cn] + a2 : 0.0;
-      double sq = 0.0;
-#pragma unroll
-      for (int k = 0; k < TRDC1_ROWS; ++k) {
-        const int i = cn + tid + k * TRDC1_NT;
-        if (i < n) {
-          double x = xr[k];
-          if (c >= 0 && tc != 0.0) x -= v[i] * wn + (tc * y[i] + a2 * v[i]);
-          cur[i] = x;
-          if (i >= cn + 2) sq += x * x;
-        }
-      }
-      sq = warp_sum(sq);
-      if (lane == 0) psq[warp] = sq;
-    }
-    __syncthreads();
-    if (cn == n - 1) {
-      if (r == 0 && tid == 0) P.d[n - 1] = cur[n - 1];
-      break;
-    }
-    // ---- reflector of column c+1 (every thread, same arithmetic) ----
-    double ss = 0.0;
-#pragma unroll
-    for (int q = 0; q < nwarps; ++q) ss += psq[q];
-    const double alpha = cur[cn + 1];
-    double beta = alpha, tcn = 0.0, scal = 0.0;
-    if (ss != 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-      tcn = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
-    }
-    if (r == 0 && tid == 0) {
-      P.d[cn] = cur[cn];
-      P.e[cn] = beta;
-      P.tau[cn] = tcn;
-    }
-    const bool own = r == cn % CL;
-    for (int i = cn + 1 + tid; i < n; i += TRDC1_NT) {
-      const double vi = (i == cn + 1) ? 1.0 : cur[i] * scal;
-      vn[i] = vi;
-      if (own && i >= cn + 2) P.A[i + (size_t)cn * ld] = vi;
-    }
-    // ---- update of the held columns j > c+1 by step c, products with v_{c+1} ----
-    const int l1 = (c + 2 - r + CL - 1) / CL > 0 ? (c + 2 - r + CL - 1) / CL : 0;
-    const bool upd = c >= 0 && tc != 0.0;
-    double sp = 0.0;
-    for (int l = l1 + 4 * warp; l < ncol; l += 4 * nwarps) {
-      const int nl = min(4, ncol - l);
-      double vj[4], wj[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int j = r + (l + min(k, nl - 1)) * CL;
-        vj[k] = upd ? v[j] : 0.0;
-        wj[k] = upd ? tc * y[j] + a2 * v[j] : 0.0;
-      }
-      double* a0 = Acol + (size_t)l * lds;
-      int i = cn + 1 + lane;
-      for (; i + 32 < n; i += 64) {
-        const double p0 = (i == cn + 1) ? 1.0 : cur[i] * scal;
-        const double p1 = cur[i + 32] * scal;
-        double x[8];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-          x[4 + k] = k < nl ? a0[(size_t)k * lds + i + 32] : 0.0;
-        }
-        if (upd) {
-          const double v0 = v[i], v1 = v[i + 32];
-          const double w0 = tc * y[i] + a2 * v0, w1 = tc * y[i + 32] + a2 * v1;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            x[k] -= v0 * wj[k] + w0 * vj[k];
-            x[4 + k] -= v1 * wj[k] + w1 * vj[k];
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) {
-              a0[(size_t)k * lds + i] = x[k];
-              a0[(size_t)k * lds + i + 32] = x[4 + k];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += x[k] * p0 + x[4 + k] * p1;
-      }
-      if (i < n) {
-        const double p0 = (i == cn + 1) ? 1.0 : cur[i] * scal;
-        double x[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) x[k] = k < nl ? a0[(size_t)k * lds + i] : 0.0;
-        if (upd) {
-          const double v0 = v[i];
-          const double w0 = tc * y[i] + a2 * v0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] -= v0 * wj[k] + w0 * vj[k];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nl) a0[(size_t)k * lds + i] = x[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += x[k] * p0;
-      }
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o2);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k >= nl) continue;
-        const int j = r + (l + k) * CL;
-        if (lane < CL) trdc_at<CL>(yn, lane)[j] = acc[k];
-        sp += acc[k] * ((j == cn + 1) ? 1.0 : cur[j] * scal);
-      }
-    }
-    if (lane < CL) trdc_at<CL>(partn, lane)[r * nwarps + warp] = sp;
-    tc = tcn;
-    trdc_sync<CL>();
-  }
-  // no CTA leaves while another may still read its shared memory
-  trdc_sync<CL>();
-}
-
-// Launch configuration of the cluster kernel for `nprob` blocks.  The
-// kernel's attributes (largest dynamic shared memory, non-portable cluster
-// size) are set once per device, at the largest size any launch uses, by the
-// solver's constructor (set_attr): setting them per launch to the launch's
-// own size would race between solver instances on other threads.
-// The cluster kernel of CL CTAs: 0 two cluster barriers per column, 1 one,
-// 2 one with the update and the next products fused.  The default (1) is
-// built for every cluster size 1..16, the comparison forms for the powers
-// of two only.
-template <int CL>
-void (*trdc_kernel(int variant))(const TrdClProb*) {
-  if constexpr ((CL & (CL - 1)) == 0) {
-    if (variant == 2) return trd_cluster2_kernel<CL>;
-    if (variant == 0) return trd_cluster_kernel<CL>;
-  }
-  return trd_cluster1_kernel<CL>;
-}
-
-// Whether the cluster kernel of this variant is built for CL CTAs.
-inline bool trdc_size_built(int variant, int CL) {
-  return CL >= 1 && CL <= TRDC_CL_MAX && (variant == 1 || (CL & (CL - 1)) == 0);
-}
-
-// f(std::integral_constant<int, CL>{}) for a runtime cluster size 1..16.
-template <class F>
-auto trdc_with_cl(int CL, F&& f) {
-  switch (CL) {
-    case 1: return f(std::integral_constant<int, 1>{});
-    case 2: return f(std::integral_constant<int, 2>{});
-    case 3: return f(std::integral_constant<int, 3>{});
-    case 4: return f(std::integral_constant<int, 4>{});
-    case 5: return f(std::integral_constant<int, 5>{});
-    case 6: return f(std::integral_constant<int, 6>{});
-    case 7: return f(std::integral_constant<int, 7>{});
-    case 8: return f(std::integral_constant<int, 8>{});
-    case 9: return f(std::integral_constant<int, 9>{});
-    case 10: return f(std::integral_constant<int, 10>{});
-    case 11: return f(std::integral_constant<int, 11>{});
-    case 12: return f(std::integral_constant<int, 12>{});
-    case 13: return f(std::integral_constant<int, 13>{});
-    case 14: return f(std::integral_constant<int, 14>{});
-    case 15: return f(std::integral_constant<int, 15>{});
-    default: return f(std::integral_constant<int, 16>{});
-  }
-}
-
-template <int CL>
-cudaError_t trdc_config(int one, size_t smem, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int nprob,
-                        cudaStream_t st, bool set_attr) {
-  cfg = cudaLaunchConfig_t{};
-  cfg.gridDim = dim3((unsigned)(nprob * CL));
-  cfg.blockDim = dim3(one ? TRDC1_NT : TRDC_NT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  if (!set_attr) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(trdc_kernel<CL>(one), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && CL > 8)
-    e = cudaFuncSetAttribute(trdc_kernel<CL>(one), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  return e;
-}
-
-// Clusters of CL CTAs with `smem` bytes each that can be resident at once
-// (0: this cluster size is not usable here); sets the kernel's attributes
-// for launches of up to `smem` bytes.
-template <int CL>
-int trdc_max_clusters(int one, size_t smem) {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
-  if (trdc_config<CL>(one, smem, cfg, at, 1, nullptr, true) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  int nc = 0;
-  if (cudaOccupancyMaxActiveClusters(&nc, trdc_kernel<CL>(one), &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return nc;
-}
-
-template <int CL>
-cudaError_t trdc_launch(int one, const TrdClProb* d, int nprob, size_t smem, cudaStream_t st) {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
-  cudaError_t e = trdc_config<CL>(one, smem, cfg, at, nprob, st, false);
-  if (e != cudaSuccess) return e;
-  return cudaLaunchKernelEx(&cfg, trdc_kernel<CL>(one), d);
 }
 
 // A kernel's largest dynamic shared memory on the current device only grows:
@@ -1980,43 +1145,13 @@ SyevBatched::SyevBatched() {
   int dev = 0;
   NRGB_CUDA(cudaGetDevice(&dev));
   NRGB_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
-  int optin = 0;
-  NRGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  cl_smem_ = std::min(TRDC_SMEM, (size_t)optin);
   // NRGB_TRD_PATH=panel keeps every block on the cooperative panel path
   // (comparisons, or a device where cluster launches are unavailable)
   const char* path = getenv("NRGB_TRD_PATH");
-  if (path && strcmp(path, "panel") == 0) cl_smem_ = 0;
-  // the cluster kernel (default: one barrier per column); for comparisons
-  // NRGB_TRDC_BARRIERS=2 selects the form with two cluster barriers per
-  // column and NRGB_TRDC_FUSED=1 the one-barrier form with the update and
-  // the next products fused (faster for a block alone, slower when many
-  // clusters run at once)
-  const char* nb = getenv("NRGB_TRDC_BARRIERS");
-  const char* nf = getenv("NRGB_TRDC_FUSED");
-  cl_one_ = (nb && strcmp(nb, "2") == 0) ? 0 : (nf && strcmp(nf, "1") == 0) ? 2 : 1;
-  // NRGB_TRDC_POW2=1 restricts the default kernel to clusters of 1, 2, 4, 8
-  // and 16 CTAs (comparisons); otherwise a block takes the smallest cluster
-  // of any size that holds it
-  const char* np2 = getenv("NRGB_TRDC_POW2");
-  const bool pow2 = np2 && strcmp(np2, "1") == 0;
-  if (cl_smem_ > 0) {
-    for (int cl = 1; cl <= TRDC_CL_MAX; ++cl) {
-      if (!trdc_size_built(cl_one_, cl) || (pow2 && (cl & (cl - 1)) != 0)) continue;
-      cl_max_[cl] = trdc_with_cl(cl, [&](auto c) { return trdc_max_clusters<decltype(c)::value>(cl_one_, cl_smem_); });
-    }
-  }
-  // largest block the cluster kernel holds (the one-barrier kernels also
-  // read at most TRDC1_ROWS rows of a column per thread)
-  for (int cl = TRDC_CL_MAX; cl >= 1 && cl_nmax_ == 0; --cl) {
-    if (cl_max_[cl] <= 0) continue;
-    int n = 1;
-    while (trdc_bytes(n + 1, cl) <= cl_smem_ && (!cl_one_ || n + 1 <= TRDC1_ROWS * TRDC1_NT)) ++n;
-    cl_nmax_ = n > SMALL_N ? n : 0;
-  }
-  // one side stream per launch group of the cluster kernel (up to 19
-  // groups: single-CTA launches in four shared-memory sizes and one per
-  // cluster size), so that no group waits behind another on a shared stream
+  if (!(path && strcmp(path, "panel") == 0)) cl_nmax_ = trdr_init();
+  if (cl_nmax_ <= SMALL_N) cl_nmax_ = 0;
+  // side streams for the launch groups of the cluster kernel (a shape and a
+  // cluster size each, up to 21), so that few groups wait behind another
   if (const char* ns = getenv("NRGB_SIDE_STREAMS")) naux_ = std::max(1, std::min(NAUX, atoi(ns)));
   for (int i = 0; i < NAUX; ++i) {
     NRGB_CUDA(cudaStreamCreateWithFlags(&aux_[i], cudaStreamNonBlocking));
@@ -2100,12 +1235,6 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
                256 * 6 * (size_t)(nmx / NBB + 4));
   pl.add<TrdClProb>(2 * ns.size() + 16);
   return pl.bytes + (size_t)ns.size() * 4096 + (1 << 20);
-}
-
-size_t SyevBatched::trdc_bytes(int n, int cl) const {
-  return (cl_one_ == 2 ? trdc2_smem_doubles(n, cl) : cl_one_ == 1 ? trdc1_smem_doubles(n, cl)
-                                                                   : trdc_smem_doubles(n, cl)) *
-         sizeof(double);
 }
 
 int SyevBatched::cl_use() const {
@@ -2232,59 +1361,40 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       ++launches_;
     }
     // ---------------- 1) tridiagonalisation ----------------
-    // Blocks whose matrix fits in the shared memory of a cluster of at most
-    // 16 CTAs: one cluster each (smallest cluster that holds the block).
-    // Launches of different cluster sizes (and, for single-CTA clusters, of
-    // different shared-memory sizes, so that small blocks share an SM) run
-    // concurrently on side streams; the panel launches for the larger
-    // blocks follow on the main stream.
+    // Blocks up to the cluster kernel's capacity: one cluster each.  The
+    // groups (a shape and a cluster size, trd_regs.cu) are launched largest
+    // first and run concurrently on side streams; the panel launches for the
+    // larger blocks follow on the main stream.
     std::vector<char> via_cluster(nbig, 0);
-    // Launch the cluster tridiagonalisation for `list`: groups by cluster size
-    // (the smallest cluster whose shared memory holds the block; single-CTA
-    // clusters split at n = 64, 96, 128), concurrently on side streams,
-    // joined into `st`.  Every entry must fit some cluster size.
+    // Launch the cluster tridiagonalisation for `list`, joined into `st`.
     auto launch_clusters = [&](const std::vector<TrdClProb>& list) {
-      constexpr int NG = TRDC_CL_MAX + 3;  // group 0..3: one CTA; group CL + 2: CL CTAs
-      std::vector<TrdClProb> grp[NG];
-      size_t gsmem[NG] = {};
+      if (list.empty()) return;
+      std::map<std::pair<int, int>, std::vector<TrdClProb>> grp;  // (-shape, -CTAs): largest first
       for (const TrdClProb& t : list) {
-        const int n = t.n;
-        for (int cl = 1; cl <= TRDC_CL_MAX; ++cl) {
-          const size_t bytes = trdc_bytes(n, cl);
-          if (cl_max_[cl] > 0 && bytes <= cl_smem_) {
-            const int g = cl > 1 ? cl + 2 : (n <= 64 ? 0 : n <= 96 ? 1 : n <= 128 ? 2 : 3);
-            grp[g].push_back(t);
-            gsmem[g] = std::max(gsmem[g], bytes);
-            break;
-          }
-        }
+        const TrdrGroup g = trdr_group(t.n);
+        grp[{-g.shape, -g.cl}].push_back(t);
       }
-      int used = 0;
-      TrdClProb* dg[NG] = {};
-      for (int g = NG - 1; g >= 0; --g) {
-        if (grp[g].empty()) continue;
-        dg[g] = arena_.alloc_n<TrdClProb>(grp[g].size());
-        NRGB_CUDA(cudaMemcpyAsync(dg[g], grp[g].data(), grp[g].size() * sizeof(TrdClProb), cudaMemcpyHostToDevice, st));
-      }
+      std::vector<TrdClProb> all;
+      for (const auto& kv : grp) all.insert(all.end(), kv.second.begin(), kv.second.end());
+      TrdClProb* dg = arena_.alloc_n<TrdClProb>(all.size());
+      NRGB_CUDA(cudaMemcpyAsync(dg, all.data(), all.size() * sizeof(TrdClProb), cudaMemcpyHostToDevice, st));
       NRGB_CUDA(cudaEventRecord(fork_, st));
-      for (int g = NG - 1; g >= 0; --g) {
-        if (grp[g].empty()) continue;
+      int used = 0;
+      for (const auto& kv : grp) {
+        const TrdrGroup g{-kv.first.first, -kv.first.second};
         cudaStream_t sx = aux_[used % naux_];
         if (used < naux_) NRGB_CUDA(cudaStreamWaitEvent(sx, fork_, 0));
         double fl = 0, by = 0;
-        for (const TrdClProb& t : grp[g]) {
+        for (const TrdClProb& t : kv.second) {
           fl += 4.0 / 3.0 * (double)t.n * t.n * t.n;
           by += 8.0 * (double)t.n * t.n;  // the block, read from HBM once
         }
         KernelStats::get().add_work("trd_cluster", fl);
         KernelStats::get().add_work("trd_cluster_hbm", by);
-        const int np = (int)grp[g].size();
-        const int cl = g > 3 ? g - 2 : 1;
         cudaError_t e = cudaSuccess;
-        NRGB_LAUNCH("trd_cluster", sx, e = trdc_with_cl(cl, [&](auto c) {
-                      return trdc_launch<decltype(c)::value>(cl_one_, dg[g], np, gsmem[g], sx);
-                    }));
+        NRGB_LAUNCH("trd_cluster", sx, e = trdr_launch(g, dg, (int)kv.second.size(), d_err_ + 3, sx));
         NRGB_CUDA(e);
+        dg += kv.second.size();
         ++launches_;
         ++used;
       }

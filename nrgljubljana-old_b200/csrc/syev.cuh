@@ -7,9 +7,11 @@
 //
 // Pipeline (all problems of a batch advance together):
 //   n <= 32 : one warp per problem, Householder + implicit QR in shared memory.
-//   n  > 32 : 1) blocked Householder tridiagonalisation (panel of 32 columns
-//                in a cooperative persistent kernel, trailing rank-64 update on
-//                the DMMA GEMM),
+//   n  > 32 : 1) Householder tridiagonalisation, up to n = 640 in one
+//                thread-block cluster with the matrix in its registers
+//                (trd_regs.cu); the leading columns of larger blocks blocked
+//                (panel of 32 columns in a cooperative persistent kernel,
+//                trailing rank-64 update on the DMMA GEMM),
 //             2) divide and conquer on the tridiagonal (Cuppen splitting,
 //                Gu-Eisenstat eigenvectors), merges of equal tree height of all
 //                problems in the same launches,
@@ -82,12 +84,7 @@ class SyevBatched : public EigSolver {
   bool inject_shortfall_ = false;
   int coop_ctas_ = 0;
   int sms_ = 0;
-  int cl_max_[17] = {};               // resident clusters of CL = 1..16 CTAs (0: not usable or not built)
-  size_t cl_smem_ = 0;                // shared memory per CTA of the cluster kernel
-  int cl_nmax_ = 0;                   // largest block it holds (0: cluster path off)
-  int cl_one_ = 1;                    // cluster kernel: 0 two barriers per column, 1 one, 2 one and fused
-  // dynamic shared memory of one CTA of the cluster kernel in use
-  size_t trdc_bytes(int n, int cl) const;
+  int cl_nmax_ = 0;  // largest block it holds (0: cluster path off)
   // blocks up to this size go to the cluster kernel whole: the capacity, or
   // the schedule's limit when it is lower (schedule.cuh)
   int cl_use() const;
