@@ -25,6 +25,7 @@
 #include "gemm_f64.cuh"
 #include "syev.cuh"
 #include "schedule.cuh"
+#include "trd_grid.cuh"
 #include "trd_regs.cuh"
 
 namespace nrgb {
@@ -1148,8 +1149,12 @@ SyevBatched::SyevBatched() {
   // NRGB_TRD_PATH=panel keeps every block on the cooperative panel path
   // (comparisons, or a device where cluster launches are unavailable)
   const char* path = getenv("NRGB_TRD_PATH");
-  if (!(path && strcmp(path, "panel") == 0)) cl_nmax_ = trdr_init();
+  if (!(path && strcmp(path, "panel") == 0)) {
+    cl_nmax_ = trdr_init();
+    grid_nmax_ = trd_grid_init(&grid_ctas_);
+  }
   if (cl_nmax_ <= SMALL_N) cl_nmax_ = 0;
+  if (cl_nmax_ == 0) grid_nmax_ = 0;
   // side streams for the launch groups of the cluster kernel (a shape and a
   // cluster size each, up to 21), so that few groups wait behind another
   if (const char* ns = getenv("NRGB_SIDE_STREAMS")) naux_ = std::max(1, std::min(NAUX, atoi(ns)));
@@ -1206,6 +1211,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
     pl.add<double>((size_t)n * 16);
     pl.add<int>((size_t)n * 10);
     pl.add<double>(2 * RED);
+    pl.add<double>(trd_grid_exchange(n));
     pl.add<double>((size_t)NBB * NBB * std::max(1, bt_nblk(n)));  // G
     pl.add<double>((size_t)NBB * NBB * std::max(1, bt_nblk(n)));  // T
     pl.add<double>((size_t)NBB * n * 2);                          // X (last block), Y
@@ -1219,7 +1225,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   // outputs of the back-transformation once; cluster descriptors
   size_t zs = 0;
   for (int n : ns)
-    zs += 6 + (size_t)n * n / ZERO_CHUNK + (size_t)NBB * NBB * bt_nblk(n) / ZERO_CHUNK +
+    zs += 8 + (size_t)n * n / ZERO_CHUNK + trd_grid_exchange(n) / ZERO_CHUNK + (size_t)NBB * NBB * bt_nblk(n) / ZERO_CHUNK +
           (NBB * (size_t)n / ZERO_CHUNK + 2) * (n / NBB + 3);
   pl.add<ZeroSeg>(zs);
   // divide-and-conquer descriptors (one copy): problems, leaves, and per
@@ -1234,12 +1240,18 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   pl.add<char>(ns.size() * sizeof(BtProb) + nbt * (sizeof(GemmProb) + sizeof(GemmSeg)) +
                256 * 6 * (size_t)(nmx / NBB + 4));
   pl.add<TrdClProb>(2 * ns.size() + 16);
+  pl.add<TrdGridProb>(ns.size() + 16);
   return pl.bytes + (size_t)ns.size() * 4096 + (1 << 20);
 }
 
 int SyevBatched::cl_use() const {
   const int lim = schedule_here().cluster_limit.load(std::memory_order_relaxed);
   return (lim > 0 && lim < cl_nmax_) ? lim : cl_nmax_;
+}
+
+int SyevBatched::grid_limit(const std::vector<int>& ns, int clim) const {
+  if (grid_nmax_ == 0 || clim == 0) return 0;
+  return grid_nmax_;
 }
 
 void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
@@ -1286,7 +1298,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     std::vector<TrdProb> tp(nbig);
     std::vector<DcProb> dp(nbig);
     std::vector<BtProb> bp(nbig);
-    std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig);
+    std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig), gex(nbig, nullptr);
     std::vector<ZeroSeg> zeros;  // ranges that must start at zero, cleared in one launch
     for (int b = 0; b < nbig; ++b) {
       const SyevDesc& S = probs[big[b]];
@@ -1349,6 +1361,10 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       bt.V = W1;  // free once divide and conquer is done
       bt.G = G;
       bt.T = T;
+      if (grid_nmax_ > 0 && n > cl_use()) {
+        gex[b] = arena_.alloc_n<double>(trd_grid_exchange(n));
+        zero_add(zeros, gex[b], (long long)trd_grid_exchange(n));
+      }
       zero_add(zeros, red, 2 * RED);
       zero_add(zeros, tauT[b], n);
       zero_add(zeros, S.Z, (long long)nn);
@@ -1403,10 +1419,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         NRGB_CUDA(cudaStreamWaitEvent(st, join_[i], 0));
       }
     };
-    // Larger blocks: panel launches for their leading columns until the
-    // trailing block fits a cluster, whose tridiagonalisation finishes it.
+    // Larger blocks go to the many-CTA kernel (trd_grid.cu) whole, those
+    // beyond its capacity after panel launches for their leading columns;
+    // without it, panel launches until the trailing block fits a cluster.
     std::vector<int> jstop(nbig);
     const int clim = cl_use();
+    const int glim = grid_limit(ns, clim);
     {
       std::vector<TrdClProb> whole;
       for (int b = 0; b < nbig; ++b) {
@@ -1415,6 +1433,8 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         if (clim > 0 && n <= clim) {
           whole.push_back(TrdClProb{tp[b].A, tp[b].d, tp[b].e, tp[b].tau, n, n});
           via_cluster[b] = 1;
+        } else if (glim > 0) {
+          jstop[b] = n <= glim ? 0 : ((n - glim + NB - 1) / NB) * NB;
         } else if (clim > 0) {
           jstop[b] = ((n - clim + NB - 1) / NB) * NB;
         }
@@ -1436,7 +1456,10 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       std::vector<int> order(nbig);
       std::iota(order.begin(), order.end(), 0);
       GridBarrier* bars = arena_.alloc_n<GridBarrier>(nbig);
-      for (int j0 = 0; j0 < nmax; j0 += NB) {
+      int jmax = 0;
+      for (int b : order)
+        if (!via_cluster[b]) jmax = std::max(jmax, jstop[b]);
+      for (int j0 = 0; j0 < std::min(nmax, jmax); j0 += NB) {
         std::vector<int> act;
         for (int b : order)
           if (tp[b].n > j0 && !via_cluster[b] && j0 < jstop[b]) act.push_back(b);
@@ -1517,11 +1540,55 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         }
       }
     }
+    // the blocks A[j:, j:] (j = jstop, fully updated by the last trailing
+    // update) on many CTAs each: as many blocks to a cooperative launch as
+    // there are CTAs for, largest first, so that blocks of a launch take
+    // similar times
+    if (glim > 0) {
+      std::vector<TrdGridProb> rest;
+      for (int b = 0; b < nbig; ++b) {
+        const int j = jstop[b], n = tp[b].n;
+        if (via_cluster[b] || j >= n) continue;
+        rest.push_back(TrdGridProb{tp[b].A + j + (size_t)j * n, tp[b].d + j, tp[b].e + j, tp[b].tau + j, gex[b], n - j, n,
+                                   std::min(wait_log2_, 21), inject_shortfall_ ? 1 : 0, 0, 0, 0});
+      }
+      std::stable_sort(rest.begin(), rest.end(), [](const TrdGridProb& x, const TrdGridProb& y) { return x.n > y.n; });
+      std::vector<std::vector<TrdGridProb>> waves;
+      std::vector<int> room;
+      for (const TrdGridProb& p : rest) {
+        const int c = trd_grid_ctas(p.n);
+        size_t w = 0;
+        while (w < waves.size() && room[w] < c) ++w;
+        if (w == waves.size()) {
+          waves.emplace_back();
+          room.push_back(grid_ctas_);
+        }
+        waves[w].push_back(p);
+        room[w] -= c;
+      }
+      std::vector<TrdGridProb> all;
+      std::vector<int> ctas;
+      for (auto& w : waves) {
+        ctas.push_back(trd_grid_place(w));
+        all.insert(all.end(), w.begin(), w.end());
+      }
+      TrdGridProb* dg = arena_.alloc_n<TrdGridProb>(all.size());
+      if (!all.empty())
+        NRGB_CUDA(cudaMemcpyAsync(dg, all.data(), all.size() * sizeof(TrdGridProb), cudaMemcpyHostToDevice, st));
+      for (size_t w = 0; w < waves.size(); ++w) {
+        double fl = 0;
+        for (const TrdGridProb& p : waves[w]) fl += 4.0 / 3.0 * (double)p.n * p.n * p.n;
+        KernelStats::get().add_work("trd_grid", fl);
+        NRGB_LAUNCH("trd_grid", st, NRGB_CUDA(trd_grid_launch(dg, (int)waves[w].size(), ctas[w], d_err_ + 3, st)));
+        dg += waves[w].size();
+        ++launches_;
+      }
+    }
     if (inject_shortfall_) {
-      // fault injection (the barriers expected a CTA that was never
-      // launched): report the timed-out wait here, before any later stage
-      // reads the unfinished reduction, and leave no work of this call in
-      // flight on any stream
+      // fault injection (the waits expect a CTA that was never launched):
+      // report the timed-out wait here, before any later stage reads the
+      // unfinished reduction, and leave no work of this call in flight on any
+      // stream
       int f = 0;
       NRGB_CUDA(cudaMemcpyAsync(&f, d_err_ + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
       NRGB_CUDA(cudaStreamSynchronize(st));
@@ -1530,9 +1597,8 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         if (aux_[i]) NRGB_CUDA(cudaStreamSynchronize(aux_[i]));
       if (f) throw CudaError("syev: grid barrier timed out");
     }
-    // the trailing blocks A[j:, j:] (j = jstop) of the larger blocks, fully
-    // updated by the last trailing update, tridiagonalised in clusters
-    {
+    // without the many-CTA kernel: the trailing blocks in clusters
+    if (glim == 0) {
       std::vector<TrdClProb> tails;
       for (int b = 0; b < nbig; ++b) {
         const int j = jstop[b], n = tp[b].n;

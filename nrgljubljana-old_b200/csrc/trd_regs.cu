@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "trd_regs.cuh"
+#include "trd_regs_dev.cuh"
 
 namespace nrgb {
 
@@ -47,8 +48,6 @@ namespace {
 
 namespace trdr {
 
-constexpr int NW = 8;               // warps that hold the matrix
-constexpr int NT = 32 * NW;         // their threads
 __host__ __device__ constexpr int threads(bool one) { return one ? NT + 32 : NT; }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -93,39 +92,11 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.aligned.release;\nbarrier.cluster.wait.aligned.acquire;\n" ::: "memory");
 }
 
-// Sum over the warp: the quads by one FP64 tensor instruction with a matrix
-// of ones (two shuffle steps saved), the eight quad sums by shuffles.
-__device__ __forceinline__ double warp_sum_mma(double x) {
-  double s = 0.0, u = 0.0;
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(s), "+d"(u)
-      : "d"(x), "d"(1.0));
-  s += __shfl_xor_sync(0xffffffffu, s, 4);
-  s += __shfl_xor_sync(0xffffffffu, s, 8);
-  s += __shfl_xor_sync(0xffffffffu, s, 16);
-  return s;
-}
-
-// beta, tau and the scale of v of the reflector of a column with the entry
-// alpha below the diagonal and the squared norm nn under it.
-__device__ __forceinline__ void reflector(double alpha, double nn, double& beta, double& tau, double& scale) {
-  beta = alpha;
-  tau = scale = 0.0;
-  if (nn != 0.0) {
-    beta = -copysign(sqrt(fma(alpha, alpha, nn)), alpha);
-    tau = (beta - alpha) / beta;
-    scale = 1.0 / (alpha - beta);
-  }
-}
-
-__host__ __device__ constexpr int pow2_up(int c) { return c <= 1 ? 1 : c <= 2 ? 2 : c <= 4 ? 4 : c <= 8 ? 8 : 16; }
-
-// Shapes of the kernel <KR, C, WR>: rows and columns per CTA it can hold.
+// A CTA's message and shared memory.
 template <int KR, int C, int WR>
-struct Shape {
-  static constexpr int WC = NW / WR;       // column groups of warps
-  static constexpr int ROWS = 32 * KR * WR;
-  static constexpr int COLS = C * WC;      // columns of a CTA
+struct ClShape : Shape<KR, C, WR> {
+  using Shape<KR, C, WR>::ROWS;
+  using Shape<KR, C, WR>::COLS;
   static constexpr int LP = COLS | 1;      // a sender's entries in the exchange buffer (odd: rows in order hit all banks)
   static constexpr size_t smem(int cl) {
     return 16 * ((size_t)(ROWS + 1) + 2 * (size_t)cl * LP) +
@@ -135,49 +106,15 @@ struct Shape {
 
 }  // namespace trdr
 
-// Matrix phase of one warp: the rank-2 update of its columns and their
-// products with x, over the row chunks KS .. KR-1.  `row`: this lane holds row
-// t + 1, in chunk KS, whose updated entries go to Rs.
-template <int KS, int KR, int C, int WR>
-__device__ __forceinline__ void trdr_update(double (&a)[C][KR], double (&acc)[C], const double (&vj)[C],
-                                            const double (&wj)[C], const double2* VW, const double* X, bool row,
-                                            double* Rs) {
-#pragma unroll
-  for (int k = KS; k < KR; ++k) {
-    const double2 vw = VW[32 * WR * k];
-    const double x = X[32 * WR * k];
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      a[c][k] = fma(-vw.y, vj[c], fma(-vw.x, wj[c], a[c][k]));
-      acc[c] = fma(a[c][k], x, acc[c]);
-    }
-  }
-  if (row) {
-#pragma unroll
-    for (int c = 0; c < C; c += 2) *reinterpret_cast<double2*>(Rs + c) = make_double2(a[c][KS], a[c + 1][KS]);
-  }
-}
-
-// The same from chunk ks on (ks < KR; a warp whose chunks are all done with has nothing to do).
-template <int KS, int KR, int C, int WR>
-__device__ __forceinline__ void trdr_update_from(int ks, double (&a)[C][KR], double (&acc)[C], const double (&vj)[C],
-                                                 const double (&wj)[C], const double2* VW, const double* X, bool row,
-                                                 double* Rs) {
-  if constexpr (KS < KR) {
-    if (ks == KS) trdr_update<KS, KR, C, WR>(a, acc, vj, wj, VW, X, row, Rs);
-    else trdr_update_from<KS + 1, KR, C, WR>(ks, a, acc, vj, wj, VW, X, row, Rs);
-  }
-}
-
 template <int KR, int C, int WR, bool ONE>
 __global__ void __launch_bounds__(trdr::threads(ONE), 1)
     trd_regs_kernel(const TrdClProb* __restrict__ probs, int CL, int* fail) {
   using namespace trdr;
-  using SH = Shape<KR, C, WR>;
+  using SH = ClShape<KR, C, WR>;
   static_assert(C <= 16 && C % 2 == 0, "columns of a warp");
   constexpr int THREADS = threads(ONE);
   constexpr int WC = SH::WC, ROWS = SH::ROWS, COLS = SH::COLS, LP = SH::LP;
-  constexpr int CP = pow2_up(C), GL = 32 / CP;  // columns padded, lanes of a column's group
+  constexpr int GL = 32 / pow2_up(C);           // lanes of a column's group
   constexpr int M = (ROWS + NT - 1) / NT;       // rows of the vectors a thread computes
   extern __shared__ __align__(16) double sm[];
   double2* VW = reinterpret_cast<double2*>(sm);  // ROWS + 1: (v, w) of the rows; the last entry stays zero
@@ -319,25 +256,9 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       double accP = 0.0;
 #pragma unroll
       for (int c = 0; c < C; ++c) accP = fma(X[jc[c]], acc[c], accP);
-      // sums over the lanes: the GL lanes of group g end with column g's
-      double red[CP];
-#pragma unroll
-      for (int c = 0; c < CP; ++c) red[c] = c < C ? acc[c < C ? c : 0] : 0.0;
-      int off = 16;
-#pragma unroll
-      for (int w2 = CP / 2; w2 >= 1; w2 >>= 1) {
-        const bool up = (lane & off) != 0;
-#pragma unroll
-        for (int c = 0; c < w2; ++c) {
-          const double keep = up ? red[c + w2] : red[c], send = up ? red[c] : red[c + w2];
-          red[c] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-        off >>= 1;
-      }
-#pragma unroll
-      for (int o = GL / 2; o >= 1; o >>= 1) red[0] += __shfl_xor_sync(0xffffffffu, red[0], o);
+      const double red = columns_sum<C>(acc, lane);
       accP = warp_sum_mma(accP);
-      if (lane % GL == 0 && lane / GL < C) Sp[(wr * WC + wc) * C + lane / GL] = red[0];
+      if (lane % GL == 0 && lane / GL < C) Sp[(wr * WC + wc) * C + lane / GL] = red;
       if (lane == 0) Pp[warp] = accP;
       if (!ONE) {
         double ss = 0.0;
@@ -375,7 +296,6 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       for (int g = 1; g < WR; ++g) s += Sp[g * COLS + at];
       return make_double2(s, Rs[at]);
     };
-    auto sum8 = [](const double* p) { return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])); };
     if (ONE) {
       if (tid < COLS) SR[(t & 1) * LP + tid] = column(tid);
       if (tid == NT) PS[(t & 1) * 16] = sum8(Pp);
@@ -449,7 +369,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
 // 0.87 ms, 15 CTAs 0.73 ms).
 template <class F>
 auto with_shape(int s, F&& f) {
-#define NRGB_TRDR(KR, C, WR, ONE) return f(trdr::Shape<KR, C, WR>{}, trd_regs_kernel<KR, C, WR, ONE>)
+#define NRGB_TRDR(KR, C, WR, ONE) return f(trdr::ClShape<KR, C, WR>{}, trd_regs_kernel<KR, C, WR, ONE>)
   switch (s) {
     case 0: NRGB_TRDR(2, 8, 1, true);
     case 1: NRGB_TRDR(3, 8, 1, false);
