@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <numeric>
 
+#include "bt_apply.cuh"
 #include "gemm_f64.cuh"
 #include "syev.cuh"
 #include "schedule.cuh"
@@ -35,7 +36,7 @@ namespace {
 constexpr int SMALL_N = 32;     // warp-per-problem path
 constexpr int LEAF = 16;        // D&C leaf size
 constexpr int NB = 32;          // tridiagonalisation panel width
-constexpr int NBB = 64;         // back-transformation block of reflectors
+constexpr int NBB = BT_NB;      // back-transformation block of reflectors
 constexpr int TRD_NT = 256;     // threads of the panel kernel
 constexpr double EPS = 2.220446049250313e-16;
 
@@ -1241,6 +1242,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
                256 * 6 * (size_t)(nmx / NBB + 4));
   pl.add<TrdClProb>(2 * ns.size() + 16);
   pl.add<TrdGridProb>(ns.size() + 16);
+  pl.add<BtSlabProb>(ns.size() + 16);
   return pl.bytes + (size_t)ns.size() * 4096 + (1 << 20);
 }
 
@@ -1297,7 +1299,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     // per-problem workspaces
     std::vector<TrdProb> tp(nbig);
     std::vector<DcProb> dp(nbig);
-    std::vector<BtProb> bp(nbig);
+    std::vector<BtProb> bt(nbig);
     std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig), gex(nbig, nullptr);
     std::vector<ZeroSeg> zeros;  // ranges that must start at zero, cleared in one launch
     for (int b = 0; b < nbig; ++b) {
@@ -1354,13 +1356,13 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       q.rotp = ivec + 5 * n;
       q.rotj = ivec + 6 * n;
       q.nrot = ivec + 7 * n;
-      BtProb& bt = bp[b];
-      bt.n = n;
-      bt.A = S.A;
-      bt.tau = tauT[b];
-      bt.V = W1;  // free once divide and conquer is done
-      bt.G = G;
-      bt.T = T;
+      BtProb& u = bt[b];
+      u.n = n;
+      u.A = S.A;
+      u.tau = tauT[b];
+      u.V = W1;  // free once divide and conquer is done
+      u.G = G;
+      u.T = T;
       if (grid_nmax_ > 0 && n > cl_use()) {
         gex[b] = arena_.alloc_n<double>(trd_grid_exchange(n));
         zero_add(zeros, gex[b], (long long)trd_grid_exchange(n));
@@ -1607,6 +1609,46 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       }
       launch_clusters(tails);
     }
+    // WY factors of the blocks that take the slab back-transformation, beside
+    // the divide and conquer
+    const int slab_max = bt_slab_nmax();
+    std::vector<BtSlabProb> slab;
+    std::vector<BtProb> bp;   // the others
+    std::vector<int> bp_of;   // their place in `big`
+    int slab_nmax = 0, slab_ctas = 0, slab_cols = 8;
+    BtSlabProb* d_slab = nullptr;
+    {
+      std::vector<int> ord;
+      long cols = 0;
+      for (int b = 0; b < nbig; ++b) {
+        if (tp[b].n <= slab_max) {
+          ord.push_back(b);
+          cols += tp[b].n;
+          slab_nmax = std::max(slab_nmax, tp[b].n);
+        } else {
+          bp.push_back(bt[b]);
+          bp_of.push_back(b);
+        }
+      }
+      slab_cols = bt_slab_columns(cols, slab_nmax);
+      std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return tp[x].n > tp[y].n; });
+      int blocks = 0;
+      for (int b : ord) {
+        const int n = tp[b].n;
+        slab.push_back(BtSlabProb{tp[b].A, tauT[b], bt[b].T, dp[b].Q, n, blocks, slab_ctas});
+        blocks += bt_nblk(n);
+        slab_ctas += ceil_div(n, slab_cols);
+      }
+      if (!slab.empty()) {
+        d_slab = arena_.alloc_n<BtSlabProb>(slab.size());
+        NRGB_CUDA(cudaMemcpyAsync(d_slab, slab.data(), slab.size() * sizeof(BtSlabProb), cudaMemcpyHostToDevice, st));
+        NRGB_CUDA(cudaEventRecord(fork_, st));
+        NRGB_CUDA(cudaStreamWaitEvent(aux_[0], fork_, 0));
+        NRGB_CUDA(bt_wy_launch(d_slab, (int)slab.size(), blocks, aux_[0]));
+        NRGB_CUDA(cudaEventRecord(join_[0], aux_[0]));
+        ++launches_;
+      }
+    }
     // ---------------- 2) divide and conquer ----------------
     // Leaves in one launch, then the merges level by level (all problems'
     // nodes of a level together); every level's descriptors go to the
@@ -1693,6 +1735,13 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       // problems that are a single leaf already have D, Q in place
     }
     // ---------------- 3) back-transformation ----------------
+    // Column slabs in one launch (bt_apply.cu) for the blocks they hold.
+    if (!slab.empty()) {
+      NRGB_CUDA(cudaStreamWaitEvent(st, join_[0], 0));
+      NRGB_CUDA(bt_apply_launch(d_slab, (int)slab.size(), slab_cols, slab_ctas, slab_nmax, st));
+      ++launches_;
+    }
+    // The larger ones:
     // Z = H_0 H_1 ... H_{n-2} Z in blocks of NBB reflectors, last block
     // first: Z[r0:, :] -= V_k T_k (V_k^T Z[r0:, :]).  V (all reflectors, in
     // W1), every G_k = V_k^T V_k and every T_k are formed up front in four
@@ -1700,18 +1749,20 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     // their own slots (U, free after divide and conquer, holds blocks
     // k with (k+1) NBB <= n; the last block uses X), zeroed once.  All
     // descriptors go to the device in one copy.
-    {
-      int kmax = 0;
-      for (int b = 0; b < nbig; ++b) kmax = std::max(kmax, bt_nblk(bp[b].n));
+    if (!bp.empty()) {
+      const int nbt = (int)bp.size();
+      int kmax = 0, nmaxb = 0;
+      for (const BtProb& P : bp) nmaxb = std::max(nmaxb, P.n);
+      for (int b = 0; b < nbt; ++b) kmax = std::max(kmax, bt_nblk(bp[b].n));
       auto xslot = [&](int b, int k) {
         const int n = bp[b].n;
-        return (k + 1) * NBB <= n ? dp[b].U + (size_t)k * NBB * n : bt_X[b];
+        return (k + 1) * NBB <= n ? dp[bp_of[b]].U + (size_t)k * NBB * n : bt_X[bp_of[b]];
       };
       auto xsplit = [](int mrows) { return std::max(1, std::min(16, mrows / 128)); };
       auto gsplit = [](int mrows) { return std::max(1, std::min(16, mrows / 256)); };
       std::vector<ZeroSeg> bz;
       GemmBatch gg;  // every G_k
-      for (int b = 0; b < nbig; ++b) {
+      for (int b = 0; b < nbt; ++b) {
         const BtProb& P = bp[b];
         const int n = P.n;
         for (int k = 0; k < bt_nblk(n); ++k) {
@@ -1739,12 +1790,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       std::vector<Step> steps(kmax);
       for (int k = kmax - 1; k >= 0; --k) {
         Step& S = steps[k];
-        for (int b = 0; b < nbig; ++b) {
+        for (int b = 0; b < nbt; ++b) {
           const BtProb& P = bp[b];
           const int n = P.n;
           if (k >= bt_nblk(n)) continue;
           const int j0 = k * NBB, nb = std::min(NBB, n - 1 - j0), r0 = j0 + 1, mrows = n - r0;
-          double* Z = probs[big[b]].Z;
+          double* Z = probs[big[bp_of[b]]].Z;
           double* Xk = xslot(b, k);
           GemmSeg s{};
           s.A = P.V + r0 + (size_t)j0 * n;
@@ -1765,12 +1816,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           t.transB = 0;
           t.k = nb;
           t.alpha = 1.0;
-          S.gy.add(bt_Y[b], NBB, nb, n, 0.0, {t});
+          S.gy.add(bt_Y[bp_of[b]], NBB, nb, n, 0.0, {t});
           GemmSeg u{};
           u.A = P.V + r0 + (size_t)j0 * n;
           u.lda = n;
           u.transA = 0;
-          u.B = bt_Y[b];
+          u.B = bt_Y[bp_of[b]];
           u.ldb = NBB;
           u.transB = 0;
           u.k = nb;
@@ -1803,7 +1854,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         ++launches_;
       };
       if (kmax > 0) {
-        NRGB_LAUNCH("bt_buildV", st, bt_buildV_kernel<<<dim3(std::max(1, nmax - 1), nbig), 128, 0, st>>>(d_bp));
+        NRGB_LAUNCH("bt_buildV", st, bt_buildV_kernel<<<dim3(std::max(1, nmaxb - 1), nbt), 128, 0, st>>>(d_bp));
         NRGB_CUDA(cudaGetLastError());
         ++launches_;
         if (!bz.empty()) {
@@ -1814,7 +1865,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         }
         gemm(gg);
         NRGB_CUDA(raise_smem_attr((const void*)bt_T_kernel, (int)BT_T_SMEM));
-        NRGB_LAUNCH("bt_T", st, bt_T_kernel<<<dim3(kmax, nbig), BT_T_NT, BT_T_SMEM, st>>>(d_bp));
+        NRGB_LAUNCH("bt_T", st, bt_T_kernel<<<dim3(kmax, nbt), BT_T_NT, BT_T_SMEM, st>>>(d_bp));
         NRGB_CUDA(cudaGetLastError());
         ++launches_;
         for (int k = kmax - 1; k >= 0; --k) {
