@@ -98,7 +98,8 @@ struct TileLoader {
 
 __global__ void __launch_bounds__(NT) gemm_grouped_kernel(const GemmProb* __restrict__ probs,
                                                           int nprob,
-                                                          const GemmSeg* __restrict__ segs) {
+                                                          const GemmSeg* __restrict__ segs,
+                                                          const int* const* __restrict__ cmaps) {
   __shared__ __align__(16) double As[2][BK][LDS];
   __shared__ __align__(16) double Bs[2][BK][LDS];
 
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(NT) gemm_grouped_kernel(const GemmProb* __rest
 
   // Epilogue: C = acc + beta*C.
   const double beta = P.beta;
+  const int* cmap = cmaps ? cmaps[lo] : nullptr;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = row0 + wm + i * 8 + g;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(NT) gemm_grouped_kernel(const GemmProb* __rest
       for (int h = 0; h < 2; ++h) {
         const int c = col0 + wn + j * 8 + 2 * tq + h;
         if (c < n) {
-          double* dst = P.C + (size_t)c * P.ldc + r;
+          double* dst = P.C + (size_t)(cmap ? cmap[c] : c) * P.ldc + r;
           const double v = acc[i][j][h];
           if (ks > 1) atomicAdd(dst, v);
           else *dst = (beta == 0.0) ? v : v + beta * (*dst);
@@ -238,7 +240,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 __global__ void __launch_bounds__(LNT) gemm_grouped_large_kernel(const GemmProb* __restrict__ probs,
                                                                  int nprob,
-                                                                 const GemmSeg* __restrict__ segs) {
+                                                                 const GemmSeg* __restrict__ segs,
+                                                                 const int* const* __restrict__ cmaps) {
   extern __shared__ __align__(16) double lsm[];
   double* As = lsm;                               // [LSTAGES][BK][LLDS]
   double* Bs = lsm + LSTAGES * BK * LLDS;         // [LSTAGES][BK][LLDS]
@@ -363,6 +366,7 @@ __global__ void __launch_bounds__(LNT) gemm_grouped_large_kernel(const GemmProb*
   }
   cp_async_wait<0>();
   const double beta = P.beta;
+  const int* cmap = cmaps ? cmaps[lo] : nullptr;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = row0 + wm + i * 8 + g;
@@ -373,7 +377,7 @@ __global__ void __launch_bounds__(LNT) gemm_grouped_large_kernel(const GemmProb*
       for (int h = 0; h < 2; ++h) {
         const int c = col0 + wn + j * 8 + 2 * tq + h;
         if (c < n) {
-          double* dst = P.C + (size_t)c * P.ldc + r;
+          double* dst = P.C + (size_t)(cmap ? cmap[c] : c) * P.ldc + r;
           const double v = acc[i][j][h];
           if (ks > 1) atomicAdd(dst, v);
           else *dst = (beta == 0.0) ? v : v + beta * (*dst);
@@ -472,7 +476,8 @@ __device__ __forceinline__ bool pipe_vec_ok(const double* p, int ld) {
 template <int S, int KB>
 __global__ void __launch_bounds__(NT, 4) gemm_grouped_pipe_kernel(const GemmProb* __restrict__ probs,
                                                                int nprob,
-                                                               const GemmSeg* __restrict__ segs) {
+                                                               const GemmSeg* __restrict__ segs,
+                                                               const int* const* __restrict__ cmaps) {
   extern __shared__ __align__(16) double psm[];
   constexpr int PTILE = ptile<KB>();
   double* As = psm;                  // [S][PTILE]
@@ -589,6 +594,7 @@ __global__ void __launch_bounds__(NT, 4) gemm_grouped_pipe_kernel(const GemmProb
   cp_async_wait<0>();
 
   const double beta = P.beta;
+  const int* cmap = cmaps ? cmaps[lo] : nullptr;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = row0 + wm + i * 8 + g;
@@ -599,7 +605,7 @@ __global__ void __launch_bounds__(NT, 4) gemm_grouped_pipe_kernel(const GemmProb
       for (int h = 0; h < 2; ++h) {
         const int c = col0 + wn + j * 8 + 2 * tq + h;
         if (c < n) {
-          double* dst = P.C + (size_t)c * P.ldc + r;
+          double* dst = P.C + (size_t)(cmap ? cmap[c] : c) * P.ldc + r;
           const double v = acc[i][j][h];
           if (ks > 1) atomicAdd(dst, v);
           else *dst = (beta == 0.0) ? v : v + beta * (*dst);
@@ -635,7 +641,7 @@ int gemm_pipe_stages() {
 
 template <int S, int KB>
 cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
-                        cudaStream_t stream, const char* tag) {
+                        cudaStream_t stream, const char* tag, const int* const* cmaps) {
   static std::atomic<bool> attr[64];
   int dev = 0;
   cudaGetDevice(&dev);
@@ -646,7 +652,7 @@ cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_seg
     if (dev < 64) attr[dev].store(true, std::memory_order_release);
   }
   NRGB_LAUNCH(tag, stream,
-              gemm_grouped_pipe_kernel<S, KB><<<total_tiles, NT, pipe_smem<S, KB>(), stream>>>(d_probs, nprob, d_segs));
+              gemm_grouped_pipe_kernel<S, KB><<<total_tiles, NT, pipe_smem<S, KB>(), stream>>>(d_probs, nprob, d_segs, cmaps));
   return cudaGetLastError();
 }
 // The 128x128 cp.async variant is used only where the device's schedule
@@ -675,7 +681,8 @@ double gemm_flops(const GemmProb* probs, int nprob, const GemmSeg* segs) {
 }
 
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                int total_tiles, cudaStream_t stream, const char* tag, int total_stiles) {
+                                int total_tiles, cudaStream_t stream, const char* tag, int total_stiles,
+                                const int* const* cmaps) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
   // 128x128 tiles when the schedule selects them for this problem size,
   // they cover at most 30% more area than the 64x64 ones and they still give
@@ -696,22 +703,22 @@ cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSe
       if (dev < 64) attr[dev].store(true, std::memory_order_release);
     }
     NRGB_LAUNCH(tag, stream,
-                gemm_grouped_large_kernel<<<total_stiles, LNT, LSMEM, stream>>>(d_probs, nprob, d_segs));
+                gemm_grouped_large_kernel<<<total_stiles, LNT, LSMEM, stream>>>(d_probs, nprob, d_segs, cmaps));
     return cudaGetLastError();
   }
   const int stages = gemm_pipe_stages();
-  if (stages == 3) return pipe_launch<3, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag);
-  if (stages == 4) return pipe_launch<4, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag);
-  if (stages == 232) return pipe_launch<2, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag);
-  if (stages == 332) return pipe_launch<3, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag);
-  NRGB_LAUNCH(tag, stream, gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs));
+  if (stages == 3) return pipe_launch<3, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
+  if (stages == 4) return pipe_launch<4, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
+  if (stages == 232) return pipe_launch<2, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
+  if (stages == 332) return pipe_launch<3, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
+  NRGB_LAUNCH(tag, stream, gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs, cmaps));
   return cudaGetLastError();
 }
 
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                             int total_tiles, cudaStream_t stream) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
-  gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs);
+  gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs, nullptr);
   return cudaGetLastError();
 }
 

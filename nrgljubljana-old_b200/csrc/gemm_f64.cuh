@@ -50,9 +50,11 @@ void gemm_assign_tiles(GemmProb& p, int& tiles, int& stiles);
 // `tag` names the call site in the launch accounting (KernelStats).
 // total_stiles > 0 allows the 128x128-tile kernel, chosen when the launch's
 // problems are large enough that the bigger tiles waste little work.
+// cmaps (device, a pointer per problem; null: none): column j of problem p's
+// product goes to column cmaps[p][j] of its C.
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                 int total_tiles, cudaStream_t stream, const char* tag = "gemm_f64",
-                                int total_stiles = 0);
+                                int total_stiles = 0, const int* const* cmaps = nullptr);
 
 // Same launch without the library's launch accounting (no host bookkeeping,
 // no events): used by the allocation-free entry point.

@@ -23,6 +23,8 @@
 #include <numeric>
 
 #include "bt_apply.cuh"
+#include "dc_base.cuh"
+#include "dc_secular.cuh"
 #include "gemm_f64.cuh"
 #include "syev.cuh"
 #include "schedule.cuh"
@@ -33,209 +35,12 @@ namespace nrgb {
 
 namespace {
 
-constexpr int SMALL_N = 32;     // warp-per-problem path
-constexpr int LEAF = 16;        // D&C leaf size
+constexpr int SMALL_N = SYEV_TINY;  // blocks solved whole in one CTA
+constexpr int LEAF = DC_BASE;   // subtrees solved in one CTA (dc_base.cu)
 constexpr int NB = 32;          // tridiagonalisation panel width
 constexpr int NBB = BT_NB;      // back-transformation block of reflectors
 constexpr int TRD_NT = 256;     // threads of the panel kernel
 constexpr double EPS = 2.220446049250313e-16;
-
-// --------------------------------------------------------------------------
-// Small path: one warp per problem (n <= 32), everything in shared memory.
-// --------------------------------------------------------------------------
-struct SmallProb {
-  const double* A;
-  double* w;
-  double* Z;
-  int n;
-};
-
-constexpr int SMALL_WARPS = 2;
-
-// Implicit symmetric QR with Wilkinson shift on tridiagonal (d, e),
-// rotations accumulated into the columns of Z (Z <- Z G^T).  dn, en: 32
-// doubles each of scratch (the step's new d, e).
-__device__ void givens_qr_sweep_warp(double* d, double* e, double (*Z)[33], int n, int lane,
-                                     double* cs, double* dn, double* en, int* fail) {
-  int iter = 0;
-  const int maxiter = 40 * n + 40;
-  int hi = n - 1;
-  while (hi > 0) {
-    // lane 0 drives the sequential part; all lanes follow the same control flow
-    int lo;
-    if (lane == 0) {
-      // deflate from the bottom
-      while (hi > 0 && fabs(e[hi - 1]) <= EPS * (fabs(d[hi - 1]) + fabs(d[hi]))) {
-        e[hi - 1] = 0.0;
-        --hi;
-      }
-      lo = hi;
-      while (lo > 0 && fabs(e[lo - 1]) > EPS * (fabs(d[lo - 1]) + fabs(d[lo]))) --lo;
-      cs[2] = (double)hi;
-      cs[3] = (double)lo;
-    }
-    __syncwarp();
-    hi = (int)cs[2];
-    lo = (int)cs[3];
-    __syncwarp();
-    if (hi <= 0) break;
-    if (++iter > maxiter) {
-      if (lane == 0) atomicExch(fail, 1);
-      break;
-    }
-    // One implicit QR step on [lo, hi].  Every lane runs the same scalar
-    // recurrence (so no lane waits for another's rotation), carrying the
-    // running d[k], e[k], the bulge and the next x in registers.  The step
-    // reads only d, e and stores only into dn, en (lane 0), which are copied
-    // back after the step, so lanes need no synchronisation inside it.
-    double a = d[lo], b = e[lo];
-    double x, z = b;
-    {
-      const double dl = (d[hi - 1] - d[hi]) * 0.5;
-      const double eh = e[hi - 1];
-      const double den = dl + copysign(hypot(dl, eh), dl == 0.0 ? 1.0 : dl);
-      x = a - (d[hi] - eh * eh / den);
-    }
-    for (int k = lo; k < hi; ++k) {
-      const double dd = d[k + 1];
-      const double ekn = (k + 1 < hi) ? e[k + 1] : 0.0;
-      double c = 1.0, s = 0.0, r = 0.0;
-      const double r2 = x * x + z * z;
-      if (r2 > 0.0 && r2 < 1e300) {
-        r = sqrt(r2);
-        const double ri = 1.0 / r;
-        c = x * ri;
-        s = z * ri;
-      } else if (x != 0.0 || z != 0.0) {  // squares out of range
-        r = hypot(x, z);
-        c = x / r;
-        s = z / r;
-      }
-      const double cc = c * c, ss = s * s, csb = 2.0 * c * s * b;
-      const double dk = cc * a + csb + ss * dd;
-      const double dk1 = ss * a - csb + cc * dd;
-      const double ek = c * s * (dd - a) + (cc - ss) * b;
-      if (lane == 0) {
-        if (k > lo) en[k - 1] = r;
-        dn[k] = dk;
-      }
-      if (lane < n) {
-        const double zk = Z[lane][k], zk1 = Z[lane][k + 1];
-        Z[lane][k] = c * zk + s * zk1;
-        Z[lane][k + 1] = -s * zk + c * zk1;
-      }
-      a = dk1;  // d[k+1]
-      x = ek;   // e[k], the next rotation's x
-      b = c * ekn;
-      z = s * ekn;  // bulge
-    }
-    if (lane == 0) {
-      dn[hi] = a;
-      en[hi - 1] = x;
-    }
-    __syncwarp();
-    if (lane >= lo && lane <= hi) d[lane] = dn[lane];
-    if (lane >= lo && lane < hi) e[lane] = en[lane];
-    __syncwarp();
-  }
-  __syncwarp();
-}
-
-__global__ void __launch_bounds__(32 * SMALL_WARPS) syev_small_kernel(const SmallProb* probs,
-                                                                       int nprob, int* fail) {
-  __shared__ double As[SMALL_WARPS][32][33];
-  __shared__ double Zs[SMALL_WARPS][32][33];
-  __shared__ double dv[SMALL_WARPS][32], ev[SMALL_WARPS][32], vv[SMALL_WARPS][32],
-      wv[SMALL_WARPS][32], tv[SMALL_WARPS][32];
-  __shared__ double csv[SMALL_WARPS][4];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = blockIdx.x * SMALL_WARPS + warp;
-  if (p >= nprob) return;
-  const SmallProb P = probs[p];
-  const int n = P.n;
-  double(*A)[33] = As[warp];
-  double(*Z)[33] = Zs[warp];
-  double *d = dv[warp], *e = ev[warp], *v = vv[warp], *w = wv[warp], *tau = tv[warp];
-  for (int j = 0; j < n; ++j) A[lane][j] = (lane < n) ? P.A[lane + (size_t)j * n] : 0.0;
-  __syncwarp();
-  // Householder tridiagonalisation: columns c = 0 .. n-3
-  for (int c = 0; c + 2 < n; ++c) {
-    const double xi = (lane >= c + 2 && lane < n) ? A[lane][c] : 0.0;
-    const double xn2 = warp_sum(xi * xi);
-    const double alpha = A[c + 1][c];
-    double tc = 0.0, beta = alpha, scal = 0.0;
-    if (xn2 != 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-      tc = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
-    }
-    const double vi = (lane == c + 1) ? 1.0 : ((lane >= c + 2 && lane < n) ? A[lane][c] * scal : 0.0);
-    v[lane] = vi;
-    __syncwarp();
-    // p = tau A22 v
-    double pi = 0.0;
-    if (lane >= c + 1 && lane < n)
-      for (int j = c + 1; j < n; ++j) pi += A[lane][j] * v[j];
-    pi *= tc;
-    const double pv = warp_sum(pi * vi);
-    const double wi = pi - 0.5 * tc * pv * vi;
-    w[lane] = wi;
-    __syncwarp();
-    if (lane >= c + 1 && lane < n)
-      for (int j = c + 1; j < n; ++j) A[lane][j] -= vi * w[j] + wi * v[j];
-    __syncwarp();
-    if (lane >= c + 2 && lane < n) A[lane][c] = vi;  // store reflector
-    if (lane == 0) {
-      e[c] = beta;
-      tau[c] = tc;
-    }
-    __syncwarp();
-  }
-  if (lane < n) d[lane] = A[lane][lane];
-  if (lane == 0 && n >= 2) e[n - 2] = A[n - 1][n - 2];
-  // Form Q = H_0 H_1 ... H_{n-3} explicitly (Z <- I, then Z <- H_c Z for c descending)
-  for (int j = 0; j < n; ++j) Z[lane][j] = (lane == j) ? 1.0 : 0.0;
-  __syncwarp();
-  for (int c = n - 3; c >= 0; --c) {
-    const double tc = tau[c];
-    if (tc == 0.0) continue;
-    // lane j handles column j of Z
-    if (lane < n) {
-      double s = Z[c + 1][lane];
-      for (int i = c + 2; i < n; ++i) s += A[i][c] * Z[i][lane];
-      s *= tc;
-      Z[c + 1][lane] -= s;
-      for (int i = c + 2; i < n; ++i) Z[i][lane] -= A[i][c] * s;
-    }
-    __syncwarp();
-  }
-  givens_qr_sweep_warp(d, e, Z, n, lane, csv[warp], v, w, fail);
-  // sort ascending (selection sort by lane 0, swap columns by all lanes)
-  for (int i = 0; i < n - 1; ++i) {
-    if (lane == 0) {
-      int kmin = i;
-      for (int k = i + 1; k < n; ++k)
-        if (d[k] < d[kmin]) kmin = k;
-      csv[warp][0] = (double)kmin;
-      if (kmin != i) {
-        const double t = d[i];
-        d[i] = d[kmin];
-        d[kmin] = t;
-      }
-    }
-    __syncwarp();
-    const int kmin = (int)csv[warp][0];
-    if (kmin != i && lane < n) {
-      const double t = Z[lane][i];
-      Z[lane][i] = Z[lane][kmin];
-      Z[lane][kmin] = t;
-    }
-    __syncwarp();
-  }
-  if (lane < n) P.w[lane] = d[lane];
-  for (int j = 0; j < n; ++j)
-    if (lane < n) P.Z[lane + (size_t)j * n] = Z[lane][j];
-}
 
 // --------------------------------------------------------------------------
 // Tridiagonalisation panel (cooperative persistent kernel).
@@ -522,18 +327,19 @@ struct DcProb {
   double* Q;      // n x n (ld n): eigenvectors of T
   double* W1;     // n x n workspace
   double* U;      // n x n workspace
-  double* ds;     // n sorted d (then compacted dK in [lo, lo+k))
-  double* zs;     // n sorted z (then zK)
-  double* dD;     // n deflated values (at [lo+k, hi))
-  int* src;       // n source column of sorted position
-  int* flag;      // n per sorted position: 1 = nondeflated, 0 = deflated
+  double* ds;     // n: poles of the secular equation at [lo, lo+k), ascending, scaled by sc
+  double* zs;     // n: their weights
+  double* val;    // n: the node's new eigenvalues: roots at [lo, lo+k), deflated values after
+  int* src;       // n child column of a sorted position
+  int* cmap;      // n child column of a compacted position (nondeflated first)
   double* tau;    // n
   int* orig;      // n
   double* zhat;   // n
   int* kcnt;      // n (value at index lo of a node)
-  double* rho;    // n (value at index lo)
-  int* rank;      // n final position
-  int* rotp;      // n rotation pairs (p index)
+  double* rho;    // n (value at index lo; scaled by sc)
+  double* sc;     // n (value at index lo): power of two that brings the node's scale near 1
+  int* rank;      // n final column of a compacted position
+  int* rotp;      // n rotation pairs (compacted positions)
   int* rotj;      // n
   double* rotc;   // n
   double* rots;   // n
@@ -544,214 +350,230 @@ struct DcNode {
   int prob, lo, mid, hi;
 };
 
-// Leaf: tridiagonal QR on [lo, hi) of one problem, one warp per leaf.
-__global__ void __launch_bounds__(64) dc_leaf_kernel(const DcProb* __restrict__ probs,
-                                                     const DcNode* __restrict__ leaves, int nleaf,
-                                                     int* fail) {
-  __shared__ double Zs[2][32][33];
-  __shared__ double dv[2][32], ev[2][32], csv[2][4], dnv[2][32], env[2][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int li = blockIdx.x * 2 + warp;
-  if (li >= nleaf) return;
-  const DcNode L = leaves[li];
-  const DcProb P = probs[L.prob];
-  const int n = P.n, lo = L.lo, s = L.hi - L.lo;
-  double* d = dv[warp];
-  double* e = ev[warp];
-  double(*Z)[33] = Zs[warp];
-  if (lane < s) {
-    double dd = P.dT[lo + lane];
-    if (lane == 0 && lo > 0) dd -= fabs(P.e[lo - 1]);
-    if (lane == s - 1 && L.hi < n) dd -= fabs(P.e[L.hi - 1]);
-    d[lane] = dd;
-    if (lane < s - 1) e[lane] = P.e[lo + lane];
-  }
-  for (int j = 0; j < s; ++j) Z[lane][j] = (lane == j) ? 1.0 : 0.0;
-  __syncwarp();
-  givens_qr_sweep_warp(d, e, Z, s, lane, csv[warp], dnv[warp], env[warp], fail);
-  for (int i = 0; i < s - 1; ++i) {
-    if (lane == 0) {
-      int kmin = i;
-      for (int k = i + 1; k < s; ++k)
-        if (d[k] < d[kmin]) kmin = k;
-      csv[warp][0] = (double)kmin;
-      if (kmin != i) {
-        const double t = d[i];
-        d[i] = d[kmin];
-        d[kmin] = t;
-      }
-    }
-    __syncwarp();
-    const int kmin = (int)csv[warp][0];
-    if (kmin != i && lane < s) {
-      const double t = Z[lane][i];
-      Z[lane][i] = Z[lane][kmin];
-      Z[lane][kmin] = t;
-    }
-    __syncwarp();
-  }
-  if (lane < s) P.D[lo + lane] = d[lane];
-  for (int j = 0; j < s; ++j)
-    if (lane < s) P.Q[(size_t)(lo + lane) + (size_t)(lo + j) * n] = Z[lane][j];
-}
-
-// Merge, step 1: z, sort, deflation, rotations, compaction.  One CTA per node.
-// The sorted d and z and the deflation flags live in a work area: dynamic
-// shared memory when the node has at most `cap` entries (the launch's
-// shared memory holds 2 cap doubles and cap ints), else the node's slices
-// of zhat, tau and flag in global memory, which are free at this point.  The
-// two sequential scans (deflation, compaction order) run on the work area.
+// Merge of a node, step 1: z, sorted order, deflation, compaction.  One CTA per
+// node.  The values live in shared memory (40 bytes an entry) when the node has
+// at most `cap` entries, else in the node's slices of its work arrays in global
+// memory.  Deflation by a close pair changes the pair, so the scan is sequential
+// in the pairs that deflate; a warp tests 32 pairs at a time and stops at the
+// first close one, which makes the scan of a node without close pairs
+// parallel (one thread tested them one by one before: 48 us of an n = 301 node).
 constexpr int DC_NT = 256;
-constexpr int DC_PREP_CAP = 8192;  // largest node staged in shared memory (160 KB)
+constexpr int DC_PREP_CAP = 5600;  // largest node staged in shared memory (219 KB)
 
-__host__ __device__ inline size_t dc_prep_smem(int cap) { return (size_t)cap * (2 * sizeof(double) + sizeof(int)); }
+__host__ __device__ inline size_t dc_prep_smem(int cap) { return (size_t)cap * (3 * sizeof(double) + 4 * sizeof(int)); }
+
+// Exclusive prefix sum of f(j) over 0 <= j < n by the CTA (each thread a run of
+// consecutive j); g(j, prefix) for every j; returns the total.
+template <class F, class H>
+__device__ __forceinline__ int dc_prefix(int n, int* scratch, F&& f, H&& g) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (n + DC_NT - 1) / DC_NT, j0 = min(n, tid * per), j1 = min(n, j0 + per);
+  int c = 0;
+  for (int j = j0; j < j1; ++j) c += f(j);
+  int inc = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  __syncthreads();
+  if (lane == 31) scratch[warp] = inc;
+  __syncthreads();
+  int base = 0, tot = 0;
+#pragma unroll
+  for (int w = 0; w < DC_NT / 32; ++w) {
+    base += w < warp ? scratch[w] : 0;
+    tot += scratch[w];
+  }
+  int at = base + inc - c;
+  for (int j = j0; j < j1; ++j) {
+    const int v = f(j);
+    g(j, at);
+    at += v;
+  }
+  __syncthreads();
+  return tot;
+}
 
 __global__ void __launch_bounds__(DC_NT) dc_prep_kernel(const DcProb* __restrict__ probs,
                                                         const DcNode* __restrict__ nodes,
                                                         GemmProb* gprob, GemmSeg* gseg, int cap) {
   extern __shared__ double dcsm[];
   __shared__ double mx[2][DC_NT / 32];
-  __shared__ int sk[2];
+  __shared__ int scratch[DC_NT / 32], s_rot;
   const DcNode N = nodes[blockIdx.x];
   const DcProb P = probs[N.prob];
   const int n = P.n, lo = N.lo, mid = N.mid, hi = N.hi;
   const int n1 = mid - lo, np = hi - lo;
   const size_t ld = (size_t)n;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool staged = np <= cap;
-  double* wd = staged ? dcsm : P.zhat + lo;
-  double* wz = staged ? dcsm + cap : P.tau + lo;
-  int* wf = staged ? reinterpret_cast<int*>(dcsm + 2 * (size_t)cap) : P.flag + lo;
+  double* dl = staged ? dcsm : P.D + lo;             // the two children's values
+  double* wd = staged ? dcsm + cap : P.val + lo;     // sorted d, z
+  double* wz = staged ? dcsm + 2 * (size_t)cap : P.tau + lo;
+  int* wi = reinterpret_cast<int*>(dcsm + 3 * (size_t)cap);
+  int* wf = staged ? wi : P.orig + lo;               // 1: stays in the secular equation
+  int* list = staged ? wi + cap : P.rank + lo;       // sorted positions with a z that is not small
+  int* src = staged ? wi + 2 * (size_t)cap : P.src + lo;
+  int* pos = staged ? wi + 3 * (size_t)cap : P.cmap + lo;  // compacted position of a sorted one
   const double beta = P.e[mid - 1];
   const double rho = 2.0 * fabs(beta);
   const double sgn = beta >= 0.0 ? 1.0 : -1.0;
   const double isq2 = 0.70710678118654752440;
+  if (staged)
+    for (int i = tid; i < np; i += DC_NT) dl[i] = P.D[lo + i];
+  for (int i = tid; i < np; i += DC_NT) src[i] = i;
+  __syncthreads();
   // sorted positions by merging the two ascending halves
   double dmax = 0.0, zmax = 0.0;
   for (int i = tid; i < np; i += DC_NT) {
-    const double di = P.D[lo + i];
+    const double di = dl[i];
     double zi;
-    int pos;
+    int p;
     if (i < n1) {
       zi = P.Q[(size_t)(mid - 1) + (size_t)(lo + i) * ld] * isq2;
-      // count of second-half values strictly less than di
-      int a = 0, b = np - n1;
+      int a = n1, b = np;  // second-half values less than di
       while (a < b) {
         const int m = (a + b) >> 1;
-        if (P.D[mid + m] < di) a = m + 1; else b = m;
+        if (dl[m] < di) a = m + 1;
+        else b = m;
       }
-      pos = i + a;
+      p = i + (a - n1);
     } else {
       zi = sgn * P.Q[(size_t)mid + (size_t)(lo + i) * ld] * isq2;
       int a = 0, b = n1;
       while (a < b) {
         const int m = (a + b) >> 1;
-        if (P.D[lo + m] <= di) a = m + 1; else b = m;
+        if (dl[m] <= di) a = m + 1;
+        else b = m;
       }
-      pos = (i - n1) + a;
+      p = (i - n1) + a;
     }
-    wd[pos] = di;
-    wz[pos] = zi;
-    P.src[lo + pos] = i;
+    wd[p] = di;
+    wz[p] = zi;
+    src[p] = i;
     dmax = fmax(dmax, fabs(di));
     zmax = fmax(zmax, fabs(zi));
   }
-  // block max of |d| and |z|
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
     zmax = fmax(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
   }
-  if ((tid & 31) == 0) {
-    mx[0][tid >> 5] = dmax;
-    mx[1][tid >> 5] = zmax;
+  if (lane == 0) {
+    mx[0][warp] = dmax;
+    mx[1][warp] = zmax;
   }
   __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < DC_NT / 32; ++w) {
-      dmax = fmax(dmax, mx[0][w]);
-      zmax = fmax(zmax, mx[1][w]);
-    }
-    // deflation scan (sequential)
-    const double tol = 8.0 * EPS * fmax(dmax, rho * zmax);
-    int nr = 0, k = 0, prev = -1;
-    for (int j = 0; j < np; ++j) {
-      wf[j] = 0;
-      if (rho * fabs(wz[j]) <= tol) continue;  // deflated by small z
-      if (prev < 0) {
-        prev = j;
+#pragma unroll
+  for (int w = 0; w < DC_NT / 32; ++w) {
+    dmax = fmax(dmax, mx[0][w]);
+    zmax = fmax(zmax, mx[1][w]);
+  }
+  const double big = fmax(dmax, rho * zmax), tol = 8.0 * EPS * big, sc = scale_near_one(big);
+  // deflation: small z
+  const int m = dc_prefix(
+      np, scratch, [&](int j) { return rho * fabs(wz[j]) <= tol ? 0 : 1; },
+      [&](int j, int at) {
+        const int f = rho * fabs(wz[j]) <= tol ? 0 : 1;
+        wf[j] = f;
+        if (f) list[at] = j;
+      });
+  // close pairs, in order: |dt c s| <= tol with c = z_j / t, s = -z_p / t,
+  // t = |(z_j, z_p)|, tested as |dt z_j z_p| <= tol t^2 (both |z| exceed
+  // tol / rho here, so t^2 is normal)
+  if (warp == 0) {
+    int nr = 0;
+    auto close = [&](int p, int j) {
+      const double zp = wz[p], zj = wz[j], dt = wd[j] - wd[p];
+      return fabs(dt * zj * zp) <= tol * (zj * zj + zp * zp);
+    };
+    int i = 1;
+    while (i < m) {
+      const int q = i + lane;
+      const unsigned hit = __ballot_sync(0xffffffffu, q < m && close(list[q - 1], list[q]));
+      if (!hit) {
+        i += 32;
         continue;
       }
-      // |dt c s| <= tol with c = z_j / t, s = -z_p / t, t = |(z_j, z_p)|,
-      // tested as |dt z_j z_p| <= tol t^2: no root or division for the
-      // entries that stay (both |z| exceed tol / rho here, so t^2 is normal)
-      const double zp = wz[prev], zj = wz[j];
-      const double dt = wd[j] - wd[prev];
-      if (fabs(dt * zj * zp) <= tol * (zj * zj + zp * zp)) {
-        const double t = hypot(zj, zp);
-        const double c = zj / t, s = -zp / t;
-        wz[j] = t;
-        wz[prev] = 0.0;
-        const double dp = wd[prev], dj = wd[j];
-        wd[prev] = dp * c * c + dj * s * s;
-        wd[j] = dp * s * s + dj * c * c;
-        P.rotp[lo + nr] = prev;
-        P.rotj[lo + nr] = j;
-        P.rotc[lo + nr] = c;
-        P.rots[lo + nr] = s;
+      i += __ffs(hit) - 1;
+      // from here one pair after another until a pair is not close
+      do {
+        if (lane == 0) {
+          const int p = list[i - 1], j = list[i];
+          const double zp = wz[p], zj = wz[j];
+          const double t = hypot(zj, zp);
+          const double c = zj / t, s = -zp / t;
+          const double dp = wd[p], dj = wd[j];
+          wz[j] = t;
+          wz[p] = 0.0;
+          wd[p] = dp * c * c + dj * s * s;
+          wd[j] = dp * s * s + dj * c * c;
+          wf[p] = 0;
+          P.rotp[lo + nr] = p;
+          P.rotj[lo + nr] = j;
+          P.rotc[lo + nr] = c;
+          P.rots[lo + nr] = s;
+        }
+        __syncwarp();
         ++nr;
-        prev = j;  // prev deflated (flag stays 0)
-      } else {
-        wf[prev] = 1;
-        ++k;
-        prev = j;
-      }
+        ++i;
+      } while (i < m && close(list[i - 1], list[i]));
+      ++i;  // the pair (i - 1, i) was tested just now
     }
-    if (prev >= 0) {
-      wf[prev] = 1;
-      ++k;
-    }
-    sk[0] = k;
-    sk[1] = nr;
-    P.kcnt[lo] = k;
-    P.rho[lo] = rho;
-    P.nrot[lo] = nr;
-    // compaction order: nondeflated first (in order), then deflated (in
-    // order); rank holds, for now, the sorted position of each target
-    int kk = 0, dd = 0;
-    for (int j = 0; j < np; ++j) {
-      if (wf[j]) {
-        P.rank[lo + kk] = j;
-        ++kk;
-      } else {
-        P.rank[lo + k + dd] = j;
-        ++dd;
-      }
-    }
+    if (lane == 0) s_rot = nr;
   }
   __syncthreads();
-  const int k = sk[0];
-  // compact the values out of the work area
-  for (int a = tid; a < np; a += DC_NT) {
-    const int j = P.rank[lo + a];
-    if (a < k) {
-      P.ds[lo + a] = wd[j];
-      P.zs[lo + a] = wz[j];
-    } else {
-      P.dD[lo + a] = wd[j];
+  const int nr = s_rot;
+  // compaction: nondeflated first (in order), then deflated (in order)
+  const int k = dc_prefix(
+      np, scratch, [&](int j) { return wf[j]; }, [&](int j, int at) { pos[j] = at; });
+  for (int j = tid; j < np; j += DC_NT) {
+    const int at = wf[j] ? pos[j] : k + (j - pos[j]);
+    const int col = min(max(src[j], 0), np - 1);
+    if (staged) {
+      P.cmap[lo + at] = col;
+      if (wf[j]) {
+        P.ds[lo + at] = wd[j] * sc;
+        P.zs[lo + at] = wz[j];
+      } else {
+        P.val[lo + at] = wd[j];
+      }
+    } else {  // the work arrays double as outputs: through others
+      P.zhat[lo + at] = wd[j];
+      P.ds[lo + at] = wd[j] * sc;
+      P.zs[lo + at] = wz[j];
+      P.kcnt[lo + at] = col;
     }
   }
-  // GEMM descriptor: W1[lo:hi, lo:lo+k] = Q[lo:hi, lo:lo+k] * U[lo:lo+k, lo:lo+k]
+  for (int r = tid; r < nr; r += DC_NT) {
+    const int p = P.rotp[lo + r], j = P.rotj[lo + r];
+    P.rotp[lo + r] = k + (p - pos[p]);
+    P.rotj[lo + r] = wf[j] ? pos[j] : k + (j - pos[j]);
+  }
+  __syncthreads();
+  if (!staged) {
+    for (int a = tid; a < np; a += DC_NT) {
+      P.cmap[lo + a] = P.kcnt[lo + a];
+      P.val[lo + a] = P.zhat[lo + a];
+    }
+    __syncthreads();
+  }
   if (tid == 0) {
+    P.kcnt[lo] = k;
+    P.rho[lo] = rho * sc;
+    P.sc[lo] = sc;
+    P.nrot[lo] = nr;
+    // GEMM descriptor (columns placed by rank): Q[lo:hi, :] = W1[lo:hi, lo:lo+k] * U[lo:lo+k, lo:lo+k]
     GemmProb g = gprob[blockIdx.x];  // tile0/tiles_n preset by the host
-    g.C = P.W1 + lo + (size_t)lo * ld;
+    g.C = P.Q + lo + (size_t)lo * ld;
     g.ldc = n;
     g.m = np;
     g.n = k;
     g.beta = 0.0;
     gprob[blockIdx.x] = g;
     GemmSeg s;
-    s.A = P.Q + lo + (size_t)lo * ld;
+    s.A = P.W1 + lo + (size_t)lo * ld;
     s.lda = n;
     s.B = P.U + lo + (size_t)lo * ld;
     s.ldb = n;
@@ -763,16 +585,12 @@ __global__ void __launch_bounds__(DC_NT) dc_prep_kernel(const DcProb* __restrict
   }
 }
 
-// Merge, step 2, in three launches over the node's block Q[lo:hi, lo:hi]
-// (rows independent throughout):
-//   gather:  W1[:, pos] = Q[:, src[pos]], the child eigenvector columns in
-//            sorted order (a CTA per 128 rows x DC_PCOLS columns);
-//   rotate:  the deflation rotations in order, one thread per row (nothing
-//            to do when the node has none);
-//   compact: Q[:, a] = W1[:, rank[a]], nondeflated columns first.
+// Step 2: the child eigenvector columns in compacted order, W1[:, a] =
+// Q[:, cmap[a]] (a CTA per 128 rows x DC_PCOLS columns), then the deflation
+// rotations in order, one thread per row (nothing to do when there are none).
 constexpr int DC_PCOLS = 8;
 
-__global__ void dc_gather_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes, int compact) {
+__global__ void dc_gather_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes) {
   const DcNode N = nodes[blockIdx.z];
   const DcProb P = probs[N.prob];
   const int lo = N.lo, np = N.hi - N.lo;
@@ -780,9 +598,9 @@ __global__ void dc_gather_kernel(const DcProb* __restrict__ probs, const DcNode*
   const int c0 = blockIdx.y * DC_PCOLS;
   if (r >= np || c0 >= np) return;
   const size_t ld = (size_t)P.n;
-  const int* map = compact ? P.rank + lo : P.src + lo;
-  const double* from = (compact ? P.W1 : P.Q) + (size_t)(lo + r) + (size_t)lo * ld;
-  double* to = (compact ? P.Q : P.W1) + (size_t)(lo + r) + (size_t)lo * ld;
+  const int* map = P.cmap + lo;
+  const double* from = P.Q + (size_t)(lo + r) + (size_t)lo * ld;
+  double* to = P.W1 + (size_t)(lo + r) + (size_t)lo * ld;
   const int c1 = min(np, c0 + DC_PCOLS);
   for (int c = c0; c < c1; ++c) to[(size_t)c * ld] = from[(size_t)map[c] * ld];
 }
@@ -805,212 +623,89 @@ __global__ void dc_rotate_kernel(const DcProb* __restrict__ probs, const DcNode*
   }
 }
 
-// Secular equation roots, one warp per root: lanes share the pole sums.
+// Step 3: secular equation roots, one warp per root.
 __global__ void dc_secular_warp_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes,
                                        int* fail) {
-  const int node = blockIdx.y;
   const int j = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const DcNode N = nodes[node];
+  const DcNode N = nodes[blockIdx.y];
   const DcProb P = probs[N.prob];
   const int lo = N.lo;
   const int k = P.kcnt[lo];
   if (j >= k) return;
-  const double* d = P.ds + lo;
-  const double* z = P.zs + lo;
-  const double rho = P.rho[lo];
+  double t;
   int o;
-  double tlo, thi;
-  if (j < k - 1) {
-    const double mid = 0.5 * (d[j + 1] - d[j]);
-    double f = 0.0;
-    for (int i = lane; i < k; i += 32) f += z[i] * z[i] / ((d[i] - d[j]) - mid);
-    f = 1.0 + rho * warp_sum(f);
-    if (f >= 0.0) {
-      o = j;
-      tlo = 0.0;
-      thi = mid;
-    } else {
-      o = j + 1;
-      tlo = -mid;
-      thi = 0.0;
-    }
-  } else {
-    double zz = 0.0;
-    for (int i = lane; i < k; i += 32) zz += z[i] * z[i];
-    zz = warp_sum(zz);
-    o = j;
-    tlo = 0.0;
-    thi = rho * zz;
-  }
-  const double dorig = d[o];
-  const double dL = d[j] - dorig;
-  const double dR = (j < k - 1) ? d[j + 1] - dorig : 0.0;
-  double t = 0.5 * (tlo + thi);
-  bool done = false;
-  for (int it = 0; it < 400; ++it) {
-    double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
-    for (int i = lane; i < k; i += 32) {
-      const double del = (d[i] - dorig) - t;
-      const double q = z[i] / del;
-      if (i <= j) {
-        psi += z[i] * q;
-        dpsi += q * q;
-      } else {
-        phi += z[i] * q;
-        dphi += q * q;
-      }
-    }
-    psi = warp_sum(psi);
-    dpsi = warp_sum(dpsi);
-    phi = warp_sum(phi);
-    dphi = warp_sum(dphi);
-    // all lanes hold identical sums and run the same scalar update
-    const double f = 1.0 + rho * (psi + phi);
-    if (f == 0.0) {
-      done = true;
-      break;
-    }
-    if (f < 0.0) tlo = t; else thi = t;
-    double tn;
-    const double DL = dL - t;
-    if (j < k - 1) {
-      const double DR = dR - t;
-      const double sL = rho * dpsi * DL * DL, sR = rho * dphi * DR * DR;
-      const double cc = f - sL / DL - sR / DR;
-      const double bb = cc * (DL + DR) + sL + sR;
-      const double c0 = DL * DR * f;
-      double eta;
-      if (cc == 0.0) {
-        eta = c0 / bb;
-      } else {
-        const double sq = sqrt(fmax(bb * bb - 4.0 * cc * c0, 0.0));
-        const double qq = (bb >= 0.0) ? bb + sq : bb - sq;
-        const double e1 = qq / (2.0 * cc), e2 = 2.0 * c0 / qq;
-        eta = (e1 > DL && e1 < DR) ? e1 : e2;
-      }
-      tn = t + eta;
-    } else {
-      const double sL = rho * dpsi * DL * DL;
-      const double cc = f - sL / DL;
-      tn = (cc > 0.0) ? t + DL + sL / cc : 0.5 * (tlo + thi);
-    }
-    if (fabs(tn - t) <= 2.0 * EPS * fabs(t) || fabs(f) <= EPS * (8.0 + 8.0 * rho * (phi - psi))) {
-      done = true;
-      break;
-    }
-    if (!(tn > tlo && tn < thi)) tn = 0.5 * (tlo + thi);
-    if (thi - tlo <= 4.0 * EPS * fmax(fabs(tlo), fabs(thi))) {
-      t = tn;
-      done = true;
-      break;
-    }
-    t = tn;
-  }
+  bool bad;
+  secular_root<32>(P.ds + lo, P.zs + lo, k, j, P.rho[lo], lane, true, t, o, bad);
   if (lane == 0) {
-    if (!done && thi - tlo > 1e-10 * fmax(fabs(tlo), fabs(thi))) atomicExch(fail, 2);
+    if (bad) atomicExch(fail, 2);
     P.tau[lo + j] = t;
     P.orig[lo + j] = o;
+    P.val[lo + j] = (P.ds[lo + o] + t) / P.sc[lo];
   }
 }
 
-// Loewner z-hat.  One warp per i; lanes share the product over j.
+// Step 4: Loewner z-hat of the nondeflated entries and the final column of
+// every entry (its rank among the node's new eigenvalues), one warp per
+// entry; writes D.
 __global__ void dc_lowner_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes) {
-  const int node = blockIdx.y;
   const int i = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const DcNode N = nodes[node];
+  const DcNode N = nodes[blockIdx.y];
   const DcProb P = probs[N.prob];
-  const int lo = N.lo;
+  const int lo = N.lo, np = N.hi - N.lo;
+  if (i >= np) return;
   const int k = P.kcnt[lo];
+  const double x = P.val[lo + i];
+  unsigned r = 0;
+  for (int b = lane; b < np; b += 32) {
+    const double y = P.val[lo + b];
+    r += (y < x) || (y == x && b < i);
+  }
+  r = __reduce_add_sync(0xffffffffu, r);
+  if (lane == 0) {
+    P.rank[lo + i] = (int)r;
+    P.D[lo + r] = x;
+  }
   if (i >= k) return;
   const double* d = P.ds + lo;
-  const double rho = P.rho[lo];
-  const double di = d[i];
-  auto lam_minus = [&](int j) { return (d[P.orig[lo + j]] - di) + P.tau[lo + j]; };
-  double prod = 1.0;
-  for (int j = lane; j < k - 1; j += 32) prod *= lam_minus(j) / ((j < i ? d[j] : d[j + 1]) - di);
+  double prod = lowner_product<32>(d, P.orig + lo, P.tau + lo, k, i, lane);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, o);
-  prod *= lam_minus(k - 1) / rho;
+  prod *= ((d[P.orig[lo + k - 1]] - d[i]) + P.tau[lo + k - 1]) / P.rho[lo];
   if (lane == 0) P.zhat[lo + i] = copysign(sqrt(fmax(prod, 0.0)), P.zs[lo + i]);
 }
 
-// Eigenvectors of the rank-one problem.  One warp per column j.
+// Step 5: eigenvectors of the rank-one problem, one warp per column j < k; the
+// deflated columns go from W1 to their place in Q.
 __global__ void dc_vectors_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes) {
-  const int node = blockIdx.y;
   const int j = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const DcNode N = nodes[node];
+  const DcNode N = nodes[blockIdx.y];
   const DcProb P = probs[N.prob];
-  const int lo = N.lo;
+  const int lo = N.lo, np = N.hi - N.lo;
+  if (j >= np) return;
   const int k = P.kcnt[lo];
-  if (j >= k) return;
+  const size_t ld = (size_t)P.n;
+  if (j >= k) {
+    const double* s = P.W1 + lo + (size_t)(lo + j) * ld;
+    double* t = P.Q + lo + (size_t)(lo + P.rank[lo + j]) * ld;
+    for (int i = lane; i < np; i += 32) t[i] = s[i];
+    return;
+  }
   const double* d = P.ds + lo;
   const double dor = d[P.orig[lo + j]];
   const double tj = P.tau[lo + j];
-  double* col = P.U + lo + (size_t)(lo + j) * P.n;
+  double* col = P.U + lo + (size_t)(lo + j) * ld;
   double ss = 0.0;
   for (int i = lane; i < k; i += 32) {
-    const double u = -P.zhat[lo + i] / ((dor - d[i]) + tj);
+    const double u = -P.zhat[lo + i] * rcp_newton((dor - d[i]) + tj);
     col[i] = u;
     ss += u * u;
   }
   ss = warp_sum(ss);
   const double inv = 1.0 / sqrt(ss);
   for (int i = lane; i < k; i += 32) col[i] *= inv;
-}
-
-// Final order: rank of every eigenvalue of the node (one warp per value,
-// lanes share the comparisons); writes D and the rank.
-__global__ void dc_rank_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes) {
-  const int node = blockIdx.y;
-  const int a = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const DcNode N = nodes[node];
-  const DcProb P = probs[N.prob];
-  const int lo = N.lo, np = N.hi - N.lo;
-  if (a >= np) return;
-  const int k = P.kcnt[lo];
-  const double* d = P.ds + lo;
-  auto val = [&](int b) {
-    return b < k ? d[P.orig[lo + b]] + P.tau[lo + b] : P.dD[lo + b];
-  };
-  const double x = val(a);
-  unsigned r = 0;
-  for (int b = lane; b < np; b += 32) {
-    const double y = val(b);
-    r += (y < x) || (y == x && b < a);
-  }
-  r = __reduce_add_sync(0xffffffffu, r);
-  if (lane == 0) {
-    P.rank[lo + a] = (int)r;
-    P.D[lo + r] = x;
-  }
-}
-
-// Deflated columns Q[:, lo+a] (a >= k) -> W1[:, lo+a]; then all columns of
-// W1 -> Q[:, lo + rank[a]].  Two launches of the same kernel (mode 0/1).
-__global__ void dc_copy_kernel(const DcProb* __restrict__ probs, const DcNode* __restrict__ nodes,
-                               int mode) {
-  const int node = blockIdx.y;
-  const int a = blockIdx.x;
-  const DcNode N = nodes[node];
-  const DcProb P = probs[N.prob];
-  const int lo = N.lo, np = N.hi - N.lo;
-  if (a >= np) return;
-  const int k = P.kcnt[lo];
-  const size_t ld = (size_t)P.n;
-  if (mode == 0) {
-    if (a < k) return;
-    const double* s = P.Q + lo + (size_t)(lo + a) * ld;
-    double* t = P.W1 + lo + (size_t)(lo + a) * ld;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) t[i] = s[i];
-  } else {
-    const double* s = P.W1 + lo + (size_t)(lo + a) * ld;
-    double* t = P.Q + lo + (size_t)(lo + P.rank[lo + a]) * ld;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) t[i] = s[i];
-  }
 }
 
 // --------------------------------------------------------------------------
@@ -1233,8 +928,8 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   // merge node a node, a GEMM problem and a segment; 3 aligned arrays per level
   size_t ndc = 0;
   for (int n : ns) ndc += 2 * (size_t)(n / LEAF + 2);
-  pl.add<char>(ns.size() * sizeof(DcProb) + ndc * (sizeof(DcNode) + sizeof(GemmProb) + sizeof(GemmSeg)) +
-               256 * 3 * 40 + 1024);
+  pl.add<char>(ns.size() * sizeof(DcProb) + ndc * (sizeof(DcBaseProb) + sizeof(DcNode) + sizeof(GemmProb) + sizeof(GemmSeg) + sizeof(int*)) +
+               256 * 4 * 40 + 1024);
   // back-transformation GEMM descriptors (4 batches per block of reflectors)
   size_t nbt = 0;
   for (int n : ns) nbt += 4 * (size_t)(bt_nblk(n) + 1);
@@ -1277,17 +972,14 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
 
   // ---------------- small problems ----------------
   if (!small.empty()) {
-    std::vector<SmallProb> sp;
-    for (int i : small) sp.push_back(SmallProb{probs[i].A, probs[i].w, probs[i].Z, probs[i].n});
-    SmallProb* d_sp = arena_.alloc_n<SmallProb>(sp.size());
-    NRGB_CUDA(cudaMemcpyAsync(d_sp, sp.data(), sp.size() * sizeof(SmallProb), cudaMemcpyHostToDevice, st));
+    std::vector<TinyProb> sp;
+    for (int i : small) sp.push_back(TinyProb{probs[i].A, probs[i].w, probs[i].Z, probs[i].n});
+    TinyProb* d_sp = arena_.alloc_n<TinyProb>(sp.size());
+    NRGB_CUDA(cudaMemcpyAsync(d_sp, sp.data(), sp.size() * sizeof(TinyProb), cudaMemcpyHostToDevice, st));
     // on its own stream, beside the larger blocks; joined before the flags are read
     NRGB_CUDA(cudaEventRecord(fork_, st));
     NRGB_CUDA(cudaStreamWaitEvent(small_st_, fork_, 0));
-    NRGB_LAUNCH("syev_small", small_st_,
-                syev_small_kernel<<<ceil_div((int)sp.size(), SMALL_WARPS), 32 * SMALL_WARPS, 0, small_st_>>>(
-                    d_sp, (int)sp.size(), d_err_));
-    NRGB_CUDA(cudaGetLastError());
+    NRGB_CUDA(syev_tiny_launch(d_sp, (int)sp.size(), d_err_ + 2, small_st_));
     NRGB_CUDA(cudaEventRecord(small_done_, small_st_));
     ++launches_;
   }
@@ -1342,14 +1034,15 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       q.U = U;
       q.ds = vec + 5 * n;
       q.zs = vec + 6 * n;
-      q.dD = vec + 7 * n;
+      q.val = vec + 7 * n;
       q.tau = vec + 8 * n;
       q.zhat = vec + 9 * n;
       q.rho = vec + 10 * n;
       q.rotc = vec + 11 * n;
       q.rots = vec + 12 * n;
       q.src = ivec;
-      q.flag = ivec + n;
+      q.cmap = ivec + n;
+      q.sc = vec + 13 * n;
       q.orig = ivec + 2 * n;
       q.kcnt = ivec + 3 * n;
       q.rank = ivec + 4 * n;
@@ -1666,13 +1359,21 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         std::vector<DcNode> nodes;
         GemmBatch gb;
         int maxnp = 0;
-        size_t o_nodes = 0, o_gp = 0, o_gs = 0;
+        std::vector<const int*> cmaps;  // where the product's columns go: the ranks
+        size_t o_nodes = 0, o_gp = 0, o_gs = 0, o_cm = 0;
       };
       std::vector<Level> levels(hmax + 1);
       for (auto& m : merges) levels[m.first].nodes.push_back(m.second);
       DescPack pk;
       const size_t o_dp = pk.add(dp);
-      const size_t o_leaves = pk.add(leaves);
+      // the subtrees, those beyond half of DC_BASE first (their own launch)
+      std::vector<DcBaseProb> base;
+      for (const DcNode& L : leaves)
+        base.push_back(DcBaseProb{dp[L.prob].dT, dp[L.prob].e, dp[L.prob].D, dp[L.prob].Q, dp[L.prob].n, L.lo, L.hi - L.lo});
+      std::stable_sort(base.begin(), base.end(), [](const DcBaseProb& x, const DcBaseProb& y) { return x.s > y.s; });
+      int nwide = 0;
+      while (nwide < (int)base.size() && base[nwide].s > DC_BASE / 2) ++nwide;
+      const size_t o_base = pk.add(base);
       for (int h = 1; h <= hmax; ++h) {
         Level& L = levels[h];
         for (auto& nd : L.nodes) {
@@ -1680,19 +1381,30 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           L.maxnp = std::max(L.maxnp, np);
           GemmSeg sg{};
           L.gb.add(nullptr, 0, np, np, 0.0, {sg});  // shapes fixed on device (n = k <= np)
+          L.cmaps.push_back(dp[nd.prob].rank + nd.lo);
         }
         // segments too, even though dc_prep fills them in: the copy sizes them
         L.o_nodes = pk.add(L.nodes);
         L.o_gp = pk.add(L.gb.probs);
         L.o_gs = pk.add(L.gb.segs);
+        L.o_cm = pk.add(L.cmaps);
       }
       char* dev = pk.upload(arena_, st);
       const DcProb* d_dp = reinterpret_cast<const DcProb*>(dev + o_dp);
-      NRGB_LAUNCH("dc_leaf", st,
-                  dc_leaf_kernel<<<ceil_div((int)leaves.size(), 2), 64, 0, st>>>(
-                      d_dp, reinterpret_cast<const DcNode*>(dev + o_leaves), (int)leaves.size(), d_err_ + 1));
-      NRGB_CUDA(cudaGetLastError());
-      ++launches_;
+      const DcBaseProb* d_base = reinterpret_cast<const DcBaseProb*>(dev + o_base);
+      const int nrest = (int)base.size() - nwide;
+      const bool both = nwide > 0 && nrest > 0;  // two launches: side by side
+      if (both) {
+        NRGB_CUDA(cudaEventRecord(fork_, st));
+        NRGB_CUDA(cudaStreamWaitEvent(aux_[1], fork_, 0));
+      }
+      if (nwide > 0) NRGB_CUDA(dc_base_launch(d_base, nwide, base[0].s, d_err_ + 2, st));
+      if (nrest > 0) NRGB_CUDA(dc_base_launch(d_base + nwide, nrest, base[nwide].s, d_err_ + 2, both ? aux_[1] : st));
+      if (both) {
+        NRGB_CUDA(cudaEventRecord(join_[1], aux_[1]));
+        NRGB_CUDA(cudaStreamWaitEvent(st, join_[1], 0));
+      }
+      launches_ += 1 + (both ? 1 : 0);
       NRGB_CUDA(raise_smem_attr((const void*)dc_prep_kernel, (int)dc_prep_smem(DC_PREP_CAP)));
       for (int h = 1; h <= hmax; ++h) {
         Level& L = levels[h];
@@ -1708,29 +1420,20 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         NRGB_CUDA(cudaGetLastError());
         dim3 g1(ceil_div(maxnp, 128), nn);
         dim3 gp(ceil_div(maxnp, 128), ceil_div(maxnp, DC_PCOLS), nn);
-        NRGB_LAUNCH("dc_permute", st, dc_gather_kernel<<<gp, 128, 0, st>>>(d_dp, d_nodes, 0));
+        NRGB_LAUNCH("dc_permute", st, dc_gather_kernel<<<gp, 128, 0, st>>>(d_dp, d_nodes));
         NRGB_CUDA(cudaGetLastError());
         NRGB_LAUNCH("dc_permute", st, dc_rotate_kernel<<<g1, 128, 0, st>>>(d_dp, d_nodes));
-        NRGB_CUDA(cudaGetLastError());
-        NRGB_LAUNCH("dc_permute", st, dc_gather_kernel<<<gp, 128, 0, st>>>(d_dp, d_nodes, 1));
         NRGB_CUDA(cudaGetLastError());
         dim3 gw(ceil_div(maxnp, 8), nn);
         NRGB_LAUNCH("dc_secular", st, dc_secular_warp_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes, d_err_ + 2));
         NRGB_CUDA(cudaGetLastError());
         NRGB_LAUNCH("dc_lowner", st, dc_lowner_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes));
         NRGB_CUDA(cudaGetLastError());
-        dim3 g2(ceil_div(maxnp, 8), nn);
-        NRGB_LAUNCH("dc_vectors", st, dc_vectors_kernel<<<g2, 256, 0, st>>>(d_dp, d_nodes));
+        NRGB_LAUNCH("dc_vectors", st, dc_vectors_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes));
         NRGB_CUDA(cudaGetLastError());
-        NRGB_CUDA(gemm_grouped_launch(d_gp, nn, d_gs, L.gb.tiles, st, "gemm_f64_dc", L.gb.stiles));
-        NRGB_LAUNCH("dc_rank", st, dc_rank_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes));
-        NRGB_CUDA(cudaGetLastError());
-        dim3 g3(maxnp, nn);
-        NRGB_LAUNCH("dc_copy", st, dc_copy_kernel<<<g3, 128, 0, st>>>(d_dp, d_nodes, 0));
-        NRGB_CUDA(cudaGetLastError());
-        NRGB_LAUNCH("dc_copy", st, dc_copy_kernel<<<g3, 128, 0, st>>>(d_dp, d_nodes, 1));
-        NRGB_CUDA(cudaGetLastError());
-        launches_ += 11;
+        NRGB_CUDA(gemm_grouped_launch(d_gp, nn, d_gs, L.gb.tiles, st, "gemm_f64_dc", L.gb.stiles,
+                                      reinterpret_cast<const int* const*>(dev + L.o_cm)));
+        launches_ += 7;
       }
       // problems that are a single leaf already have D, Q in place
     }
@@ -1884,7 +1587,6 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
   NRGB_CUDA(cudaMemcpyAsync(&hb, d_bar_, sizeof(hb), cudaMemcpyDeviceToHost, st));
   NRGB_CUDA(cudaStreamSynchronize(st));
   hb.error |= herr[3];
-  if (herr[0] || herr[1]) throw CudaError("syev: QR iteration did not converge");
   if (herr[2]) throw CudaError("syev: secular equation iteration did not converge");
   if (hb.error) throw CudaError("syev: grid barrier timed out");
 }
