@@ -774,8 +774,7 @@ def run_split_micro(edge, slices, nprob):
 
 
 def run_gemm_micro():
-    """Grouped FP64 GEMM (the kernel NRGB_GEMM_PIPE selects in this process)
-    on square problems in all four transpose combinations, and cuBLAS DGEMM
+    """Grouped FP64 GEMM on square problems in all four transpose combinations, and cuBLAS DGEMM
     (torch.bmm) on the same untransposed problems; device-resident inputs,
     CUDA events on the launch stream, best of 5.  Prints one JSON object of
     TF/s per case."""
@@ -801,9 +800,7 @@ def run_gemm_micro():
             best = min(best, t0.elapsed_time(t1))
         return best
 
-    forms = {"0": "register-staged", "3": "pipelined, K step 16, 3 stages", "4": "pipelined, K step 16, 4 stages",
-             "232": "pipelined, K step 32, 2 stages", "332": "pipelined, K step 32, 3 stages"}
-    out = {"kernel": forms.get(os.environ.get("NRGB_GEMM_PIPE") or "3", "pipelined, K step 16, 3 stages")}
+    out = {"kernel": "pipelined, K step 16, 3 stages"}
     for edge, nprob, nseg in ((2048, 4, 1), (1024, 16, 1), (512, 64, 1), (384, 64, 3), (256, 128, 2)):
         for ta, tb in ((0, 0), (1, 0), (0, 1), (1, 1)):
             A = [torch.randn(edge, edge, generator=g, device=dev, dtype=torch.float64) for _ in range(nprob * nseg)]

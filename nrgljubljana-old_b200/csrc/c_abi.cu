@@ -160,15 +160,11 @@ int nrgb_gemm_grouped_dev(nrgb_ctx* ctx, int nout, const nrgb_gemm_out* outs, in
     }
     if (P.empty()) return;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t bytes = P.size() * sizeof(nrgb::GemmProb) + S.size() * sizeof(nrgb::GemmSeg) + 1024;
-    ctx->scratch.reserve(bytes);
+    ctx->scratch.reserve(nrgb::gemm_desc_bytes((int)P.size(), (int)S.size()));
     ctx->scratch.reset();
-    auto* dP = ctx->scratch.alloc_n<nrgb::GemmProb>(P.size());
-    auto* dS = ctx->scratch.alloc_n<nrgb::GemmSeg>(S.size());
-    NRGB_CUDA(cudaMemcpyAsync(dP, P.data(), P.size() * sizeof(nrgb::GemmProb), cudaMemcpyHostToDevice, st));
-    NRGB_CUDA(cudaMemcpyAsync(dS, S.data(), S.size() * sizeof(nrgb::GemmSeg), cudaMemcpyHostToDevice, st));
     nrgb::KernelStats::get().add_work("gemm_f64", nrgb::gemm_flops(P.data(), (int)P.size(), S.data()));
-    NRGB_CUDA(nrgb::gemm_grouped_launch(dP, (int)P.size(), dS, tiles, st, "gemm_f64", stiles));
+    NRGB_CUDA(nrgb::gemm_grouped_launch_host(P.data(), (int)P.size(), S.data(), (int)S.size(), tiles, st, "gemm_f64",
+                                             stiles, ctx->scratch));
     NRGB_CUDA(cudaStreamSynchronize(st));
   });
 }
@@ -202,18 +198,12 @@ void recalc_pairs(nrgb_ctx* ctx, int nops, const int* n, const int* bra, const i
     add(p2, s2, t2, u2, out[o], nb, nk, nrgb::GemmSeg{Z[bra[o]], T, nb, nb, nb, 1, 0, 1.0});
   }
   if (p1.empty()) return;
-  auto* d1 = scr.alloc_n<nrgb::GemmProb>(p1.size());
-  auto* e1 = scr.alloc_n<nrgb::GemmSeg>(s1.size());
-  auto* d2 = scr.alloc_n<nrgb::GemmProb>(p2.size());
-  auto* e2 = scr.alloc_n<nrgb::GemmSeg>(s2.size());
-  NRGB_CUDA(cudaMemcpyAsync(d1, p1.data(), p1.size() * sizeof(p1[0]), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(e1, s1.data(), s1.size() * sizeof(s1[0]), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(d2, p2.data(), p2.size() * sizeof(p2[0]), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(e2, s2.data(), s2.size() * sizeof(s2[0]), cudaMemcpyHostToDevice, st));
   nrgb::KernelStats::get().add_work("gemm_f64_recalc", nrgb::gemm_flops(p1.data(), (int)p1.size(), s1.data()) +
                                                            nrgb::gemm_flops(p2.data(), (int)p2.size(), s2.data()));
-  NRGB_CUDA(nrgb::gemm_grouped_launch(d1, (int)p1.size(), e1, t1, st, "gemm_f64_recalc", u1));
-  NRGB_CUDA(nrgb::gemm_grouped_launch(d2, (int)p2.size(), e2, t2, st, "gemm_f64_recalc", u2));
+  NRGB_CUDA(nrgb::gemm_grouped_launch_host(p1.data(), (int)p1.size(), s1.data(), (int)s1.size(), t1, st,
+                                           "gemm_f64_recalc", u1, scr));
+  NRGB_CUDA(nrgb::gemm_grouped_launch_host(p2.data(), (int)p2.size(), s2.data(), (int)s2.size(), t2, st,
+                                           "gemm_f64_recalc", u2, scr));
 }
 
 size_t recalc_scratch(int nops, const int* n, const int* bra, const int* ket) {

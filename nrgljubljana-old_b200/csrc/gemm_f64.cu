@@ -1,16 +1,16 @@
 // Grouped, segmented-K FP64 GEMM on the DMMA tensor-core path (sm_100a).
 // See gemm_f64.cuh for the contract.
 //
-// Tile: 64x64 per CTA, 4 warps of 32x32, K staged 16 at a time through
-// shared memory laid out so that the DMMA fragment loads are bank-conflict
-// free: by default a cp.async ring of three K steps of 16
-// (gemm_grouped_pipe_kernel<3, 16>), else
-// register-staged double buffering (gemm_grouped_kernel; also the kernel of
-// the allocation-free entry point) or 128x128 tiles where the schedule picks
-// them.  mma.sync.m8n8k4.f64 (the m16n8k4/k8/k16 f64 shapes run at the same
-// rate on B200): A fragment A[g][t], B fragment B[t][g], accumulator
+// 64x64 tiles per CTA on 4 warps of 32x32 (32x32 tiles for launches with few
+// of them), K staged 16 at a time through a cp.async ring laid out so that
+// the DMMA fragment loads are bank-conflict free; 128x128 tiles where the
+// schedule picks them.  mma.sync.m8n8k4.f64 (the m16n8k4/k8/k16 f64 shapes run
+// at the same rate on B200): A fragment A[g][t], B fragment B[t][g], accumulator
 // C[g][2t..2t+1] with g = lane/4, t = lane%4.
+#include <string.h>
+
 #include <atomic>
+
 #include "common.cuh"
 #include "gemm_f64.cuh"
 #include "schedule.cuh"
@@ -20,8 +20,6 @@ namespace nrgb {
 namespace {
 
 constexpr int BM = GEMM_BM, BN = GEMM_BN, BK = GEMM_BK;
-constexpr int PAD = 4;          // row stride 68 doubles: t*68+g hits 16 distinct bank pairs
-constexpr int LDS = BM + PAD;   // BM == BN
 constexpr int NT = 128;
 
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
@@ -29,196 +27,6 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
 }
-
-struct TileLoader {
-  // 8 A values and 8 B values per thread per K-tile.
-  double ra[8], rb[8];
-
-  __device__ __forceinline__ void load(const GemmSeg& s, int k0, int row0, int col0, int m, int n,
-                                       int tid) {
-    const double alpha = s.alpha;
-    if (!s.transA) {  // A[i + p*lda], contiguous in i
-      const int i = tid & 63, pb = tid >> 6;
-      const int gi = row0 + i;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int p = pb + 2 * r, gp = k0 + p;
-        ra[r] = (gi < m && gp < s.k) ? alpha * __ldg(s.A + (size_t)gp * s.lda + gi) : 0.0;
-      }
-    } else {  // op(A)[i,p] = A[p + i*lda], contiguous in p
-      const int p = tid & 15, ib = tid >> 4;
-      const int gp = k0 + p;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int gi = row0 + ib + 8 * r;
-        ra[r] = (gi < m && gp < s.k) ? alpha * __ldg(s.A + (size_t)gi * s.lda + gp) : 0.0;
-      }
-    }
-    if (!s.transB) {  // op(B)[p,j] = B[p + j*ldb], contiguous in p
-      const int p = tid & 15, jb = tid >> 4;
-      const int gp = k0 + p;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int gj = col0 + jb + 8 * r;
-        rb[r] = (gj < n && gp < s.k) ? __ldg(s.B + (size_t)gj * s.ldb + gp) : 0.0;
-      }
-    } else {  // op(B)[p,j] = B[j + p*ldb], contiguous in j
-      const int j = tid & 63, pb = tid >> 6;
-      const int gj = col0 + j;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int p = pb + 2 * r, gp = k0 + p;
-        rb[r] = (gj < n && gp < s.k) ? __ldg(s.B + (size_t)gp * s.ldb + gj) : 0.0;
-      }
-    }
-  }
-
-  __device__ __forceinline__ void store(const GemmSeg& s, double (*As)[LDS], double (*Bs)[LDS],
-                                        int tid) {
-    if (!s.transA) {
-      const int i = tid & 63, pb = tid >> 6;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) As[pb + 2 * r][i] = ra[r];
-    } else {
-      const int p = tid & 15, ib = tid >> 4;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) As[p][ib + 8 * r] = ra[r];
-    }
-    if (!s.transB) {
-      const int p = tid & 15, jb = tid >> 4;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) Bs[p][jb + 8 * r] = rb[r];
-    } else {
-      const int j = tid & 63, pb = tid >> 6;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) Bs[pb + 2 * r][j] = rb[r];
-    }
-  }
-};
-
-__global__ void __launch_bounds__(NT) gemm_grouped_kernel(const GemmProb* __restrict__ probs,
-                                                          int nprob,
-                                                          const GemmSeg* __restrict__ segs,
-                                                          const int* const* __restrict__ cmaps) {
-  __shared__ __align__(16) double As[2][BK][LDS];
-  __shared__ __align__(16) double Bs[2][BK][LDS];
-
-  // Locate the problem owning this tile (probs sorted by tile0).
-  const int tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-  }
-  const GemmProb P = probs[lo];
-  const int ks = P.ksplit > 1 ? P.ksplit : 1;
-  const int t = (tile - P.tile0) / ks;
-  const int kc = (tile - P.tile0) % ks;
-  const int row0 = (t / P.tiles_n) * BM;
-  const int col0 = (t % P.tiles_n) * BN;
-  const int m = P.m, n = P.n;
-  if (row0 >= m || col0 >= n) return;  // shapes may be set on the device below the planned bound
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, tq = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-
-  double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  // Flattened (segment, k-tile) iteration over this CTA's share of the K tiles.
-  const int send = P.seg0 + P.nseg;
-  int ktot = 0;
-  for (int q = P.seg0; q < send; ++q) ktot += segs[q].k > 0 ? (segs[q].k + BK - 1) / BK : 0;
-  const int per = (ktot + ks - 1) / ks;
-  const int kt0 = kc * per;
-  int remaining = min(ktot, kt0 + per) - kt0;
-  int s = P.seg0, k0 = 0;
-  {
-    int kt = 0;
-    while (s < send) {
-      const int nt = segs[s].k > 0 ? (segs[s].k + BK - 1) / BK : 0;
-      if (kt + nt > kt0) break;
-      kt += nt;
-      ++s;
-    }
-    k0 = (kt0 - kt) * BK;
-  }
-  if (remaining > 0 && s < send) {
-    TileLoader L;
-    GemmSeg cur = segs[s];
-    L.load(cur, k0, row0, col0, m, n, tid);
-    L.store(cur, As[0], Bs[0], tid);
-    __syncthreads();
-    int buf = 0;
-    while (true) {
-      --remaining;
-      // advance to next (segment, k0)
-      GemmSeg nxt = cur;
-      int nk0 = k0 + BK;
-      int ns = s;
-      bool more = remaining > 0;
-      if (more && nk0 >= cur.k) {
-        ns = s + 1;
-        while (ns < send && segs[ns].k <= 0) ++ns;
-        if (ns < send) {
-          nxt = segs[ns];
-          nk0 = 0;
-        } else {
-          more = false;
-        }
-      }
-      if (more) L.load(nxt, nk0, row0, col0, m, n, tid);
-
-#pragma unroll
-      for (int kk = 0; kk < BK; kk += 4) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[buf][kk + tq][wm + i * 8 + g];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk + tq][wn + j * 8 + g];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-      }
-      if (!more) break;
-      L.store(nxt, As[buf ^ 1], Bs[buf ^ 1], tid);
-      __syncthreads();
-      buf ^= 1;
-      cur = nxt;
-      s = ns;
-      k0 = nk0;
-    }
-  }
-
-  // Epilogue: C = acc + beta*C.
-  const double beta = P.beta;
-  const int* cmap = cmaps ? cmaps[lo] : nullptr;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = row0 + wm + i * 8 + g;
-    if (r >= m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = col0 + wn + j * 8 + 2 * tq + h;
-        if (c < n) {
-          double* dst = P.C + (size_t)(cmap ? cmap[c] : c) * P.ldc + r;
-          const double v = acc[i][j][h];
-          if (ks > 1) atomicAdd(dst, v);
-          else *dst = (beta == 0.0) ? v : v + beta * (*dst);
-        }
-      }
-    }
-  }
-}
-
 
 // ---------------------------------------------------------------------------
 // Large-tile variant: 128x128 per CTA, 8 warps of 64x32, K staged 16 at a
@@ -390,217 +198,264 @@ __global__ void __launch_bounds__(LNT) gemm_grouped_large_kernel(const GemmProb*
 constexpr size_t LSMEM = 2 * (size_t)LSTAGES * BK * LLDS * sizeof(double);
 
 // ---------------------------------------------------------------------------
-// Pipelined variant: the same 64x64 tile and 4 warps of 32x32, with the
-// operands copied by cp.async into an S-stage ring of K steps of KB (no
-// register staging, S-1 K tiles in flight).  Each operand tile keeps the direction in
-// which it is contiguous in global memory:
-//   mn-contiguous (A as stored, B transposed): [KB][64 + 4]
-//   k-contiguous  (A transposed, B as stored): [64][KB], the 16-byte pairs of
+// Pipelined kernel: T x T tiles (64 or 32) on 4 warps of T/2 x T/2, operands
+// copied by cp.async into a ring of three K steps of 16.  Each operand tile
+// keeps the direction in which it is contiguous in global memory:
+//   mn-contiguous (A as stored, B transposed): [16][T + 4]
+//   k-contiguous  (A transposed, B as stored): [T][16], the 16-byte pairs of
 //     row r at pair index (p/2) ^ (2r mod 8)
 // and both are read bank-conflict free by the fragment loads (within a
 // half-warp, lanes g, t hit double offsets 4t + g, resp. 2((k/2 + t/2) ^ 2g)
-// + t%2, mod 16, all distinct).  A segment whose base address
-// and leading dimension are 16-byte aligned is copied in element pairs
-// (16-byte cp.async; the half of a pair outside the matrix is zero-filled),
-// any other segment element by element.
+// + t%2, mod 16, all distinct).  A segment whose base address and leading
+// dimension are 16-byte aligned is copied in element pairs (16-byte cp.async;
+// the half of a pair outside the matrix is zero-filled), any other segment
+// (sub-blocks of eigenvector matrices mostly) element by element.
+//
+// What bounds it is the FP64 tensor pipe (16 cycles an m8n8k4) and the issue
+// slots around it, so everything that does not change from K step to K step
+// (source pointers, strides, row bounds, the swizzled offsets) stays in
+// registers: nine instructions went with every tensor instruction when each
+// step derived them from the segment again.  A CTA finds its problem with one
+// or two loads by all lanes (a binary search was a chain of up to ten), and
+// small launches get their descriptors as kernel parameters instead of copies.
 // ---------------------------------------------------------------------------
-constexpr int PLD_MN = BM + 4;        // 68
+constexpr int KB = BK, STAGES = 3;
 
-// doubles per operand tile of K step KB: KB * 68 >= 64 * KB
-template <int KB>
-__host__ __device__ constexpr int ptile() { return KB * PLD_MN; }
-
-// offset of element (row r, K index p) in a k-contiguous tile of K step KB
-template <int KB>
-__device__ __forceinline__ int pipe_kofs(int r, int p) {
-  return r * KB + (((p >> 1) ^ ((2 * r) & 7)) << 1) + (p & 1);
-}
+template <int T>
+__host__ __device__ constexpr int ptile() { return KB * (T + 4); }
 
 __device__ __forceinline__ void cp_async16(double* smem, const double* gmem, int bytes) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 
-// Copy one 64 x KB operand tile: rows mn0 .. mn0+63 (< mnlim) and K columns
-// k0 .. k0+KB-1 (< klim) of a matrix whose element (mn, k) sits at
-// base[mn + k*ld] (mn-contiguous) or base[k + mn*ld] (k-contiguous).
-template <int KB>
-__device__ __forceinline__ void pipe_load_tile(double* dst, const double* base, int ld, bool kcontig,
-                                               bool vec, int mn0, int mnlim, int k0, int klim, int tid) {
-  if (!kcontig) {
-    if (vec) {
+// One operand's copies of a thread: a T x 16 tile of a matrix whose element
+// (mn, k) sits at base[mn + k ld] (mn-contiguous) or base[k + mn ld].
+template <int T>
+struct Operand {
+  const double* p;  // the thread's first element of the next K step
+  int ld, lim;      // leading dimension; rows of the tile inside the matrix
+  int mode;         // bit 0: pairs, bit 1: k-contiguous
+
+  __device__ __forceinline__ void set(const double* base, int ld_, bool kcont, int mn0, int mnlim, int k0, int tid) {
+    ld = ld_;
+    lim = mnlim - mn0;
+    const bool vec = ((reinterpret_cast<uintptr_t>(base) & 15) == 0) && ((ld & 1) == 0);
+    mode = (vec ? 1 : 0) | (kcont ? 2 : 0);
+    int i, k;
+    if (mode == 0) {
+      i = tid & (T - 1);
+      k = tid / T;
+    } else if (mode == 1) {
+      i = 2 * (tid & (T / 2 - 1));
+      k = tid / (T / 2);
+    } else if (mode == 2) {
+      i = tid >> 4;
+      k = tid & 15;
+    } else {
+      i = tid >> 3;
+      k = 2 * (tid & 7);
+    }
+    p = base + (kcont ? (size_t)(mn0 + i) * ld + (k0 + k) : (size_t)(k0 + k) * ld + (mn0 + i));
+  }
+  // Copies the tile (krem columns are inside the matrix) and steps on.
+  __device__ __forceinline__ void issue(double* dst, int krem, int tid) {
+    if (mode == 0) {
+      const int i = tid & (T - 1), k = tid / T;
+      const size_t step = (size_t)(NT / T) * ld;
+      const bool in = i < lim;
+      const double* q = p;
 #pragma unroll
-      for (int r = 0; r < KB / 4; ++r) {
-        const int c = tid + NT * r, p = c >> 5, i = 2 * (c & 31);
-        const int gi = mn0 + i, gp = k0 + p;
-        const int bytes = gp < klim ? (gi + 1 < mnlim ? 16 : (gi < mnlim ? 8 : 0)) : 0;
-        cp_async16(dst + p * PLD_MN + i, bytes ? base + (size_t)gp * ld + gi : base, bytes);
+      for (int r = 0; r < KB * T / NT; ++r) {
+        cp_async8(dst + (k + NT / T * r) * (T + 4) + i, q, in && k + NT / T * r < krem);
+        q += step;
+      }
+    } else if (mode == 1) {
+      const int i = 2 * (tid & (T / 2 - 1)), k = tid / (T / 2);
+      const size_t step = (size_t)(2 * NT / T) * ld;
+      const int bytes = min(max(lim - i, 0), 2) * 8;
+      const double* q = p;
+#pragma unroll
+      for (int r = 0; r < KB * T / (2 * NT); ++r) {
+        cp_async16(dst + (k + 2 * NT / T * r) * (T + 4) + i, q, k + 2 * NT / T * r < krem ? bytes : 0);
+        q += step;
+      }
+    } else if (mode == 2) {
+      const int i = tid >> 4, k = tid & 15;
+      const size_t step = (size_t)8 * ld;
+      double* d = dst + i * KB + (((k >> 1) ^ ((2 * i) & 7)) << 1) + (k & 1);
+      const int rows = k < krem ? lim - i : 0;
+      const double* q = p;
+#pragma unroll
+      for (int r = 0; r < T / 8; ++r) {
+        cp_async8(d + 8 * KB * r, q, 8 * r < rows);
+        q += step;
       }
     } else {
+      const int i = tid >> 3, k = 2 * (tid & 7);
+      const size_t step = (size_t)16 * ld;
+      double* d = dst + i * KB + (((k >> 1) ^ ((2 * i) & 7)) << 1);
+      const int bytes = min(max(krem - k, 0), 2) * 8, rows = lim - i;
+      const double* q = p;
 #pragma unroll
-      for (int r = 0; r < KB / 2; ++r) {
-        const int e = tid + NT * r, p = e >> 6, i = e & 63;
-        const int gi = mn0 + i, gp = k0 + p;
-        const bool ok = gi < mnlim && gp < klim;
-        cp_async8(dst + p * PLD_MN + i, ok ? base + (size_t)gp * ld + gi : base, ok);
+      for (int r = 0; r < T / 16; ++r) {
+        cp_async16(d + 16 * KB * r, q, 16 * r < rows ? bytes : 0);
+        q += step;
       }
     }
-  } else {
-    if (vec) {
+    p += (mode & 2) ? (size_t)KB : (size_t)KB * ld;
+  }
+};
+
+// The products of one K step; FL: bit 0 A k-contiguous, bit 1 B k-contiguous.
+template <int T, int FL>
+__device__ __forceinline__ void tile_step(double (&acc)[T / 16][T / 16][2], const double* as, const double* bs,
+                                          double alpha, int wm, int wn, int g, int tq, const int (&ko)[4]) {
+  constexpr int W = T / 16;
+  const double* ap = (FL & 1) ? as + (wm + g) * KB : as + tq * (T + 4) + wm + g;
+  const double* bp = (FL & 2) ? bs + (wn + g) * KB : bs + tq * (T + 4) + wn + g;
 #pragma unroll
-      for (int r = 0; r < KB / 4; ++r) {
-        const int c = tid + NT * r, i = c / (KB / 2), p = 2 * (c % (KB / 2));
-        const int gi = mn0 + i, gp = k0 + p;
-        const int bytes = gi < mnlim ? (gp + 1 < klim ? 16 : (gp < klim ? 8 : 0)) : 0;
-        cp_async16(dst + pipe_kofs<KB>(i, p), bytes ? base + (size_t)gi * ld + gp : base, bytes);
-      }
-    } else {
+  for (int kk = 0; kk < KB; kk += 4) {
+    double a[W], b[W];
 #pragma unroll
-      for (int r = 0; r < KB / 2; ++r) {
-        const int e = tid + NT * r, i = e / KB, p = e % KB;
-        const int gi = mn0 + i, gp = k0 + p;
-        const bool ok = gi < mnlim && gp < klim;
-        cp_async8(dst + pipe_kofs<KB>(i, p), ok ? base + (size_t)gi * ld + gp : base, ok);
-      }
+    for (int i = 0; i < W; ++i) a[i] = (FL & 1) ? ap[ko[kk / 4] + i * 8 * KB] : ap[kk * (T + 4) + i * 8];
+#pragma unroll
+    for (int j = 0; j < W; ++j) b[j] = (FL & 2) ? bp[ko[kk / 4] + j * 8 * KB] : bp[kk * (T + 4) + j * 8];
+    if (alpha != 1.0) {
+#pragma unroll
+      for (int i = 0; i < W; ++i) a[i] *= alpha;
     }
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+#pragma unroll
+      for (int j = 0; j < W; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
   }
 }
 
-__device__ __forceinline__ bool pipe_vec_ok(const double* p, int ld) {
-  return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((ld & 1) == 0);
+// Last problem whose tile0 is at most `tile` (all lanes of a warp call it).
+__device__ __forceinline__ int find_problem(const GemmProb* probs, int nprob, int tile, int lane) {
+  int lo = 0, len = nprob;
+  while (len > 1) {
+    const int step = (len + 31) / 32, i = lo + lane * step;
+    const bool le = lane * step < len && (lane == 0 || probs[i].tile0 <= tile);
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, le));
+    lo += last * step;
+    len = min(step, len - last * step);
+  }
+  return lo;
 }
 
-// 128 registers at most, so that shared memory alone sets the CTAs per SM:
-// four with KB = 16 and 3 stages (52 KB each), three with KB = 32 and 2
-// stages (70 KB each)
-template <int S, int KB>
-__global__ void __launch_bounds__(NT, 4) gemm_grouped_pipe_kernel(const GemmProb* __restrict__ probs,
-                                                               int nprob,
-                                                               const GemmSeg* __restrict__ segs,
-                                                               const int* const* __restrict__ cmaps) {
+template <int T>
+__device__ __forceinline__ void gemm_tile(const GemmProb* __restrict__ probs, int nprob, const GemmSeg* __restrict__ segs,
+                                          const int* const* __restrict__ cmaps) {
+  constexpr int W = T / 16, PT = ptile<T>(), SUB = 64 / T;  // SUB^2 CTAs share a 64 x 64 tile
   extern __shared__ __align__(16) double psm[];
-  constexpr int PTILE = ptile<KB>();
-  double* As = psm;                  // [S][PTILE]
-  double* Bs = psm + S * PTILE;      // [S][PTILE]
-  __shared__ double salpha[S];
-  __shared__ int sflags[S];          // bit 0: A k-contiguous, bit 1: B k-contiguous
+  double* As = psm;                 // [STAGES][PT]
+  double* Bs = psm + STAGES * PT;   // [STAGES][PT]
+  __shared__ double salpha[STAGES];
+  __shared__ int sflags[STAGES];    // bit 0: A k-contiguous, bit 1: B k-contiguous
 
-  const int tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (probs[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tile = blockIdx.x / (SUB * SUB), sub = blockIdx.x % (SUB * SUB);
+  const int lo = find_problem(probs, nprob, tile, lane);
   const GemmProb P = probs[lo];
   const int ks = P.ksplit > 1 ? P.ksplit : 1;
   const int t = (tile - P.tile0) / ks;
   const int kc = (tile - P.tile0) % ks;
-  const int row0 = (t / P.tiles_n) * BM;
-  const int col0 = (t % P.tiles_n) * BN;
+  const int row0 = (t / P.tiles_n) * BM + (sub / SUB) * T;
+  const int col0 = (t % P.tiles_n) * BN + (sub % SUB) * T;
   const int m = P.m, n = P.n;
-  if (row0 >= m || col0 >= n) return;  // shapes may be set on the device below the planned bound
+  if (row0 >= m || col0 >= n) return;  // also shapes set on the device below the planned bound
 
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, tq = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-
-  double acc[4][4][2];
+  const int wm = (warp & 1) * (T / 2), wn = (warp >> 1) * (T / 2);
+  int ko[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int q = 0; q < 4; ++q) ko[q] = (((2 * q + (tq >> 1)) ^ ((2 * g) & 7)) << 1) + (tq & 1);
 
-  // this CTA's share of the flattened (segment, K tile) sequence
+  double acc[W][W][2];
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+#pragma unroll
+    for (int j = 0; j < W; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+  // this CTA's share of the flattened (segment, K step) sequence
   const int send = P.seg0 + P.nseg;
   int ktot = 0;
-  for (int q = P.seg0; q < send; ++q) ktot += segs[q].k > 0 ? (segs[q].k + KB - 1) / KB : 0;
+  for (int q = P.seg0 + lane; q < send; q += 32) ktot += segs[q].k > 0 ? (segs[q].k + KB - 1) / KB : 0;
+  ktot = __reduce_add_sync(0xffffffffu, ktot);
   const int per = (ktot + ks - 1) / ks;
   const int kt0 = kc * per;
   const int nk = max(0, min(ktot, kt0 + per) - kt0);
-  int ls = P.seg0, lk0 = 0;
-  {
+  int ls = P.seg0, kleft = 0;  // current segment, its K columns not yet copied
+  Operand<T> oa, ob;
+  double alpha_l = 1.0;
+  auto open = [&](int k0) {
+    const GemmSeg G = segs[ls];
+    // op(A)[i, p]: A[i + p lda] as stored, A[p + i lda] transposed
+    oa.set(G.A, G.lda, G.transA != 0, row0, m, k0, tid);
+    // op(B)[p, j]: B[p + j ldb] as stored (k-contiguous), B[j + p ldb] transposed
+    ob.set(G.B, G.ldb, G.transB == 0, col0, n, k0, tid);
+    alpha_l = G.alpha;
+    kleft = G.k - k0;
+  };
+  if (nk > 0) {
     int kt = 0;
-    while (ls < send) {
-      const int nt = segs[ls].k > 0 ? (segs[ls].k + KB - 1) / KB : 0;
+    while (true) {
+      const int k = segs[ls].k, nt = k > 0 ? (k + KB - 1) / KB : 0;
       if (kt + nt > kt0) break;
       kt += nt;
       ++ls;
     }
-    lk0 = (kt0 - kt) * KB;
+    open((kt0 - kt) * KB);
   }
   auto issue = [&](int stage) {
-    const GemmSeg G = segs[ls];
-    // op(A)[i, p]: A[i + p*lda] as stored, A[p + i*lda] transposed
-    pipe_load_tile<KB>(As + stage * PTILE, G.A, G.lda, G.transA != 0, pipe_vec_ok(G.A, G.lda), row0, m, lk0, G.k,
-                   tid);
-    // op(B)[p, j]: B[p + j*ldb] as stored (k-contiguous), B[j + p*ldb] transposed
-    pipe_load_tile<KB>(Bs + stage * PTILE, G.B, G.ldb, G.transB == 0, pipe_vec_ok(G.B, G.ldb), col0, n, lk0, G.k,
-                   tid);
-    if (tid == 0) {
-      salpha[stage] = G.alpha;
-      sflags[stage] = (G.transA != 0 ? 1 : 0) | (G.transB == 0 ? 2 : 0);
+    if (kleft <= 0) {
+      do ++ls;
+      while (segs[ls].k <= 0);
+      open(0);
     }
-    lk0 += KB;
-    if (lk0 >= G.k) {
-      ++ls;
-      while (ls < send && segs[ls].k <= 0) ++ls;
-      lk0 = 0;
+    oa.issue(As + stage * PT, kleft, tid);
+    ob.issue(Bs + stage * PT, kleft, tid);
+    kleft -= KB;
+    if (tid == 0) {
+      salpha[stage] = alpha_l;
+      sflags[stage] = (oa.mode >> 1) | (ob.mode & 2);
     }
   };
 #pragma unroll
-  for (int st = 0; st < S - 1; ++st) {
+  for (int st = 0; st < STAGES - 1; ++st) {
     if (st < nk) issue(st);
     cp_async_commit();
   }
+  int stg = 0, nxt = STAGES - 1;
   for (int kt = 0; kt < nk; ++kt) {
-    cp_async_wait<S - 2>();
+    cp_async_wait<STAGES - 2>();
     __syncthreads();
-    const int nxt = kt + S - 1;
-    if (nxt < nk) issue(nxt % S);
+    if (kt + STAGES - 1 < nk) issue(nxt);
     cp_async_commit();
-    const int stg = kt % S;
-    const double* as = As + stg * PTILE;
-    const double* bs = Bs + stg * PTILE;
+    const double* as = As + stg * PT;
+    const double* bs = Bs + stg * PT;
     const double alpha = salpha[stg];
-    const int fl = sflags[stg];
-#pragma unroll
-    for (int kk = 0; kk < KB; kk += 4) {
-      double a[4], b[4];
-      if (fl & 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = as[pipe_kofs<KB>(wm + i * 8 + g, kk + tq)];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = as[(kk + tq) * PLD_MN + wm + i * 8 + g];
-      }
-      if (fl & 2) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = bs[pipe_kofs<KB>(wn + j * 8 + g, kk + tq)];
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = bs[(kk + tq) * PLD_MN + wn + j * 8 + g];
-      }
-      if (alpha != 1.0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] *= alpha;
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    switch (sflags[stg]) {
+      case 0: tile_step<T, 0>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      case 1: tile_step<T, 1>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      case 2: tile_step<T, 2>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      default: tile_step<T, 3>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
     }
+    stg = stg + 1 == STAGES ? 0 : stg + 1;
+    nxt = nxt + 1 == STAGES ? 0 : nxt + 1;
   }
   cp_async_wait<0>();
 
   const double beta = P.beta;
   const int* cmap = cmaps ? cmaps[lo] : nullptr;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < W; ++i) {
     const int r = row0 + wm + i * 8 + g;
     if (r >= m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < W; ++j) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int c = col0 + wn + j * 8 + 2 * tq + h;
@@ -615,50 +470,86 @@ __global__ void __launch_bounds__(NT, 4) gemm_grouped_pipe_kernel(const GemmProb
   }
 }
 
-template <int S, int KB>
-constexpr size_t pipe_smem() { return 2 * (size_t)S * ptile<KB>() * sizeof(double); }
-
-// Form of the grouped GEMM: the pipelined kernel with K step 16 and 3 stages
-// by default (3).  Measured on B200: 28.0-29.2 TF/s on grouped 2048^3
-// problems and 20.5-20.9 TF/s on 256^3 ones, over the four transpose
-// combinations, against 24.8-28.2 and 14.5-19.0 TF/s for the register-staged
-// kernel; over the eigensolver's own launches of a 12-block step (trailing
-// updates, merges, back-transforms, basis changes) 4 % less GEMM time than
-// either the register-staged kernel or K step 32 with 2 stages.  That last
-// form (232) is 3 % faster on large square problems but up to 50 % slower on
-// launches with short K.  NRGB_GEMM_PIPE selects another form: 4 (K step 16,
-// 4 stages), 232, 332 (K step 32, 2 or 3 stages) or 0 (register-staged);
-// read once per process.
-int gemm_pipe_stages() {
-  static const int s = [] {
-    const char* e = getenv("NRGB_GEMM_PIPE");
-    if (!e || !*e) return 3;
-    const int v = atoi(e);
-    return (v == 0 || v == 3 || v == 4 || v == 232 || v == 332) ? v : 3;
-  }();
-  return s;
+// 128 registers at most, so that shared memory alone sets the CTAs per SM
+// (52 KB each with T = 64: four).
+template <int T>
+__global__ void __launch_bounds__(NT, T == 64 ? 4 : 6) gemm_grouped_pipe_kernel(const GemmProb* __restrict__ probs, int nprob,
+                                                                  const GemmSeg* __restrict__ segs,
+                                                                  const int* const* __restrict__ cmaps) {
+  gemm_tile<T>(probs, nprob, segs, cmaps);
 }
 
-template <int S, int KB>
-cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
-                        cudaStream_t stream, const char* tag, const int* const* cmaps) {
-  static std::atomic<bool> attr[64];
+// The descriptors of a small launch as a kernel parameter: problems, then segments.
+template <int BYTES>
+struct InlineDesc {
+  alignas(16) unsigned char b[BYTES];
+};
+template <int T, int BYTES>
+__global__ void __launch_bounds__(NT, T == 64 ? 4 : 6) gemm_grouped_inline_kernel(const __grid_constant__ InlineDesc<BYTES> d,
+                                                                    int nprob) {
+  const GemmProb* probs = reinterpret_cast<const GemmProb*>(d.b);
+  gemm_tile<T>(probs, nprob, reinterpret_cast<const GemmSeg*>(probs + nprob), nullptr);
+}
+
+template <int T>
+constexpr size_t pipe_smem() { return 2 * (size_t)STAGES * ptile<T>() * sizeof(double); }
+
+// Dynamic shared memory of the kernels above, once per device (every caller
+// sets the same values, so threads that race here agree).
+cudaError_t pipe_attributes() {
+  static std::atomic<bool> set[64];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !attr[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_grouped_pipe_kernel<S, KB>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pipe_smem<S, KB>());
-    if (e != cudaSuccess) return e;
-    if (dev < 64) attr[dev].store(true, std::memory_order_release);
-  }
-  NRGB_LAUNCH(tag, stream,
-              gemm_grouped_pipe_kernel<S, KB><<<total_tiles, NT, pipe_smem<S, KB>(), stream>>>(d_probs, nprob, d_segs, cmaps));
+  if (dev < 64 && set[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  auto one = [&](auto* k, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  one(gemm_grouped_pipe_kernel<64>, pipe_smem<64>());
+  one(gemm_grouped_pipe_kernel<32>, pipe_smem<32>());
+  one(gemm_grouped_inline_kernel<64, 4096>, pipe_smem<64>());
+  one(gemm_grouped_inline_kernel<32, 4096>, pipe_smem<32>());
+  one(gemm_grouped_inline_kernel<64, GEMM_INLINE_MAX>, pipe_smem<64>());
+  one(gemm_grouped_inline_kernel<32, GEMM_INLINE_MAX>, pipe_smem<32>());
+  if (e == cudaSuccess && dev < 64) set[dev].store(true, std::memory_order_release);
+  return e;
+}
+
+// Tile edge of a launch: four 32 x 32 CTAs for each 64 x 64 tile where those
+// would leave SMs idle, or where the problems are so small (60 tiles: an edge
+// of 480) that the tiles' rims outweigh the operands read twice as often.
+// Measured (64 / 32, us): one 500^3 44.9 / 26.5, four 300^3 32.0 / 25.7, twelve of
+// 400-500 130.6 / 116.7, eighty of 100-300 86 / 79, two 700^3 78.5 / 88.1, forty
+// 512^3 399 / 450, sixteen 1024^3 1172 / 1351.
+bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || total_tiles <= 60L * nprob; }
+
+cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
+                        cudaStream_t stream, const int* const* cmaps) {
+  const cudaError_t e = pipe_attributes();
+  if (e != cudaSuccess) return e;
+  if (use_small_tiles(total_tiles, nprob))
+    gemm_grouped_pipe_kernel<32><<<4 * total_tiles, NT, pipe_smem<32>(), stream>>>(d_probs, nprob, d_segs, cmaps);
+  else
+    gemm_grouped_pipe_kernel<64><<<total_tiles, NT, pipe_smem<64>(), stream>>>(d_probs, nprob, d_segs, cmaps);
+  return cudaGetLastError();
+}
+
+template <int BYTES>
+cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
+                          cudaStream_t stream) {
+  InlineDesc<BYTES> d;
+  memcpy(d.b, probs, nprob * sizeof(GemmProb));
+  memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
+  if (use_small_tiles(total_tiles, nprob))
+    gemm_grouped_inline_kernel<32, BYTES><<<4 * total_tiles, NT, pipe_smem<32>(), stream>>>(d, nprob);
+  else
+    gemm_grouped_inline_kernel<64, BYTES><<<total_tiles, NT, pipe_smem<64>(), stream>>>(d, nprob);
   return cudaGetLastError();
 }
 // The 128x128 cp.async variant is used only where the device's schedule
 // (schedule.cuh, set by the autotuner's measurements) says it wins: by
 // default never (measured on B200 at first: 21-25 TF/s against 25-28 TF/s
-// for the 64x64 register-staged kernel on the same shapes).
+// for a register-staged 64x64 kernel on the same shapes).
 
 }  // namespace
 
@@ -706,20 +597,48 @@ cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSe
                 gemm_grouped_large_kernel<<<total_stiles, LNT, LSMEM, stream>>>(d_probs, nprob, d_segs, cmaps));
     return cudaGetLastError();
   }
-  const int stages = gemm_pipe_stages();
-  if (stages == 3) return pipe_launch<3, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
-  if (stages == 4) return pipe_launch<4, 16>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
-  if (stages == 232) return pipe_launch<2, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
-  if (stages == 332) return pipe_launch<3, 32>(d_probs, nprob, d_segs, total_tiles, stream, tag, cmaps);
-  NRGB_LAUNCH(tag, stream, gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs, cmaps));
-  return cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  NRGB_LAUNCH(tag, stream, e = pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, cmaps));
+  return e;
 }
 
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                             int total_tiles, cudaStream_t stream) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
-  gemm_grouped_kernel<<<total_tiles, NT, 0, stream>>>(d_probs, nprob, d_segs, nullptr);
-  return cudaGetLastError();
+  return pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, nullptr);
+}
+
+size_t gemm_desc_bytes(int nprob, int nseg) {
+  return nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) + 1024;
+}
+
+cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
+                                     cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch) {
+  if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  if (gemm_inline_fits(nprob, nseg) && schedule_here().gemm_large_from.load(std::memory_order_relaxed) == 0) {
+    NRGB_LAUNCH(tag, stream, e = gemm_grouped_launch_inline(probs, nprob, segs, nseg, total_tiles, stream));
+    return e;
+  }
+  GemmProb* dp = scratch.alloc_n<GemmProb>(nprob);
+  GemmSeg* ds = scratch.alloc_n<GemmSeg>(nseg);
+  if ((e = cudaMemcpyAsync(dp, probs, nprob * sizeof(GemmProb), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(ds, segs, nseg * sizeof(GemmSeg), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
+  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles);
+}
+
+bool gemm_inline_fits(int nprob, int nseg) {
+  return nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= (size_t)GEMM_INLINE_MAX;
+}
+
+cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg,
+                                       int total_tiles, cudaStream_t stream) {
+  if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
+  const cudaError_t e = pipe_attributes();
+  if (e != cudaSuccess) return e;
+  if (nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= 4096)
+    return inline_launch<4096>(probs, nprob, segs, nseg, total_tiles, stream);
+  return inline_launch<GEMM_INLINE_MAX>(probs, nprob, segs, nseg, total_tiles, stream);
 }
 
 }  // namespace nrgb

@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace nrgb {
 
 struct GemmSeg {
@@ -60,6 +62,20 @@ cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSe
 // no events): used by the allocation-free entry point.
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                             int total_tiles, cudaStream_t stream);
+
+// The same with the descriptors in host memory, passed as a kernel parameter
+// (gemm_inline_fits: up to GEMM_INLINE_MAX bytes): no copy to the device.
+constexpr int GEMM_INLINE_MAX = 32000;
+bool gemm_inline_fits(int nprob, int nseg);
+cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg,
+                                       int total_tiles, cudaStream_t stream);
+
+// A launch described on the host: inline when the descriptors fit (and the
+// schedule does not ask for 128 x 128 tiles), else through copies into `scratch`,
+// which must have room for both arrays (gemm_desc_bytes).
+size_t gemm_desc_bytes(int nprob, int nseg);
+cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
+                                     cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch);
 
 // Algorithmic flops of a grouped launch described on the host
 // (sum over problems and their segments of 2 m n k); for the launch

@@ -129,17 +129,22 @@ extern "C" int nrgb_basis_change_noalloc(int nops, const int* n_bra, const int* 
     ++np;
   }
   if (np == 0) return 0;
-  if (cudaMemcpyAsync(d_p1, g_p1, np * sizeof(g_p1[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(d_s1, g_s1, np * sizeof(g_s1[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(d_p2, g_p2, np * sizeof(g_p2[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(d_s2, g_s2, np * sizeof(g_s2[0]), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return 6;
-  if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p1), np,
-                                            reinterpret_cast<nrgb::GemmSeg*>(d_s1), t1, st) != cudaSuccess)
-    return 6;
-  if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p2), np,
-                                            reinterpret_cast<nrgb::GemmSeg*>(d_s2), t2, st) != cudaSuccess)
-    return 6;
+  if (nrgb::gemm_inline_fits(np, np)) {  // descriptors as kernel parameters: no copies
+    if (nrgb::gemm_grouped_launch_inline(g_p1, np, g_s1, np, t1, st) != cudaSuccess) return 6;
+    if (nrgb::gemm_grouped_launch_inline(g_p2, np, g_s2, np, t2, st) != cudaSuccess) return 6;
+  } else {
+    if (cudaMemcpyAsync(d_p1, g_p1, np * sizeof(g_p1[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(d_s1, g_s1, np * sizeof(g_s1[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(d_p2, g_p2, np * sizeof(g_p2[0]), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemcpyAsync(d_s2, g_s2, np * sizeof(g_s2[0]), cudaMemcpyHostToDevice, st) != cudaSuccess)
+      return 6;
+    if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p1), np,
+                                              reinterpret_cast<nrgb::GemmSeg*>(d_s1), t1, st) != cudaSuccess)
+      return 6;
+    if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p2), np,
+                                              reinterpret_cast<nrgb::GemmSeg*>(d_s2), t2, st) != cudaSuccess)
+      return 6;
+  }
   // the static host staging is reused by the next call: wait until the GPU is done
   if (cudaStreamSynchronize(st) != cudaSuccess) return 6;
   return 0;

@@ -379,10 +379,9 @@ int nrgb_recalc(nrgb_ctx* ctx, int nout, const nrgb_recalc_out* outs, int nterms
     }
     auto launch = [&](std::vector<GemmProb>& P, std::vector<GemmSeg>& Sg, int tiles, int stiles) {
       if (P.empty()) return;
-      GemmProb* dP = stage(ctx, P);
-      GemmSeg* dS = stage(ctx, Sg);
       KernelStats::get().add_work("gemm_f64_recalc", gemm_flops(P.data(), (int)P.size(), Sg.data()));
-      NRGB_CUDA(gemm_grouped_launch(dP, (int)P.size(), dS, tiles, st, "gemm_f64_recalc", stiles));
+      NRGB_CUDA(gemm_grouped_launch_host(P.data(), (int)P.size(), Sg.data(), (int)Sg.size(), tiles, st, "gemm_f64_recalc",
+                                         stiles, ctx->scratch));
     };
     launch(p1, s1, t1, st1);
     launch(p2, s2, t2, st2);
@@ -460,10 +459,9 @@ int nrgb_dm_backward(nrgb_ctx* ctx, int nout, const nrgb_dm_out* outs, int nterm
     }
     auto launch = [&](std::vector<GemmProb>& P, std::vector<GemmSeg>& Sg, int tiles, int stiles) {
       if (P.empty()) return;
-      GemmProb* dP = stage(ctx, P);
-      GemmSeg* dS = stage(ctx, Sg);
       KernelStats::get().add_work("gemm_f64_dm", gemm_flops(P.data(), (int)P.size(), Sg.data()));
-      NRGB_CUDA(gemm_grouped_launch(dP, (int)P.size(), dS, tiles, st, "gemm_f64_dm", stiles));
+      NRGB_CUDA(gemm_grouped_launch_host(P.data(), (int)P.size(), Sg.data(), (int)Sg.size(), tiles, st, "gemm_f64_dm",
+                                         stiles, ctx->scratch));
     };
     launch(p1, s1, t1, st1);
     launch(p2, s2, t2, st2);
@@ -566,9 +564,8 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
       maxe = std::max(maxe, allj * alli);
     }
     if (!gp.empty()) {
-      GemmProb* dP = stage(ctx, gp);
-      GemmSeg* dS = stage(ctx, gs);
-      NRGB_CUDA(gemm_grouped_launch(dP, (int)gp.size(), dS, tiles, st, "gemm_f64_spec", stiles));
+      NRGB_CUDA(gemm_grouped_launch_host(gp.data(), (int)gp.size(), gs.data(), (int)gs.size(), tiles, st,
+                                         "gemm_f64_spec", stiles, ctx->scratch));
     }
     double* dbins = static_cast<double*>(ctx->scratch.alloc(2 * (size_t)nbins * sizeof(double)));
     NRGB_CUDA(cudaMemsetAsync(dbins, 0, 2 * (size_t)nbins * sizeof(double), st));
@@ -647,9 +644,8 @@ int nrgb_spectrum_dmnrg(nrgb_ctx* ctx, int npairs, const nrgb_dmnrg_pair* pairs,
       maxe = std::max(maxe, d1 * dp);
     }
     if (!gp.empty()) {
-      GemmProb* dP = stage(ctx, gp);
-      GemmSeg* dS = stage(ctx, gs);
-      NRGB_CUDA(gemm_grouped_launch(dP, (int)gp.size(), dS, tiles, st, "gemm_f64_spec", stiles));
+      NRGB_CUDA(gemm_grouped_launch_host(gp.data(), (int)gp.size(), gs.data(), (int)gs.size(), tiles, st,
+                                         "gemm_f64_spec", stiles, ctx->scratch));
     }
     double* dbins = static_cast<double*>(ctx->scratch.alloc(2 * (size_t)nbins * sizeof(double)));
     NRGB_CUDA(cudaMemsetAsync(dbins, 0, 2 * (size_t)nbins * sizeof(double), st));

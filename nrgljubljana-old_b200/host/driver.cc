@@ -333,10 +333,9 @@ struct NrgDriver::Impl {
       launches += 3;
       return;
     }
-    GemmProb* dp = upload(g.probs);
-    GemmSeg* ds = upload(g.segs);
     KernelStats::get().add_work("gemm_f64_nrg", gemm_flops(g.probs.data(), (int)g.probs.size(), g.segs.data()));
-    NRGB_CUDA(gemm_grouped_launch(dp, (int)g.probs.size(), ds, g.tiles, st, "gemm_f64_nrg", g.stiles));
+    NRGB_CUDA(gemm_grouped_launch_host(g.probs.data(), (int)g.probs.size(), g.segs.data(), (int)g.segs.size(), g.tiles, st,
+                                       "gemm_f64_nrg", g.stiles, desc));
     launches += 1;
   }
   DevMat upload_mat(const HostMat& M, Slab& slab) {
