@@ -80,6 +80,9 @@ cudaError_t spec_dmnrg_launch(const SpecDmnrgPair* d_pairs, int npairs, int max_
 cudaError_t spec_fdm_launch(const SpecFdmPair* d_pairs, int npairs, int max_elems, BinGrid g,
                             double T, double wnf, double msign, double* bins, cudaStream_t st);
 
+// Writes XEj = exp(-Ej / T) and XEi = exp(-Ei / T) of every pair.
+cudaError_t boltzmann_launch(const SpecFdmPair* d_pairs, int npairs, int max_states, double T, cudaStream_t st);
+
 // Merge chain bins into the full spectrum: FDM adds; DM-NRG applies the
 // N/N+2 window (src/spectrumrealfreq.cc:96-185) to bins with Emin<e<Emax.
 cudaError_t merge_bins_launch(const double* chain, double* full, const double* ebins, BinGrid g,

@@ -488,7 +488,7 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
     // per pair: the two products with the density matrices and the
     // Boltzmann factors of both blocks' states
     size_t bytes = 2 * (size_t)nbins * sizeof(double) + (size_t)npairs * sizeof(SpecFdmPair) + 8192;
-    std::vector<double> hx;  // every pair's two energy lists, back to back, then exp(-E/T) in place
+    size_t nx = 0;  // every pair's two lists of Boltzmann factors, back to back
     std::vector<size_t> xo(2 * (size_t)npairs);
     for (int k = 0; k < npairs; ++k) {
       const nrgb_fdm_pair& q = pairs[k];
@@ -502,25 +502,14 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
         const PlanMatrix& E = mat(ctx, side ? q.e_j : q.e_i);
         const int want = side ? A.rows : A.cols;
         if ((long)E.rows * E.cols != want) throw CudaError("nrgb_spectrum_fdm: energy list length differs from the block");
-        xo[2 * k + side] = hx.size();
-        hx.resize(hx.size() + want);
+        xo[2 * k + side] = nx;
+        nx += want;
       }
     }
-    for (int k = 0; k < npairs; ++k)
-      for (int side = 0; side < 2; ++side) {
-        const PlanMatrix& E = mat(ctx, side ? pairs[k].e_j : pairs[k].e_i);
-        const size_t want = (size_t)E.rows * E.cols;
-        if (want)
-          NRGB_CUDA(cudaMemcpyAsync(hx.data() + xo[2 * k + side], E.p, want * sizeof(double), cudaMemcpyDeviceToHost,
-                                    st));
-      }
-    NRGB_CUDA(cudaStreamSynchronize(st));
-    for (double& x : hx) x = exp(-x / T);
-    bytes += hx.size() * sizeof(double) + (size_t)(4 * npairs + 16) * 512;  // allocations and their alignment
+    bytes += nx * sizeof(double) + (size_t)(4 * npairs + 16) * 512;  // allocations and their alignment
     ctx->scratch.reserve(bytes + (size_t)(2 * npairs + 8) * (sizeof(GemmProb) + sizeof(GemmSeg)));
     ctx->scratch.reset();
-    double* dx = static_cast<double*>(ctx->scratch.alloc(std::max<size_t>(1, hx.size()) * sizeof(double)));
-    if (!hx.empty()) NRGB_CUDA(cudaMemcpyAsync(dx, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    double* dx = static_cast<double*>(ctx->scratch.alloc(std::max<size_t>(1, nx) * sizeof(double)));
     std::vector<GemmProb> gp;
     std::vector<GemmSeg> gs;
     int tiles = 0, stiles = 0;
@@ -538,7 +527,7 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
       gs.push_back(GemmSeg{a, b, lda, ldb, k, 0, 0, 1.0});
     };
     std::vector<SpecFdmPair> sp;
-    int maxe = 0;
+    int maxe = 0, maxs = 0;
     for (int k = 0; k < npairs; ++k) {
       const nrgb_fdm_pair& q = pairs[k];
       const PlanMatrix& A = mat(ctx, q.op1);
@@ -562,6 +551,7 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
       sp.push_back(SpecFdmPair{A.p, B.p, O2R, RO2, mat(ctx, q.e_j).p, mat(ctx, q.e_i).p, dx + xo[2 * k + 1],
                                dx + xo[2 * k], A.rows, allj, alli, q.retj, q.reti, q.factor});
       maxe = std::max(maxe, allj * alli);
+      maxs = std::max(maxs, std::max(allj, alli));
     }
     if (!gp.empty()) {
       NRGB_CUDA(gemm_grouped_launch_host(gp.data(), (int)gp.size(), gs.data(), (int)gs.size(), tiles, st,
@@ -569,8 +559,11 @@ int nrgb_spectrum_fdm(nrgb_ctx* ctx, int npairs, const nrgb_fdm_pair* pairs, dou
     }
     double* dbins = static_cast<double*>(ctx->scratch.alloc(2 * (size_t)nbins * sizeof(double)));
     NRGB_CUDA(cudaMemsetAsync(dbins, 0, 2 * (size_t)nbins * sizeof(double), st));
-    if (!sp.empty())
-      NRGB_CUDA(spec_fdm_launch(stage(ctx, sp), (int)sp.size(), maxe, grid, T, wn, fermionic ? 1.0 : -1.0, dbins, st));
+    if (!sp.empty()) {
+      const SpecFdmPair* dsp = stage(ctx, sp);
+      NRGB_CUDA(boltzmann_launch(dsp, (int)sp.size(), maxs, T, st));
+      NRGB_CUDA(spec_fdm_launch(dsp, (int)sp.size(), maxe, grid, T, wn, fermionic ? 1.0 : -1.0, dbins, st));
+    }
     std::vector<double> hb(2 * (size_t)nbins);
     NRGB_CUDA(cudaMemcpyAsync(hb.data(), dbins, hb.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     NRGB_CUDA(cudaStreamSynchronize(st));
