@@ -3,29 +3,46 @@
 // operands staged in shared memory by bulk asynchronous copies); see
 // gemm_split.cuh for the arithmetic.
 //
-// Operand packing.  A slicing pass writes every operand as ready-made
-// shared-memory images: op(A) in tiles of 128 rows x 64 K-bytes, op(B)^T in
-// tiles of 64 rows x 64 K-bytes, each in the canonical K-major layout
-// without swizzle (core matrices of 8 rows x 16 bytes; consecutive core
-// matrices along K 128 bytes apart, along the rows 512 bytes apart).  The S
-// slices of one (row tile, K chunk) follow each other, so one stage of the
-// GEMM is two contiguous bulk copies: S x 8 KB of A and S x 4 KB of B.
+// Operand packing.  Two passes over the operands: one finds the row exponents,
+// one writes the digits as ready-made shared-memory images: op(A) in tiles of
+// 128 rows x 32 K-bytes, op(B)^T in tiles of 64 rows x 32 K-bytes, each in the
+// canonical K-major layout without swizzle (core matrices of 8 rows x 16
+// bytes; consecutive core matrices along K 128 bytes apart, along the rows 256
+// bytes apart).  The digits of one (row tile, K chunk) follow each other, so
+// one stage of the GEMM is two contiguous bulk copies: D x 4 KB of A and D x
+// 2 KB of B.  Both passes are meant to run at the rate of memory: their blocks
+// take 128 K entries of a row tile (many blocks also for few problems), an
+// element is converted to an integer once, and its digits are the bytes of
+// that integer plus a bias.  (One block per row tile for the exponents, and a
+// multiply, truncate, subtract and convert per digit, took 0.43 ms for eight
+// products of edges 900 to 1500; the two passes take 0.11 ms.)
 //
-// GEMM kernel.  One CTA (4 warps) per 128 x 64 output tile of a problem.
-// Warp 1 lane 0 issues the bulk copies into a two-stage ring
-// (cp.async.bulk with mbarrier transaction counts); warp 0 lane 0 issues
-// the tcgen05.mma instructions: for every chunk, the slice pairs (p, q) with
-// p + q <= S + 1, two K = 32 instructions each, into the accumulator of
-// p + q (S accumulators of 64 INT32 columns: up to 512 tensor-memory
-// columns), and commits to the stage's "empty" barrier.  After a segment's
-// last chunk a commit to the "done" barrier releases the epilogue: each warp
-// reads its 32 rows (tensor-memory lanes) with tcgen05.ld, recombines the
-// accumulators in FP64 and adds alpha times the result into C.  Every wait
-// on a barrier is bounded; a wait that gives up sets an error flag, ends
-// the CTA's work (waiting, bounded, for its copies in flight), frees the
-// tensor memory and returns.
+// GEMM kernel.  Persistent CTAs, each over 128 x 64 output tiles: one warp issues
+// the bulk copies into a ring of 32-byte-deep chunks (mbarrier transaction
+// counts), another the tcgen05.mma instructions: for every chunk the digit pairs
+// (p, q) with p + q <= D + 1 into the accumulator of p + q (D accumulators of
+// 64 INT32 columns: up to 448 of the 512 tensor-memory columns), and commits to
+// the stage's "empty" barrier.  Pairs of one p follow each other, so the A
+// image is read from shared memory once and kept in the tensor core's collector
+// buffer.  After a segment's last chunk a commit to the "done" barrier releases
+// eight warps: each reads half the columns of its 32 rows (tensor-memory lanes) with tcgen05.ld,
+// recombines the accumulators exactly in 64-bit integers and adds alpha times
+// the result into C, while the ring already fills for the next tile.
+//
+// What bounds it: the shape of the instruction.  D accumulators of N columns
+// must fit in 512 columns, so N = 64, and a 128 x 64 x 32 product reads 6 KB of
+// operands from shared memory for 32 cycles of arithmetic: measured alone, 48
+// cycles an instruction and 45 with the collector (N = 128: 64).  A chunk's 28
+// products of 8 slices take 1300 to 1500 cycles here.  The eight products above:
+// 0.74 ms with 36 products a chunk, issued by one thread of a divergent branch,
+// and a compensated FP64 recombination; 0.27 ms now.
+// Every wait on a barrier is bounded; a wait that gives up sets an error flag,
+// ends the CTA's work (waiting, bounded, for its copies and products in
+// flight), frees the tensor memory and returns.
 #include "gemm_split.cuh"
 
+#include <float.h>
+#include <limits.h>
 #include <math.h>
 #include <string.h>
 
@@ -37,11 +54,23 @@ namespace {
 
 constexpr int SBM = 128;              // output rows per CTA (tensor-memory lanes)
 constexpr int SBN = 64;               // output columns per CTA
-constexpr int SBK = 64;               // K bytes per stage
-constexpr int A_TILE = SBM * SBK;     // 8 KB
-constexpr int B_TILE = SBN * SBK;     // 4 KB
-constexpr int SPLIT_NT = 128;
+constexpr int SBK = 32;               // K bytes per stage
+constexpr int A_TILE = SBM * SBK;     // 4 KB
+constexpr int B_TILE = SBN * SBK;     // 2 KB
+constexpr int EPI_WARPS = 8;          // two per quarter of the tensor-memory lanes
+constexpr int SPLIT_NT = 32 * EPI_WARPS + 64;  // and a warp for the copies, one for the products
+constexpr int SLICE_NT = 256;
+constexpr int PIECE = 4;              // K chunks per block of the slicing passes
+constexpr int MAX_STAGES = 16;
+constexpr size_t RING_BYTES = 216 * 1024;
 constexpr long long WAIT_LIMIT = 1ll << 24;
+constexpr int NO_EXP = (int)0x80808080;  // what memset leaves: a row of zeros
+
+// Digits of 8 bits that carry what `slices` truncated digits of 7 bits do: D
+// balanced digits (the leading one with 7 bits and the sign) leave a remainder
+// of at most 2^-8D, so 7 of them replace 8 slices, and fewer slices become as
+// many digits.
+constexpr int split_digits(int slices) { return slices < 8 ? slices : 7; }
 
 __device__ int g_split_err = 0;
 
@@ -50,10 +79,11 @@ struct SliceJob {
   long long rs, ls;
   int rows, K;
   int tile_rows;     // 128 (A) or 64 (B)
-  int kch;           // K chunks of 64
-  int tile0;         // first row tile of this job in the launch
-  signed char* out;  // packed slices: [row tile][K chunk][slice] images
-  int* exps;         // tile rows of exponents (rows past `rows`: 0)
+  int kch;           // K chunks of 32
+  int pieces;        // blocks of PIECE chunks
+  int block0;        // first (row tile, piece) of this job in the launch
+  signed char* out;  // packed digits: [row tile][K chunk][digit] images
+  int* exps;         // tile rows of exponents (rows of zeros and past `rows`: NO_EXP)
 };
 
 struct SplitSeg {
@@ -78,88 +108,154 @@ __device__ __forceinline__ int find_job(const SliceJob* jobs, int njobs, int t) 
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].tile0 <= t) lo = mid; else hi = mid - 1;
+    if (jobs[mid].block0 <= t) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
 
-// Row exponents: E_r with max_l |X(r, l)| < 2^E_r (0 for a zero row).
-__global__ void __launch_bounds__(SPLIT_NT) split_exp_kernel(const SliceJob* __restrict__ jobs, int njobs) {
+// Largest integer whose D balanced digits fit: D bytes 0x7F.
+__device__ __forceinline__ long long digit_limit(int D) { return 0x7F7F7F7F7F7F7F7Fll >> (8 * (8 - D)); }
+
+// Exponent of a row whose largest magnitude is mx > 0: the least e for which mx
+// scaled by 2^(8 D - 1 - e) rounds to an integer of D balanced digits.
+__device__ __forceinline__ int digit_exp(double mx, int D) {
+  int e;
+  const double f = frexp(fmin(mx, DBL_MAX), &e);  // [0.5, 1)
+  return __double2ll_rn(ldexp(f, 8 * D - 1)) > digit_limit(D) ? e + 1 : e;
+}
+
+__device__ __forceinline__ int row_exp(const int* exps, int r) {
+  const int e = exps[r];
+  return e == NO_EXP ? 0 : e;
+}
+
+// Row exponents: the largest of the pieces' exponents.
+__global__ void __launch_bounds__(SLICE_NT) split_exp_kernel(const SliceJob* __restrict__ jobs, int njobs, int D) {
   const SliceJob J = jobs[find_job(jobs, njobs, blockIdx.x)];
-  const int t = blockIdx.x - J.tile0;
-  const int r0 = t * J.tile_rows;
+  const int local = blockIdx.x - J.block0;
+  const int t = local / J.pieces, l0 = (local % J.pieces) * PIECE * SBK;
+  const int l1 = min(J.K, l0 + PIECE * SBK), R = J.tile_rows;
   if (J.rs == 1) {
-    // consecutive rows are adjacent: one thread per row, coalesced over rows
-    for (int rr = threadIdx.x; rr < J.tile_rows; rr += blockDim.x) {
-      const int r = r0 + rr;
-      double mx = 0.0;
-      if (r < J.rows)
-        for (int l = 0; l < J.K; ++l) mx = fmax(mx, fabs(J.X[(long long)r + l * J.ls]));
-      int e = 0;
-      if (mx > 0.0) frexp(mx, &e);
-      J.exps[r0 + rr] = e;
+    // consecutive rows are adjacent: a thread takes one row and every
+    // (SLICE_NT / R)-th of its entries
+    const int rr = threadIdx.x % R, r = t * R + rr, step = SLICE_NT / R;
+    double mx = 0.0;
+    if (r < J.rows) {
+      const double* x = J.X + r;
+#pragma unroll 8
+      for (int l = l0 + threadIdx.x / R; l < l1; l += step) mx = fmax(mx, fabs(x[l * J.ls]));
     }
+    if (mx > 0.0) atomicMax(&J.exps[t * R + rr], digit_exp(mx, D));
   } else {
     // the K entries of a row are adjacent: one warp per row
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int rr = warp; rr < J.tile_rows; rr += blockDim.x >> 5) {
-      const int r = r0 + rr;
+#pragma unroll 2
+    for (int rr = warp; rr < R; rr += SLICE_NT / 32) {
+      const int r = t * R + rr;
       double mx = 0.0;
-      if (r < J.rows)
-        for (int l = lane; l < J.K; l += 32) mx = fmax(mx, fabs(J.X[(long long)r * J.rs + (long long)l * J.ls]));
+      if (r < J.rows) {
+        const double* x = J.X + r * J.rs;
+#pragma unroll
+        for (int u = 0; u < PIECE * SBK / 32; ++u) {
+          const int l = l0 + lane + 32 * u;
+          if (l < l1) mx = fmax(mx, fabs(x[l * J.ls]));
+        }
+      }
       for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      int e = 0;
-      if (mx > 0.0) frexp(mx, &e);
-      if (lane == 0) J.exps[r0 + rr] = e;
+      if (lane == 0 && mx > 0.0) atomicMax(&J.exps[t * R + rr], digit_exp(mx, D));
     }
   }
 }
 
-// Digits: one item = 16 consecutive K entries of one row, written as 16
-// bytes into each of the S slice images of its (row tile, K chunk).
-__global__ void __launch_bounds__(SPLIT_NT) split_digits_kernel(const SliceJob* __restrict__ jobs, int njobs,
-                                                                 int slices) {
-  // blockIdx.x enumerates (row tile, K chunk) pairs: tile0 counts row tiles
-  // times K chunks here
-  const SliceJob J = jobs[find_job(jobs, njobs, blockIdx.x)];
-  const int local = blockIdx.x - J.tile0;
-  const int t = local / J.kch, kc = local % J.kch;
+// Bytes of four words, byte j of word u to byte u of word j.
+__device__ __forceinline__ void transpose4(unsigned (&w)[4]) {
+  const unsigned a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+  const unsigned c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+  w[0] = __byte_perm(a, b, 0x5410);
+  w[1] = __byte_perm(a, b, 0x7632);
+  w[2] = __byte_perm(c, d, 0x5410);
+  w[3] = __byte_perm(c, d, 0x7632);
+}
+
+// The digits of 16 consecutive K entries x of a row (scaled by f1 * f2 they
+// are rounded to integers), 16 bytes into each of the D images.
+// With 0x80 in every byte as a bias the balanced digits carry by themselves:
+// digit = byte of (y + bias), less 0x80.
+__device__ __forceinline__ void write_digits(const double (&x)[16], double f1, double f2, int D, signed char* dst,
+                                             size_t image) {
+  unsigned out[8][4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    unsigned a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long y = __double2ll_rn(x[4 * q + u] * f1 * f2);
+      const unsigned long long z = ((unsigned long long)y + 0x8080808080808080ull) ^ 0x8080808080808080ull;
+      a[u] = (unsigned)z;
+      b[u] = (unsigned)(z >> 32);
+    }
+    transpose4(a);
+    transpose4(b);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      out[j][q] = a[j];
+      out[4 + j][q] = b[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 7; ++j)  // byte j is digit D - j
+    if (j < D)
+      *reinterpret_cast<uint4*>(dst + (size_t)(D - 1 - j) * image) =
+          make_uint4(out[j][0], out[j][1], out[j][2], out[j][3]);
+}
+
+// Power of two 2^s, -1022 <= s <= 1023.
+__device__ __forceinline__ double pow2(int s) { return __longlong_as_double((long long)(s + 1023) << 52); }
+
+__global__ void __launch_bounds__(SLICE_NT) split_digits_kernel(const SliceJob* __restrict__ jobs, int njobs, int D) {
+  __shared__ double tile[SBM][SBK + 1];
+  // backwards: what the exponents' pass read last is still in L2
+  const int block = gridDim.x - 1 - blockIdx.x;
+  const SliceJob J = jobs[find_job(jobs, njobs, block)];
+  const int local = block - J.block0;
+  const int t = local / J.pieces, c0 = (local % J.pieces) * PIECE, c1 = min(J.kch, c0 + PIECE);
   const int R = J.tile_rows;
-  const int items = R * (SBK / 16);
-  const size_t tile_bytes = (size_t)R * SBK;
-  signed char* base = J.out + ((size_t)t * J.kch + kc) * slices * tile_bytes;
-  for (int it = threadIdx.x; it < items; it += blockDim.x) {
-    int rr, g;
-    if (J.rs == 1) {  // rows fastest: coalesced reads across the warp
-      rr = it % R;
-      g = it / R;
-    } else {          // K groups fastest: each thread reads 128 contiguous bytes
-      rr = it / (SBK / 16);
-      g = it % (SBK / 16);
-    }
-    const int r = t * R + rr;
-    const int l0 = kc * SBK + g * 16;
-    double x[16];
-    const int e = J.exps[r];
+  const size_t image = (size_t)R * SBK;
+  signed char* base = J.out + (size_t)t * J.kch * D * image;
+  // 16 entries of row rr, K group g of chunk c
+  auto write = [&](const double(&x)[16], int rr, int c, int g) {
+    const int s = 8 * D - 1 - row_exp(J.exps, t * R + rr), h = s / 2;
+    write_digits(x, pow2(h), pow2(s - h), D,
+                 base + (size_t)c * D * image + (rr >> 3) * 256 + g * 128 + (rr & 7) * 16, image);
+  };
+  if (J.rs == 1) {  // rows fastest: coalesced reads across the warp
+    for (int it = threadIdx.x; it < R * 2 * (c1 - c0); it += SLICE_NT) {
+      const int rr = it % R, cg = it / R, c = c0 + (cg >> 1), g = cg & 1;
+      const int r = t * R + rr, l0 = c * SBK + g * 16;
+      double x[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int l = l0 + u;
-      double v = 0.0;
-      if (r < J.rows && l < J.K) v = J.X[(long long)r * J.rs + (long long)l * J.ls];
-      x[u] = ldexp(v, -e);  // |x| < 1, exact
+      for (int u = 0; u < 16; ++u)
+        x[u] = (r < J.rows && l0 + u < J.K) ? J.X[(long long)r + (l0 + u) * J.ls] : 0.0;
+      write(x, rr, c, g);
     }
-    const size_t off = (size_t)(rr >> 3) * 512 + (size_t)g * 128 + (size_t)(rr & 7) * 16;
-    for (int p = 0; p < slices; ++p) {
-      unsigned w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const double tt = x[u] * 128.0;  // exact
-        const double d = trunc(tt);      // |d| <= 127
-        x[u] = tt - d;                   // exact remainder, |x| < 1
-        const unsigned byte = (unsigned)((int)d) & 0xffu;
-        w[u >> 2] |= byte << (8 * (u & 3));
+  } else {  // the K entries of a row are adjacent: through shared memory
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c = c0; c < c1; ++c) {
+      const int l = c * SBK + lane;
+#pragma unroll 8
+      for (int rr = warp; rr < R; rr += SLICE_NT / 32) {
+        const int r = t * R + rr;
+        tile[rr][lane] = (r < J.rows && l < J.K) ? J.X[(long long)r * J.rs + l * J.ls] : 0.0;
       }
-      *reinterpret_cast<uint4*>(base + (size_t)p * tile_bytes + off) = make_uint4(w[0], w[1], w[2], w[3]);
+      __syncthreads();
+      for (int it = threadIdx.x; it < R * 2; it += SLICE_NT) {
+        const int rr = it % R, g = it / R;
+        double x[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) x[u] = tile[rr][16 * g + u];
+        write(x, rr, c, g);
+      }
+      __syncthreads();
     }
   }
 }
@@ -191,6 +287,20 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
   return ok != 0;
 }
 
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred P;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+      "selp.b32 %0, 1, 0, P;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait for the phase with parity `parity` to complete.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
   for (long long it = 0; it < WAIT_LIMIT; ++it) {
@@ -198,6 +308,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
     if (*abort_flag) return false;
   }
   return false;
+}
+
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -225,8 +339,41 @@ constexpr unsigned IDESC_I8 = (2u << 4)            // D format S32
                               | ((SBN >> 3) << 17)  // N / 8
                               | ((SBM >> 4) << 24); // M / 16
 
+// Use of the collector buffer of A: filled by the first product of an A image,
+// read by the later ones.
+enum Collector { A_ONCE, A_FILL, A_USE, A_LASTUSE };
+
+template <Collector COL>
 __device__ __forceinline__ void mma_i8(unsigned dtmem, unsigned long long adesc, unsigned long long bdesc,
                                        unsigned accumulate) {
+  if constexpr (COL == A_FILL)
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::i8.collector::a::fill [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(IDESC_I8), "r"(accumulate)
+      : "memory");
+  else if constexpr (COL == A_USE)
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::i8.collector::a::use [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(IDESC_I8), "r"(accumulate)
+      : "memory");
+  else if constexpr (COL == A_LASTUSE)
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::i8.collector::a::lastuse [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(IDESC_I8), "r"(accumulate)
+      : "memory");
+  else
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
@@ -237,6 +384,19 @@ __device__ __forceinline__ void mma_i8(unsigned dtmem, unsigned long long adesc,
       : "memory");
 }
 
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile(
+      "{\n"
+      ".reg .pred P;\n"
+      "elect.sync _|P, 0xffffffff;\n"
+      "selp.b32 %0, 1, 0, P;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
                : "memory");
@@ -245,14 +405,66 @@ __device__ __forceinline__ void mma_commit(unsigned bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld16(unsigned taddr, int (&v)[16]) {
-  asm volatile(
+// 16 columns of N accumulators, SBN columns apart (loads and their wait in one
+// statement: nothing may read the registers before the wait).
+template <int N>
+__device__ __forceinline__ void tmem_ld16(unsigned taddr, int (&v)[N][16]) {
+  static_assert(N >= 1 && N <= 4);
+  if constexpr (N == 1)
+    asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(v[0][0]), "=r"(v[0][1]), "=r"(v[0][2]), "=r"(v[0][3]), "=r"(v[0][4]), "=r"(v[0][5]), "=r"(v[0][6]),
+        "=r"(v[0][7]), "=r"(v[0][8]), "=r"(v[0][9]), "=r"(v[0][10]), "=r"(v[0][11]), "=r"(v[0][12]), "=r"(v[0][13]),
+        "=r"(v[0][14]), "=r"(v[0][15])
+      : "r"(taddr + 0 * SBN)
       : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+  else if constexpr (N == 2)
+    asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(v[0][0]), "=r"(v[0][1]), "=r"(v[0][2]), "=r"(v[0][3]), "=r"(v[0][4]), "=r"(v[0][5]), "=r"(v[0][6]),
+        "=r"(v[0][7]), "=r"(v[0][8]), "=r"(v[0][9]), "=r"(v[0][10]), "=r"(v[0][11]), "=r"(v[0][12]), "=r"(v[0][13]),
+        "=r"(v[0][14]), "=r"(v[0][15]), "=r"(v[1][0]), "=r"(v[1][1]), "=r"(v[1][2]), "=r"(v[1][3]), "=r"(v[1][4]),
+        "=r"(v[1][5]), "=r"(v[1][6]), "=r"(v[1][7]), "=r"(v[1][8]), "=r"(v[1][9]), "=r"(v[1][10]), "=r"(v[1][11]),
+        "=r"(v[1][12]), "=r"(v[1][13]), "=r"(v[1][14]), "=r"(v[1][15])
+      : "r"(taddr + 0 * SBN), "r"(taddr + 1 * SBN)
+      : "memory");
+  else if constexpr (N == 3)
+    asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%48];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%49];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%50];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(v[0][0]), "=r"(v[0][1]), "=r"(v[0][2]), "=r"(v[0][3]), "=r"(v[0][4]), "=r"(v[0][5]), "=r"(v[0][6]),
+        "=r"(v[0][7]), "=r"(v[0][8]), "=r"(v[0][9]), "=r"(v[0][10]), "=r"(v[0][11]), "=r"(v[0][12]), "=r"(v[0][13]),
+        "=r"(v[0][14]), "=r"(v[0][15]), "=r"(v[1][0]), "=r"(v[1][1]), "=r"(v[1][2]), "=r"(v[1][3]), "=r"(v[1][4]),
+        "=r"(v[1][5]), "=r"(v[1][6]), "=r"(v[1][7]), "=r"(v[1][8]), "=r"(v[1][9]), "=r"(v[1][10]), "=r"(v[1][11]),
+        "=r"(v[1][12]), "=r"(v[1][13]), "=r"(v[1][14]), "=r"(v[1][15]), "=r"(v[2][0]), "=r"(v[2][1]), "=r"(v[2][2]),
+        "=r"(v[2][3]), "=r"(v[2][4]), "=r"(v[2][5]), "=r"(v[2][6]), "=r"(v[2][7]), "=r"(v[2][8]), "=r"(v[2][9]),
+        "=r"(v[2][10]), "=r"(v[2][11]), "=r"(v[2][12]), "=r"(v[2][13]), "=r"(v[2][14]), "=r"(v[2][15])
+      : "r"(taddr + 0 * SBN), "r"(taddr + 1 * SBN), "r"(taddr + 2 * SBN)
+      : "memory");
+  else if constexpr (N == 4)
+    asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%64];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%65];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%66];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%67];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(v[0][0]), "=r"(v[0][1]), "=r"(v[0][2]), "=r"(v[0][3]), "=r"(v[0][4]), "=r"(v[0][5]), "=r"(v[0][6]),
+        "=r"(v[0][7]), "=r"(v[0][8]), "=r"(v[0][9]), "=r"(v[0][10]), "=r"(v[0][11]), "=r"(v[0][12]), "=r"(v[0][13]),
+        "=r"(v[0][14]), "=r"(v[0][15]), "=r"(v[1][0]), "=r"(v[1][1]), "=r"(v[1][2]), "=r"(v[1][3]), "=r"(v[1][4]),
+        "=r"(v[1][5]), "=r"(v[1][6]), "=r"(v[1][7]), "=r"(v[1][8]), "=r"(v[1][9]), "=r"(v[1][10]), "=r"(v[1][11]),
+        "=r"(v[1][12]), "=r"(v[1][13]), "=r"(v[1][14]), "=r"(v[1][15]), "=r"(v[2][0]), "=r"(v[2][1]), "=r"(v[2][2]),
+        "=r"(v[2][3]), "=r"(v[2][4]), "=r"(v[2][5]), "=r"(v[2][6]), "=r"(v[2][7]), "=r"(v[2][8]), "=r"(v[2][9]),
+        "=r"(v[2][10]), "=r"(v[2][11]), "=r"(v[2][12]), "=r"(v[2][13]), "=r"(v[2][14]), "=r"(v[2][15]),
+        "=r"(v[3][0]), "=r"(v[3][1]), "=r"(v[3][2]), "=r"(v[3][3]), "=r"(v[3][4]), "=r"(v[3][5]), "=r"(v[3][6]),
+        "=r"(v[3][7]), "=r"(v[3][8]), "=r"(v[3][9]), "=r"(v[3][10]), "=r"(v[3][11]), "=r"(v[3][12]), "=r"(v[3][13]),
+        "=r"(v[3][14]), "=r"(v[3][15])
+      : "r"(taddr + 0 * SBN), "r"(taddr + 1 * SBN), "r"(taddr + 2 * SBN), "r"(taddr + 3 * SBN)
+      : "memory");
 }
 
 __device__ __forceinline__ int find_prob(const SplitProb* probs, int nprob, int b) {
@@ -265,27 +477,140 @@ __device__ __forceinline__ int find_prob(const SplitProb* probs, int nprob, int 
 }
 
 // ------------------------------------------------------------------ GEMM
+// sum_d v_d 256^(D - 1 - d) of 16 columns as hi 2^L + low, 0 <= low < 2^L: the
+// first four terms and the rest are exact in 64 bits each (|v| < 2^31).
+template <int D>
+struct Recombine {
+  static constexpr int NH = D < 4 ? D : 4, NL = D - NH, L = 8 * NL;
+  long long hi[16];
+  int low[16];
+
+  __device__ __forceinline__ void load(unsigned taddr) {
+    {
+      int v[NH][16];
+      tmem_ld16<NH>(taddr, v);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        hi[u] = 0;
+#pragma unroll
+        for (int d = 0; d < NH; ++d) hi[u] += (long long)v[d][u] * (1ll << (8 * (NH - 1 - d)));
+      }
+    }
+    if constexpr (NL > 0) {
+      int v[NL][16];
+      tmem_ld16<NL>(taddr + NH * SBN, v);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        long long x = 0;
+#pragma unroll
+        for (int d = 0; d < NL; ++d) x += (long long)v[d][u] * (1ll << (8 * (NL - 1 - d)));
+        hi[u] += x >> L;
+        low[u] = (int)x & ((1 << L) - 1);
+      }
+    }
+  }
+  // the sum, rounded once to FP64
+  __device__ __forceinline__ double value(int u) const {
+    long long bottom = (hi[u] & 0xFFFFF) << L;  // below 2^44: exact
+    if constexpr (NL > 0) bottom |= low[u];
+    return fma((double)(hi[u] >> 20), (double)(1ll << (20 + L)), (double)bottom);
+  }
+};
+
+// Barriers and the ring of one CTA, as shared-memory addresses.
+struct Ring {
+  unsigned data, full0, empty0, done, drained, last;
+};
+
+constexpr int FIRST = 1, LAST = 2, END = 4;  // of a stage's chunk: see flag_s
+
+// The warp that issues the products.  (A function of its own: inlined beside
+// the recombination its loop issues 28 products in 1426 cycles instead of 1304.)
+template <int D>
+__device__ __noinline__ void split_products(Ring ring, unsigned tmem, int stages, const volatile int* flag_s,
+                                            volatile int* abort_flag) {
+  constexpr unsigned STAGE = (unsigned)D * (A_TILE + B_TILE);
+  auto give_up = [&] {
+    atomicExch(&g_split_err, 1);
+    *abort_flag = 1;
+  };
+  // products.  The whole warp takes the loop and one lane issues: with the
+  // operands' descriptors in uniform registers an issue is short.  The tensor
+  // core queues few products, and what the next chunk needs is looked up while
+  // the last ones of this chunk wait.
+  const bool leader = elect_one();
+  int st = 0, round = 0, item = 0;
+  bool ready = false;
+  for (;;) {
+    if (!ready && !mbar_wait(ring.full0 + 8 * st, round & 1, abort_flag)) {
+      give_up();
+      break;
+    }
+    const int flag = __shfl_sync(0xffffffffu, flag_s[st], 0);
+    if (flag & END) break;
+    if ((flag & FIRST) && !mbar_wait(ring.drained, (item & 1) ^ 1, abort_flag)) {
+      give_up();
+      break;
+    }
+    tc_fence_after();
+    const unsigned sa = ring.data + (unsigned)st * STAGE;
+    const unsigned long long ad = smem_desc(sa, 128, 256), bd = smem_desc(sa + D * A_TILE, 128, 256);
+    const unsigned more = !(flag & FIRST);
+    const unsigned empty = ring.empty0 + 8 * st;
+    if (++st == stages) {
+      st = 0;
+      ++round;
+    }
+#pragma unroll
+    for (int p = 0; p < D; ++p) {
+      if (p == (D > 2 ? 2 : 1)) ready = __all_sync(0xffffffffu, mbar_test(ring.full0 + 8 * st, round & 1));
+      if (leader) {
+#pragma unroll
+        for (int q = 0; q < D - p; ++q) {
+          const unsigned dt = tmem + (unsigned)((p + q) * SBN);
+          const unsigned long long a = ad + (unsigned)(p * A_TILE >> 4), b = bd + (unsigned)(q * B_TILE >> 4);
+          const unsigned acc = p > 0 ? 1u : more;
+          if (D - p == 1) mma_i8<A_ONCE>(dt, a, b, acc);
+          else if (q == 0) mma_i8<A_FILL>(dt, a, b, acc);
+          else if (q == D - p - 1) mma_i8<A_LASTUSE>(dt, a, b, acc);
+          else mma_i8<A_USE>(dt, a, b, acc);
+        }
+      }
+    }
+    if (leader) {
+      mma_commit(empty);  // the stage is free once these products have read it
+      if (flag & LAST) mma_commit(ring.done);  // every product of the segment has completed
+    }
+    __syncwarp();
+    if (flag & LAST) ++item;
+  }
+  // nothing is in flight when the tensor memory is released
+  if (leader) mma_commit(ring.last);
+  for (long long it = 0; it < WAIT_LIMIT && !mbar_try_wait(ring.last, 0); ++it) {
+  }
+}
+
+template <int D>
 __global__ void __launch_bounds__(SPLIT_NT, 1) split_gemm_kernel(const SplitProb* __restrict__ probs, int nprob,
-                                                                  const SplitSeg* __restrict__ segs, int slices,
-                                                                  unsigned tmem_cols) {
+                                                                  const SplitSeg* __restrict__ segs, int tiles,
+                                                                  int stages, unsigned tmem_cols) {
   extern __shared__ __align__(1024) unsigned char dsm[];
-  // 1024-aligned stage buffers: [stage][A: S x 8 KB | B: S x 4 KB]
+  // ring of stages, 1024-aligned: [A: D x 4 KB | B: D x 2 KB]
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<size_t>(dsm) + 1023) & ~size_t(1023));
-  const unsigned stage_bytes = (unsigned)slices * (A_TILE + B_TILE);
-  __shared__ __align__(8) unsigned long long bars[5];  // full[2], empty[2], done
+  constexpr unsigned STAGE = (unsigned)D * (A_TILE + B_TILE);
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_STAGES + 3];  // full, empty, done, drained, last
+  // per stage: first, last chunk of a segment (set by the copies' thread, so that
+  // the products' thread looks nothing up), end of the work
+  __shared__ volatile int flag_s[MAX_STAGES];
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
-  __shared__ int issued_s;  // chunks whose copies have been issued (ring position)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  const SplitProb P = probs[find_prob(probs, nprob, blockIdx.x)];
-  const int local = blockIdx.x - P.tile0;
-  const int mt = local / P.tiles_n, nt = local % P.tiles_n;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES]);
+  const unsigned done = smem_u32(&bars[2 * MAX_STAGES]), drained = done + 8, last = done + 16;
 
   if (tid == 0) {
-    for (int i = 0; i < 5; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    for (int i = 0; i < 2 * MAX_STAGES + 3; ++i) mbar_init(smem_u32(&bars[i]), i == 2 * MAX_STAGES + 1 ? EPI_WARPS : 1);
     abort_s = 0;
-    issued_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
@@ -299,126 +624,101 @@ __global__ void __launch_bounds__(SPLIT_NT, 1) split_gemm_kernel(const SplitProb
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tmem_base_s;
-  const unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[2]), done = smem_u32(&bars[4]);
   volatile int* abort_flag = &abort_s;
+  const Ring ring{smem_u32(sm), full0, empty0, done, drained, last};
+  auto give_up = [&] {
+    atomicExch(&g_split_err, 1);
+    *abort_flag = 1;
+  };
 
-  int g0 = 0;  // chunks issued so far in this CTA (ring position and phases)
-  for (int si = 0; si < P.nseg; ++si) {
-    const SplitSeg S = segs[P.seg0 + si];
-    const int nk = S.kch;
-    if (warp == 1 && lane == 0) {
-      // producer: bulk copies of each chunk's S A images and S B images
-      const signed char* a0 = S.A + (size_t)mt * nk * slices * A_TILE;
-      const signed char* b0 = S.B + (size_t)nt * nk * slices * B_TILE;
-      for (int c = 0; c < nk && !*abort_flag; ++c) {
-        const int g = g0 + c, st = g & 1;
-        if (g >= 2 && !mbar_wait(empty0 + 8 * st, ((g >> 1) - 1) & 1, abort_flag)) {
-          atomicExch(&g_split_err, 1);
-          *abort_flag = 1;
-          break;
+  if (warp == EPI_WARPS && lane == 0) {
+    // copies: each chunk's D images of A and of B
+    int st = 0, round = 0;
+    for (int t = blockIdx.x; t < tiles && !*abort_flag; t += gridDim.x) {
+      const SplitProb P = probs[find_prob(probs, nprob, t)];
+      const int local = t - P.tile0, mt = local / P.tiles_n, nt = local % P.tiles_n;
+      for (int si = 0; si < P.nseg; ++si) {
+        const SplitSeg S = segs[P.seg0 + si];
+        const signed char* a = S.A + (size_t)mt * S.kch * D * A_TILE;
+        const signed char* b = S.B + (size_t)nt * S.kch * D * B_TILE;
+        for (int c = 0; c < S.kch && !*abort_flag; ++c) {
+          if (!mbar_wait(empty0 + 8 * st, (round & 1) ^ 1, abort_flag)) {
+            give_up();
+            break;
+          }
+          const unsigned dst = smem_u32(sm) + (unsigned)st * STAGE, bar = full0 + 8 * st;
+          flag_s[st] = (c == 0 ? FIRST : 0) | (c == S.kch - 1 ? LAST : 0);
+          mbar_expect_tx(bar, STAGE);
+          bulk_g2s(dst, a + (size_t)c * D * A_TILE, D * A_TILE, bar);
+          bulk_g2s(dst + D * A_TILE, b + (size_t)c * D * B_TILE, D * B_TILE, bar);
+          if (++st == stages) {
+            st = 0;
+            ++round;
+          }
         }
-        const unsigned dst = smem_u32(sm + (size_t)st * stage_bytes);
-        mbar_expect_tx(full0 + 8 * st, stage_bytes);
-        bulk_g2s(dst, a0 + (size_t)c * slices * A_TILE, (unsigned)slices * A_TILE, full0 + 8 * st);
-        bulk_g2s(dst + (unsigned)slices * A_TILE, b0 + (size_t)c * slices * B_TILE, (unsigned)slices * B_TILE,
-                 full0 + 8 * st);
-        issued_s = g + 1;
       }
-    } else if (warp == 0 && lane == 0) {
-      // MMA issuer
-      unsigned started = 0;  // accumulators written in this segment
-      for (int c = 0; c < nk && !*abort_flag; ++c) {
-        const int g = g0 + c, st = g & 1;
-        if (!mbar_wait(full0 + 8 * st, (g >> 1) & 1, abort_flag)) {
-          atomicExch(&g_split_err, 1);
-          *abort_flag = 1;
+    }
+    if (!*abort_flag) {
+      if (mbar_wait(empty0 + 8 * st, (round & 1) ^ 1, abort_flag)) {
+        flag_s[st] = END;
+        mbar_arrive(full0 + 8 * st);
+      } else {
+        give_up();
+      }
+    }
+    if (*abort_flag) {  // the copies in flight land before the memory is released
+      for (int i = 0; i < stages; ++i) {
+        const int n = round + (i < st ? 1 : 0);  // copies into stage i so far
+        if (n == 0) continue;
+        for (long long it = 0; it < WAIT_LIMIT && !mbar_try_wait(full0 + 8 * i, (n - 1) & 1); ++it) {
+        }
+      }
+    }
+  } else if (warp == EPI_WARPS + 1) {
+    split_products<D>(ring, tmem, stages, flag_s, &abort_s);
+  } else if (warp < EPI_WARPS) {
+    // recombination and C: a warp takes 32 rows and half of the columns
+    const int quarter = warp & 3, half = warp >> 2;
+    int item = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+      const SplitProb P = probs[find_prob(probs, nprob, t)];
+      const int local = t - P.tile0, mt = local / P.tiles_n, nt = local % P.tiles_n;
+      const int row = mt * SBM + quarter * 32 + lane;
+      bool ok = true;
+      for (int si = 0; si < P.nseg && ok; ++si, ++item) {
+        const SplitSeg S = segs[P.seg0 + si];
+        // lane u holds the exponent of column u of the half
+        const int ea = row_exp(S.eA, row) - 8 * D - 6, eb = row_exp(S.eB, nt * SBN + half * 32 + lane);
+        if (lane == 0) ok = mbar_wait(done, item & 1, abort_flag);
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok) {
+          give_up();
           break;
         }
         tc_fence_after();
-        const unsigned sa = smem_u32(sm + (size_t)st * stage_bytes);
-        const unsigned sb = sa + (unsigned)slices * A_TILE;
-        for (int p = 1; p <= slices; ++p)
-          for (int q = 1; p + q <= slices + 1; ++q) {
-            const int d = p + q - 2;  // accumulator index 0 .. S-1
-            const unsigned dt = tmem + (unsigned)(d * SBN);
+        Recombine<D> x[2];  // 16 columns each
 #pragma unroll
-            for (int ks = 0; ks < SBK / 32; ++ks) {
-              const unsigned long long ad = smem_desc(sa + (p - 1) * A_TILE + ks * 256, 128, 512);
-              const unsigned long long bd = smem_desc(sb + (q - 1) * B_TILE + ks * 256, 128, 512);
-              mma_i8(dt, ad, bd, (started >> d) & 1u);
-              started |= 1u << d;
-            }
-          }
-        mma_commit(empty0 + 8 * st);  // the stage is free once these MMAs have read it
-      }
-      mma_commit(done);  // every MMA of the segment has completed
-    }
-    __syncwarp();
-    // epilogue: wait for the segment's MMAs, then recombine in FP64
-    bool ok = mbar_wait(done, si & 1, abort_flag);
-    __syncwarp();
-    if (!ok) {
-      if (tid == 0) atomicExch(&g_split_err, 1);
-      *abort_flag = 1;
-    }
-    tc_fence_after();
-    if (!*abort_flag) {
-      const int row = mt * SBM + warp * 32 + lane;
-      const int ea = (row < P.m) ? S.eA[row] : 0;
-      for (int cg = 0; cg < SBN / 16; ++cg) {
-        double sum[16], cmp[16];
+        for (int h = 0; h < 2; ++h)
+          x[h].load(tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(half * 32 + h * 16));
+        // the accumulators may be overwritten
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(drained);
+        const int col0 = nt * SBN + half * 32;
+        double* cp = P.C + (size_t)col0 * P.ldc + row;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) sum[u] = cmp[u] = 0.0;
-        for (int d = slices - 1; d >= 0; --d) {  // smallest scale first
-          int v[16];
-          tmem_ld16(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(d * SBN + cg * 16), v);
-          const double sc = ldexp(1.0, -7 * (d + 2));
-#pragma unroll
-          for (int u = 0; u < 16; ++u) {
-            const double t = (double)v[u] * sc;  // exact
-            const double s2 = sum[u] + t;        // TwoSum
-            const double bp = s2 - sum[u];
-            cmp[u] += (sum[u] - (s2 - bp)) + (t - bp);
-            sum[u] = s2;
-          }
-        }
-        if (row < P.m) {
-#pragma unroll
-          for (int u = 0; u < 16; ++u) {
-            const int col = nt * SBN + cg * 16 + u;
-            if (col >= P.n) continue;
-            const double val = S.alpha * ldexp(sum[u] + cmp[u], ea + S.eB[col]);
-            double* cp = P.C + (size_t)col * P.ldc + row;
-            double base = 0.0;
-            if (si > 0) base = *cp;
-            else if (P.beta != 0.0) base = P.beta * *cp;
-            *cp = base + val;
-          }
+        for (int u = 0; u < 32; ++u) {
+          const int e = ea + __shfl_sync(0xffffffffu, eb, u);
+          if (row >= P.m || col0 + u >= P.n) continue;
+          const double f = x[u / 16].value(u % 16);
+          double val = S.alpha * (abs(e) < 900 ? f * pow2(e) : ldexp(f, e));
+          double* c = cp + (size_t)u * P.ldc;
+          if (si > 0) val += *c;
+          else if (P.beta != 0.0) val += P.beta * *c;
+          *c = val;
         }
       }
-    }
-    g0 += nk;
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (*abort_flag) {
-      // a wait gave up: before the shared memory and the tensor memory are
-      // released, let this CTA's copies in flight land and its MMAs finish
-      // (both bounded; the MMA thread committed `done` after its last MMA)
-      if (tid == 32) {
-        const int issued = issued_s;
-        for (int st = 0; st < 2; ++st) {
-          int last = issued - 1;
-          if (last >= 0 && (last & 1) != st) last -= 1;
-          if (last < 0) continue;
-          for (long long it = 0; it < WAIT_LIMIT && !mbar_try_wait(full0 + 8 * st, (last >> 1) & 1); ++it) {
-          }
-        }
-      }
-      if (tid == 0)
-        for (long long it = 0; it < WAIT_LIMIT && !mbar_try_wait(done, si & 1); ++it) {
-        }
-      break;
+      if (!ok) break;
     }
   }
   tc_fence_before();
@@ -429,16 +729,30 @@ __global__ void __launch_bounds__(SPLIT_NT, 1) split_gemm_kernel(const SplitProb
   }
 }
 
-size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
+template <int D>
+cudaError_t split_gemm_launch(const SplitProb* probs, int nprob, const SplitSeg* segs, int tiles, cudaStream_t st) {
+  constexpr size_t stage = (size_t)D * (A_TILE + B_TILE);
+  constexpr int stages = RING_BYTES / stage < MAX_STAGES ? (int)(RING_BYTES / stage) : MAX_STAGES;
+  constexpr size_t smem = stages * stage + 1024;
+  static std::once_flag once;
+  static cudaError_t err = cudaSuccess;
+  std::call_once(once, [] {
+    err = cudaFuncSetAttribute(split_gemm_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (err != cudaSuccess) return err;
+  unsigned cols = 32;
+  while (cols < (unsigned)(D * SBN)) cols <<= 1;
+  split_gemm_kernel<D><<<std::min(tiles, 148), SPLIT_NT, smem, st>>>(probs, nprob, segs, tiles, stages, cols);
+  return cudaGetLastError();
+}
 
-struct SegShape {
-  int m, n, k;
-};
+size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 
 }  // namespace
 
 size_t split_gemm_workspace(const GemmProb* probs, int nprob, const GemmSeg* segs, int slices) {
   size_t b = 1 << 16;
+  const size_t D = split_digits(slices);
   for (int p = 0; p < nprob; ++p)
     for (int s = 0; s < probs[p].nseg; ++s) {
       const GemmSeg& g = segs[probs[p].seg0 + s];
@@ -446,12 +760,12 @@ size_t split_gemm_workspace(const GemmProb* probs, int nprob, const GemmSeg* seg
         const size_t kk = std::min(SPLIT_MAX_K, g.k - k0);
         const size_t kch = ceil_div(kk, SBK);
         const size_t tm = ceil_div(probs[p].m, SBM), tn = ceil_div(probs[p].n, SBN);
-        b += (size_t)slices * kch * (tm * A_TILE + tn * B_TILE) + 512;
+        b += D * kch * (tm * A_TILE + tn * B_TILE) + 512;
         b += (tm * SBM + tn * SBN) * sizeof(int) + 512;
       }
-      b += 2 * sizeof(SliceJob) + sizeof(SplitSeg) + 64;
+      b += 2 * sizeof(SliceJob) + sizeof(SplitSeg);
     }
-  b += (size_t)nprob * (sizeof(SplitProb) + 64);
+  b += (size_t)nprob * sizeof(SplitProb);
   return b;
 }
 
@@ -462,9 +776,11 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
   std::vector<SliceJob> jobs;
   std::vector<SplitSeg> ss;
   std::vector<SplitProb> ps;
-  int exp_tiles = 0, dig_blocks = 0, tiles = 0;
+  int blocks = 0, tiles = 0;
   double flops = 0;
-  std::vector<std::pair<int, int>> jobs_dig;  // digit-block prefix per job
+  const int D = split_digits(slices);
+  std::vector<size_t> eoff;  // per job: its exponents within those of the launch
+  size_t nexp = 0;
   for (int p = 0; p < nprob; ++p) {
     const GemmProb& G = probs[p];
     if (G.m <= 0 || G.n <= 0) continue;
@@ -492,8 +808,7 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
         ja.X = g.A + (size_t)k0 * ja.ls;
         ja.tile_rows = SBM;
         ja.kch = kch;
-        ja.out = ws.alloc_n<signed char>((size_t)slices * kch * sp.tiles_m * A_TILE);
-        ja.exps = ws.alloc_n<int>((size_t)sp.tiles_m * SBM);
+        ja.out = ws.alloc_n<signed char>((size_t)D * kch * sp.tiles_m * A_TILE);
         // op(B)^T(j, l) = op(B)(l, j) = B[l + j ldb] (as stored) or B[j + l ldb]
         SliceJob jb{};
         jb.rows = G.n;
@@ -503,22 +818,21 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
         jb.X = g.B + (size_t)k0 * jb.ls;
         jb.tile_rows = SBN;
         jb.kch = kch;
-        jb.out = ws.alloc_n<signed char>((size_t)slices * kch * sp.tiles_n * B_TILE);
-        jb.exps = ws.alloc_n<int>((size_t)sp.tiles_n * SBN);
+        jb.out = ws.alloc_n<signed char>((size_t)D * kch * sp.tiles_n * B_TILE);
         SplitSeg q{};
         q.A = ja.out;
         q.B = jb.out;
-        q.eA = ja.exps;
-        q.eB = jb.exps;
         q.kch = kch;
         q.alpha = g.alpha;
         ss.push_back(q);
         for (SliceJob* j : {&ja, &jb}) {
           const int t = (int)ceil_div(j->rows, j->tile_rows);
+          j->pieces = (int)ceil_div(kch, PIECE);
+          j->block0 = blocks;
+          blocks += t * j->pieces;
           jobs.push_back(*j);
-          jobs_dig.push_back({exp_tiles, dig_blocks});
-          exp_tiles += t;
-          dig_blocks += t * j->kch;
+          eoff.push_back(nexp);
+          nexp += (size_t)t * j->tile_rows;
         }
       }
     }
@@ -537,38 +851,36 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
     ps.push_back(sp);
   }
   if (ps.empty()) return;
-  // the two slicing launches index the jobs by their own prefix counts
-  std::vector<SliceJob> je = jobs, jd = jobs;
-  for (size_t i = 0; i < jobs.size(); ++i) {
-    je[i].tile0 = jobs_dig[i].first;
-    jd[i].tile0 = jobs_dig[i].second;
+  int* exps = ws.alloc_n<int>(nexp);
+  for (size_t i = 0; i < jobs.size(); ++i) jobs[i].exps = exps + eoff[i];
+  for (size_t i = 0; i < ss.size(); ++i) {  // two jobs per segment, A's and B's
+    ss[i].eA = exps + eoff[2 * i];
+    ss[i].eB = exps + eoff[2 * i + 1];
   }
-  SliceJob* d_je = ws.alloc_n<SliceJob>(je.size());
-  SliceJob* d_jd = ws.alloc_n<SliceJob>(jd.size());
-  SplitSeg* d_ss = ws.alloc_n<SplitSeg>(ss.size());
-  SplitProb* d_ps = ws.alloc_n<SplitProb>(ps.size());
-  NRGB_CUDA(cudaMemcpyAsync(d_je, je.data(), je.size() * sizeof(SliceJob), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(d_jd, jd.data(), jd.size() * sizeof(SliceJob), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(d_ss, ss.data(), ss.size() * sizeof(SplitSeg), cudaMemcpyHostToDevice, st));
-  NRGB_CUDA(cudaMemcpyAsync(d_ps, ps.data(), ps.size() * sizeof(SplitProb), cudaMemcpyHostToDevice, st));
-  const int nj = (int)jobs.size();
-  NRGB_LAUNCH("split_slice", st, split_exp_kernel<<<exp_tiles, SPLIT_NT, 0, st>>>(d_je, nj));
+  // the descriptors in one copy
+  const size_t bj = jobs.size() * sizeof(SliceJob), bs = ss.size() * sizeof(SplitSeg), bp = ps.size() * sizeof(SplitProb);
+  std::vector<unsigned char> desc(bj + bs + bp);
+  memcpy(desc.data(), jobs.data(), bj);
+  memcpy(desc.data() + bj, ss.data(), bs);
+  memcpy(desc.data() + bj + bs, ps.data(), bp);
+  unsigned char* d = ws.alloc_n<unsigned char>(desc.size());
+  NRGB_CUDA(cudaMemcpyAsync(d, desc.data(), desc.size(), cudaMemcpyHostToDevice, st));
+  const SliceJob* d_j = reinterpret_cast<const SliceJob*>(d);
+  const SplitSeg* d_ss = reinterpret_cast<const SplitSeg*>(d + bj);
+  const SplitProb* d_ps = reinterpret_cast<const SplitProb*>(d + bj + bs);
+  const int nj = (int)jobs.size(), np = (int)ps.size();
+  NRGB_CUDA(cudaMemsetAsync(exps, 0x80, nexp * sizeof(int), st));
+  NRGB_LAUNCH("split_slice", st, split_exp_kernel<<<blocks, SLICE_NT, 0, st>>>(d_j, nj, D));
   NRGB_CUDA(cudaGetLastError());
-  NRGB_LAUNCH("split_slice", st, split_digits_kernel<<<dig_blocks, SPLIT_NT, 0, st>>>(d_jd, nj, slices));
+  NRGB_LAUNCH("split_slice", st, split_digits_kernel<<<blocks, SLICE_NT, 0, st>>>(d_j, nj, D));
   NRGB_CUDA(cudaGetLastError());
-  const size_t smem = 2 * (size_t)slices * (A_TILE + B_TILE) + 1024;
-  static std::once_flag attr_once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(attr_once, [&] {
-    attr_err = cudaFuncSetAttribute(split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(2 * (size_t)SPLIT_MAX_SLICES * (A_TILE + B_TILE) + 1024));
-  });
-  NRGB_CUDA(attr_err);
-  unsigned cols = 32;
-  while (cols < (unsigned)(slices * SBN)) cols <<= 1;
+  cudaError_t (*launch)(const SplitProb*, int, const SplitSeg*, int, cudaStream_t) =
+      D == 2 ? split_gemm_launch<2> : D == 3 ? split_gemm_launch<3> : D == 4 ? split_gemm_launch<4>
+      : D == 5 ? split_gemm_launch<5> : D == 6 ? split_gemm_launch<6> : split_gemm_launch<7>;
   KernelStats::get().add_work(tag, flops);
-  NRGB_LAUNCH(tag, st, split_gemm_kernel<<<tiles, SPLIT_NT, smem, st>>>(d_ps, (int)ps.size(), d_ss, slices, cols));
-  NRGB_CUDA(cudaGetLastError());
+  cudaError_t err = cudaSuccess;
+  NRGB_LAUNCH(tag, st, err = launch(d_ps, np, d_ss, tiles, st));
+  NRGB_CUDA(err);
 }
 
 int split_gemm_take_error(cudaStream_t st) {

@@ -5,20 +5,23 @@
 //   C_p = beta_p * C_p + sum_{s in segments(p)} alpha_s * op(A_s) op(B_s)
 //
 // Same problem/segment description as the FP64 grouped GEMM (GemmProb,
-// GemmSeg; column-major, op = as stored or transposed).  Each row i of op(A)
-// is scaled by a power of two 2^eA_i (and each column j of op(B) by 2^eB_j)
-// so that its entries lie in (-1, 1), and cut into `slices` signed 7-bit
-// digits:  op(A)_il = 2^eA_i sum_{p=1..S} a^(p)_il 2^(-7p) + r_il with
-// |r_il| < 2^(eA_i - 7S)  (Ozaki-type splitting, Ozaki, Ogita, Oishi and
+// GemmSeg; column-major, op = as stored or transposed).  `slices` asks for the
+// precision of that many truncated 7-bit slices per operand.  Each row i of
+// op(A) is scaled by a power of two 2^eA_i (and each column j of op(B) by
+// 2^eB_j) so that its entries lie in (-1, 1), rounded to 8 D - 1 bits and cut
+// into D balanced 8-bit digits, D = slices, or 7 for 8 slices:
+//   op(A)_il = 2^eA_i sum_{p=1..D} a^(p)_il 2^(1-8p) + r_il,
+// |r_il| <= 2^(eA_i - 8D)  (Ozaki-type splitting, Ozaki, Ogita, Oishi and
 // Rump 2012, with integer slices as in the INT8 emulation of DGEMM).  Every
-// slice product a^(p) b^(q) is exact in INT32; the products with the same
-// p + q share one accumulator; products with p + q > S + 1 are dropped (they
-// lie below the slicing error).  The result is recombined in FP64 with a
-// compensated (TwoSum) sum of the S scaled accumulators, then scaled by
-// 2^(eA_i + eB_j).  The error per entry is bounded by about
-// k * 2^(eA_i + eB_j) * 2^(-7S) * (S + 1): with S = 8 that is below the
-// rounding error bound of an FP64 product (k 2^-53 |A||B|) for rows and
-// columns whose entries are of similar size.
+// digit product a^(p) b^(q) is exact in INT32; the products with the same
+// p + q share one accumulator; products with p + q > D + 1 are dropped (they
+// lie at the rounding's level).  The D accumulators are recombined exactly in
+// 64-bit integers, rounded once to FP64 and scaled by 2^(eA_i + eB_j).  The
+// error per entry is bounded by about k * 2^(eA_i + eB_j) * 2^(-8D) * (D + 2):
+// for 8 slices, 9 k 2^-56 of the scales, which is below the rounding error bound
+// of an FP64 product (k 2^-53 |A||B|) for rows and columns whose entries are of
+// similar size.  Eight truncated 7-bit slices have (8 + 1) k 2^-56, from 36
+// products instead of 28.
 //
 // This replaces the BLAS gemm calls of the operator recalculation
 // (src/recalc.cc:90-91, 268-272) and of the density matrices
@@ -36,7 +39,7 @@ namespace nrgb {
 constexpr int SPLIT_MIN_SLICES = 2;
 constexpr int SPLIT_MAX_SLICES = 8;
 // Largest inner dimension of one segment: the accumulator of p + q = d sums
-// d - 1 <= S slice products of magnitude <= 127^2 k, which must stay below
+// d - 1 <= 7 digit products of magnitude <= 128^2 k, which must stay below
 // 2^31.  Longer segments are cut into pieces of this length.
 constexpr int SPLIT_MAX_K = 16000;
 
