@@ -123,15 +123,11 @@ class KernelStats {
     ks__.end(slot__, stream);                               \
   } while (0)
 
-// Device-side state of a grid barrier.  The arrival counter and the
-// generation word sit on separate 128-byte lines, so CTAs polling the
-// generation do not contend with the atomics on the counter.
+// Device-side state of a grid barrier, zero at the launch.
 struct GridBarrier {
-  unsigned int count;
-  int error;     // set when a wait gave up
-  unsigned int pad0[30];
-  unsigned int gen;
-  unsigned int pad1[31];
+  unsigned int count;  // arrivals since the launch
+  int error;           // set when a wait gave up
+  unsigned int pad[30];
 };
 
 #ifdef __CUDACC__
@@ -141,46 +137,27 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   return v;
 }
 
-// Generation barrier for co-resident CTAs (cooperative launch).  Thread 0
-// of each CTA arrives with a release-acquire atomic and polls the
-// generation with acquire loads and exponential back-off.  Every wait is
-// bounded: after 2^limit_log2 polls (2^23, about a second, by default) the
-// CTA records an error, and a waiting CTA that sees the error leaves too;
-// once the error is set all later barriers return immediately.  Returns
-// true (in every thread of the CTA) when the error is set, so that the
+// Barrier for co-resident CTAs (cooperative launch): one thread of each CTA, after
+// a barrier of the CTA, adds its arrival with release order and polls the counter
+// with acquire loads until all `nblocks` of barrier number `round` (counting from
+// 1) are in: two trips to L2 beside the slowest CTA.  (An arrival whose result
+// chose the CTA that opens a second word, with the error flag read on either
+// side, made seven.)  Every wait is bounded: after 2^limit_log2 polls (2^23,
+// about a second, by default) the CTA records an error, and a waiting CTA that
+// sees the error leaves too.  Returns true when the wait gave up, so that the
 // caller can end the launch instead of computing on unsynchronised data.
-__device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned int nblocks, int limit_log2 = 23) {
-  __shared__ int s_failed;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const long long limit = 1ll << limit_log2;
-    if (*reinterpret_cast<volatile int*>(&b->error) == 0) {
-      const unsigned int g = ld_acquire_u32(&b->gen);
-      __threadfence();
-      unsigned int arrived;
-      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(arrived) : "l"(&b->count) : "memory");
-      if (arrived + 1u == nblocks) {
-        b->count = 0;
-        __threadfence();
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(&b->gen) : "memory");
-      } else {
-        long long it = 0;
-        unsigned ns = 8;
-        while (ld_acquire_u32(&b->gen) == g) {
-          if (++it > limit || *reinterpret_cast<volatile int*>(&b->error)) {
-            atomicExch(&b->error, 1);
-            break;
-          }
-          __nanosleep(ns);
-          if (ns < 128) ns <<= 1;
-        }
-      }
-      __threadfence();
+__device__ __forceinline__ bool grid_barrier_thread(GridBarrier* b, unsigned nblocks, unsigned round, int limit_log2) {
+  const long long limit = 1ll << limit_log2;
+  const unsigned target = nblocks * round;
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(&b->count) : "memory");
+  for (long long it = 0; (int)(ld_acquire_u32(&b->count) - target) < 0; ++it) {
+    if (it > limit || ((it & 15) == 15 && *reinterpret_cast<volatile int*>(&b->error))) {
+      atomicExch(&b->error, 1);
+      return true;
     }
-    s_failed = *reinterpret_cast<volatile int*>(&b->error);
+    __nanosleep(16);
   }
-  __syncthreads();
-  return s_failed != 0;
+  return false;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

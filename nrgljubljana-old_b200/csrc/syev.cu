@@ -38,8 +38,9 @@ namespace {
 constexpr int SMALL_N = SYEV_TINY;  // blocks solved whole in one CTA
 constexpr int LEAF = DC_BASE;   // subtrees solved in one CTA (dc_base.cu)
 constexpr int NB = 32;          // tridiagonalisation panel width
+constexpr int TRAIL_STRIP = 256;  // columns of a strip of the trailing update
 constexpr int NBB = BT_NB;      // back-transformation block of reflectors
-constexpr int TRD_NT = 256;     // threads of the panel kernel
+constexpr int TRD_NT = 512;     // threads of the panel kernel, one CTA per SM
 constexpr double EPS = 2.220446049250313e-16;
 
 // --------------------------------------------------------------------------
@@ -52,8 +53,7 @@ struct TrdProb {
   double* tau;  // n-1
   double* Vp;   // n x NB panel reflectors, row-major (row i at Vp + i*NB)
   double* W;    // n x NB, row-major
-  double* v;    // n
-  double* y;    // n
+  double* y;    // slots of A22 v: see SymvShape
   double* red;  // 2 slots x (2 + 2*NB)
   GridBarrier* bar;  // this problem's barrier: only its own CTAs synchronise
   int n;
@@ -68,29 +68,167 @@ __device__ __forceinline__ double ld_volatile(const double* p) {
   return *reinterpret_cast<const volatile double*>(p);
 }
 
-// One panel of NB columns for every problem (cooperative launch).  Per column
-// c two phases separated by grid barriers; every load of data written by
-// other CTAs during the launch bypasses L1 (__ldcg).
+// Tiles of the product A22 v: 64 rows x 32 columns, one warp each, anchored at the
+// panel's first row and column (base = j0 + 1; columns that the panel has finished
+// meet zeros of v).  A tile on or below the diagonal gives its row sums to slot J
+// of yr and the sums over its rows, of the elements below the diagonal, to slot I
+// of yc: y_i = sum_{J <= i/32} yr[J][i] + sum_{I >= i/64} yc[I][i].
+constexpr int SY_M = 64, SY_N = 32;
+constexpr int TRD_SMEM = 32 + 4 * NB + 8 + (TRD_NT / 32) * 2 * NB;  // doubles before v
+
+struct SymvShape {
+  int M, nbm, nbn, mp;  // rows; blocks of 64 and of 32; padded rows
+  __host__ __device__ explicit SymvShape(int rows)
+      : M(rows), nbm((rows + SY_M - 1) / SY_M), nbn((rows + SY_N - 1) / SY_N), mp(nbm * SY_M) {}
+};
+
+// y_i (relative row) from every step-th of its slots, from the g-th on (yc lies
+// behind yr, so that a slot is a multiple of mp away).
+__device__ __forceinline__ double symv_sum(const SymvShape& S, const double* yr, int i, int g, int step) {
+  const int nr = i / SY_N + 1, count = nr + S.nbm - i / SY_M, skip = S.nbn + i / SY_M - nr;
+  double s = 0.0;
+  for (int k = g; k < count; k += 16 * step) {
+    double x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int q = k + u * step;
+      x[u] = q < count ? __ldcg(&yr[(size_t)(q < nr ? q : q + skip) * S.mp + i]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += x[u];
+  }
+  return s;
+}
+
+// d (8 x 8) += a (8 x 4) b (4 x 8), one warp; a lane holds a[lane / 4][lane % 4],
+// b[lane % 4][lane / 4] and d[lane / 4][2 (lane % 4) + {0, 1}].
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// A warp's walk through its tiles, 8 columns at a time, with the elements of the
+// next 8 in registers: a lane holds rows lane and 32 + lane of the tile.  Column
+// blocks 2 s and 2 s + 1 have nbm - s tiles; blocks s and nbm - 1 - s together
+// nbm + 1, so tile numbers decode with one division.
+struct SymvWalk {
+  const double* A;  // relative (0, 0)
+  size_t ld;
+  int M, nbm, nbn;
+  int t, step;      // tile number
+  int I, J, strip;  // where the elements in x are
+  double x[16];
+
+  __device__ __forceinline__ bool live() const { return I >= 0; }
+  __device__ __forceinline__ int row() const { return I * SY_M + (threadIdx.x & 31); }
+  __device__ __forceinline__ int col() const { return J * SY_N + 8 * strip; }
+  // every column of the strip lies below the diagonal (and so within the matrix,
+  // the tile's first row being one)
+  __device__ __forceinline__ bool below() const { return col() + 7 < I * SY_M; }
+  // the first tile from number t on
+  __device__ __forceinline__ void settle() {
+    const int folds = (nbm + 1) / 2;
+    I = -1;
+    for (; t < 2 * folds * (nbm + 1); t += step) {
+      const int q = t >> 1, f = q / (nbm + 1), k = q - f * (nbm + 1);
+      const bool first = k < nbm - f;
+      const int s = first ? f : nbm - 1 - f;
+      if (!first && s == f) continue;  // the middle block, counted once
+      J = 2 * s + (t & 1);
+      if (J >= nbn) continue;
+      I = s + (first ? k : k - (nbm - f));
+      break;
+    }
+    strip = 0;
+  }
+  __device__ __forceinline__ void advance() { skip(1); }
+  __device__ __forceinline__ void skip(int strips) {  // up to the end of the tile
+    strip += strips;
+    if (strip == SY_N / 8) {
+      t += step;
+      settle();
+    }
+  }
+  // Below the diagonal rows beyond the last are read as they come: at least eight
+  // columns of the matrix follow, their v is zero and nobody reads their sums.
+  __device__ __forceinline__ void load() {
+    const int r = row(), c = col();
+    const double* a = A + (r + c * ld);
+    if (below()) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u, a += ld) {
+        x[u] = __ldcg(a);
+        x[8 + u] = __ldcg(a + 32);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u, a += ld) {
+        x[u] = (r < M && c + u <= r) ? __ldcg(a) : 0.0;
+        x[8 + u] = (r + 32 < M && c + u <= r + 32) ? __ldcg(a + 32) : 0.0;
+      }
+    }
+  }
+};
+
+// A grid barrier of all threads.  first() runs in warp 0 between the barrier of
+// the CTA and its arrival, over() in the other warps while the barrier is under
+// way and in warp 0 after it.
+template <class F, class G>
+__device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned nblocks, unsigned round, int limit_log2, F&& first,
+                                             G&& over) {
+  __shared__ bool failed;
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    over();
+  } else {
+    first();
+    __syncwarp();
+    if (threadIdx.x == 0) failed = grid_barrier_thread(b, nblocks, round, limit_log2);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) over();
+  return failed;
+}
+
+// One panel of NB columns for every problem (cooperative launch).  A CTA owns a
+// chunk of rows: it alone reads and writes their rows of V and W, through L1.
+// Per column c two phases separated by grid barriers; every load of data written
+// by other CTAs during the launch bypasses L1 (__ldcg).
 //   A: finish the previous column: y = y' - V p - W q (p = W^T v, q = V^T v
 //      of that column), W[:, jj-1] = tau y + a2 v with
 //      a2 = -tau^2/2 * (y'^T v - 2 p^T q);  then
 //      a = A[c:, c] - V W[c,:]^T - W V[c,:]^T and its norm below c+1.
 //   B: Householder vector v of column c (every CTA forms all of it in shared
-//      memory), partial p = W^T v, q = V^T v over this CTA's row chunk, and
-//      y' = A22 v (one warp per column of A22), with y'^T v.
+//      memory), partial p = W^T v, q = V^T v over this CTA's rows, and
+//      y' = A22 v with y'^T v from the lower triangle alone, in tiles whose
+//      sums go to slots that phase A adds up.  The first tile of a CTA is
+//      loaded during the barrier, and strips of it stay in shared memory: A22 is
+//      the same for all columns of a panel.
 // Deferring the V p + W q correction of y to the next column's phase A saves
 // the third grid barrier per column that an eager correction needs.  The
 // entries below the subdiagonal of column c are overwritten with v one
 // phase later too, because every CTA reads the updated column in phase B.
-__global__ void __launch_bounds__(TRD_NT) trd_panel_kernel(const TrdProb* __restrict__ probs,
-                                                           int nprob, int j0, int* fail) {
+//
+// What bounds a column is the chain of round trips to L2 around the two barriers
+// (20000 of 34000 cycles at 2640 rows), then reading A22 and its two sums; while
+// the lower triangles together exceed L2, HBM.  Two blocks of 3600 and 3533 rows
+// together, down to 1776: 36 us a column when both triangles were read and a
+// barrier took seven round trips, 28 with one triangle in tiles that the warps of
+// a CTA shared, 18.3 with a tile to a warp, two round trips to a barrier and the
+// first strips in shared memory.
+// V_SMEM: v in shared memory; otherwise (blocks above 27000 rows) a copy per CTA
+// behind the slots of y.
+template <bool V_SMEM>
+__global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __restrict__ probs,
+                                                              int nprob, int j0, int nres, int* fail) {
   extern __shared__ double sm[];
   double* scratch = sm;          // 32
   double* VWc = sm + 32;         // 2*NB: row c of V and W
   double* pq = VWc + 2 * NB;     // 2*NB: p, q of the previous column
   double* misc = pq + 2 * NB;    // 8
-  double* pqw = misc + 8;        // (TRD_NT/32) x 2*NB partial p,q
-  double* vs = pqw + (TRD_NT / 32) * 2 * NB;  // n_max
+  double* pqw = misc + 8;        // (TRD_NT/32) x 2*NB partial p, q (phase B)
+  double* ypart = pqw;           // 8 x 64 partial sums of y (phase A)
   const int b = blockIdx.x;
   int lo = 0, hi = nprob - 1;
   while (lo < hi) {
@@ -107,67 +245,134 @@ __global__ void __launch_bounds__(TRD_NT) trd_panel_kernel(const TrdProb* __rest
   const size_t ld = (size_t)n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int nwarps = TRD_NT / 32;
-  const int gw = rank * nwarps + warp, tw = P.ncta * nwarps;  // warp index within the problem
+  const int chunk = (n - j0 + P.ncta - 1) / P.ncta;
+  const int R0 = min(n, j0 + rank * chunk), R1 = min(n, R0 + chunk);  // this CTA's rows
+  const int base = j0 + 1;
+  const SymvShape S(max(0, n - base));
+  double* yr = P.y;
+  double* yc = P.y + (size_t)S.nbn * S.mp;
+  double* vs = V_SMEM ? sm + TRD_SMEM : yc + (size_t)S.nbm * S.mp + (size_t)rank * S.mp;  // padded rows
+  // this lane's elements of the strips that stay in shared memory
+  double* res = sm + TRD_SMEM + (V_SMEM ? S.mp : 0) + warp * nres * 512 + lane;
 
+  // W[:, kp] = tprev (y' - V p - W q) + a2 v of the previous column for this CTA's
+  // rows from i0 on, W[i][kp] stored; then f(i, v_i, a) in one lane with
+  // a = A[i][c] - V[i] . W[c] - W[i] . V[c].  Warps take four rows at a time.
+  // scalars() fills pq, VWc and misc[0] = a2 (warp 0, before the first use).
+  auto rows = [&](int i0, int jj, double tprev, auto&& scalars, auto&& f) {
+    const int kp = jj - 1;
+    for (int rb = R0 + ((i0 - R0) / 64) * 64; rb < R1; rb += 64) {
+      // every load of the block at once
+      double vik[4], wik[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = rb + warp * 4 + u;
+        const bool on = i >= i0 && i < R1;
+        vik[u] = on && lane < jj ? P.Vp[(size_t)i * NB + lane] : 0.0;
+        wik[u] = on && lane < kp ? P.W[(size_t)i * NB + lane] : 0.0;
+      }
+      const int il = rb + warp * 4 + lane;  // the row that lanes 0 .. 3 finish
+      const bool fin = lane < 4 && il >= i0 && il < R1;
+      const double acol = fin && jj < NB ? __ldcg(&P.A[il + (size_t)(j0 + jj) * ld]) : 0.0;
+      if (jj > 0) {
+        const int i = rb + (tid & 63), g = tid >> 6;
+        ypart[tid] = (i >= i0 && i < R1) ? symv_sum(S, yr, i - base, g, TRD_NT / 64) : 0.0;
+      }
+      if (warp == 0 && rb <= i0) scalars();
+      __syncthreads();
+      const double pk = pq[lane], qk = pq[NB + lane], vck = VWc[lane], wck = VWc[NB + lane];
+      const double vckp = jj > 0 ? VWc[kp] : 0.0, a2 = jj > 0 ? misc[0] : 0.0;
+      double ys[4], ts[4], vi[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int rr = warp * 4 + u;
+        ys[u] = (jj > 0 && lane < TRD_NT / 64 ? ypart[lane * 64 + rr] : 0.0) - (vik[u] * pk + wik[u] * qk);
+        ts[u] = vik[u] * wck + wik[u] * vck;
+        vi[u] = jj > 0 ? __shfl_sync(0xffffffffu, vik[u], max(kp, 0)) : 0.0;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          ys[u] += __shfl_xor_sync(0xffffffffu, ys[u], o);
+          ts[u] += __shfl_xor_sync(0xffffffffu, ts[u], o);
+        }
+      if (lane < 4) {
+        double y = ys[0], t = ts[0], v = vi[0];
+#pragma unroll
+        for (int u = 1; u < 4; ++u)
+          if (lane == u) {
+            y = ys[u];
+            t = ts[u];
+            v = vi[u];
+          }
+        if (fin) {
+          const double wl = tprev * y + a2 * v;
+          if (jj > 0) P.W[(size_t)il * NB + kp] = wl;
+          f(il, v, acol - (t + wl * vckp));
+        }
+      }
+      __syncthreads();  // ypart is read
+    }
+  };
+
+  // A22 and the tiles of a warp stay as they are within a panel: the first nres
+  // strips of its first tile are read from global memory for the first column
+  // only
+  SymvWalk first{P.A + (size_t)base * (ld + 1), ld, S.M, S.nbm, S.nbn, rank + P.ncta * warp, P.ncta * nwarps, 0, 0, 0, {}};
+  first.settle();
   for (int jj = 0; jj < NB; ++jj) {
     const int c = j0 + jj;
     const bool act = c < n;
     double* R = P.red + (c & 1) * RED;         // this column's sums
     double* Ro = P.red + ((c + 1) & 1) * RED;  // previous column's sums (next column's slot)
+    SymvWalk walk = first;
+    if (jj > 0 && first.live()) walk.skip(nres);
     // ---------------- phase A ----------------
     if (act) {
       const int kp = jj - 1;  // columns of V, W before the previous one
-      double tprev = 0.0;
-      if (jj > 0) tprev = __ldcg(&P.tau[c - 1]);
-      if (tid < NB) {
-        const int k = tid;
-        pq[k] = (k < kp) ? ld_volatile(&Ro[2 + k]) : 0.0;
-        pq[NB + k] = (k < kp) ? ld_volatile(&Ro[2 + NB + k]) : 0.0;
-        VWc[k] = (k < jj) ? __ldcg(&P.Vp[(size_t)c * NB + k]) : 0.0;
-        VWc[NB + k] = (k < kp) ? __ldcg(&P.W[(size_t)c * NB + k]) : 0.0;
-      }
-      __syncthreads();
-      if (jj > 0 && warp == 0) {
-        // scalar a2 and row c of the previous column of W (every CTA)
-        const double ptq = warp_sum(pq[lane] * pq[NB + lane]);
-        const double corr = warp_sum(VWc[lane] * pq[lane] + VWc[NB + lane] * pq[NB + lane]);
-        const double a2 = -0.5 * tprev * tprev * (ld_volatile(&Ro[1]) - 2.0 * ptq);
-        if (lane == 0) {
-          misc[0] = a2;
-          VWc[NB + kp] = tprev * (__ldcg(&P.y[c]) - corr) + a2 * __ldcg(&P.v[c]);
-        }
-      }
-      __syncthreads();
-      const double a2 = (jj > 0) ? misc[0] : 0.0;
-      const double pk = pq[lane], qk = pq[NB + lane];
-      const double vck = VWc[lane], wck = VWc[NB + lane];
-      double ss = 0.0;
-      for (int i = c + gw; i < n; i += tw) {
-        double vik = 0.0, wik = 0.0;
-        if (lane < jj) vik = __ldcg(&P.Vp[(size_t)i * NB + lane]);
-        if (lane < kp) wik = __ldcg(&P.W[(size_t)i * NB + lane]);
-        double wl = 0.0;
+      const double tprev = jj > 0 ? __ldcg(&P.tau[c - 1]) : 0.0;
+      auto scalars = [&] {
+        const double p = (lane < kp) ? ld_volatile(&Ro[2 + lane]) : 0.0, q = (lane < kp) ? ld_volatile(&Ro[2 + NB + lane]) : 0.0;
+        const double vc = (lane < jj) ? __ldcg(&P.Vp[(size_t)c * NB + lane]) : 0.0;
+        double wc = (lane < kp) ? __ldcg(&P.W[(size_t)c * NB + lane]) : 0.0;
         if (jj > 0) {
-          const double corr = warp_sum(vik * pk + wik * qk);
-          wl = tprev * (__ldcg(&P.y[i]) - corr) + a2 * __ldcg(&P.v[i]);
-          if (lane == kp) wik = wl;
+          // scalar a2 and row c of the previous column of W (every CTA)
+          const double yv = ld_volatile(&Ro[1]);
+          const double ptq = warp_sum(p * q);
+          const double y = warp_sum(symv_sum(S, yr, c - base, lane, 32) - (vc * p + wc * q));
+          const double a2 = -0.5 * tprev * tprev * (yv - 2.0 * ptq);
+          if (lane == kp) wc = tprev * y + a2 * vc;
+          if (lane == 0) misc[0] = a2;
         }
-        const double t = warp_sum(vik * wck + wik * vck);
-        if (lane == 0) {
-          if (jj > 0) {
-            P.W[(size_t)i * NB + kp] = wl;
-            if (i >= c + 1) P.A[i + (size_t)(c - 1) * ld] = __ldcg(&P.v[i]);
-          }
-          const double a = __ldcg(&P.A[i + c * ld]) - t;
-          P.A[i + c * ld] = a;
-          if (i == c) P.d[c] = a;
-          if (i >= c + 2) ss += a * a;
-        }
-      }
-      ss = block_sum(ss, scratch);
-      if (tid == 0 && ss != 0.0) atomicAdd(&R[0], ss);
+        pq[lane] = p;
+        pq[NB + lane] = q;
+        VWc[lane] = vc;
+        VWc[NB + lane] = wc;
+      };
+      double ss = 0.0;
+      rows(max(R0, c), jj, tprev, scalars, [&](int i, double v, double a) {
+        if (jj > 0 && i >= c + 1) P.A[i + (size_t)(c - 1) * ld] = v;
+        P.A[i + c * ld] = a;
+        if (i == c) P.d[c] = a;
+        if (i >= c + 2) ss += a * a;
+      });
+      ss += __shfl_xor_sync(0xffffffffu, ss, 1);  // of lanes 0 .. 3
+      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+      if (lane == 0) scratch[warp] = ss;
     }
-    if (grid_barrier(bar, nblocks, P.wait_log2)) {
+    auto add_sum = [&](double* r) {  // of the warps' sums in scratch
+      const double x = warp_sum(lane < nwarps ? scratch[lane] : 0.0);
+      if (lane == 0 && x != 0.0) atomicAdd(r, x);
+    };
+    if (grid_barrier(
+            bar, nblocks, 2 * jj + 1, P.wait_log2,
+            [&] {
+              if (act) add_sum(&R[0]);
+            },
+            [&] {
+              if (c < n - 1 && walk.live()) walk.load();
+            })) {
       // a wait gave up: end the launch and report it (the host throws)
       if (tid == 0) atomicExch(fail, 1);
       return;
@@ -177,75 +382,139 @@ __global__ void __launch_bounds__(TRD_NT) trd_panel_kernel(const TrdProb* __rest
       const double alpha = __ldcg(&P.A[c + 1 + c * ld]);
       const double xn2 = ld_volatile(&R[0]);
       double beta = alpha, tc = 0.0, scal = 0.0;
-      if (xn2 != 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-        tc = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
+      // W and V of this warp's first rows, on the way while v is formed
+      double wr[4], vr[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = max(R0, c + 1) + warp + u * nwarps;
+        wr[u] = i < R1 && lane < jj ? P.W[(size_t)i * NB + lane] : 0.0;
+        vr[u] = i < R1 && lane < jj ? P.Vp[(size_t)i * NB + lane] : 0.0;
+      }
+      for (int r0 = 0; r0 < S.mp; r0 += 8 * TRD_NT) {
+        double a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int r = r0 + tid + u * TRD_NT;
+          a[u] = (r > jj && r < S.M) ? __ldcg(&P.A[base + r + c * ld]) : 0.0;
+        }
+        if (r0 == 0 && xn2 != 0.0) {
+          beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
+          tc = (beta - alpha) / beta;
+          scal = 1.0 / (alpha - beta);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int r = r0 + tid + u * TRD_NT;
+          if (r < S.mp) vs[r] = r == jj ? 1.0 : a[u] * scal;
+        }
       }
       if (rank == 0 && tid == 0) {
         P.e[c] = beta;
         P.tau[c] = tc;
       }
       if (rank == 0 && tid < RED) Ro[tid] = 0.0;  // read in phase A, refilled from the next phase A on
-      const int m = n - c - 1;
-      for (int i = tid; i < m; i += TRD_NT) vs[i] = (i == 0) ? 1.0 : __ldcg(&P.A[c + 1 + i + c * ld]) * scal;
       __syncthreads();
-      const int chunk = (m + P.ncta - 1) / P.ncta;
-      const int r0 = c + 1 + rank * chunk, r1 = min(n, r0 + chunk);
-      for (int i = r0 + tid; i < r1; i += TRD_NT) {
-        const double vi = vs[i - c - 1];
-        P.v[i] = vi;
-        P.Vp[(size_t)i * NB + jj] = vi;
+      double sp = 0.0, sq = 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = max(R0, c + 1) + warp + u * nwarps;
+        if (i >= R1) break;
+        const double vi = vs[i - base];
+        sp += wr[u] * vi;
+        sq += vr[u] * vi;
+        if (lane == jj) P.Vp[(size_t)i * NB + jj] = vi;
       }
-      if (jj > 0) {
-        double sp = 0.0, sq = 0.0;
-        for (int i = r0 + warp; i < r1; i += nwarps) {
-          const double vi = vs[i - c - 1];
-          if (lane < jj) {
-            sp += __ldcg(&P.W[(size_t)i * NB + lane]) * vi;
-            sq += __ldcg(&P.Vp[(size_t)i * NB + lane]) * vi;
+      for (int i = max(R0, c + 1) + warp + 4 * nwarps; i < R1; i += nwarps) {
+        const double vi = vs[i - base];
+        if (lane < jj) {
+          sp += P.W[(size_t)i * NB + lane] * vi;
+          sq += P.Vp[(size_t)i * NB + lane] * vi;
+        }
+        if (lane == jj) P.Vp[(size_t)i * NB + jj] = vi;
+      }
+      pqw[warp * 2 * NB + lane] = sp;
+      pqw[warp * 2 * NB + NB + lane] = sq;
+      __syncthreads();
+      if (tid < 2 * NB && (tid & (NB - 1)) < jj) {
+        double a = 0.0;
+#pragma unroll
+        for (int w = 0; w < nwarps; ++w) a += pqw[w * 2 * NB + tid];
+        if (a != 0.0) atomicAdd(&R[2 + tid], a);
+      }
+      double yvp = 0.0, a0 = 0.0, a1 = 0.0;
+      // one strip; next() may overwrite x and move `at` on
+      auto strip = [&](const SymvWalk& at, double (&x)[16], auto&& next) {
+        const int I = at.I, J = at.J, r = at.row(), cc = at.col();
+        const bool ends = at.strip == SY_N / 8 - 1;
+        const double v0 = vs[r], v1 = vs[r + 32];
+        double b0 = 0.0, b1 = 0.0, t[8];
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          const double w0 = vs[cc + u], w1 = vs[cc + u + 1];
+          a0 += x[u] * w0;
+          a1 += x[8 + u] * w0;
+          b0 += x[u + 1] * w1;
+          b1 += x[9 + u] * w1;
+        }
+        a0 += b0;
+        a1 += b1;
+        if (at.below()) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) t[u] = x[u] * v0 + x[8 + u] * v1;
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const double p = x[u] * v0, q = x[8 + u] * v1;
+            t[u] = (cc + u == r ? 0.0 : p) + (cc + u == r + 32 ? 0.0 : q);
+            yvp -= (cc + u == r ? p * v0 : 0.0) + (cc + u == r + 32 ? q * v1 : 0.0);
           }
         }
-        pqw[warp * 2 * NB + lane] = sp;
-        pqw[warp * 2 * NB + NB + lane] = sq;
-        __syncthreads();
-        if (tid < jj) {
-          double a = 0.0, bq = 0.0;
-          for (int w = 0; w < nwarps; ++w) {
-            a += pqw[w * 2 * NB + tid];
-            bq += pqw[w * 2 * NB + NB + tid];
+        next();
+        // column sums over the lanes on the tensor core: product u adds the sums
+        // over groups of four lanes of column u to row u of an 8 x 8 accumulator
+        double e[2] = {0, 0}, o[2] = {0, 0};
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          dmma(e, (lane >> 2) == u ? 1.0 : 0.0, t[u]);
+          dmma(o, (lane >> 2) == u + 1 ? 1.0 : 0.0, t[u + 1]);
+        }
+        double cs = (e[0] + o[0]) + (e[1] + o[1]);
+        cs += __shfl_xor_sync(0xffffffffu, cs, 1);
+        cs += __shfl_xor_sync(0xffffffffu, cs, 2);
+        if (!(lane & 3)) yc[I * S.mp + cc + (lane >> 2)] = cs;
+        if (ends) {
+          yr[J * S.mp + r] = a0;
+          yr[J * S.mp + r + 32] = a1;
+          yvp += 2.0 * (a0 * v0 + a1 * v1);
+          a0 = a1 = 0.0;
+        }
+      };
+      if (jj > 0 && first.live()) {
+        SymvWalk at = first;
+        for (at.strip = 0; at.strip < nres; ++at.strip) {
+#pragma unroll
+          for (int u = 0; u < 16; ++u) at.x[u] = res[at.strip * 512 + 32 * u];
+          strip(at, at.x, [] {});
+        }
+      }
+      while (walk.live())
+        strip(walk, walk.x, [&] {
+          if (jj == 0 && walk.t == first.t && walk.strip < nres) {
+#pragma unroll
+            for (int u = 0; u < 16; ++u) res[walk.strip * 512 + 32 * u] = walk.x[u];
           }
-          if (a != 0.0) atomicAdd(&R[2 + tid], a);
-          if (bq != 0.0) atomicAdd(&R[2 + NB + tid], bq);
-        }
-      }
-      double yvp = 0.0;
-      for (int j = c + 1 + gw; j < n; j += tw) {
-        const double* col = P.A + (size_t)j * ld + (c + 1);
-        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        int i = lane;
-        for (; i + 480 < m; i += 512) {
-          double x[16];
-#pragma unroll
-          for (int u = 0; u < 16; ++u) x[u] = __ldcg(&col[i + 32 * u]);
-#pragma unroll
-          for (int u = 0; u < 16; ++u) s[u & 7] += x[u] * vs[i + 32 * u];
-        }
-        for (; i + 224 < m; i += 256) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) s[u] += __ldcg(&col[i + 32 * u]) * vs[i + 32 * u];
-        }
-        for (; i < m; i += 32) s[0] += __ldcg(&col[i]) * vs[i];
-        const double yj = warp_sum(((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
-        if (lane == 0) {
-          P.y[j] = yj;
-          yvp += yj * vs[j - c - 1];
-        }
-      }
-      yvp = block_sum(yvp, scratch);
-      if (tid == 0 && yvp != 0.0) atomicAdd(&R[1], yvp);
+          walk.advance();
+          if (walk.live()) walk.load();
+        });
+      yvp = warp_sum(yvp);
+      if (lane == 0) scratch[warp] = yvp;
     }
-    if (grid_barrier(bar, nblocks, P.wait_log2)) {
+    if (grid_barrier(
+            bar, nblocks, 2 * jj + 2, P.wait_log2,
+            [&] {
+              if (act && c < n - 1) add_sum(&R[1]);
+            },
+            [] {})) {
       // a wait gave up: end the launch and report it (the host throws)
       if (tid == 0) atomicExch(fail, 1);
       return;
@@ -257,27 +526,46 @@ __global__ void __launch_bounds__(TRD_NT) trd_panel_kernel(const TrdProb* __rest
   if (c < n - 1) {
     const double* R = P.red + (c & 1) * RED;
     const double tc = __ldcg(&P.tau[c]);
-    if (tid < NB) {
-      pq[tid] = (tid < NB - 1) ? ld_volatile(&R[2 + tid]) : 0.0;
-      pq[NB + tid] = (tid < NB - 1) ? ld_volatile(&R[2 + NB + tid]) : 0.0;
-    }
-    __syncthreads();
-    const double pk = pq[lane], qk = pq[NB + lane];
-    const double a2 = -0.5 * tc * tc * (ld_volatile(&R[1]) - 2.0 * warp_sum(pk * qk));
-    for (int i = c + 1 + gw; i < n; i += tw) {
-      double corr = 0.0;
-      if (lane < NB - 1)
-        corr = __ldcg(&P.Vp[(size_t)i * NB + lane]) * pk + __ldcg(&P.W[(size_t)i * NB + lane]) * qk;
-      corr = warp_sum(corr);
-      if (lane == 0) {
-        const double vi = __ldcg(&P.v[i]);
-        P.W[(size_t)i * NB + NB - 1] = tc * (__ldcg(&P.y[i]) - corr) + a2 * vi;
-        if (i >= c + 2) P.A[i + c * ld] = vi;
-      }
-    }
+    auto scalars = [&] {
+      const double p = (lane < NB - 1) ? ld_volatile(&R[2 + lane]) : 0.0, q = (lane < NB - 1) ? ld_volatile(&R[2 + NB + lane]) : 0.0;
+      const double a2 = -0.5 * tc * tc * (ld_volatile(&R[1]) - 2.0 * warp_sum(p * q));
+      pq[lane] = p;
+      pq[NB + lane] = q;
+      VWc[lane] = VWc[NB + lane] = 0.0;
+      if (lane == 0) misc[0] = a2;
+    };
+    rows(max(R0, c + 1), NB, tc, scalars, [&](int i, double v, double) {
+      if (i >= c + 2) P.A[i + c * ld] = v;
+    });
   }
   // a barrier that gave up is reported to the host (the barriers are reset per launch)
   if (tid == 0 && *reinterpret_cast<volatile int*>(&bar->error)) atomicExch(fail, 1);
+}
+
+// --------------------------------------------------------------------------
+// The upper triangle from the lower: the panels keep only the lower one, the
+// kernels that take the rest of a block read columns of both.
+// --------------------------------------------------------------------------
+struct MirrorProb {
+  double* A;
+  int n, ld;
+};
+
+constexpr int MIRROR_T = 32;
+
+__global__ void __launch_bounds__(256) mirror_kernel(const MirrorProb* __restrict__ probs) {
+  __shared__ double tile[MIRROR_T][MIRROR_T + 1];
+  const MirrorProb P = probs[blockIdx.z];
+  const int r0 = blockIdx.x * MIRROR_T, c0 = blockIdx.y * MIRROR_T;  // a tile on or below the diagonal
+  if (r0 >= P.n || c0 > r0) return;
+  const int x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+  for (int y = y0; y < MIRROR_T; y += 8)
+    if (r0 + x < P.n && c0 + y < P.n) tile[y][x] = P.A[r0 + x + (size_t)(c0 + y) * P.ld];
+  __syncthreads();
+  for (int y = y0; y < MIRROR_T; y += 8) {
+    const int r = r0 + y, c = c0 + x;  // of the lower triangle; written at (c, r)
+    if (r < P.n && c < r) P.A[c + (size_t)r * P.ld] = tile[x][y];
+  }
 }
 
 // A kernel's largest dynamic shared memory on the current device only grows:
@@ -916,7 +1204,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   int nmx = 0;
   for (int n : ns) nmx = std::max(nmx, n);
   // per-panel launch descriptors
-  pl.add<char>((size_t)(nmx / NB + 2) * (ns.size() * (sizeof(TrdProb) + 2 * sizeof(GemmSeg) + sizeof(GemmProb)) + 2048));
+  pl.add<char>((size_t)(nmx / NB + 2) * (ns.size() * (sizeof(TrdProb) + (size_t)(nmx / TRAIL_STRIP + 1) * (2 * sizeof(GemmSeg) + sizeof(GemmProb))) + 2048));
   // zero-fill descriptors: the per-problem buffers once, the split-K
   // outputs of the back-transformation once; cluster descriptors
   size_t zs = 0;
@@ -937,6 +1225,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
                256 * 6 * (size_t)(nmx / NBB + 4));
   pl.add<TrdClProb>(2 * ns.size() + 16);
   pl.add<TrdGridProb>(ns.size() + 16);
+  pl.add<MirrorProb>(ns.size() + 16);
   pl.add<BtSlabProb>(ns.size() + 16);
   return pl.bytes + (size_t)ns.size() * 4096 + (1 << 20);
 }
@@ -1020,8 +1309,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       t.tau = tauT[b];
       t.Vp = Vp;
       t.W = Wp;
-      t.v = vec + 3 * n;
-      t.y = vec + 4 * n;
+      t.y = W1;  // free until divide and conquer
       t.red = red;
       t.n = n;
       DcProb& q = dp[b];
@@ -1137,12 +1425,11 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       launch_clusters(whole);
     }
     {
-      const size_t smem = (size_t)(32 + 4 * NB + 8 + (TRD_NT / 32) * 2 * NB + nmax) * sizeof(double);
-      NRGB_CUDA(raise_smem_attr((const void*)trd_panel_kernel, (int)smem));
-      int per_sm = 0;
-      NRGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trd_panel_kernel, TRD_NT, smem));
-      per_sm = std::max(1, std::min(per_sm, 4));
-      const int cap = per_sm * sms_;
+      constexpr size_t SMEM_CAP = 227 * 1024 - 64;
+      const bool v_smem = ((size_t)TRD_SMEM + SymvShape(nmax).mp) * sizeof(double) <= SMEM_CAP;
+      const void* panel = v_smem ? (const void*)trd_panel_kernel<true> : (const void*)trd_panel_kernel<false>;
+      NRGB_CUDA(raise_smem_attr(panel, (int)SMEM_CAP));
+      const int cap = sms_;  // one CTA per SM: few to synchronise, and v formed once per SM
       // One cooperative launch per panel of NB columns.  All problems advance
       // column by column in lockstep, so a column costs the maximum over
       // problems of (trailing size)^2 / CTAs: the CTAs of each launch are
@@ -1174,7 +1461,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
             t.expect_extra = inject_shortfall_ ? 1 : 0;
             const double w = pow((double)(t.n - j0), 2.0) / wsum;
             int nc = 1 + (int)floor(w * extra);
-            nc = std::min(nc, std::max(1, (t.n - j0) / 8));
+            nc = std::min(nc, std::max(1, (t.n - j0) / (TRD_NT / 32)));
             t.cta0 = tot;
             t.ncta = nc;
             tot += nc;
@@ -1185,54 +1472,73 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           int np_ = cnt;
           int j0_ = j0;
           int* fail = d_err_ + 3;
-          void* args[] = {(void*)&d_tp, (void*)&np_, (void*)&j0_, (void*)&fail};
+          int mrows = 0;
+          for (const TrdProb& t : sub) mrows = std::max(mrows, t.n - j0 - 1);
+          const size_t fixed = ((size_t)TRD_SMEM + (v_smem ? SymvShape(mrows).mp : 0)) * sizeof(double);
+          constexpr size_t STRIP_BYTES = (size_t)(TRD_NT / 32) * 512 * sizeof(double);  // of every warp
+          int nres = (int)std::min<size_t>(SY_N / 8, (SMEM_CAP - fixed) / STRIP_BYTES);
+          const size_t smem = fixed + nres * STRIP_BYTES;
+          void* args[] = {(void*)&d_tp, (void*)&np_, (void*)&j0_, (void*)&nres, (void*)&fail};
           {
-            // algorithmic bytes: column c reads its trailing (n-c-1)^2 block once
+            // algorithmic bytes: column c reads the lower triangle of its trailing block once
             double wb = 0;
             for (const TrdProb& t : sub)
-              for (int c = j0; c < std::min(j0 + NB, t.n - 1); ++c) wb += 8.0 * (double)(t.n - c - 1) * (t.n - c - 1);
+              for (int c = j0; c < std::min(j0 + NB, t.n - 1); ++c) wb += 4.0 * (double)(t.n - c - 1) * (t.n - c);
             KernelStats::get().add_work("trd_panel", wb);
           }
           NRGB_LAUNCH("trd_panel", st,
-                      NRGB_CUDA(cudaLaunchCooperativeKernel((void*)trd_panel_kernel, dim3(tot), dim3(TRD_NT),
+                      NRGB_CUDA(cudaLaunchCooperativeKernel(panel, dim3(tot), dim3(TRD_NT),
                                                             args, smem, st)));
           ++launches_;
-          // trailing update A22 -= V W^T + W V^T for rows/cols >= j0+NB
+          // trailing update A22 -= V W^T + W V^T for rows/cols >= j0+NB of the
+          // lower triangle, in strips of columns
           GemmBatch gb;
           for (const TrdProb& t : sub) {
             const int n = t.n;
-            const int r0 = j0 + NB;
-            if (r0 >= n) continue;
-            const int m2 = n - r0;
-            // Vp, W are row-major n x NB: as column-major matrices they are
-            // NB x n with ld NB, so op(A) = stored^T and op(B) = stored.
-            GemmSeg s1{}, s2{};
-            s1.A = t.Vp + (size_t)r0 * NB;
-            s1.lda = NB;
-            s1.B = t.W + (size_t)r0 * NB;
-            s1.ldb = NB;
-            s1.k = NB;
-            s1.transA = 1;
-            s1.transB = 0;
-            s1.alpha = -1.0;
-            s2 = s1;
-            s2.A = t.W + (size_t)r0 * NB;
-            s2.B = t.Vp + (size_t)r0 * NB;
-            gb.add(t.A + r0 + (size_t)r0 * n, n, m2, m2, 1.0, {s1, s2});
+            for (int r0 = j0 + NB; r0 < n; r0 += TRAIL_STRIP) {
+              // Vp, W are row-major n x NB: as column-major matrices they are
+              // NB x n with ld NB, so op(A) = stored^T and op(B) = stored.
+              GemmSeg s1{}, s2{};
+              s1.A = t.Vp + (size_t)r0 * NB;
+              s1.lda = NB;
+              s1.B = t.W + (size_t)r0 * NB;
+              s1.ldb = NB;
+              s1.k = NB;
+              s1.transA = 1;
+              s1.transB = 0;
+              s1.alpha = -1.0;
+              s2 = s1;
+              s2.A = t.W + (size_t)r0 * NB;
+              s2.B = t.Vp + (size_t)r0 * NB;
+              gb.add(t.A + r0 + (size_t)r0 * n, n, n - r0, std::min(TRAIL_STRIP, n - r0), 1.0, {s1, s2});
+            }
           }
           if (!gb.empty()) {
-            GemmProb* d_gp = arena_.alloc_n<GemmProb>(gb.probs.size());
-            GemmSeg* d_gs = arena_.alloc_n<GemmSeg>(gb.segs.size());
-            NRGB_CUDA(cudaMemcpyAsync(d_gp, gb.probs.data(), gb.probs.size() * sizeof(GemmProb),
-                                      cudaMemcpyHostToDevice, st));
-            NRGB_CUDA(cudaMemcpyAsync(d_gs, gb.segs.data(), gb.segs.size() * sizeof(GemmSeg),
-                                      cudaMemcpyHostToDevice, st));
             KernelStats::get().add_work("gemm_f64_trailing",
                                         gemm_flops(gb.probs.data(), (int)gb.probs.size(), gb.segs.data()));
-            NRGB_CUDA(gemm_grouped_launch(d_gp, (int)gb.probs.size(), d_gs, gb.tiles, st, "gemm_f64_trailing", gb.stiles));
+            NRGB_CUDA(gemm_grouped_launch_host(gb.probs.data(), (int)gb.probs.size(), gb.segs.data(), (int)gb.segs.size(),
+                                               gb.tiles, st, "gemm_f64_trailing", gb.stiles, arena_));
             ++launches_;
           }
         }
+      }
+    }
+    {
+      std::vector<MirrorProb> mp;
+      int mm = 0;
+      for (int b = 0; b < nbig; ++b) {
+        const int j = jstop[b], n = tp[b].n;
+        if (via_cluster[b] || j == 0 || j >= n) continue;
+        mp.push_back(MirrorProb{tp[b].A + j + (size_t)j * n, n - j, n});
+        mm = std::max(mm, n - j);
+      }
+      if (!mp.empty()) {
+        MirrorProb* d_mp = arena_.alloc_n<MirrorProb>(mp.size());
+        NRGB_CUDA(cudaMemcpyAsync(d_mp, mp.data(), mp.size() * sizeof(MirrorProb), cudaMemcpyHostToDevice, st));
+        const unsigned g = (unsigned)((mm + MIRROR_T - 1) / MIRROR_T);
+        NRGB_LAUNCH("trd_mirror", st, mirror_kernel<<<dim3(g, g, (unsigned)mp.size()), 256, 0, st>>>(d_mp));
+        NRGB_CUDA(cudaGetLastError());
+        ++launches_;
       }
     }
     // the blocks A[j:, j:] (j = jstop, fully updated by the last trailing
