@@ -59,11 +59,66 @@ struct DevMat {
 };
 using DevBlocks = std::map<Twoinvar, DevMat>;
 
-// Device bytes held by the slabs of one run (current and peak).
+// The device memory of one run's slabs: bytes held (current and peak, including
+// the chunks kept for reuse) and the chunks that slabs gave back.  Every step
+// frees and allocates its slabs anew, and the allocator's default pool returns
+// free memory to the device at each synchronisation; mapping it again took 30 ms
+// of a run of 190.  The chunks kept are at most KEEP bytes, are used by the run's
+// own stream alone (so that reuse is ordered with the work before it) and are
+// freed at the end of the run.
 struct MemCount {
+  static constexpr size_t KEEP = size_t(256) << 20;
   size_t cur = 0, peak = 0;
+  size_t kept = 0;
+  std::vector<std::pair<void*, size_t>> chunks;
+
+  // A chunk of at least sz bytes; its size in sz.
+  void* take(size_t& sz, cudaStream_t st) {
+    size_t best = chunks.size();
+    for (size_t i = 0; i < chunks.size(); ++i)
+      if (chunks[i].second >= sz && chunks[i].second <= 2 * sz && (best == chunks.size() || chunks[i].second < chunks[best].second))
+        best = i;
+    if (best < chunks.size()) {
+      void* p = chunks[best].first;
+      sz = chunks[best].second;
+      kept -= sz;
+      chunks[best] = chunks.back();
+      chunks.pop_back();
+      return p;
+    }
+    void* p = nullptr;
+    cudaError_t e = cudaMallocAsync(&p, sz, st);
+    if (e == cudaErrorMemoryAllocation && !chunks.empty()) {
+      cudaGetLastError();
+      clear(st);
+      NRGB_CUDA(cudaStreamSynchronize(st));
+      e = cudaMallocAsync(&p, sz, st);
+    }
+    NRGB_CUDA(e);
+    cur += sz;
+    peak = std::max(peak, cur);
+    return p;
+  }
+  void give(void* p, size_t sz, cudaStream_t st) {
+    if (kept + sz <= KEEP) {
+      chunks.push_back({p, sz});
+      kept += sz;
+    } else {
+      cudaFreeAsync(p, st);
+      cur -= sz;
+    }
+  }
+  void clear(cudaStream_t st) {
+    for (auto& c : chunks) {
+      cudaFreeAsync(c.first, st);
+      cur -= c.second;
+    }
+    chunks.clear();
+    kept = 0;
+  }
 };
-// The run executing on this host thread (set for the duration of run()).
+
+// The run whose slabs are made on this host thread (set for the duration of run()).
 thread_local MemCount* tl_mem = nullptr;
 
 // Stream-ordered device memory owned by one generation of data.  Requests
@@ -80,16 +135,13 @@ class Slab {
     if (n == 0) return nullptr;
     const size_t bytes = (n * sizeof(double) + 255) & ~size_t(255);
     if (chunks_.empty() || off_ + bytes > chunks_.back().second) {
-      const size_t sz = std::max(bytes, next_);
+      size_t sz = std::max(bytes, next_);
       next_ = std::min(next_ * 2, size_t(64) << 20);
       void* p = nullptr;
-      NRGB_CUDA(cudaMallocAsync(&p, sz, st_));
+      if (mc_) p = mc_->take(sz, st_);
+      else NRGB_CUDA(cudaMallocAsync(&p, sz, st_));
       chunks_.push_back({p, sz});
       off_ = 0;
-      if (mc_) {
-        mc_->cur += sz;
-        mc_->peak = std::max(mc_->peak, mc_->cur);
-      }
     }
     char* p = static_cast<char*>(chunks_.back().first) + off_;
     off_ += bytes;
@@ -97,8 +149,8 @@ class Slab {
   }
   void release() {
     for (auto& c : chunks_) {
-      cudaFreeAsync(c.first, st_);
-      if (mc_) mc_->cur -= c.second;
+      if (mc_) mc_->give(c.first, c.second, st_);
+      else cudaFreeAsync(c.first, st_);
     }
     chunks_.clear();
     off_ = 0;
@@ -192,6 +244,7 @@ std::string fmt_g(double x, int prec) {
 }  // namespace
 
 struct NrgDriver::Impl {
+  MemCount mem;  // before everything that holds slabs
   cudaStream_t st;
   EigSolver* syev;
   Params P;
@@ -278,12 +331,12 @@ struct NrgDriver::Impl {
     tstate.map_cap = cap;
   }
 
-  MemCount mem;
   double eig_calls = 0;
   std::vector<double> wstage;  // host staging of per-step eigenvalue uploads
 
   Impl(cudaStream_t s, EigSolver* e) : st(s), syev(e) {}
   ~Impl() {
+    release_run_data();
     free_trunc();
     cudaStreamSynchronize(st);
     if (desc_pin) cudaFreeHost(desc_pin);
@@ -980,6 +1033,7 @@ struct NrgDriver::Impl {
   // ---------------- density matrices ----------------
   std::map<int, DevBlocks> rho, rhofdm;
   std::vector<double> ZnD, wn, wnfactor;
+  std::vector<std::vector<long double>> boltz;  // per step: exp(-E/T) of the discarded states, block after block
   std::vector<std::unique_ptr<Slab>> rho_slabs;
 
   DevMat diag_matrix(const std::vector<double>& d, Slab& slab) {
@@ -1036,6 +1090,19 @@ struct NrgDriver::Impl {
     Slab tmp(st);
     std::vector<ColScale> cs;
     int maxr = 0, maxc = 0;
+    // the diagonals of all blocks in one copy
+    std::map<Invar, double*> dpos;
+    if (dd) {
+      std::vector<double> all;
+      std::vector<size_t> at;
+      for (const auto& kv : *dd) {
+        at.push_back(all.size());
+        all.insert(all.end(), kv.second.begin(), kv.second.end());
+      }
+      double* p = upload(all);
+      size_t k = 0;
+      for (const auto& kv : *dd) dpos[kv.first] = p + at[k++];
+    }
     for (const auto& kv : Sp.blocks) {
       const Invar& I = kv.first;
       const int dim = kv.second.kept;
@@ -1069,10 +1136,7 @@ struct NrgDriver::Impl {
             const int lo = Bc.kept, hi = Bc.dim;
             if (hi > lo) {
               double* T = tmp.alloc((size_t)dim * (hi - lo));
-              double* s = tmp.alloc(hi - lo);
-              NRGB_CUDA(cudaMemcpyAsync(s, di->second.data() + lo, (hi - lo) * sizeof(double), cudaMemcpyHostToDevice, st));
-              h2d += (hi - lo) * sizeof(double);
-              cs.push_back(ColScale{Zs + (size_t)lo * Bc.dim, T, s, dim, hi - lo, Bc.dim, dim});
+              cs.push_back(ColScale{Zs + (size_t)lo * Bc.dim, T, dpos.at(child) + lo, dim, hi - lo, Bc.dim, dim});
               maxr = std::max(maxr, dim);
               maxc = std::max(maxc, hi - lo);
               ss.push_back(seg(T, dim, 0, Zs + (size_t)lo * Bc.dim, Bc.dim, 1, hi - lo, coef));
@@ -1121,13 +1185,18 @@ struct NrgDriver::Impl {
 
   void calc_ZnD() {
     ZnD.assign(Nmax, 0.0);
+    boltz.assign(Nmax, {});
     for (int N = Ninit; N < Nmax; ++N) {
       long double Z = 0;
       for (const auto& kv : steps[N - Ninit].blocks) {
         const int lo = last(N) ? 0 : kv.second.kept;
         for (int i = lo; i < kv.second.dim; ++i) {
           const long double Eabs = kv.second.absE[i] - GSenergy;
-          Z += sym->mult(kv.first) * expl(-Eabs / P.T);
+          // below the smallest subnormal (exp(-11399)) the result is zero; the
+          // library takes its slow path there
+          const long double x = -Eabs / P.T, b = x < -11500.0L ? 0.0L : expl(x);
+          boltz[N].push_back(b);
+          Z += sym->mult(kv.first) * b;
         }
       }
       ZnD[N] = (double)Z;
@@ -1149,15 +1218,16 @@ struct NrgDriver::Impl {
 
   std::map<Invar, std::vector<double>> rho_fdm_diag(int N) {
     std::map<Invar, std::vector<double>> out;
+    const long double w = (long double)wn[N] / ZnD[N];
+    size_t q = 0;
     for (const auto& kv : steps[N - Ninit].blocks) {
       std::vector<double> d(kv.second.dim, 0.0);
       const int lo = last(N) ? 0 : kv.second.kept;
       for (int i = lo; i < kv.second.dim; ++i) {
-        const long double Eabs = kv.second.absE[i] - GSenergy;
-        long double v = expl(-Eabs / P.T) * ((long double)wn[N] / ZnD[N]);
+        const long double v = boltz[N][q++] * w;
         d[i] = std::isfinite((double)v) ? (double)v : 0.0;
       }
-      out[kv.first] = d;
+      out[kv.first] = std::move(d);
     }
     return out;
   }
@@ -1541,11 +1611,14 @@ struct NrgDriver::Impl {
     rhofdm.clear();
     rho_slabs.clear();
     steps.clear();
+    expv_slab.reset();
+    boltz.clear();
+    mem.clear(st);
   }
 
   void run(const std::string& wd, const std::string& od, double* stats, RunExtra* extra) {
     release_run_data();
-    mem = MemCount();
+    mem.cur = mem.peak = 0;
     eig_calls = 0;
     struct MemScope {
       explicit MemScope(MemCount* m) { tl_mem = m; }
