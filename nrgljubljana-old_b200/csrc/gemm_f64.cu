@@ -307,8 +307,11 @@ struct Operand {
   }
 };
 
-// The products of one K step; FL: bit 0 A k-contiguous, bit 1 B k-contiguous.
-template <int T, int FL>
+// The products of one K step; FL: bit 0 A k-contiguous, bit 1 B k-contiguous;
+// SC: A is scaled by alpha.  (A test of alpha between the loads and the products
+// kept the compiler from loading ahead: 29.5 TF/s on 37 products of edge 1024,
+// 32.5 without scaling, 29.2 with.)
+template <int T, bool SC, int FL>
 __device__ __forceinline__ void tile_step(double (&acc)[T / 16][T / 16][2], const double* as, const double* bs,
                                           double alpha, int wm, int wn, int g, int tq, const int (&ko)[4]) {
   constexpr int W = T / 16;
@@ -321,14 +324,17 @@ __device__ __forceinline__ void tile_step(double (&acc)[T / 16][T / 16][2], cons
     for (int i = 0; i < W; ++i) a[i] = (FL & 1) ? ap[ko[kk / 4] + i * 8 * KB] : ap[kk * (T + 4) + i * 8];
 #pragma unroll
     for (int j = 0; j < W; ++j) b[j] = (FL & 2) ? bp[ko[kk / 4] + j * 8 * KB] : bp[kk * (T + 4) + j * 8];
-    if (alpha != 1.0) {
+    if constexpr (SC) {
 #pragma unroll
       for (int i = 0; i < W; ++i) a[i] *= alpha;
     }
 #pragma unroll
     for (int i = 0; i < W; ++i)
 #pragma unroll
-      for (int j = 0; j < W; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+      for (int q = 0; q < W; ++q) {
+        const int j = (i & 1) ? W - 1 - q : q;  // back and forth: one fragment stays
+        dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+      }
   }
 }
 
@@ -345,7 +351,7 @@ __device__ __forceinline__ int find_problem(const GemmProb* probs, int nprob, in
   return lo;
 }
 
-template <int T>
+template <int T, bool SC>
 __device__ __forceinline__ void gemm_tile(const GemmProb* __restrict__ probs, int nprob, const GemmSeg* __restrict__ segs,
                                           const int* const* __restrict__ cmaps) {
   constexpr int W = T / 16, PT = ptile<T>(), SUB = 64 / T;  // SUB^2 CTAs share a 64 x 64 tile
@@ -353,7 +359,7 @@ __device__ __forceinline__ void gemm_tile(const GemmProb* __restrict__ probs, in
   double* As = psm;                 // [STAGES][PT]
   double* Bs = psm + STAGES * PT;   // [STAGES][PT]
   __shared__ double salpha[STAGES];
-  __shared__ int sflags[STAGES];    // bit 0: A k-contiguous, bit 1: B k-contiguous
+  __shared__ int sflags[STAGES];    // see tile_step
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x / (SUB * SUB), sub = blockIdx.x % (SUB * SUB);
@@ -438,10 +444,10 @@ __device__ __forceinline__ void gemm_tile(const GemmProb* __restrict__ probs, in
     const double* bs = Bs + stg * PT;
     const double alpha = salpha[stg];
     switch (sflags[stg]) {
-      case 0: tile_step<T, 0>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
-      case 1: tile_step<T, 1>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
-      case 2: tile_step<T, 2>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
-      default: tile_step<T, 3>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      case 0: tile_step<T, SC, 0>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      case 1: tile_step<T, SC, 1>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      case 2: tile_step<T, SC, 2>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
+      default: tile_step<T, SC, 3>(acc, as, bs, alpha, wm, wn, g, tq, ko); break;
     }
     stg = stg + 1 == STAGES ? 0 : stg + 1;
     nxt = nxt + 1 == STAGES ? 0 : nxt + 1;
@@ -471,12 +477,12 @@ __device__ __forceinline__ void gemm_tile(const GemmProb* __restrict__ probs, in
 }
 
 // 128 registers at most, so that shared memory alone sets the CTAs per SM
-// (52 KB each with T = 64: four).
-template <int T>
+// (52 KB each with T = 64: four).  SC: some segment's alpha is not one.
+template <int T, bool SC>
 __global__ void __launch_bounds__(NT, T == 64 ? 4 : 6) gemm_grouped_pipe_kernel(const GemmProb* __restrict__ probs, int nprob,
                                                                   const GemmSeg* __restrict__ segs,
                                                                   const int* const* __restrict__ cmaps) {
-  gemm_tile<T>(probs, nprob, segs, cmaps);
+  gemm_tile<T, SC>(probs, nprob, segs, cmaps);
 }
 
 // The descriptors of a small launch as a kernel parameter: problems, then segments.
@@ -484,11 +490,11 @@ template <int BYTES>
 struct InlineDesc {
   alignas(16) unsigned char b[BYTES];
 };
-template <int T, int BYTES>
+template <int T, bool SC, int BYTES>
 __global__ void __launch_bounds__(NT, T == 64 ? 4 : 6) gemm_grouped_inline_kernel(const __grid_constant__ InlineDesc<BYTES> d,
                                                                     int nprob) {
   const GemmProb* probs = reinterpret_cast<const GemmProb*>(d.b);
-  gemm_tile<T>(probs, nprob, reinterpret_cast<const GemmSeg*>(probs + nprob), nullptr);
+  gemm_tile<T, SC>(probs, nprob, reinterpret_cast<const GemmSeg*>(probs + nprob), nullptr);
 }
 
 template <int T>
@@ -505,12 +511,18 @@ cudaError_t pipe_attributes() {
   auto one = [&](auto* k, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  one(gemm_grouped_pipe_kernel<64>, pipe_smem<64>());
-  one(gemm_grouped_pipe_kernel<32>, pipe_smem<32>());
-  one(gemm_grouped_inline_kernel<64, 4096>, pipe_smem<64>());
-  one(gemm_grouped_inline_kernel<32, 4096>, pipe_smem<32>());
-  one(gemm_grouped_inline_kernel<64, GEMM_INLINE_MAX>, pipe_smem<64>());
-  one(gemm_grouped_inline_kernel<32, GEMM_INLINE_MAX>, pipe_smem<32>());
+  auto both = [&](auto* plain, auto* scaled, size_t bytes) {
+    one(plain, bytes);
+    one(scaled, bytes);
+  };
+  both(gemm_grouped_pipe_kernel<64, false>, gemm_grouped_pipe_kernel<64, true>, pipe_smem<64>());
+  both(gemm_grouped_pipe_kernel<32, false>, gemm_grouped_pipe_kernel<32, true>, pipe_smem<32>());
+  both(gemm_grouped_inline_kernel<64, false, 4096>, gemm_grouped_inline_kernel<64, true, 4096>, pipe_smem<64>());
+  both(gemm_grouped_inline_kernel<32, false, 4096>, gemm_grouped_inline_kernel<32, true, 4096>, pipe_smem<32>());
+  both(gemm_grouped_inline_kernel<64, false, GEMM_INLINE_MAX>, gemm_grouped_inline_kernel<64, true, GEMM_INLINE_MAX>,
+       pipe_smem<64>());
+  both(gemm_grouped_inline_kernel<32, false, GEMM_INLINE_MAX>, gemm_grouped_inline_kernel<32, true, GEMM_INLINE_MAX>,
+       pipe_smem<32>());
   if (e == cudaSuccess && dev < 64) set[dev].store(true, std::memory_order_release);
   return e;
 }
@@ -524,13 +536,13 @@ cudaError_t pipe_attributes() {
 bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || total_tiles <= 60L * nprob; }
 
 cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
-                        cudaStream_t stream, const int* const* cmaps) {
+                        cudaStream_t stream, const int* const* cmaps, bool scaled) {
   const cudaError_t e = pipe_attributes();
   if (e != cudaSuccess) return e;
-  if (use_small_tiles(total_tiles, nprob))
-    gemm_grouped_pipe_kernel<32><<<4 * total_tiles, NT, pipe_smem<32>(), stream>>>(d_probs, nprob, d_segs, cmaps);
-  else
-    gemm_grouped_pipe_kernel<64><<<total_tiles, NT, pipe_smem<64>(), stream>>>(d_probs, nprob, d_segs, cmaps);
+  const bool small = use_small_tiles(total_tiles, nprob);
+  const auto k = small ? (scaled ? gemm_grouped_pipe_kernel<32, true> : gemm_grouped_pipe_kernel<32, false>)
+                       : (scaled ? gemm_grouped_pipe_kernel<64, true> : gemm_grouped_pipe_kernel<64, false>);
+  k<<<(small ? 4 : 1) * total_tiles, NT, small ? pipe_smem<32>() : pipe_smem<64>(), stream>>>(d_probs, nprob, d_segs, cmaps);
   return cudaGetLastError();
 }
 
@@ -540,12 +552,13 @@ cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs,
   InlineDesc<BYTES> d;
   memcpy(d.b, probs, nprob * sizeof(GemmProb));
   memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
-  if (use_small_tiles(total_tiles, nprob))
-    gemm_grouped_inline_kernel<32, BYTES><<<4 * total_tiles, NT, pipe_smem<32>(), stream>>>(d, nprob);
-  else
-    gemm_grouped_inline_kernel<64, BYTES><<<total_tiles, NT, pipe_smem<64>(), stream>>>(d, nprob);
+  const bool small = use_small_tiles(total_tiles, nprob), scaled = gemm_scaled(segs, nseg);
+  const auto k = small ? (scaled ? gemm_grouped_inline_kernel<32, true, BYTES> : gemm_grouped_inline_kernel<32, false, BYTES>)
+                       : (scaled ? gemm_grouped_inline_kernel<64, true, BYTES> : gemm_grouped_inline_kernel<64, false, BYTES>);
+  k<<<(small ? 4 : 1) * total_tiles, NT, small ? pipe_smem<32>() : pipe_smem<64>(), stream>>>(d, nprob);
   return cudaGetLastError();
 }
+
 // The 128x128 cp.async variant is used only where the device's schedule
 // (schedule.cuh, set by the autotuner's measurements) says it wins: by
 // default never (measured on B200 at first: 21-25 TF/s against 25-28 TF/s
@@ -563,6 +576,12 @@ void gemm_assign_tiles(GemmProb& p, int& tiles, int& stiles) {
   stiles += ((p.m + LBM - 1) / LBM) * p.stiles_n * ks;
 }
 
+bool gemm_scaled(const GemmSeg* segs, int nseg) {
+  for (int s = 0; s < nseg; ++s)
+    if (segs[s].alpha != 1.0) return true;
+  return false;
+}
+
 double gemm_flops(const GemmProb* probs, int nprob, const GemmSeg* segs) {
   double f = 0;
   for (int p = 0; p < nprob; ++p)
@@ -573,7 +592,7 @@ double gemm_flops(const GemmProb* probs, int nprob, const GemmSeg* segs) {
 
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                 int total_tiles, cudaStream_t stream, const char* tag, int total_stiles,
-                                const int* const* cmaps) {
+                                const int* const* cmaps, bool scaled) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
   // 128x128 tiles when the schedule selects them for this problem size,
   // they cover at most 30% more area than the 64x64 ones and they still give
@@ -598,14 +617,14 @@ cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSe
     return cudaGetLastError();
   }
   cudaError_t e = cudaSuccess;
-  NRGB_LAUNCH(tag, stream, e = pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, cmaps));
+  NRGB_LAUNCH(tag, stream, e = pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, cmaps, scaled));
   return e;
 }
 
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                            int total_tiles, cudaStream_t stream) {
+                                            int total_tiles, cudaStream_t stream, bool scaled) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
-  return pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, nullptr);
+  return pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, nullptr, scaled);
 }
 
 size_t gemm_desc_bytes(int nprob, int nseg) {
@@ -624,7 +643,7 @@ cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const Gem
   GemmSeg* ds = scratch.alloc_n<GemmSeg>(nseg);
   if ((e = cudaMemcpyAsync(dp, probs, nprob * sizeof(GemmProb), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(ds, segs, nseg * sizeof(GemmSeg), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
-  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles);
+  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles, nullptr, gemm_scaled(segs, nseg));
 }
 
 bool gemm_inline_fits(int nprob, int nseg) {

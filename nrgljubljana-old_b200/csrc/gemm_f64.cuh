@@ -54,14 +54,15 @@ void gemm_assign_tiles(GemmProb& p, int& tiles, int& stiles);
 // problems are large enough that the bigger tiles waste little work.
 // cmaps (device, a pointer per problem; null: none): column j of problem p's
 // product goes to column cmaps[p][j] of its C.
+// scaled: some segment's alpha may differ from one (gemm_scaled).
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
                                 int total_tiles, cudaStream_t stream, const char* tag = "gemm_f64",
-                                int total_stiles = 0, const int* const* cmaps = nullptr);
+                                int total_stiles = 0, const int* const* cmaps = nullptr, bool scaled = true);
 
 // Same launch without the library's launch accounting (no host bookkeeping,
 // no events): used by the allocation-free entry point.
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                            int total_tiles, cudaStream_t stream);
+                                            int total_tiles, cudaStream_t stream, bool scaled);
 
 // The same with the descriptors in host memory, passed as a kernel parameter
 // (gemm_inline_fits: up to GEMM_INLINE_MAX bytes): no copy to the device.
@@ -76,6 +77,9 @@ cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const G
 size_t gemm_desc_bytes(int nprob, int nseg);
 cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
                                      cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch);
+
+// Some alpha differs from one.
+bool gemm_scaled(const GemmSeg* segs, int nseg);
 
 // Algorithmic flops of a grouped launch described on the host
 // (sum over problems and their segments of 2 m n k); for the launch

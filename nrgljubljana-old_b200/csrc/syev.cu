@@ -1738,7 +1738,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         NRGB_LAUNCH("dc_vectors", st, dc_vectors_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes));
         NRGB_CUDA(cudaGetLastError());
         NRGB_CUDA(gemm_grouped_launch(d_gp, nn, d_gs, L.gb.tiles, st, "gemm_f64_dc", L.gb.stiles,
-                                      reinterpret_cast<const int* const*>(dev + L.o_cm)));
+                                      reinterpret_cast<const int* const*>(dev + L.o_cm), false));
         launches_ += 7;
       }
       // problems that are a single leaf already have D, Q in place
@@ -1792,7 +1792,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           if (xsplit(mrows) > 1) zero_add(bz, xslot(b, k), (long long)NBB * n);
         }
       }
-      // per block k (descending): X_k = V_k^T Z, Y = T_k X_k, Z -= V_k Y
+      // per block k (descending): X_k = V_k^T Z, Y = -T_k X_k, Z += V_k Y
       struct Step {
         GemmBatch gx, gy, gz;
       };
@@ -1824,7 +1824,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           t.ldb = NBB;
           t.transB = 0;
           t.k = nb;
-          t.alpha = 1.0;
+          t.alpha = -1.0;
           S.gy.add(bt_Y[bp_of[b]], NBB, nb, n, 0.0, {t});
           GemmSeg u{};
           u.A = P.V + r0 + (size_t)j0 * n;
@@ -1834,7 +1834,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           u.ldb = NBB;
           u.transB = 0;
           u.k = nb;
-          u.alpha = -1.0;
+          u.alpha = 1.0;
           S.gz.add(Z + r0, n, mrows, n, 1.0, {u});
         }
       }
@@ -1859,7 +1859,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         KernelStats::get().add_work("gemm_f64_bt", gemm_flops(g.probs.data(), (int)g.probs.size(), g.segs.data()));
         NRGB_CUDA(gemm_grouped_launch(reinterpret_cast<const GemmProb*>(dev + o.first), (int)g.probs.size(),
                                       reinterpret_cast<const GemmSeg*>(dev + o.second), g.tiles, st, "gemm_f64_bt",
-                                      g.stiles));
+                                      g.stiles, nullptr, gemm_scaled(g.segs.data(), (int)g.segs.size())));
         ++launches_;
       };
       if (kmax > 0) {
