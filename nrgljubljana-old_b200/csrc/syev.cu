@@ -1198,7 +1198,9 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
     pl.add<double>(trd_grid_exchange(n));
     pl.add<double>((size_t)NBB * NBB * std::max(1, bt_nblk(n)));  // G
     pl.add<double>((size_t)NBB * NBB * std::max(1, bt_nblk(n)));  // T
-    pl.add<double>((size_t)NBB * n * 2);                          // X (last block), Y
+    pl.add<double>((size_t)NBB * n * 2);                          // X (last pair)
+    pl.add<double>((size_t)NBB * n * 2);                          // Y
+    pl.add<double>((size_t)NBB * NBB * ((std::max(1, bt_nblk(n)) + 1) / 2));  // G12
   }
   pl.add<double>(64 * 1024);
   int nmx = 0;
@@ -1209,7 +1211,7 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   // outputs of the back-transformation once; cluster descriptors
   size_t zs = 0;
   for (int n : ns)
-    zs += 8 + (size_t)n * n / ZERO_CHUNK + trd_grid_exchange(n) / ZERO_CHUNK + (size_t)NBB * NBB * bt_nblk(n) / ZERO_CHUNK +
+    zs += 8 + (size_t)n * n / ZERO_CHUNK + trd_grid_exchange(n) / ZERO_CHUNK + 2 * ((size_t)NBB * NBB / ZERO_CHUNK + 1) * bt_nblk(n) +
           (NBB * (size_t)n / ZERO_CHUNK + 2) * (n / NBB + 3);
   pl.add<ZeroSeg>(zs);
   // divide-and-conquer descriptors (one copy): problems, leaves, and per
@@ -1218,9 +1220,9 @@ size_t SyevBatched::workspace_bytes(const std::vector<int>& ns) {
   for (int n : ns) ndc += 2 * (size_t)(n / LEAF + 2);
   pl.add<char>(ns.size() * sizeof(DcProb) + ndc * (sizeof(DcBaseProb) + sizeof(DcNode) + sizeof(GemmProb) + sizeof(GemmSeg) + sizeof(int*)) +
                256 * 4 * 40 + 1024);
-  // back-transformation GEMM descriptors (4 batches per block of reflectors)
+  // back-transformation GEMM descriptors (nine products of ten segments per pair of blocks)
   size_t nbt = 0;
-  for (int n : ns) nbt += 4 * (size_t)(bt_nblk(n) + 1);
+  for (int n : ns) nbt += 5 * (size_t)(bt_nblk(n) + 2);
   pl.add<char>(ns.size() * sizeof(BtProb) + nbt * (sizeof(GemmProb) + sizeof(GemmSeg)) +
                256 * 6 * (size_t)(nmx / NBB + 4));
   pl.add<TrdClProb>(2 * ns.size() + 16);
@@ -1281,7 +1283,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     std::vector<TrdProb> tp(nbig);
     std::vector<DcProb> dp(nbig);
     std::vector<BtProb> bt(nbig);
-    std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig), gex(nbig, nullptr);
+    std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig), bt_G12(nbig), gex(nbig, nullptr);
     std::vector<ZeroSeg> zeros;  // ranges that must start at zero, cleared in one launch
     for (int b = 0; b < nbig; ++b) {
       const SyevDesc& S = probs[big[b]];
@@ -1297,8 +1299,9 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       const int nblk = std::max(1, bt_nblk(n));
       double* G = arena_.alloc_n<double>((size_t)NBB * NBB * nblk);
       double* T = arena_.alloc_n<double>((size_t)NBB * NBB * nblk);
-      bt_X[b] = arena_.alloc_n<double>((size_t)NBB * n);
-      bt_Y[b] = arena_.alloc_n<double>((size_t)NBB * n);
+      bt_X[b] = arena_.alloc_n<double>(2 * (size_t)NBB * n);
+      bt_Y[b] = arena_.alloc_n<double>(2 * (size_t)NBB * n);
+      bt_G12[b] = arena_.alloc_n<double>((size_t)NBB * NBB * ((nblk + 1) / 2));
       dT[b] = vec;
       eT[b] = vec + n;
       tauT[b] = vec + 2 * n;
@@ -1751,91 +1754,92 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       ++launches_;
     }
     // The larger ones:
-    // Z = H_0 H_1 ... H_{n-2} Z in blocks of NBB reflectors, last block
-    // first: Z[r0:, :] -= V_k T_k (V_k^T Z[r0:, :]).  V (all reflectors, in
-    // W1), every G_k = V_k^T V_k and every T_k are formed up front in four
-    // launches; then three GEMMs per block.  Split-K outputs X_k live in
-    // their own slots (U, free after divide and conquer, holds blocks
-    // k with (k+1) NBB <= n; the last block uses X), zeroed once.  All
-    // descriptors go to the device in one copy.
+    // Z = H_0 H_1 ... H_{n-2} Z in pairs of blocks of NBB reflectors, last pair
+    // first: Z[r0:, :] -= V T (V^T Z[r0:, :]), V = [V_k V_k+1] and
+    // T = [T_k, -T_k (V_k^T V_k+1) T_k+1; 0, T_k+1].  V (all reflectors, in W1),
+    // every T_k and every T12 are formed up front; then three GEMMs per pair.
+    // Split-K outputs X live in their own slots (U, free after divide and
+    // conquer, holds those of pairs that end by row n; the last pair uses X),
+    // zeroed once.  All descriptors go to the device in one copy.  What bounds
+    // them is the FP64 tensor pipe; by single blocks the last product had four
+    // steps of 16 to a tile, and the five blocks of 1777 to 3600 rows of one call
+    // took 18.1 ms instead of 12.7.
     if (!bp.empty()) {
       const int nbt = (int)bp.size();
-      int kmax = 0, nmaxb = 0;
+      int kmax = 0, pmax = 0, nmaxb = 0;
       for (const BtProb& P : bp) nmaxb = std::max(nmaxb, P.n);
       for (int b = 0; b < nbt; ++b) kmax = std::max(kmax, bt_nblk(bp[b].n));
-      auto xslot = [&](int b, int k) {
+      pmax = (kmax + 1) / 2;
+      constexpr int PB = 2 * NBB;  // reflectors of a pair
+      auto xslot = [&](int b, int q) {
         const int n = bp[b].n;
-        return (k + 1) * NBB <= n ? dp[bp_of[b]].U + (size_t)k * NBB * n : bt_X[bp_of[b]];
+        return (q + 1) * PB <= n ? dp[bp_of[b]].U + (size_t)q * PB * n : bt_X[bp_of[b]];
       };
-      auto xsplit = [](int mrows) { return std::max(1, std::min(16, mrows / 128)); };
+      auto xsplit = [](int mrows) { return std::max(1, std::min(16, mrows / 256)); };
       auto gsplit = [](int mrows) { return std::max(1, std::min(16, mrows / 256)); };
+      auto seg = [](const double* A, int lda, int ta, const double* B, int ldb, int k, double alpha) {
+        GemmSeg s{};
+        s.A = A;
+        s.lda = lda;
+        s.transA = ta;
+        s.B = B;
+        s.ldb = ldb;
+        s.k = k;
+        s.alpha = alpha;
+        return s;
+      };
       std::vector<ZeroSeg> bz;
-      GemmBatch gg;  // every G_k
+      GemmBatch gg, gm, gt;  // every G_k and V_k^T V_k+1; T_k of that; T12
+      constexpr size_t NB2 = (size_t)NBB * NBB;
       for (int b = 0; b < nbt; ++b) {
         const BtProb& P = bp[b];
-        const int n = P.n;
-        for (int k = 0; k < bt_nblk(n); ++k) {
+        const int n = P.n, nblk = bt_nblk(n);
+        for (int k = 0; k < nblk; ++k) {
           const int j0 = k * NBB, nb = std::min(NBB, n - 1 - j0), r0 = j0 + 1, mrows = n - r0;
-          GemmSeg s{};
-          s.A = P.V + r0 + (size_t)j0 * n;
-          s.lda = n;
-          s.transA = 1;
-          s.B = s.A;
-          s.ldb = n;
-          s.transB = 0;
-          s.k = mrows;
-          s.alpha = 1.0;
+          const double* Vk = P.V + r0 + (size_t)j0 * n;
           const int kg = gsplit(mrows);
-          double* Gk = P.G + (size_t)k * NBB * NBB;
-          if (kg > 1) zero_add(bz, Gk, (long long)NBB * NBB);
-          gg.add(Gk, NBB, nb, nb, 0.0, {s}, kg);
-          if (xsplit(mrows) > 1) zero_add(bz, xslot(b, k), (long long)NBB * n);
+          double* Gk = P.G + k * NB2;
+          if (kg > 1) zero_add(bz, Gk, (long long)NB2);
+          gg.add(Gk, NBB, nb, nb, 0.0, {seg(Vk, n, 1, Vk, n, mrows, 1.0)}, kg);
+          if (k & 1) {  // with the block before
+            double* G12 = bt_G12[bp_of[b]] + (k / 2) * NB2;
+            if (kg > 1) zero_add(bz, G12, (long long)NB2);
+            gg.add(G12, NBB, NBB, nb, 0.0, {seg(P.V + r0 + (size_t)(j0 - NBB) * n, n, 1, Vk, n, mrows, 1.0)}, kg);
+            // G_k-1 and G_k are free once the T are formed
+            gm.add(Gk - NB2, NBB, NBB, nb, 0.0, {seg(P.T + (k - 1) * NB2, NBB, 0, G12, NBB, NBB, 1.0)});
+            gt.add(Gk, NBB, NBB, nb, 0.0, {seg(Gk - NB2, NBB, 0, P.T + k * NB2, NBB, nb, -1.0)});
+          }
         }
+        for (int q = 0; q < (nblk + 1) / 2; ++q)
+          if (xsplit(n - q * PB) > 1) zero_add(bz, xslot(b, q), (long long)PB * n);
       }
-      // per block k (descending): X_k = V_k^T Z, Y = -T_k X_k, Z += V_k Y
+      // per pair (descending): X = V^T Z, Y = -T X, Z += V Y
       struct Step {
         GemmBatch gx, gy, gz;
       };
-      std::vector<Step> steps(kmax);
-      for (int k = kmax - 1; k >= 0; --k) {
-        Step& S = steps[k];
+      std::vector<Step> steps(pmax);
+      for (int q = pmax - 1; q >= 0; --q) {
+        Step& S = steps[q];
         for (int b = 0; b < nbt; ++b) {
           const BtProb& P = bp[b];
-          const int n = P.n;
-          if (k >= bt_nblk(n)) continue;
-          const int j0 = k * NBB, nb = std::min(NBB, n - 1 - j0), r0 = j0 + 1, mrows = n - r0;
+          const int n = P.n, nblk = bt_nblk(n), k = 2 * q;
+          if (k >= nblk) continue;
+          // from the row before the first reflector's one on, where V is zero: with
+          // an even n the operands are aligned
+          const int j0 = q * PB, nb = std::min(PB, n - 1 - j0), r0 = j0, mrows = n - r0;
+          const int n1 = std::min(NBB, nb), n2 = nb - n1;
           double* Z = probs[big[bp_of[b]]].Z;
-          double* Xk = xslot(b, k);
-          GemmSeg s{};
-          s.A = P.V + r0 + (size_t)j0 * n;
-          s.lda = n;
-          s.transA = 1;
-          s.B = Z + r0;
-          s.ldb = n;
-          s.transB = 0;
-          s.k = mrows;
-          s.alpha = 1.0;
-          S.gx.add(Xk, NBB, nb, n, 0.0, {s}, xsplit(mrows));
-          GemmSeg t{};
-          t.A = P.T + (size_t)k * NBB * NBB;
-          t.lda = NBB;
-          t.transA = 0;
-          t.B = Xk;
-          t.ldb = NBB;
-          t.transB = 0;
-          t.k = nb;
-          t.alpha = -1.0;
-          S.gy.add(bt_Y[bp_of[b]], NBB, nb, n, 0.0, {t});
-          GemmSeg u{};
-          u.A = P.V + r0 + (size_t)j0 * n;
-          u.lda = n;
-          u.transA = 0;
-          u.B = bt_Y[bp_of[b]];
-          u.ldb = NBB;
-          u.transB = 0;
-          u.k = nb;
-          u.alpha = 1.0;
-          S.gz.add(Z + r0, n, mrows, n, 1.0, {u});
+          double *X = xslot(b, q), *Y = bt_Y[bp_of[b]];
+          const double* V = P.V + r0 + (size_t)j0 * n;
+          const double *T1 = P.T + k * NB2, *T12 = P.G + (k + 1) * NB2;
+          S.gx.add(X, PB, nb, n, 0.0, {seg(V, n, 1, Z + r0, n, mrows, 1.0)}, xsplit(mrows));
+          if (n2 > 0) {
+            S.gy.add(Y, PB, n1, n, 0.0, {seg(T1, NBB, 0, X, PB, n1, -1.0), seg(T12, NBB, 0, X + NBB, PB, n2, -1.0)});
+            S.gy.add(Y + NBB, PB, n2, n, 0.0, {seg(T1 + NB2, NBB, 0, X + NBB, PB, n2, -1.0)});
+          } else {
+            S.gy.add(Y, PB, n1, n, 0.0, {seg(T1, NBB, 0, X, PB, n1, -1.0)});
+          }
+          S.gz.add(Z + r0, n, mrows, n, 1.0, {seg(V, n, 0, Y, PB, nb, 1.0)});
         }
       }
       // one upload: problems, zero ranges, then the GEMM batches
@@ -1845,10 +1849,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       std::vector<std::pair<size_t, size_t>> og;  // (probs, segs) offsets, batch order below
       auto put = [&](const GemmBatch& g) { og.push_back({pk.add(g.probs), pk.add(g.segs)}); };
       put(gg);
-      for (int k = kmax - 1; k >= 0; --k) {
-        put(steps[k].gx);
-        put(steps[k].gy);
-        put(steps[k].gz);
+      put(gm);
+      put(gt);
+      for (int q = pmax - 1; q >= 0; --q) {
+        put(steps[q].gx);
+        put(steps[q].gy);
+        put(steps[q].gz);
       }
       char* dev = pk.upload(arena_, st);
       const BtProb* d_bp = reinterpret_cast<const BtProb*>(dev + o_bp);
@@ -1877,10 +1883,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         NRGB_LAUNCH("bt_T", st, bt_T_kernel<<<dim3(kmax, nbt), BT_T_NT, BT_T_SMEM, st>>>(d_bp));
         NRGB_CUDA(cudaGetLastError());
         ++launches_;
-        for (int k = kmax - 1; k >= 0; --k) {
-          gemm(steps[k].gx);
-          gemm(steps[k].gy);
-          gemm(steps[k].gz);
+        gemm(gm);
+        gemm(gt);
+        for (int q = pmax - 1; q >= 0; --q) {
+          gemm(steps[q].gx);
+          gemm(steps[q].gy);
+          gemm(steps[q].gz);
         }
       }
     }
