@@ -423,11 +423,10 @@ struct TinySm {
   double w[SYEV_TINY], tau[SYEV_TINY];
 };
 
-__global__ void __launch_bounds__(G * SYEV_TINY) syev_tiny_kernel(const TinyProb* __restrict__ probs, int* fail) {
+__device__ __forceinline__ void syev_tiny(const TinyProb P, int* fail) {
   constexpr int N = SYEV_TINY;
   extern __shared__ __align__(16) unsigned char raw[];
   TinySm& m = *reinterpret_cast<TinySm*>(raw);
-  const TinyProb P = probs[blockIdx.x];
   const int n = P.n, tid = threadIdx.x, lane = tid & 31;
   if (tid < 32) {
     double a[N];
@@ -530,11 +529,31 @@ cudaError_t dc_base_launch(const DcBaseProb* d, int nprob, int smax, int* fail, 
   return cudaGetLastError();
 }
 
-cudaError_t syev_tiny_launch(const TinyProb* d, int nprob, int* fail, cudaStream_t st) {
+__global__ void __launch_bounds__(G * SYEV_TINY) syev_tiny_kernel(const TinyProb* __restrict__ probs, int* fail) {
+  syev_tiny(probs[blockIdx.x], fail);
+}
+
+// The descriptors of a call with few blocks, as a kernel parameter: no copy.
+struct TinyArgs {
+  TinyProb p[TINY_INLINE];
+};
+__global__ void __launch_bounds__(G * SYEV_TINY) syev_tiny_inline_kernel(const __grid_constant__ TinyArgs args, int* fail) {
+  syev_tiny(args.p[blockIdx.x], fail);
+}
+
+cudaError_t syev_tiny_launch(const TinyProb* h, const TinyProb* d, int nprob, int* fail, cudaStream_t st) {
   if (nprob <= 0) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(syev_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TinySm));
+  cudaError_t e = d ? cudaFuncSetAttribute(syev_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TinySm))
+                    : cudaFuncSetAttribute(syev_tiny_inline_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(TinySm));
   if (e != cudaSuccess) return e;
-  NRGB_LAUNCH("syev_small", st, syev_tiny_kernel<<<nprob, G * SYEV_TINY, sizeof(TinySm), st>>>(d, fail));
+  if (d) {
+    NRGB_LAUNCH("syev_small", st, syev_tiny_kernel<<<nprob, G * SYEV_TINY, sizeof(TinySm), st>>>(d, fail));
+  } else {
+    TinyArgs args;
+    for (int i = 0; i < nprob; ++i) args.p[i] = h[i];
+    NRGB_LAUNCH("syev_small", st, syev_tiny_inline_kernel<<<nprob, G * SYEV_TINY, sizeof(TinySm), st>>>(args, fail));
+  }
   return cudaGetLastError();
 }
 

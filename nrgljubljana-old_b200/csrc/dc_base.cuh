@@ -26,6 +26,9 @@ struct TinyProb {
   double* Z;        // n x n
   int n;
 };
-cudaError_t syev_tiny_launch(const TinyProb* d, int nprob, int* fail, cudaStream_t st);
+// Up to TINY_INLINE descriptors are taken from the host (d null), more from the
+// device.
+constexpr int TINY_INLINE = 96;
+cudaError_t syev_tiny_launch(const TinyProb* h, const TinyProb* d, int nprob, int* fail, cudaStream_t st);
 
 }  // namespace nrgb

@@ -338,9 +338,9 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
         double wc = (lane < kp) ? __ldcg(&P.W[(size_t)c * NB + lane]) : 0.0;
         if (jj > 0) {
           // scalar a2 and row c of the previous column of W (every CTA)
-          const double yv = ld_volatile(&Ro[1]);
+          const double yv = ld_volatile(&Ro[1]), yc = symv_sum(S, yr, c - base, lane, 32);
           const double ptq = warp_sum(p * q);
-          const double y = warp_sum(symv_sum(S, yr, c - base, lane, 32) - (vc * p + wc * q));
+          const double y = warp_sum(yc - (vc * p + wc * q));
           const double a2 = -0.5 * tprev * tprev * (yv - 2.0 * ptq);
           if (lane == kp) wc = tprev * y + a2 * vc;
           if (lane == 0) misc[0] = a2;
@@ -1126,7 +1126,7 @@ struct GemmBatch {
 
 SyevBatched::SyevBatched() {
   NRGB_CUDA(cudaMalloc(&d_err_, 4 * sizeof(int)));
-  NRGB_CUDA(cudaMalloc(&d_bar_, sizeof(GridBarrier)));
+  NRGB_CUDA(cudaMallocHost(&h_err_, 4 * sizeof(int)));
   int dev = 0;
   NRGB_CUDA(cudaGetDevice(&dev));
   NRGB_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
@@ -1153,7 +1153,7 @@ SyevBatched::SyevBatched() {
 
 SyevBatched::~SyevBatched() {
   if (d_err_) cudaFree(d_err_);
-  if (d_bar_) cudaFree(d_bar_);
+  if (h_err_) cudaFreeHost(h_err_);
   for (int i = 0; i < NAUX; ++i) {
     if (aux_[i]) cudaStreamDestroy(aux_[i]);
     if (join_[i]) cudaEventDestroy(join_[i]);
@@ -1245,7 +1245,6 @@ int SyevBatched::grid_limit(const std::vector<int>& ns, int clim) const {
 void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
   launches_ = 0;
   NRGB_CUDA(cudaMemsetAsync(d_err_, 0, 4 * sizeof(int), st));
-  NRGB_CUDA(cudaMemsetAsync(d_bar_, 0, sizeof(GridBarrier), st));
   std::vector<int> small, big;
   for (int i = 0; i < (int)probs.size(); ++i) {
     if (probs[i].n <= 0) continue;
@@ -1265,13 +1264,19 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
   if (!small.empty()) {
     std::vector<TinyProb> sp;
     for (int i : small) sp.push_back(TinyProb{probs[i].A, probs[i].w, probs[i].Z, probs[i].n});
-    TinyProb* d_sp = arena_.alloc_n<TinyProb>(sp.size());
-    NRGB_CUDA(cudaMemcpyAsync(d_sp, sp.data(), sp.size() * sizeof(TinyProb), cudaMemcpyHostToDevice, st));
+    TinyProb* d_sp = nullptr;
+    if (sp.size() > (size_t)TINY_INLINE) {
+      d_sp = arena_.alloc_n<TinyProb>(sp.size());
+      NRGB_CUDA(cudaMemcpyAsync(d_sp, sp.data(), sp.size() * sizeof(TinyProb), cudaMemcpyHostToDevice, st));
+    }
     // on its own stream, beside the larger blocks; joined before the flags are read
-    NRGB_CUDA(cudaEventRecord(fork_, st));
-    NRGB_CUDA(cudaStreamWaitEvent(small_st_, fork_, 0));
-    NRGB_CUDA(syev_tiny_launch(d_sp, (int)sp.size(), d_err_ + 2, small_st_));
-    NRGB_CUDA(cudaEventRecord(small_done_, small_st_));
+    cudaStream_t sx = big.empty() ? st : small_st_;
+    if (sx != st) {
+      NRGB_CUDA(cudaEventRecord(fork_, st));
+      NRGB_CUDA(cudaStreamWaitEvent(sx, fork_, 0));
+    }
+    NRGB_CUDA(syev_tiny_launch(sp.data(), d_sp, (int)sp.size(), d_err_ + 2, sx));
+    if (sx != st) NRGB_CUDA(cudaEventRecord(small_done_, sx));
     ++launches_;
   }
 
@@ -1893,16 +1898,12 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       }
     }
   }
-  if (!small.empty()) NRGB_CUDA(cudaStreamWaitEvent(st, small_done_, 0));
+  if (!small.empty() && !big.empty()) NRGB_CUDA(cudaStreamWaitEvent(st, small_done_, 0));
   // error flags
-  int herr[4] = {0, 0, 0, 0};
-  GridBarrier hb{};
-  NRGB_CUDA(cudaMemcpyAsync(herr, d_err_, sizeof(herr), cudaMemcpyDeviceToHost, st));
-  NRGB_CUDA(cudaMemcpyAsync(&hb, d_bar_, sizeof(hb), cudaMemcpyDeviceToHost, st));
+  NRGB_CUDA(cudaMemcpyAsync(h_err_, d_err_, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
   NRGB_CUDA(cudaStreamSynchronize(st));
-  hb.error |= herr[3];
-  if (herr[2]) throw CudaError("syev: secular equation iteration did not converge");
-  if (hb.error) throw CudaError("syev: grid barrier timed out");
+  if (h_err_[2]) throw CudaError("syev: secular equation iteration did not converge");
+  if (h_err_[3]) throw CudaError("syev: grid barrier timed out");
 }
 
 }  // namespace nrgb

@@ -78,7 +78,7 @@ class SyevBatched : public EigSolver {
  private:
   DeviceArena arena_;
   int* d_err_ = nullptr;
-  GridBarrier* d_bar_ = nullptr;
+  int* h_err_ = nullptr;  // pinned copy of d_err_
   int launches_ = 0;
   int wait_log2_ = 23;
   bool inject_shortfall_ = false;
