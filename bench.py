@@ -153,20 +153,14 @@ def fp64_gemm_peak(torch, dev):
     return 2.0 * n ** 3 / best / 1e12
 
 
-KERNELS = ("trd_panel", "trd_cluster", "gemm_f64_trailing", "gemm_f64_dc", "gemm_f64_bt", "gemm_f64_recalc", "gemm_f64_nrg",
-           "dc_prep", "dc_permute", "dc_secular", "dc_lowner", "dc_vectors", "dc_rank", "dc_copy", "dc_leaf",
-           "bt_T", "bt_buildV", "syev_small", "assemble*", "spec_dmnrg", "spec_fdm", "merge_bins",
-           "gather_diag", "col_scale")
+KERNELS = ("trd_panel", "trd_grid", "trd_cluster", "trd_mirror", "bt_apply", "gemm_f64_trailing", "gemm_f64_dc", "gemm_f64_bt", "gemm_f64_recalc", "gemm_f64_nrg",
+           "dc_prep", "dc_permute", "dc_secular", "dc_lowner", "dc_vectors", "dc_leaf",
+           "bt_T", "bt_buildV", "syev_small", "assemble*", "spec_dmnrg", "spec_fdm", "boltzmann", "merge_bins",
+           "gather_diag", "col_scale", "truncate")
 
 
 def kernel_table(ctx):
     return {k.rstrip("*"): ctx.kernel_stats(k) for k in KERNELS}
-
-
-# DRAM bytes of the cluster tridiagonalisation per algorithmic byte (each
-# block read once, 8 n^2), from the ncu capture of the small profiling case:
-# 6.010 MB read, 0 written (the results stay in L2), against 5.913 MB.
-TRDC_TRAFFIC_RATIO = 6.010368 / 5.912680
 
 
 def roofline(ctx, ks, torch, dev):
@@ -179,11 +173,10 @@ def roofline(ctx, ks, torch, dev):
         return None
     work = ctx.kernel_work(name)
     if name == "trd_panel":
-        # symv bytes (each column's trailing block read once) per second,
-        # against the HBM copy rate for scale only: the trailing block is
-        # re-read from L2 (85 % hit rate, 0.6 % of DRAM peak in the ncu
-        # capture) and the kernel waits at grid barriers, so it is bound by
-        # barrier latency, not by HBM
+        # bytes of the lower triangle of each column's trailing block per
+        # second, against the HBM copy rate for scale only: the triangle is
+        # re-read from L2 and the kernel waits at grid barriers, so it is
+        # bound by their latency, not by HBM
         peak = peaks.get("hbm_gbs", 6650.0)
         achieved = work / (ms / 1000.0) / 1e9
         return {"kernel": name, "bound": "latency (grid barriers; trailing block L2-resident)",
@@ -200,10 +193,8 @@ def roofline(ctx, ks, torch, dev):
         hbm = ctx.kernel_work("trd_cluster_hbm")
         return {"kernel": name, "bound": "fp64", "achieved": achieved, "peak": peak,
                 "peak_source": "measured cuBLAS DGEMM 8192^3 in this run", "unit": "TFLOP/s",
-                "frac": achieved / peak, "traffic": TRDC_TRAFFIC_RATIO * hbm / nl,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the small-case capture "
-                                  "(3 blocks, n = 402..580) = %.3f x 8 n^2 per block, scaled to this run's "
-                                  "blocks" % TRDC_TRAFFIC_RATIO,
+                "frac": achieved / peak, "traffic": hbm / nl,
+                "traffic_source": "8 n^2 bytes per block, read once into registers (counted by the launching code)",
                 "algorithmic_bytes_per_launch": hbm / nl, "launches": nl, "avg_launch_ms": ms / nl,
                 "algorithmic_flops_per_launch": work / nl}
     if name.startswith("gemm_f64"):

@@ -314,9 +314,9 @@ int nrgb_run(nrgb_ctx* ctx, const char* workdir, const char* outdir, double* sta
  * by every context of the process (no counterpart in the reference, whose
  * only schedule is a sort of the blocks by size, src/nrg.cc:2785-2803):
  *   cluster_limit    blocks up to this size are tridiagonalised whole in one
- *                    thread-block cluster, larger ones take cooperative
- *                    panel launches until their trailing block is this small
- *                    (0 = the cluster kernel's capacity);
+ *                    thread-block cluster, larger ones on many SMs (beyond
+ *                    1776 rows after cooperative panel launches for their
+ *                    leading columns) (0 = the cluster kernel's capacity);
  *   gemm_large_from  grouped FP64 GEMM launches whose problems average at
  *                    least this output edge use 128 x 128 tiles (0 = never).
  * nrgb_autotune measures both choices on the device (a few seconds of

@@ -541,9 +541,9 @@ cudaError_t pipe_attributes() {
 // Tile edge of a launch: four 32 x 32 CTAs for each 64 x 64 tile where those
 // would leave SMs idle, or where the problems are so small (60 tiles: an edge
 // of 480) that the tiles' rims outweigh the operands read twice as often.
-// Measured (64 / 32, us): one 500^3 44.9 / 26.5, four 300^3 32.0 / 25.7, twelve of
-// 400-500 130.6 / 116.7, eighty of 100-300 86 / 79, two 700^3 78.5 / 88.1, forty
-// 512^3 399 / 450, sixteen 1024^3 1172 / 1351.
+// Measured (64 / 32, us): one 500^3 44.8 / 29.8, four 300^3 30.2 / 22.5, eight of
+// 300-400 42.3 / 45.4, twelve of 400-500 121 / 106, eighty of 100-300 80 / 74, two
+// 700^3 70 / 78, forty 512^3 361 / 402, sixteen 1024^3 1064 / 1202.
 bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || total_tiles <= 60L * nprob; }
 
 cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,

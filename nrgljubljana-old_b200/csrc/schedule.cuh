@@ -4,8 +4,7 @@
 // process; readers take the current values at each launch.
 //
 //   cluster_limit   blocks up to this size are tridiagonalised whole inside
-//                   one thread-block cluster; larger ones take cooperative
-//                   panel launches until their trailing block is this small
+//                   one thread-block cluster; larger ones on many SMs
 //                   (0: the cluster kernel's capacity, the default)
 //   gemm_large_from grouped FP64 GEMM launches whose problems average at
 //                   least this edge (sqrt of the output area) use 128 x 128

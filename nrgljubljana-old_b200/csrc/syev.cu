@@ -5,8 +5,6 @@
 //    H x = beta e_1, beta = -sign(x_0) ||x||, tau = (beta - x_0)/beta.
 //  * Blocked tridiagonalisation with the panel formulation A22 <- A22 - V W^T
 //    - W V^T (Dongarra, Sorensen, Hammarling 1989).
-//  * Implicit symmetric QR step with Wilkinson shift (Golub & Van Loan,
-//    Matrix Computations, Alg. 8.3.2) for the leaves and the small path.
 //  * Divide and conquer: Cuppen's rank-one tearing, deflation of small z_i
 //    and of close d_i by Givens rotations, secular-equation roots by a
 //    safeguarded two-pole rational iteration (Bunch-Nielsen-Sorensen / Li

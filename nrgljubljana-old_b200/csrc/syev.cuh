@@ -97,7 +97,7 @@ class SyevBatched : public EigSolver {
   int naux_ = NAUX;  // side streams in use (NRGB_SIDE_STREAMS, for comparisons)
   cudaStream_t aux_[NAUX] = {};
   cudaEvent_t fork_ = nullptr, join_[NAUX] = {};
-  // the warp solver for blocks up to 32 runs beside the larger blocks' work
+  // blocks up to 32 run beside the larger blocks' work
   cudaStream_t small_st_ = nullptr;
   cudaEvent_t small_done_ = nullptr;
 };
