@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
   const int n = P.n;
   const size_t ld = (size_t)n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int nwarps = TRD_NT / 32;
+  constexpr int nwarps = TRD_NT / 32, YG = TRD_NT / 64 - 1;
   const int chunk = (n - j0 + P.ncta - 1) / P.ncta;
   const int R0 = min(n, j0 + rank * chunk), R1 = min(n, R0 + chunk);  // this CTA's rows
   const int base = j0 + 1;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
   // W[:, kp] = tprev (y' - V p - W q) + a2 v of the previous column for this CTA's
   // rows from i0 on, W[i][kp] stored; then f(i, v_i, a) in one lane with
   // a = A[i][c] - V[i] . W[c] - W[i] . V[c].  Warps take four rows at a time.
-  // scalars() fills pq, VWc and misc[0] = a2 (warp 0, before the first use).
+  // scalars() fills pq, VWc and misc[0] = a2 (the last warp, before the first use).
   auto rows = [&](int i0, int jj, double tprev, auto&& scalars, auto&& f) {
     const int kp = jj - 1;
     for (int rb = R0 + ((i0 - R0) / 64) * 64; rb < R1; rb += 64) {
@@ -272,11 +272,12 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
       const int il = rb + warp * 4 + lane;  // the row that lanes 0 .. 3 finish
       const bool fin = lane < 4 && il >= i0 && il < R1;
       const double acol = fin && jj < NB ? __ldcg(&P.A[il + (size_t)(j0 + jj) * ld]) : 0.0;
-      if (jj > 0) {
+      // the sums by all warps but two, of which one forms the scalars meanwhile
+      if (jj > 0 && tid < YG * 64) {
         const int i = rb + (tid & 63), g = tid >> 6;
-        ypart[tid] = (i >= i0 && i < R1) ? symv_sum(S, yr, i - base, g, TRD_NT / 64) : 0.0;
+        ypart[tid] = (i >= i0 && i < R1) ? symv_sum(S, yr, i - base, g, YG) : 0.0;
       }
-      if (warp == 0 && rb <= i0) scalars();
+      if (warp == nwarps - 1 && rb <= i0) scalars();
       __syncthreads();
       const double pk = pq[lane], qk = pq[NB + lane], vck = VWc[lane], wck = VWc[NB + lane];
       const double vckp = jj > 0 ? VWc[kp] : 0.0, a2 = jj > 0 ? misc[0] : 0.0;
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int rr = warp * 4 + u;
-        ys[u] = (jj > 0 && lane < TRD_NT / 64 ? ypart[lane * 64 + rr] : 0.0) - (vik[u] * pk + wik[u] * qk);
+        ys[u] = (jj > 0 && lane < YG ? ypart[lane * 64 + rr] : 0.0) - (vik[u] * pk + wik[u] * qk);
         ts[u] = vik[u] * wck + wik[u] * vck;
         vi[u] = jj > 0 ? __shfl_sync(0xffffffffu, vik[u], max(kp, 0)) : 0.0;
       }
