@@ -530,6 +530,10 @@ cudaError_t pipe_attributes() {
   both(gemm_grouped_pipe_kernel<32, false>, gemm_grouped_pipe_kernel<32, true>, pipe_smem<32>());
   both(gemm_grouped_inline_kernel<64, false, 4096>, gemm_grouped_inline_kernel<64, true, 4096>, pipe_smem<64>());
   both(gemm_grouped_inline_kernel<32, false, 4096>, gemm_grouped_inline_kernel<32, true, 4096>, pipe_smem<32>());
+  both(gemm_grouped_inline_kernel<64, false, 8192>, gemm_grouped_inline_kernel<64, true, 8192>, pipe_smem<64>());
+  both(gemm_grouped_inline_kernel<32, false, 8192>, gemm_grouped_inline_kernel<32, true, 8192>, pipe_smem<32>());
+  both(gemm_grouped_inline_kernel<64, false, 16384>, gemm_grouped_inline_kernel<64, true, 16384>, pipe_smem<64>());
+  both(gemm_grouped_inline_kernel<32, false, 16384>, gemm_grouped_inline_kernel<32, true, 16384>, pipe_smem<32>());
   both(gemm_grouped_inline_kernel<64, false, GEMM_INLINE_MAX>, gemm_grouped_inline_kernel<64, true, GEMM_INLINE_MAX>,
        pipe_smem<64>());
   both(gemm_grouped_inline_kernel<32, false, GEMM_INLINE_MAX>, gemm_grouped_inline_kernel<32, true, GEMM_INLINE_MAX>,
@@ -661,6 +665,8 @@ bool gemm_inline_fits(int nprob, int nseg) {
   return nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= (size_t)GEMM_INLINE_MAX;
 }
 
+// (a launch copies the whole parameter: four sizes of it; an allocation-free basis
+// change of 40 operators, 4.2 KB twice, 39.0 us with 32000 bytes, 34.8 with 8192)
 cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg,
                                        int total_tiles, cudaStream_t stream) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
@@ -668,6 +674,10 @@ cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const G
   if (e != cudaSuccess) return e;
   if (nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= 4096)
     return inline_launch<4096>(probs, nprob, segs, nseg, total_tiles, stream);
+  if (nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= 8192)
+    return inline_launch<8192>(probs, nprob, segs, nseg, total_tiles, stream);
+  if (nprob * sizeof(GemmProb) + nseg * sizeof(GemmSeg) <= 16384)
+    return inline_launch<16384>(probs, nprob, segs, nseg, total_tiles, stream);
   return inline_launch<GEMM_INLINE_MAX>(probs, nprob, segs, nseg, total_tiles, stream);
 }
 
