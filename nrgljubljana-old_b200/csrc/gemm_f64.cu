@@ -9,7 +9,9 @@
 // C[g][2t..2t+1] with g = lane/4, t = lane%4.
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
+#include <vector>
 
 #include "common.cuh"
 #include "gemm_f64.cuh"
@@ -550,6 +552,33 @@ cudaError_t pipe_attributes() {
 // 700^3 70 / 78, forty 512^3 361 / 402, sixteen 1024^3 1064 / 1202.
 bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || total_tiles <= 60L * nprob; }
 
+// Copies the problems of a launch described on the host into `out`, those whose
+// tiles have the most K steps first where the launch takes more than one wave of
+// CTAs (six per SM with T = 32, four with 64): the last wave then ends with short
+// tiles.  64 outputs of four terms (K 15 to 115 each), 3544 CTAs: 112.9 us in the
+// caller's order, 105.1 sorted.  key, idx: scratch of nprob each.
+void order_problems(const GemmProb* probs, int nprob, const GemmSeg* segs, int total_tiles, GemmProb* out, int* key,
+                    int* idx) {
+  const bool small = use_small_tiles(total_tiles, nprob);
+  if (nprob == 1 || (small ? 4L : 1L) * total_tiles <= (small ? 6L : 4L) * 148) {
+    memcpy(out, probs, nprob * sizeof(GemmProb));
+    return;
+  }
+  for (int p = 0; p < nprob; ++p) {
+    long steps = 0;
+    for (int q = probs[p].seg0; q < probs[p].seg0 + probs[p].nseg; ++q)
+      if (segs[q].k > 0) steps += (segs[q].k + KB - 1) / KB;
+    key[p] = (int)std::min(steps / std::max(1, probs[p].ksplit), 0x7fffffffL);
+    idx[p] = p;
+  }
+  std::sort(idx, idx + nprob, [&](int a, int b) { return key[a] != key[b] ? key[a] > key[b] : a < b; });
+  int tiles = 0, stiles = 0;
+  for (int i = 0; i < nprob; ++i) {
+    out[i] = probs[idx[i]];
+    gemm_assign_tiles(out[i], tiles, stiles);
+  }
+}
+
 cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
                         cudaStream_t stream, const int* const* cmaps, bool scaled) {
   const cudaError_t e = pipe_attributes();
@@ -565,7 +594,8 @@ template <int BYTES>
 cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
                           cudaStream_t stream) {
   InlineDesc<BYTES> d;
-  memcpy(d.b, probs, nprob * sizeof(GemmProb));
+  int key[GEMM_INLINE_MAX / sizeof(GemmProb)], idx[GEMM_INLINE_MAX / sizeof(GemmProb)];
+  order_problems(probs, nprob, segs, total_tiles, reinterpret_cast<GemmProb*>(d.b), key, idx);
   memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
   const bool small = use_small_tiles(total_tiles, nprob), scaled = gemm_scaled(segs, nseg);
   const auto k = small ? (scaled ? gemm_grouped_inline_kernel<32, true, BYTES> : gemm_grouped_inline_kernel<32, false, BYTES>)
@@ -656,7 +686,10 @@ cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const Gem
   }
   GemmProb* dp = scratch.alloc_n<GemmProb>(nprob);
   GemmSeg* ds = scratch.alloc_n<GemmSeg>(nseg);
-  if ((e = cudaMemcpyAsync(dp, probs, nprob * sizeof(GemmProb), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
+  std::vector<GemmProb> ordered(nprob);
+  std::vector<int> key(nprob), idx(nprob);
+  order_problems(probs, nprob, segs, total_tiles, ordered.data(), key.data(), idx.data());
+  if ((e = cudaMemcpyAsync(dp, ordered.data(), nprob * sizeof(GemmProb), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(ds, segs, nseg * sizeof(GemmSeg), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
   return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles, nullptr, gemm_scaled(segs, nseg));
 }
