@@ -851,6 +851,18 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
     ps.push_back(sp);
   }
   if (ps.empty()) return;
+  // the longest tiles first: the last wave of the persistent CTAs ends with short ones
+  auto chunks = [&](const SplitProb& p) {
+    int c = 0;
+    for (int i = p.seg0; i < p.seg0 + p.nseg; ++i) c += ss[i].kch;
+    return c;
+  };
+  std::stable_sort(ps.begin(), ps.end(), [&](const SplitProb& x, const SplitProb& y) { return chunks(x) > chunks(y); });
+  tiles = 0;
+  for (SplitProb& p : ps) {
+    p.tile0 = tiles;
+    tiles += p.tiles_m * p.tiles_n;
+  }
   int* exps = ws.alloc_n<int>(nexp);
   for (size_t i = 0; i < jobs.size(); ++i) jobs[i].exps = exps + eoff[i];
   for (size_t i = 0; i < ss.size(); ++i) {  // two jobs per segment, A's and B's
