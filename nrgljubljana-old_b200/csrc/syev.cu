@@ -213,7 +213,7 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned nblocks, u
 // the lower triangles together exceed L2, HBM.  Two blocks of 3600 and 3533 rows
 // together, down to 1776: 36 us a column when both triangles were read and a
 // barrier took seven round trips, 28 with one triangle in tiles that the warps of
-// a CTA shared, 18.3 with a tile to a warp, two round trips to a barrier and the
+// a CTA shared, 17.3 with a tile to a warp, two round trips to a barrier and the
 // first strips in shared memory.
 // V_SMEM: v in shared memory; otherwise (blocks above 27000 rows) a copy per CTA
 // behind the slots of y.
