@@ -15,10 +15,14 @@
 //    threads, one CTA per SM.
 //  * One exchange per column and no cluster barrier: every CTA sends, for its
 //    live columns j, S_j = sum_{i >= t+2} A_ij x_i (x: the updated column t,
-//    unscaled) and R_j = A_{t+1,j}, and P = sum_j S_j x_j.  From these every
-//    CTA forms y = scale S + R, y^T v = scale^2 P + 2 scale S_{t+1} + R_{t+1},
+//    unscaled) and R_j = A_{t+1,j}, and P = p sum_j S_j x_j.  From these every
+//    CTA forms y = scale S + R, y^T v = scale^2 P / p + 2 scale S_{t+1} + R_{t+1},
 //    w and the next column itself (all CTAs run the same arithmetic on the
-//    same values).  The scale of v is not needed before the products, so the
+//    same values).  p is the power of two that brings the largest |x| near one:
+//    without it P is cubic in the matrix's scale, and entries below 1e-105 gave
+//    silently wrong eigenvalues, above 1e103 not-a-numbers; with it the square
+//    of a column's norm is what limits the range, as everywhere else.  The
+//    scale of v is not needed before the products, so the
 //    norm's root and divisions run while the messages travel; R is a row
 //    of the symmetric matrix, so the owner of column t+1 broadcasts nothing.
 //  * The messages are st.async stores that count on the receiver's mbarrier,
@@ -92,6 +96,16 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.aligned.release;\nbarrier.cluster.wait.aligned.acquire;\n" ::: "memory");
 }
 
+// The power of two that brings the largest |x| of a column to [1, 2) (from the
+// upper words of the warps' largest; clamped to normal numbers), and its inverse.
+__device__ __forceinline__ double column_scale(const int* xtop, double& inverse) {
+  const int4 a = *reinterpret_cast<const int4*>(xtop), b = *reinterpret_cast<const int4*>(xtop + 4);
+  const int top = max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
+  const int e = min(max(top >> 20, 1), 2045);
+  inverse = __hiloint2double(e << 20, 0);
+  return __hiloint2double((2046 - e) << 20, 0);
+}
+
 // A CTA's message and shared memory.
 template <int KR, int C, int WR>
 struct ClShape : Shape<KR, C, WR> {
@@ -127,6 +141,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
   double* ssp = Pp + NW;                         // NW partial norms
   double* scl = ssp + NW;                        // tau, scale of v, alpha of even and of odd columns
   const unsigned bar = smem_u32(scl + 4);
+  int* xtop = reinterpret_cast<int*>(scl + 6);   // NW: by warp, the upper word of its largest |x|
   if (ONE) CL = 1;
   const int r = ONE ? 0 : (int)(blockIdx.x % CL);
   const TrdClProb P = probs[ONE ? blockIdx.x : blockIdx.x / CL];
@@ -179,6 +194,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
   if (!ONE) cluster_sync_all();
 
   double tc = 0.0, scal = 0.0;
+  double unp = 1.0;  // 1 / p of the last column
   bool ok = true;
   int tl = 0, tr = 0;  // t / CL, t % CL
   for (int t = 0; t < n; ++t) {
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       }
       const double2 st = sr[tr * LP + tl];
       const double yt = fma(scal, st.x, st.y);
-      const double ytv = fma(scal * scal, Ps, fma(scal, st.x, yt));
+      const double ytv = fma(scal * unp, scal * Ps, fma(scal, st.x, yt));
       const double a2 = -0.5 * tc * tc * ytv;
       const double wt = fma(tc, yt, a2);
 #pragma unroll
@@ -235,6 +251,11 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
           X[i] = x[m];
         }
       }
+      int top = 0;
+#pragma unroll
+      for (int m = 0; m < M; ++m) top = max(top, __double2hiint(x[m]) & 0x7fffffff);
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) xtop[warp] = top;
     }
     if (t == n - 1) break;
     __syncthreads();
@@ -253,9 +274,10 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       const int ks = kd <= 0 ? 0 : (kd + WR - 1) / WR;
       trdr_update_from<0, KR, C, WR>(ks, a, acc, vj, wj, VW + lane + 32 * wr, X + lane + 32 * wr,
                                      ks * WR == kd && lane == l1, Rs + wc * C);
+      const double p = column_scale(xtop, unp);
       double accP = 0.0;
 #pragma unroll
-      for (int c = 0; c < C; ++c) accP = fma(X[jc[c]], acc[c], accP);
+      for (int c = 0; c < C; ++c) accP = fma(X[jc[c]] * p, acc[c], accP);
       const double red = columns_sum<C>(acc, lane);
       accP = warp_sum_mma(accP);
       if (lane % GL == 0 && lane / GL < C) Sp[(wr * WC + wc) * C + lane / GL] = red;
