@@ -226,13 +226,14 @@ int nrgb_spectrum_dmnrg(nrgb_ctx* ctx, int npairs, const nrgb_dmnrg_pair* pairs,
                         double discard, int nbins, double* bins);
 
 /* Split-precision form of nrgb_gemm_grouped_dev (same descriptors): every
- * product is computed from INT8 digits of each operand that carry at least
- * `slices` (2..8) signed 7-bit slices, with power-of-two scales per row of
- * op(A) and per column of op(B), as exact INT8 tensor-core products (tcgen05
- * kind::i8, INT32 accumulators) recombined exactly and rounded once to FP64.
- * The error of an entry is at most about
- * k * 2^-7S * (S + 3) * max|op(A) row| * max|op(B) column|; S = 8 is at the
- * level of an FP64 product.  Replaces the BLAS gemm of the recalculation
+ * product is computed from `slices` (2..8) balanced 8-bit digits of each
+ * operand, which carry at least as many signed 7-bit slices, with power-of-two
+ * scales per row of op(A) and per column of op(B), as exact INT8 tensor-core
+ * products (tcgen05 kind::i8, INT32 accumulators) recombined exactly and
+ * rounded once to FP64.  The error of an entry is at most
+ * 4.2 * k * 2^-8S * (S + 2) * max|op(A) row| * max|op(B) column|, which is below
+ * k * 2^-7S * (S + 3) times the same, and the rounding of the result; S = 8 is
+ * at the level of an FP64 product.  Replaces the BLAS gemm of the recalculation
  * (src/recalc.cc:268-272) and the density matrices (src/dmnrg.h:382-387) in
  * the split-precision form.  Returns after the work completed. */
 int nrgb_gemm_grouped_split_dev(nrgb_ctx* ctx, int slices, int nout, const nrgb_gemm_out* outs, int nterms,

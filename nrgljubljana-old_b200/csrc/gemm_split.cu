@@ -21,8 +21,8 @@
 // the bulk copies into a ring of 32-byte-deep chunks (mbarrier transaction
 // counts), another the tcgen05.mma instructions: for every chunk the digit pairs
 // (p, q) with p + q <= D + 1 into the accumulator of p + q (D accumulators of
-// 64 INT32 columns: up to 448 of the 512 tensor-memory columns), and commits to
-// the stage's "empty" barrier.  Pairs of one p follow each other, so the A
+// 64 INT32 columns: up to all 512 tensor-memory columns), and commits to the
+// stage's "empty" barrier.  Pairs of one p follow each other, so the A
 // image is read from shared memory once and kept in the tensor core's collector
 // buffer.  After a segment's last chunk a commit to the "done" barrier releases
 // eight warps: each reads half the columns of its 32 rows (tensor-memory lanes) with tcgen05.ld,
@@ -32,10 +32,9 @@
 // What bounds it: the shape of the instruction.  D accumulators of N columns
 // must fit in 512 columns, so N = 64, and a 128 x 64 x 32 product reads 6 KB of
 // operands from shared memory for 32 cycles of arithmetic: measured alone, 48
-// cycles an instruction and 45 with the collector (N = 128: 64).  A chunk's 28
-// products of 8 slices take 1300 to 1500 cycles here.  The eight products above:
-// 0.74 ms with 36 products a chunk, issued by one thread of a divergent branch,
-// and a compensated FP64 recombination; 0.27 ms now.
+// cycles an instruction and 45 with the collector (N = 128: 64).  The eight
+// products above with 8 slices, 36 products a chunk: 0.74 ms issued by one thread
+// of a divergent branch, with a compensated FP64 recombination; 0.34 ms now.
 // Every wait on a barrier is bounded; a wait that gives up sets an error flag,
 // ends the CTA's work (waiting, bounded, for its copies and products in
 // flight), frees the tensor memory and returns.
@@ -65,12 +64,6 @@ constexpr int MAX_STAGES = 16;
 constexpr size_t RING_BYTES = 216 * 1024;
 constexpr long long WAIT_LIMIT = 1ll << 24;
 constexpr int NO_EXP = (int)0x80808080;  // what memset leaves: a row of zeros
-
-// Digits of 8 bits that carry what `slices` truncated digits of 7 bits do: D
-// balanced digits (the leading one with 7 bits and the sign) leave a remainder
-// of at most 2^-8D, so 7 of them replace 8 slices, and fewer slices become as
-// many digits.
-constexpr int split_digits(int slices) { return slices < 8 ? slices : 7; }
 
 __device__ int g_split_err = 0;
 
@@ -203,7 +196,7 @@ __device__ __forceinline__ void write_digits(const double (&x)[16], double f1, d
     }
   }
 #pragma unroll
-  for (int j = 0; j < 7; ++j)  // byte j is digit D - j
+  for (int j = 0; j < 8; ++j)  // byte j is digit D - j
     if (j < D)
       *reinterpret_cast<uint4*>(dst + (size_t)(D - 1 - j) * image) =
           make_uint4(out[j][0], out[j][1], out[j][2], out[j][3]);
@@ -483,7 +476,7 @@ template <int D>
 struct Recombine {
   static constexpr int NH = D < 4 ? D : 4, NL = D - NH, L = 8 * NL;
   long long hi[16];
-  int low[16];
+  unsigned low[16];
 
   __device__ __forceinline__ void load(unsigned taddr) {
     {
@@ -505,13 +498,13 @@ struct Recombine {
 #pragma unroll
         for (int d = 0; d < NL; ++d) x += (long long)v[d][u] * (1ll << (8 * (NL - 1 - d)));
         hi[u] += x >> L;
-        low[u] = (int)x & ((1 << L) - 1);
+        low[u] = (unsigned)x & (unsigned)((1ull << L) - 1);
       }
     }
   }
   // the sum, rounded once to FP64
   __device__ __forceinline__ double value(int u) const {
-    long long bottom = (hi[u] & 0xFFFFF) << L;  // below 2^44: exact
+    long long bottom = (hi[u] & 0xFFFFF) << L;  // below 2^52: exact
     if constexpr (NL > 0) bottom |= low[u];
     return fma((double)(hi[u] >> 20), (double)(1ll << (20 + L)), (double)bottom);
   }
@@ -525,7 +518,8 @@ struct Ring {
 constexpr int FIRST = 1, LAST = 2, END = 4;  // of a stage's chunk: see flag_s
 
 // The warp that issues the products.  (A function of its own: inlined beside
-// the recombination its loop issues 28 products in 1426 cycles instead of 1304.)
+// the recombination its loop issues 28 products, those of 7 slices, in 1426 cycles
+// instead of 1304.)
 template <int D>
 __device__ __noinline__ void split_products(Ring ring, unsigned tmem, int stages, const volatile int* flag_s,
                                             volatile int* abort_flag) {
@@ -752,7 +746,7 @@ size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 
 size_t split_gemm_workspace(const GemmProb* probs, int nprob, const GemmSeg* segs, int slices) {
   size_t b = 1 << 16;
-  const size_t D = split_digits(slices);
+  const size_t D = slices;
   for (int p = 0; p < nprob; ++p)
     for (int s = 0; s < probs[p].nseg; ++s) {
       const GemmSeg& g = segs[probs[p].seg0 + s];
@@ -778,7 +772,7 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
   std::vector<SplitProb> ps;
   int blocks = 0, tiles = 0;
   double flops = 0;
-  const int D = split_digits(slices);
+  const int D = slices;
   std::vector<size_t> eoff;  // per job: its exponents within those of the launch
   size_t nexp = 0;
   for (int p = 0; p < nprob; ++p) {
@@ -888,7 +882,8 @@ void split_gemm_grouped(const GemmProb* probs, int nprob, const GemmSeg* segs, i
   NRGB_CUDA(cudaGetLastError());
   cudaError_t (*launch)(const SplitProb*, int, const SplitSeg*, int, cudaStream_t) =
       D == 2 ? split_gemm_launch<2> : D == 3 ? split_gemm_launch<3> : D == 4 ? split_gemm_launch<4>
-      : D == 5 ? split_gemm_launch<5> : D == 6 ? split_gemm_launch<6> : split_gemm_launch<7>;
+      : D == 5 ? split_gemm_launch<5> : D == 6 ? split_gemm_launch<6>
+      : D == 7 ? split_gemm_launch<7> : split_gemm_launch<8>;
   KernelStats::get().add_work(tag, flops);
   cudaError_t err = cudaSuccess;
   NRGB_LAUNCH(tag, st, err = launch(d_ps, np, d_ss, tiles, st));
