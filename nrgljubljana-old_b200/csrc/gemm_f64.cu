@@ -677,21 +677,29 @@ size_t gemm_desc_bytes(int nprob, int nseg) {
 }
 
 cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
-                                     cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch) {
+                                     cudaStream_t stream, const char* tag, int total_stiles, const GemmStage& stage) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
   cudaError_t e = cudaSuccess;
   if (gemm_inline_fits(nprob, nseg) && schedule_here().gemm_large_from.load(std::memory_order_relaxed) == 0) {
     NRGB_LAUNCH(tag, stream, e = gemm_grouped_launch_inline(probs, nprob, segs, nseg, total_tiles, stream));
     return e;
   }
-  GemmProb* dp = scratch.alloc_n<GemmProb>(nprob);
-  GemmSeg* ds = scratch.alloc_n<GemmSeg>(nseg);
   std::vector<GemmProb> ordered(nprob);
   std::vector<int> key(nprob), idx(nprob);
   order_problems(probs, nprob, segs, total_tiles, ordered.data(), key.data(), idx.data());
-  if ((e = cudaMemcpyAsync(dp, ordered.data(), nprob * sizeof(GemmProb), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
-  if ((e = cudaMemcpyAsync(ds, segs, nseg * sizeof(GemmSeg), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
+  const GemmProb* dp = static_cast<const GemmProb*>(stage(ordered.data(), nprob * sizeof(GemmProb)));
+  const GemmSeg* ds = static_cast<const GemmSeg*>(stage(segs, nseg * sizeof(GemmSeg)));
   return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles, nullptr, gemm_scaled(segs, nseg));
+}
+
+cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
+                                     cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch) {
+  return gemm_grouped_launch_host(probs, nprob, segs, nseg, total_tiles, stream, tag, total_stiles,
+                                  [&](const void* src, size_t bytes) -> const void* {
+                                    void* d = scratch.alloc(bytes);
+                                    NRGB_CUDA(cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, stream));
+                                    return d;
+                                  });
 }
 
 bool gemm_inline_fits(int nprob, int nseg) {

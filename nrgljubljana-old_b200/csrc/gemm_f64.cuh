@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
+
 #include "common.cuh"
 
 namespace nrgb {
@@ -72,8 +74,15 @@ cudaError_t gemm_grouped_launch_inline(const GemmProb* probs, int nprob, const G
                                        int total_tiles, cudaStream_t stream);
 
 // A launch described on the host: inline when the descriptors fit (and the
-// schedule does not ask for 128 x 128 tiles), else through copies into `scratch`,
-// which must have room for both arrays (gemm_desc_bytes).
+// schedule does not ask for 128 x 128 tiles), else through two calls of `stage`,
+// which copies that many bytes of host memory to the device in stream order,
+// takes them before it returns (they are temporary) and gives their address.
+using GemmStage = std::function<const void*(const void*, size_t)>;
+cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
+                                     cudaStream_t stream, const char* tag, int total_stiles, const GemmStage& stage);
+
+// The same with plain copies into `scratch`, which must have room for both
+// arrays (gemm_desc_bytes).
 size_t gemm_desc_bytes(int nprob, int nseg);
 cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
                                      cudaStream_t stream, const char* tag, int total_stiles, DeviceArena& scratch);

@@ -350,23 +350,24 @@ struct NrgDriver::Impl {
   // have a pinned host mirror, so their uploads are plain DMA (a pageable
   // source goes through the CUDA driver's staging buffer, which the run
   // threads of a server share).  The mirror is rewritten only after
-  // desc_reset(), which waits for the stream.
+  // desc_reset(), which waits for the stream.  GEMM descriptors that travel as
+  // a kernel parameter are not copies and do not count in h2d.
   static constexpr size_t DESC_PINNED = 4 << 20;
   char* desc_pin = nullptr;
-  template <class T>
-  T* upload(const std::vector<T>& v) {
-    if (v.empty()) return nullptr;
-    const size_t bytes = v.size() * sizeof(T);
-    T* d = static_cast<T*>(desc.alloc(bytes));
+  void* upload(const void* src, size_t bytes) {
+    void* d = desc.alloc(bytes);
     const size_t off = desc.offset_of(d);
     if (desc_pin && off + bytes <= DESC_PINNED) {
-      memcpy(desc_pin + off, v.data(), bytes);
-      NRGB_CUDA(cudaMemcpyAsync(d, desc_pin + off, bytes, cudaMemcpyHostToDevice, st));
-    } else {
-      NRGB_CUDA(cudaMemcpyAsync(d, v.data(), bytes, cudaMemcpyHostToDevice, st));
+      memcpy(desc_pin + off, src, bytes);
+      src = desc_pin + off;
     }
+    NRGB_CUDA(cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, st));
     h2d += bytes;
     return d;
+  }
+  template <class T>
+  T* upload(const std::vector<T>& v) {
+    return v.empty() ? nullptr : static_cast<T*>(upload(v.data(), v.size() * sizeof(T)));
   }
   void desc_reset() {
     // descriptors of the previous launches must not be overwritten while in use
@@ -388,7 +389,8 @@ struct NrgDriver::Impl {
     }
     KernelStats::get().add_work("gemm_f64_nrg", gemm_flops(g.probs.data(), (int)g.probs.size(), g.segs.data()));
     NRGB_CUDA(gemm_grouped_launch_host(g.probs.data(), (int)g.probs.size(), g.segs.data(), (int)g.segs.size(), g.tiles, st,
-                                       "gemm_f64_nrg", g.stiles, desc));
+                                       "gemm_f64_nrg", g.stiles,
+                                       [this](const void* src, size_t bytes) { return upload(src, bytes); }));
     launches += 1;
   }
   DevMat upload_mat(const HostMat& M, Slab& slab) {
