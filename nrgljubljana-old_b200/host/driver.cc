@@ -288,6 +288,7 @@ struct NrgDriver::Impl {
   size_t tail_pin_bytes = 0;
   std::vector<ExpvDeferred> expv_def;
   std::unique_ptr<Slab> expv_slab;
+  std::unique_ptr<Slab> persist_slab;  // eigenvalues, bins
   void free_trunc() {
     for (int i = 0; i < 2; ++i) {
       if (tstate.map_k[i]) cudaFreeAsync(tstate.map_k[i], st);
@@ -1606,7 +1607,8 @@ struct NrgDriver::Impl {
   }
 
   // Device data of a run: freed at its end, and on the way out of a failed run
-  // so that a server can hand the memory to the next run.
+  // so that a server can hand the memory to the next run.  The chunks go last,
+  // after every slab of the run has given its own back.
   void release_run_data() {
     spectra.clear();
     rho.clear();
@@ -1614,6 +1616,7 @@ struct NrgDriver::Impl {
     rho_slabs.clear();
     steps.clear();
     expv_slab.reset();
+    persist_slab.reset();
     boltz.clear();
     mem.clear(st);
   }
@@ -1680,7 +1683,8 @@ struct NrgDriver::Impl {
     find_laststored();
     if (Nmax <= Ninit) throw std::runtime_error("zero-bandwidth runs (Nmax == Ninit) are not supported");
     if (P.dm && P.T <= 0) throw std::runtime_error("density-matrix runs need T > 0");
-    Slab persist(st);
+    persist_slab.reset(new Slab(st));
+    Slab& persist = *persist_slab;
     sec.reset();
     {
       struct Client {
