@@ -1236,11 +1236,6 @@ int SyevBatched::cl_use() const {
   return (lim > 0 && lim < cl_nmax_) ? lim : cl_nmax_;
 }
 
-int SyevBatched::grid_limit(const std::vector<int>& ns, int clim) const {
-  if (grid_nmax_ == 0 || clim == 0) return 0;
-  return grid_nmax_;
-}
-
 void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
   launches_ = 0;
   NRGB_CUDA(cudaMemsetAsync(d_err_, 0, 4 * sizeof(int), st));
@@ -1289,6 +1284,10 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     std::vector<BtProb> bt(nbig);
     std::vector<double*> dT(nbig), eT(nbig), tauT(nbig), bt_X(nbig), bt_Y(nbig), bt_G12(nbig), gex(nbig, nullptr);
     std::vector<ZeroSeg> zeros;  // ranges that must start at zero, cleared in one launch
+    // The schedule's limit is read once: another thread may change it at any
+    // time, and the buffers below must match the paths chosen further down.
+    const int clim = cl_use();
+    const int glim = clim > 0 ? grid_nmax_ : 0;
     for (int b = 0; b < nbig; ++b) {
       const SyevDesc& S = probs[big[b]];
       const int n = S.n;
@@ -1351,7 +1350,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       u.V = W1;  // free once divide and conquer is done
       u.G = G;
       u.T = T;
-      if (grid_nmax_ > 0 && n > cl_use()) {
+      if (glim > 0 && n > clim) {
         gex[b] = arena_.alloc_n<double>(trd_grid_exchange(n));
         zero_add(zeros, gex[b], (long long)trd_grid_exchange(n));
       }
@@ -1413,8 +1412,6 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
     // beyond its capacity after panel launches for their leading columns;
     // without it, panel launches until the trailing block fits a cluster.
     std::vector<int> jstop(nbig);
-    const int clim = cl_use();
-    const int glim = grid_limit(ns, clim);
     {
       std::vector<TrdClProb> whole;
       for (int b = 0; b < nbig; ++b) {

@@ -90,8 +90,6 @@ class SyevBatched : public EigSolver {
   int cl_use() const;
   // the many-CTA tridiagonalisation: largest block (0: off) and CTAs of a launch
   int grid_nmax_ = 0, grid_ctas_ = 0;
-  // blocks beyond `clim` go to it once their trailing block is this small (0: never)
-  int grid_limit(const std::vector<int>& ns, int clim) const;
   // side streams on which the cluster launches of different sizes overlap
   static constexpr int NAUX = 16;
   int naux_ = NAUX;  // side streams in use (NRGB_SIDE_STREAMS, for comparisons)
