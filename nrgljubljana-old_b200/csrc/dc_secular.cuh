@@ -10,8 +10,12 @@ namespace {
 
 // Reciprocal from the hardware's approximation by two Newton steps
 // r <- r + r (1 - x r): within an ulp for |x| in [2^-1000, 2^1000], which the
-// scaled problems below stay in.  On B200 68 cycles (with an add) and 16 issue
-// cycles a warp, where a division takes 148 and 65.
+// scaled problems below stay in: values are near 1, and poles that were not
+// deflated are at least 8 units of 2^-52 apart.  Not a number for 0, subnormal and
+// infinite x: of the callers only the quadratics' coefficients (s, c, cc, qq) can
+// vanish, and a root that is not a number fails the test of its bracket, after
+// which the other root or the bracket's middle is taken.  On B200 68 cycles (with
+// an add) and 16 issue cycles a warp, where a division takes 148 and 65.
 __device__ __forceinline__ double rcp_newton(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
