@@ -333,14 +333,17 @@ int nrgb_get_schedule(nrgb_ctx* ctx, int* cluster_limit, int* gemm_large_from, i
 
 /* Failure detection of the device waits.  Every wait of a kernel in this
  * library is bounded: a grid-barrier wait of the cooperative tridiagonalisation
- * gives up after 2^poll_log2 polls (default 23, about a second), the launch
- * ends early, and the call returns status 2 with "grid barrier timed out"
- * while the context stays usable.  poll_log2 in [4, 30].  No counterpart in
+ * gives up after 2^poll_log2 polls (default 23, about a second), a wait of the
+ * kernels that hold the matrix in registers after at most 2^21, inside a
+ * cluster after 2^12 to 2^20; the launch ends early, and the call returns
+ * status 2 with "grid barrier timed out" while the context stays usable.
+ * poll_log2 in [4, 30].  No counterpart in
  * the reference (its LAPACK calls have no waits to bound). */
 int nrgb_set_wait_limit(nrgb_ctx* ctx, int poll_log2);
 /* Host-side fault injection for tests of that path: while `on`, the panel
  * launches' barriers expect one CTA more than is launched (a CTA that never
- * arrives), so their waits run out and nrgb_syev_batched / nrgb_run return
+ * arrives) and the other tridiagonalisations' waits a word that is never sent,
+ * so the waits run out and nrgb_syev_batched / nrgb_run return
  * the timeout error.  No counterpart in the reference. */
 int nrgb_inject_barrier_shortfall(nrgb_ctx* ctx, int on);
 

@@ -1397,7 +1397,10 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         KernelStats::get().add_work("trd_cluster", fl);
         KernelStats::get().add_work("trd_cluster_hbm", by);
         cudaError_t e = cudaSuccess;
-        NRGB_LAUNCH("trd_cluster", sx, e = trdr_launch(g, dg, (int)kv.second.size(), d_err_ + 3, sx));
+        // between 4 ms and a second: a cluster's CTAs run together, its exchange takes microseconds
+        const int tries_log2 = std::max(12, std::min(wait_log2_, 20));
+        NRGB_LAUNCH("trd_cluster", sx, e = trdr_launch(g, dg, (int)kv.second.size(), tries_log2,
+                                                       inject_shortfall_ ? 1 : 0, d_err_ + 3, sx));
         NRGB_CUDA(e);
         dg += kv.second.size();
         ++launches_;

@@ -91,7 +91,6 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-constexpr int WAIT_TRIES = 1 << 20;  // about a second
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.aligned.release;\nbarrier.cluster.wait.aligned.acquire;\n" ::: "memory");
 }
@@ -122,7 +121,7 @@ struct ClShape : Shape<KR, C, WR> {
 
 template <int KR, int C, int WR, bool ONE>
 __global__ void __launch_bounds__(trdr::threads(ONE), 1)
-    trd_regs_kernel(const TrdClProb* __restrict__ probs, int CL, int* fail) {
+    trd_regs_kernel(const TrdClProb* __restrict__ probs, int CL, int tries, int extra, int* fail) {
   using namespace trdr;
   using SH = ClShape<KR, C, WR>;
   static_assert(C <= 16 && C % 2 == 0, "columns of a warp");
@@ -131,6 +130,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
   constexpr int GL = 32 / pow2_up(C);           // lanes of a column's group
   constexpr int M = (ROWS + NT - 1) / NT;       // rows of the vectors a thread computes
   extern __shared__ __align__(16) double sm[];
+  __shared__ volatile int gave_up;               // a wait of this CTA ran out
   double2* VW = reinterpret_cast<double2*>(sm);  // ROWS + 1: (v, w) of the rows; the last entry stays zero
   double2* SR = VW + ROWS + 1;                   // [2][CL][LP]: (S, R) of every column, by sender
   double* PS = reinterpret_cast<double*>(SR + 2 * CL * LP);  // [2][16]: P, by sender
@@ -184,31 +184,30 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
   }
   int l0 = CL == 1 ? 1 : 0, lr = CL == 1 ? 0 : 1;  // (t + 1) / CL and (t + 1) % CL of the phase t to be sent
   if (!ONE && tid == 0) {
+    gave_up = 0;
     mbar_init(bar, 1);
     mbar_init(bar + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect(bar, CL * ((COLS - 1 / CL) * 16 + 8));
-    mbar_expect(bar + 8, CL * ((COLS - 2 / CL) * 16 + 8));
+    mbar_expect(bar, CL * ((COLS - 1 / CL) * 16 + 8) + extra);
+    mbar_expect(bar + 8, CL * ((COLS - 2 / CL) * 16 + 8) + extra);
   }
   __syncthreads();
   if (!ONE) cluster_sync_all();
 
   double tc = 0.0, scal = 0.0;
   double unp = 1.0;  // 1 / p of the last column
-  bool ok = true;
   int tl = 0, tr = 0;  // t / CL, t % CL
   for (int t = 0; t < n; ++t) {
     const int pb = (t + 1) & 1;  // buffer of phase t - 1
-    if (!ONE && t > 0 && ok) {
+    if (!ONE && t > 0) {
       const unsigned bw = bar + 8 * pb, par = ((t - 1) >> 1) & 1;
       int it = 0;
-      while (!__all_sync(0xffffffffu, mbar_try(bw, par)))
-        if (++it > WAIT_TRIES) {  // a wait that gives up: report it and run on without waiting
-          ok = false;
-          atomicExch(fail, 1);
-          break;
-        }
-      if (tid == 0) {  // phase t + 1 (its first column to be sent: (t + 2) / CL)
+      bool ok = true;
+      while (ok && !__all_sync(0xffffffffu, mbar_try(bw, par))) ok = ++it <= tries;
+      if (!ok) {  // this CTA ends after its next barrier, the others run out too
+        atomicExch(fail, 1);
+        gave_up = 1;
+      } else if (tid == 0) {  // phase t + 1 (its first column to be sent: (t + 2) / CL)
         const int f = lr + 1 == CL ? l0 + 1 : l0;
         mbar_expect(bw, CL * ((COLS - f) * 16 + 8));
       }
@@ -259,6 +258,9 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
     }
     if (t == n - 1) break;
     __syncthreads();
+    // (nothing is armed or sent after a wait that ran out: the transaction counts
+    // would leave their range)
+    if (!ONE && gave_up) break;
     if (warp < NW) {
       // ---- matrix: rank-2 update, products of the columns with x ----
       double vj[C], wj[C], acc[C];
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
     // no CTA leaves while another may still write its shared memory
     __syncthreads();
     cluster_sync_all();
-    if (!ok)  // a wait gave up: let copies in flight land before this CTA's memory goes
+    if (gave_up)  // let copies in flight land before this CTA's memory goes
       for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
 }
@@ -469,11 +471,14 @@ int trdr_init() {
   return nmax;
 }
 
-cudaError_t trdr_launch(TrdrGroup g, const TrdClProb* d, int nprob, int* fail, cudaStream_t st) {
+cudaError_t trdr_launch(TrdrGroup g, const TrdClProb* d, int nprob, int wait_log2, int expect_extra, int* fail,
+                        cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[1];
   group_config(g, nprob, st, cfg, at);
-  return with_shape(g.shape, [&](auto, auto kern) { return cudaLaunchKernelEx(&cfg, kern, d, g.cl, fail); });
+  return with_shape(g.shape, [&](auto, auto kern) {
+    return cudaLaunchKernelEx(&cfg, kern, d, g.cl, 1 << wait_log2, 16 * expect_extra, fail);
+  });
 }
 
 }  // namespace nrgb

@@ -27,7 +27,10 @@ TrdrGroup trdr_group(int n);
 int trdr_init();
 
 // Tridiagonalises `nprob` blocks of one group.  *fail is set when a wait
-// inside a cluster gave up.
-cudaError_t trdr_launch(TrdrGroup g, const TrdClProb* d, int nprob, int* fail, cudaStream_t st);
+// inside a cluster gave up, after 2^wait_log2 tries of about a microsecond.
+// expect_extra: the waits expect so many words that no CTA sends (0; 1 injects
+// a lost message).
+cudaError_t trdr_launch(TrdrGroup g, const TrdClProb* d, int nprob, int wait_log2, int expect_extra, int* fail,
+                        cudaStream_t st);
 
 }  // namespace nrgb
