@@ -129,7 +129,8 @@ std::string autotune(EigSolver& syev, int cluster_capacity, cudaStream_t st) {
       NRGB_CUDA(cudaMemcpyAsync(dP.p, P.data(), sizeof(GemmProb) * np, cudaMemcpyHostToDevice, st));
       NRGB_CUDA(cudaMemcpyAsync(dG.p, G.data(), sizeof(GemmSeg) * np, cudaMemcpyHostToDevice, st));
       auto run = [&] {
-        NRGB_CUDA(gemm_grouped_launch(dP.as<GemmProb>(), np, dG.as<GemmSeg>(), tiles, st, "autotune", stiles));
+        NRGB_CUDA(gemm_grouped_launch(dP.as<GemmProb>(), np, dG.as<GemmSeg>(), tiles, st, "autotune",
+                                      gemm_tiles32(P.data(), np), stiles));
       };
       S.gemm_large_from.store(0);
       const double t_small = time_ms(st, 3, run);

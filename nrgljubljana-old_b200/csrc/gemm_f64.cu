@@ -545,12 +545,18 @@ cudaError_t pipe_attributes() {
 }
 
 // Tile edge of a launch: four 32 x 32 CTAs for each 64 x 64 tile where those
-// would leave SMs idle, or where the problems are so small (60 tiles: an edge
-// of 480) that the tiles' rims outweigh the operands read twice as often.
-// Measured (64 / 32, us): one 500^3 44.8 / 29.8, four 300^3 30.2 / 22.5, eight of
-// 300-400 42.3 / 45.4, twelve of 400-500 121 / 106, eighty of 100-300 80 / 74, two
-// 700^3 70 / 78, forty 512^3 361 / 402, sixteen 1024^3 1064 / 1202.
-bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || total_tiles <= 60L * nprob; }
+// would leave SMs idle, or where the problems are small (60 tiles: an edge of
+// 480) and at least 3 % of the 64 x 64 tiles' area lies outside them in quarters
+// that 32 x 32 tiles leave out, so that the rims outweigh the operands read twice
+// as often.  Measured (64 / 32, us; area that is left out): one 500^3 44.8 / 29.1
+// (idle SMs), four 300^3 32.4 / 26.0 (idle SMs), eight of 200-300 34.8 / 29.6 (14 %),
+// twelve of 400-500 120.5 / 105.8 (7 %), eighty of 100-300 84.0 / 83.9 (13 %), eight
+// 384^3 44.8 / 50.8 (none), forty 512^3 358.8 / 405.3 (none), two 700^3 70.6 / 80.9
+// (none).  Within 5 % either way, by how the last wave falls: eight of 300-400 45.7 /
+// 46.1 (4 %), sixteen of them 75.8 / 78.2 (6 %), forty of 200-400 112.8 / 117.9 (9 %).
+bool use_small_tiles(int total_tiles, int nprob, int tiles32) {
+  return total_tiles < 148 || (total_tiles <= 60L * nprob && tiles32 <= 3.88 * total_tiles);
+}
 
 // Copies the problems of a launch described on the host into `out`, those whose
 // tiles have the most K steps first where the launch takes more than one wave of
@@ -559,7 +565,7 @@ bool use_small_tiles(int total_tiles, int nprob) { return total_tiles < 148 || t
 // caller's order, 105.1 sorted.  key, idx: scratch of nprob each.
 void order_problems(const GemmProb* probs, int nprob, const GemmSeg* segs, int total_tiles, GemmProb* out, int* key,
                     int* idx) {
-  const bool small = use_small_tiles(total_tiles, nprob);
+  const bool small = use_small_tiles(total_tiles, nprob, gemm_tiles32(probs, nprob));
   if (nprob == 1 || (small ? 4L : 1L) * total_tiles <= (small ? 6L : 4L) * 148) {
     memcpy(out, probs, nprob * sizeof(GemmProb));
     return;
@@ -579,11 +585,11 @@ void order_problems(const GemmProb* probs, int nprob, const GemmSeg* segs, int t
   }
 }
 
-cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles,
+cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles, int tiles32,
                         cudaStream_t stream, const int* const* cmaps, bool scaled) {
   const cudaError_t e = pipe_attributes();
   if (e != cudaSuccess) return e;
-  const bool small = use_small_tiles(total_tiles, nprob);
+  const bool small = use_small_tiles(total_tiles, nprob, tiles32);
   const auto k = small ? (scaled ? gemm_grouped_pipe_kernel<32, true> : gemm_grouped_pipe_kernel<32, false>)
                        : (scaled ? gemm_grouped_pipe_kernel<64, true> : gemm_grouped_pipe_kernel<64, false>);
   k<<<(small ? 4 : 1) * total_tiles, NT, small ? pipe_smem<32>() : pipe_smem<64>(), stream>>>(d_probs, nprob, d_segs, cmaps);
@@ -597,7 +603,7 @@ cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs,
   int key[GEMM_INLINE_MAX / sizeof(GemmProb)], idx[GEMM_INLINE_MAX / sizeof(GemmProb)];
   order_problems(probs, nprob, segs, total_tiles, reinterpret_cast<GemmProb*>(d.b), key, idx);
   memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
-  const bool small = use_small_tiles(total_tiles, nprob), scaled = gemm_scaled(segs, nseg);
+  const bool small = use_small_tiles(total_tiles, nprob, gemm_tiles32(probs, nprob)), scaled = gemm_scaled(segs, nseg);
   const auto k = small ? (scaled ? gemm_grouped_inline_kernel<32, true, BYTES> : gemm_grouped_inline_kernel<32, false, BYTES>)
                        : (scaled ? gemm_grouped_inline_kernel<64, true, BYTES> : gemm_grouped_inline_kernel<64, false, BYTES>);
   k<<<(small ? 4 : 1) * total_tiles, NT, small ? pipe_smem<32>() : pipe_smem<64>(), stream>>>(d, nprob);
@@ -621,6 +627,13 @@ void gemm_assign_tiles(GemmProb& p, int& tiles, int& stiles) {
   stiles += ((p.m + LBM - 1) / LBM) * p.stiles_n * ks;
 }
 
+int gemm_tiles32(const GemmProb* probs, int nprob) {
+  int t = 0;
+  for (int p = 0; p < nprob; ++p)
+    t += ((probs[p].m + 31) / 32) * ((probs[p].n + 31) / 32) * (probs[p].ksplit > 1 ? probs[p].ksplit : 1);
+  return t;
+}
+
 bool gemm_scaled(const GemmSeg* segs, int nseg) {
   for (int s = 0; s < nseg; ++s)
     if (segs[s].alpha != 1.0) return true;
@@ -636,7 +649,7 @@ double gemm_flops(const GemmProb* probs, int nprob, const GemmSeg* segs) {
 }
 
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                int total_tiles, cudaStream_t stream, const char* tag, int total_stiles,
+                                int total_tiles, cudaStream_t stream, const char* tag, int tiles32, int total_stiles,
                                 const int* const* cmaps, bool scaled) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
   // 128x128 tiles when the schedule selects them for this problem size,
@@ -662,14 +675,14 @@ cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSe
     return cudaGetLastError();
   }
   cudaError_t e = cudaSuccess;
-  NRGB_LAUNCH(tag, stream, e = pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, cmaps, scaled));
+  NRGB_LAUNCH(tag, stream, e = pipe_launch(d_probs, nprob, d_segs, total_tiles, tiles32, stream, cmaps, scaled));
   return e;
 }
 
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                            int total_tiles, cudaStream_t stream, bool scaled) {
+                                            int total_tiles, int tiles32, cudaStream_t stream, bool scaled) {
   if (total_tiles <= 0 || nprob <= 0) return cudaSuccess;
-  return pipe_launch(d_probs, nprob, d_segs, total_tiles, stream, nullptr, scaled);
+  return pipe_launch(d_probs, nprob, d_segs, total_tiles, tiles32, stream, nullptr, scaled);
 }
 
 size_t gemm_desc_bytes(int nprob, int nseg) {
@@ -689,7 +702,8 @@ cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const Gem
   order_problems(probs, nprob, segs, total_tiles, ordered.data(), key.data(), idx.data());
   const GemmProb* dp = static_cast<const GemmProb*>(stage(ordered.data(), nprob * sizeof(GemmProb)));
   const GemmSeg* ds = static_cast<const GemmSeg*>(stage(segs, nseg * sizeof(GemmSeg)));
-  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, total_stiles, nullptr, gemm_scaled(segs, nseg));
+  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, gemm_tiles32(probs, nprob), total_stiles, nullptr,
+                             gemm_scaled(segs, nseg));
 }
 
 cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,

@@ -57,14 +57,17 @@ void gemm_assign_tiles(GemmProb& p, int& tiles, int& stiles);
 // cmaps (device, a pointer per problem; null: none): column j of problem p's
 // product goes to column cmaps[p][j] of its C.
 // scaled: some segment's alpha may differ from one (gemm_scaled).
+// tiles32: the 32 x 32 tiles inside the problems (gemm_tiles32).
 cudaError_t gemm_grouped_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                int total_tiles, cudaStream_t stream, const char* tag = "gemm_f64",
-                                int total_stiles = 0, const int* const* cmaps = nullptr, bool scaled = true);
+                                int total_tiles, cudaStream_t stream, const char* tag,
+                                int tiles32, int total_stiles = 0, const int* const* cmaps = nullptr,
+                                bool scaled = true);
+int gemm_tiles32(const GemmProb* probs, int nprob);
 
 // Same launch without the library's launch accounting (no host bookkeeping,
 // no events): used by the allocation-free entry point.
 cudaError_t gemm_grouped_launch_unaccounted(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs,
-                                            int total_tiles, cudaStream_t stream, bool scaled);
+                                            int total_tiles, int tiles32, cudaStream_t stream, bool scaled);
 
 // The same with the descriptors in host memory, passed as a kernel parameter
 // (gemm_inline_fits: up to GEMM_INLINE_MAX bytes): no copy to the device.

@@ -139,10 +139,12 @@ extern "C" int nrgb_basis_change_noalloc(int nops, const int* n_bra, const int* 
         cudaMemcpyAsync(d_s2, g_s2, np * sizeof(g_s2[0]), cudaMemcpyHostToDevice, st) != cudaSuccess)
       return 6;
     if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p1), np,
-                                              reinterpret_cast<nrgb::GemmSeg*>(d_s1), t1, st, false) != cudaSuccess)
+                                              reinterpret_cast<nrgb::GemmSeg*>(d_s1), t1, nrgb::gemm_tiles32(g_p1, np), st,
+                                              false) != cudaSuccess)
       return 6;
     if (nrgb::gemm_grouped_launch_unaccounted(reinterpret_cast<nrgb::GemmProb*>(d_p2), np,
-                                              reinterpret_cast<nrgb::GemmSeg*>(d_s2), t2, st, false) != cudaSuccess)
+                                              reinterpret_cast<nrgb::GemmSeg*>(d_s2), t2, nrgb::gemm_tiles32(g_p2, np), st,
+                                              false) != cudaSuccess)
       return 6;
   }
   // the static host staging is reused by the next call: wait until the GPU is done

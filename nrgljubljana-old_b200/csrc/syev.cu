@@ -1744,7 +1744,8 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         NRGB_CUDA(cudaGetLastError());
         NRGB_LAUNCH("dc_vectors", st, dc_vectors_kernel<<<gw, 256, 0, st>>>(d_dp, d_nodes));
         NRGB_CUDA(cudaGetLastError());
-        NRGB_CUDA(gemm_grouped_launch(d_gp, nn, d_gs, L.gb.tiles, st, "gemm_f64_dc", L.gb.stiles,
+        NRGB_CUDA(gemm_grouped_launch(d_gp, nn, d_gs, L.gb.tiles, st, "gemm_f64_dc",
+                                      gemm_tiles32(L.gb.probs.data(), nn), L.gb.stiles,
                                       reinterpret_cast<const int* const*>(dev + L.o_cm), false));
         launches_ += 7;
       }
@@ -1869,7 +1870,8 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
         KernelStats::get().add_work("gemm_f64_bt", gemm_flops(g.probs.data(), (int)g.probs.size(), g.segs.data()));
         NRGB_CUDA(gemm_grouped_launch(reinterpret_cast<const GemmProb*>(dev + o.first), (int)g.probs.size(),
                                       reinterpret_cast<const GemmSeg*>(dev + o.second), g.tiles, st, "gemm_f64_bt",
-                                      g.stiles, nullptr, gemm_scaled(g.segs.data(), (int)g.segs.size())));
+                                      gemm_tiles32(g.probs.data(), (int)g.probs.size()), g.stiles, nullptr,
+                                      gemm_scaled(g.segs.data(), (int)g.segs.size())));
         ++launches_;
       };
       if (kmax > 0) {

@@ -15,7 +15,7 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("alpha", [1.0, -0.7])
 @pytest.mark.parametrize("count,lo,hi", [(30, 130, 192), (60, 66, 128), (100, 66, 128), (250, 66, 100), (400, 40, 90),
-                                         (8, 600, 640)])
+                                         (8, 600, 640), (12, 384, 384)])
 def test_every_parameter_block(count, lo, hi, alpha):
     import nrgb
     g = torch.Generator(device="cuda:0").manual_seed(count)
