@@ -548,14 +548,19 @@ cudaError_t pipe_attributes() {
 // would leave SMs idle, or where the problems are small (60 tiles: an edge of
 // 480) and at least 3 % of the 64 x 64 tiles' area lies outside them in quarters
 // that 32 x 32 tiles leave out, so that the rims outweigh the operands read twice
-// as often.  Measured (64 / 32, us; area that is left out): one 500^3 44.8 / 29.1
+// as often (12 % more time for the same area), or the SMs with one tile more than
+// the others would cost more than that.  Measured (64 / 32, us; area that is left out): one 500^3 44.8 / 29.1
 // (idle SMs), four 300^3 32.4 / 26.0 (idle SMs), eight of 200-300 34.8 / 29.6 (14 %),
 // twelve of 400-500 120.5 / 105.8 (7 %), eighty of 100-300 84.0 / 83.9 (13 %), eight
 // 384^3 44.8 / 50.8 (none), forty 512^3 358.8 / 405.3 (none), two 700^3 70.6 / 80.9
-// (none).  Within 5 % either way, by how the last wave falls: eight of 300-400 45.7 /
+// (none), sixteen 448^3 156 / 166 (none; 13 % lost to the last tiles), forty products
+// of 256^3 134 / 119 (none; 16 %).  Within 5 % either way, by how the last wave falls: eight of 300-400 45.7 /
 // 46.1 (4 %), sixteen of them 75.8 / 78.2 (6 %), forty of 200-400 112.8 / 117.9 (9 %).
 bool use_small_tiles(int total_tiles, int nprob, int tiles32) {
-  return total_tiles < 148 || (total_tiles <= 60L * nprob && tiles32 <= 3.88 * total_tiles);
+  if (total_tiles < 148) return true;
+  if (total_tiles > 60L * nprob) return false;
+  const long busiest = (total_tiles + 147) / 148;  // tiles of the SM with the most
+  return tiles32 <= 3.88 * total_tiles || 148 * busiest > 1.15 * total_tiles;
 }
 
 // Copies the problems of a launch described on the host into `out`, those whose
