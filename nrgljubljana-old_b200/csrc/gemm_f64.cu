@@ -563,32 +563,45 @@ bool use_small_tiles(int total_tiles, int nprob, int tiles32) {
   return tiles32 <= 3.88 * total_tiles || 148 * busiest > 1.15 * total_tiles;
 }
 
-// Copies the problems of a launch described on the host into `out`, those whose
-// tiles have the most K steps first where the launch takes more than one wave of
-// CTAs (six per SM with T = 32, four with 64): the last wave then ends with short
+// Order of the problems of a launch described on the host: those whose tiles
+// have the most K steps first where the launch takes more than one wave of CTAs
+// (six per SM with T = 32, four with 64), so that the last wave ends with short
 // tiles.  64 outputs of four terms (K 15 to 115 each), 3544 CTAs: 112.9 us in the
-// caller's order, 105.1 sorted.  key, idx: scratch of nprob each.
-void order_problems(const GemmProb* probs, int nprob, const GemmSeg* segs, int total_tiles, GemmProb* out, int* key,
-                    int* idx) {
-  const bool small = use_small_tiles(total_tiles, nprob, gemm_tiles32(probs, nprob));
-  if (nprob == 1 || (small ? 4L : 1L) * total_tiles <= (small ? 6L : 4L) * 148) {
-    memcpy(out, probs, nprob * sizeof(GemmProb));
-    return;
+// caller's order, 105.1 sorted.  In 64 classes of steps, in time linear in the
+// problems (a comparison sort and a copy of descriptors that stayed as they were
+// took 15 to 20 us of host time for a thousand problems, more than it gave);
+// problems of one class keep their order.
+struct ProblemOrder {
+  static constexpr int CLASSES = 64;
+  int at[CLASSES + 1] = {};  // first place of a class, the longest first
+
+  // The problems' classes in key; false: the caller's order stands.
+  bool classes(const GemmProb* probs, int nprob, const GemmSeg* segs, int total_tiles, bool small, int* key) {
+    if (nprob == 1 || (small ? 4L : 1L) * total_tiles <= (small ? 6L : 4L) * 148) return false;
+    int most = 0;
+    for (int p = 0; p < nprob; ++p) {
+      long steps = 0;
+      for (int q = probs[p].seg0; q < probs[p].seg0 + probs[p].nseg; ++q)
+        if (segs[q].k > 0) steps += (segs[q].k + KB - 1) / KB;
+      key[p] = (int)std::min(steps / std::max(1, probs[p].ksplit), 0x7fffffffL);
+      most = std::max(most, key[p]);
+    }
+    const double scale = (CLASSES - 1) / std::max(1.0, (double)most);
+    bool ordered = true;
+    for (int p = 0; p < nprob; ++p) {
+      key[p] = CLASSES - 1 - (int)(key[p] * scale);
+      ++at[key[p] + 1];
+      ordered = ordered && (p == 0 || key[p - 1] <= key[p]);
+    }
+    return !ordered;
   }
-  for (int p = 0; p < nprob; ++p) {
-    long steps = 0;
-    for (int q = probs[p].seg0; q < probs[p].seg0 + probs[p].nseg; ++q)
-      if (segs[q].k > 0) steps += (segs[q].k + KB - 1) / KB;
-    key[p] = (int)std::min(steps / std::max(1, probs[p].ksplit), 0x7fffffffL);
-    idx[p] = p;
+  void copy(const GemmProb* probs, int nprob, const int* key, GemmProb* out) {
+    for (int c = 0; c < CLASSES; ++c) at[c + 1] += at[c];
+    for (int p = 0; p < nprob; ++p) out[at[key[p]]++] = probs[p];
+    int tiles = 0, stiles = 0;
+    for (int i = 0; i < nprob; ++i) gemm_assign_tiles(out[i], tiles, stiles);
   }
-  std::sort(idx, idx + nprob, [&](int a, int b) { return key[a] != key[b] ? key[a] > key[b] : a < b; });
-  int tiles = 0, stiles = 0;
-  for (int i = 0; i < nprob; ++i) {
-    out[i] = probs[idx[i]];
-    gemm_assign_tiles(out[i], tiles, stiles);
-  }
-}
+};
 
 cudaError_t pipe_launch(const GemmProb* d_probs, int nprob, const GemmSeg* d_segs, int total_tiles, int tiles32,
                         cudaStream_t stream, const int* const* cmaps, bool scaled) {
@@ -605,10 +618,12 @@ template <int BYTES>
 cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs, int nseg, int total_tiles,
                           cudaStream_t stream) {
   InlineDesc<BYTES> d;
-  int key[GEMM_INLINE_MAX / sizeof(GemmProb)], idx[GEMM_INLINE_MAX / sizeof(GemmProb)];
-  order_problems(probs, nprob, segs, total_tiles, reinterpret_cast<GemmProb*>(d.b), key, idx);
-  memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
   const bool small = use_small_tiles(total_tiles, nprob, gemm_tiles32(probs, nprob)), scaled = gemm_scaled(segs, nseg);
+  ProblemOrder order;
+  int key[GEMM_INLINE_MAX / sizeof(GemmProb)];
+  if (order.classes(probs, nprob, segs, total_tiles, small, key)) order.copy(probs, nprob, key, reinterpret_cast<GemmProb*>(d.b));
+  else memcpy(d.b, probs, nprob * sizeof(GemmProb));
+  memcpy(d.b + nprob * sizeof(GemmProb), segs, nseg * sizeof(GemmSeg));
   const auto k = small ? (scaled ? gemm_grouped_inline_kernel<32, true, BYTES> : gemm_grouped_inline_kernel<32, false, BYTES>)
                        : (scaled ? gemm_grouped_inline_kernel<64, true, BYTES> : gemm_grouped_inline_kernel<64, false, BYTES>);
   k<<<(small ? 4 : 1) * total_tiles, NT, small ? pipe_smem<32>() : pipe_smem<64>(), stream>>>(d, nprob);
@@ -702,12 +717,18 @@ cudaError_t gemm_grouped_launch_host(const GemmProb* probs, int nprob, const Gem
     NRGB_LAUNCH(tag, stream, e = gemm_grouped_launch_inline(probs, nprob, segs, nseg, total_tiles, stream));
     return e;
   }
-  std::vector<GemmProb> ordered(nprob);
-  std::vector<int> key(nprob), idx(nprob);
-  order_problems(probs, nprob, segs, total_tiles, ordered.data(), key.data(), idx.data());
-  const GemmProb* dp = static_cast<const GemmProb*>(stage(ordered.data(), nprob * sizeof(GemmProb)));
+  const int tiles32 = gemm_tiles32(probs, nprob);
+  ProblemOrder order;
+  std::vector<GemmProb> ordered;
+  std::vector<int> key(nprob);
+  if (order.classes(probs, nprob, segs, total_tiles, use_small_tiles(total_tiles, nprob, tiles32), key.data())) {
+    ordered.resize(nprob);
+    order.copy(probs, nprob, key.data(), ordered.data());
+    probs = ordered.data();
+  }
+  const GemmProb* dp = static_cast<const GemmProb*>(stage(probs, nprob * sizeof(GemmProb)));
   const GemmSeg* ds = static_cast<const GemmSeg*>(stage(segs, nseg * sizeof(GemmSeg)));
-  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, gemm_tiles32(probs, nprob), total_stiles, nullptr,
+  return gemm_grouped_launch(dp, nprob, ds, total_tiles, stream, tag, tiles32, total_stiles, nullptr,
                              gemm_scaled(segs, nseg));
 }
 
