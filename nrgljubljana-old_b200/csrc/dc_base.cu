@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "dc_base.cuh"
 #include "dc_secular.cuh"
+#include "reflector.cuh"
 
 namespace nrgb {
 
@@ -439,11 +440,12 @@ __device__ __forceinline__ void syev_tiny(const TinyProb P, int* fail) {
       const double xi = lane >= c + 2 ? ac : 0.0;
       const double xn2 = warp_sum(xi * xi);
       const double alpha = __shfl_sync(0xffffffffu, ac, c + 1);
-      double tc = 0.0, beta = alpha, scal = 0.0;
-      if (xn2 != 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-        tc = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
+      double tc, beta, scal;
+      reflector(alpha, xn2, beta, tc, scal);
+      if (squares_lost(alpha, xn2)) {
+        double inverse;
+        const double p = small_scale(alpha, (int)__reduce_max_sync(0xffffffffu, upper_word(xi)), inverse);
+        reflector_small(alpha, warp_sum(xi * p * (xi * p)), p, inverse, beta, tc, scal);
       }
       const double vi = lane == c + 1 ? 1.0 : xi * scal;
       m.v[c][lane] = vi;

@@ -24,6 +24,7 @@
 #include "dc_base.cuh"
 #include "dc_secular.cuh"
 #include "gemm_f64.cuh"
+#include "reflector.cuh"
 #include "syev.cuh"
 #include "schedule.cuh"
 #include "trd_grid.cuh"
@@ -381,6 +382,26 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
       const double alpha = __ldcg(&P.A[c + 1 + c * ld]);
       const double xn2 = ld_volatile(&R[0]);
       double beta = alpha, tc = 0.0, scal = 0.0;
+      const bool lost = squares_lost(alpha, xn2);
+      if (lost) {  // in every thread of every CTA, with the same sums
+        int* tops = reinterpret_cast<int*>(pqw);
+        int top = 0;
+        for (int r = jj + 1 + tid; r < S.M; r += TRD_NT) top = max(top, upper_word(__ldcg(&P.A[base + r + c * ld])));
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (lane == 0) tops[warp] = top;
+        __syncthreads();
+        for (int w = 0; w < nwarps; ++w) top = max(top, tops[w]);
+        double inverse, ss = 0.0;
+        const double p = small_scale(alpha, top, inverse);
+        for (int r = jj + 1 + tid; r < S.M; r += TRD_NT) {
+          const double x = __ldcg(&P.A[base + r + c * ld]) * p;
+          ss += x * x;
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) scratch[warp] = ss;
+        __syncthreads();
+        reflector_small(alpha, warp_sum(lane < nwarps ? scratch[lane] : 0.0), p, inverse, beta, tc, scal);
+      }
       // W and V of this warp's first rows, on the way while v is formed
       double wr[4], vr[4];
 #pragma unroll
@@ -396,11 +417,7 @@ __global__ void __launch_bounds__(TRD_NT, 1) trd_panel_kernel(const TrdProb* __r
           const int r = r0 + tid + u * TRD_NT;
           a[u] = (r > jj && r < S.M) ? __ldcg(&P.A[base + r + c * ld]) : 0.0;
         }
-        if (r0 == 0 && xn2 != 0.0) {
-          beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-          tc = (beta - alpha) / beta;
-          scal = 1.0 / (alpha - beta);
-        }
+        if (r0 == 0 && !lost) reflector(alpha, xn2, beta, tc, scal);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int r = r0 + tid + u * TRD_NT;

@@ -226,8 +226,28 @@ __device__ __forceinline__ void trd_grid_block(const TrdGridProb& P, int r, doub
     }
     if (tid == NT - 1 && jlast < t + 1) st_entry(P.ex + (t & 1) * stride + 4 * (n + 1) + 2 * r, 0.0, (unsigned long long)(t + 1));
     // ---- the reflector of column t, while the entries travel ----
+    const double nn = sum8(ssp), alpha = sc[1];
     double beta;
-    reflector(sc[1], sum8(ssp), beta, tc, scal);
+    reflector(alpha, nn, beta, tc, scal);
+    if (squares_lost(alpha, nn)) {  // in every thread or in none
+      int* xtop = reinterpret_cast<int*>(yvp);
+      int top = 0;
+#pragma unroll
+      for (int m = 0; m < M; ++m) top = max(top, upper_word(x[m]));
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) xtop[warp] = top;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < NW; ++w) top = max(top, xtop[w]);
+      double inverse, ss = 0.0;
+      const double p = small_scale(alpha, top, inverse);
+#pragma unroll
+      for (int m = 0; m < M; ++m) ss = fma(x[m] * p, x[m] * p, ss);
+      ss = warp_sum_mma(ss);
+      if (lane == 0) ssp[warp] = ss;
+      __syncthreads();
+      reflector_small(alpha, sum8(ssp), p, inverse, beta, tc, scal);
+    }
     if (r == 0 && tid == 0) {
       P.e[t] = beta;
       P.tau[t] = tc;

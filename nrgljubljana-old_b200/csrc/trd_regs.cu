@@ -97,10 +97,12 @@ __device__ __forceinline__ void cluster_sync_all() {
 
 // The power of two that brings the largest |x| of a column to [1, 2) (from the
 // upper words of the warps' largest; clamped to normal numbers), and its inverse.
-__device__ __forceinline__ double column_scale(const int* xtop, double& inverse) {
+__device__ __forceinline__ int column_top(const int* xtop) {
   const int4 a = *reinterpret_cast<const int4*>(xtop), b = *reinterpret_cast<const int4*>(xtop + 4);
-  const int top = max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
-  const int e = min(max(top >> 20, 1), 2045);
+  return max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
+}
+__device__ __forceinline__ double column_scale(const int* xtop, double& inverse) {
+  const int e = min(max(column_top(xtop) >> 20, 1), 2045);
   inverse = __hiloint2double(e << 20, 0);
   return __hiloint2double((2046 - e) << 20, 0);
 }
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       }
       int top = 0;
 #pragma unroll
-      for (int m = 0; m < M; ++m) top = max(top, __double2hiint(x[m]) & 0x7fffffff);
+      for (int m = 0; m < M; ++m) top = max(top, upper_word(x[m]));
       top = __reduce_max_sync(0xffffffffu, top);
       if (lane == 0) xtop[warp] = top;
     }
@@ -300,9 +302,19 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
         s0 = fma(u0, u0, s0);
         s1 = fma(u1, u1, s1);
       }
-      const double nn = warp_sum_mma(s0 + s1);
+      const double nn = warp_sum_mma(s0 + s1), alpha = scl[2 + (t & 1)];
       double beta;
-      reflector(scl[2 + (t & 1)], nn, beta, tc, scal);
+      reflector(alpha, nn, beta, tc, scal);
+      if (squares_lost(alpha, nn)) {
+        double inverse;
+        const double p = small_scale(alpha, column_top(xtop), inverse);
+        double s = 0.0;
+        for (int k = 0; k < KR * WR; ++k) {
+          const double u = X[lane + 32 * k] * p;
+          s = fma(u, u, s);
+        }
+        reflector_small(alpha, warp_sum_mma(s), p, inverse, beta, tc, scal);
+      }
       if (lane == 0) {
         scl[0] = tc;
         scl[1] = scal;
@@ -347,9 +359,20 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       tc = scl[0];
       scal = scl[1];
     } else {  // while the messages travel
-      const double nn = sum8(ssp);
+      const double nn = sum8(ssp), alpha = scl[2 + (t & 1)];
       double beta;
-      reflector(scl[2 + (t & 1)], nn, beta, tc, scal);
+      reflector(alpha, nn, beta, tc, scal);
+      if (squares_lost(alpha, nn)) {  // in every thread or in none
+        double inverse, ss = 0.0;
+        const double p = small_scale(alpha, column_top(xtop), inverse);
+#pragma unroll
+        for (int m = 0; m < M; ++m) ss = fma(x[m] * p, x[m] * p, ss);
+        ss = warp_sum_mma(ss);
+        __syncthreads();
+        if (lane == 0) ssp[warp] = ss;
+        __syncthreads();
+        reflector_small(alpha, sum8(ssp), p, inverse, beta, tc, scal);
+      }
       if (r == 0 && tid == 0) {
         P.e[t] = beta;
         P.tau[t] = tc;

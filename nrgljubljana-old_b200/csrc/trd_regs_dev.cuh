@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "reflector.cuh"
+
 namespace nrgb {
 namespace {
 
@@ -23,18 +25,6 @@ __device__ __forceinline__ double warp_sum_mma(double x) {
   s += __shfl_xor_sync(0xffffffffu, s, 8);
   s += __shfl_xor_sync(0xffffffffu, s, 16);
   return s;
-}
-
-// beta, tau and the scale of v of the reflector of a column with the entry
-// alpha below the diagonal and the squared norm nn under it.
-__device__ __forceinline__ void reflector(double alpha, double nn, double& beta, double& tau, double& scale) {
-  beta = alpha;
-  tau = scale = 0.0;
-  if (nn != 0.0) {
-    beta = -copysign(sqrt(fma(alpha, alpha, nn)), alpha);
-    tau = (beta - alpha) / beta;
-    scale = 1.0 / (alpha - beta);
-  }
 }
 
 __host__ __device__ constexpr int pow2_up(int c) { return c <= 1 ? 1 : c <= 2 ? 2 : c <= 4 ? 4 : c <= 8 ? 8 : 16; }
