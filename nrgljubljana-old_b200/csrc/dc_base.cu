@@ -414,20 +414,21 @@ __global__ void __launch_bounds__(G * CAP) dc_base_kernel(const DcBaseProb* __re
   if (i < P.s) P.D[P.lo + i] = m.D[i];
 }
 
-// Householder tridiagonalisation of a block of up to 32 rows by warp 0, one row
-// a lane in registers; divide and conquer by the CTA; the reflectors applied to
-// the eigenvectors, a column a thread.
+// Householder tridiagonalisation of a block of up to N rows by warp 0, one row
+// a lane in registers; divide and conquer by the CTA (4 N threads); the reflectors
+// applied to the eigenvectors, a column a thread.
+template <int N>
 struct TinySm {
-  DcSm<SYEV_TINY> dc;
-  double Z[SYEV_TINY * (SYEV_TINY + 1)];
-  double v[SYEV_TINY][SYEV_TINY + 2];  // reflectors
-  double w[SYEV_TINY], tau[SYEV_TINY];
+  DcSm<N> dc;
+  double Z[N * (N + 1)];
+  double v[N][N + 2];  // reflectors
+  double w[N], tau[N];
 };
 
+template <int N>
 __device__ __forceinline__ void syev_tiny(const TinyProb P, int* fail) {
-  constexpr int N = SYEV_TINY;
   extern __shared__ __align__(16) unsigned char raw[];
-  TinySm& m = *reinterpret_cast<TinySm*>(raw);
+  TinySm<N>& m = *reinterpret_cast<TinySm<N>*>(raw);
   const int n = P.n, tid = threadIdx.x, lane = tid & 31;
   if (tid < 32) {
     double a[N];
@@ -448,7 +449,7 @@ __device__ __forceinline__ void syev_tiny(const TinyProb P, int* fail) {
         reflector_small(alpha, warp_sum(xi * p * (xi * p)), p, inverse, beta, tc, scal);
       }
       const double vi = lane == c + 1 ? 1.0 : xi * scal;
-      m.v[c][lane] = vi;
+      if (lane < N) m.v[c][lane] = vi;
       if (lane == 0) {
         m.dc.E[c] = beta;
         m.tau[c] = tc;
@@ -467,7 +468,7 @@ __device__ __forceinline__ void syev_tiny(const TinyProb P, int* fail) {
       }
       const double pi = lane > c ? tc * ((p0 + p1) + (p2 + p3)) : 0.0;
       const double wi = pi - 0.5 * tc * warp_sum(pi * vi) * vi;
-      m.w[lane] = wi;
+      if (lane < N) m.w[lane] = wi;
       __syncwarp();
       double nx = 0.0;
 #pragma unroll
@@ -531,32 +532,51 @@ cudaError_t dc_base_launch(const DcBaseProb* d, int nprob, int smax, int* fail, 
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(G * SYEV_TINY) syev_tiny_kernel(const TinyProb* __restrict__ probs, int* fail) {
-  syev_tiny(probs[blockIdx.x], fail);
+template <int N>
+__global__ void __launch_bounds__(G * N) syev_tiny_kernel(const TinyProb* __restrict__ probs, int* fail) {
+  syev_tiny<N>(probs[blockIdx.x], fail);
 }
 
 // The descriptors of a call with few blocks, as a kernel parameter: no copy.
 struct TinyArgs {
   TinyProb p[TINY_INLINE];
 };
-__global__ void __launch_bounds__(G * SYEV_TINY) syev_tiny_inline_kernel(const __grid_constant__ TinyArgs args, int* fail) {
-  syev_tiny(args.p[blockIdx.x], fail);
+template <int N>
+__global__ void __launch_bounds__(G * N) syev_tiny_inline_kernel(const __grid_constant__ TinyArgs args, int* fail) {
+  syev_tiny<N>(args.p[blockIdx.x], fail);
 }
 
-cudaError_t syev_tiny_launch(const TinyProb* h, const TinyProb* d, int nprob, int* fail, cudaStream_t st) {
-  if (nprob <= 0) return cudaSuccess;
-  cudaError_t e = d ? cudaFuncSetAttribute(syev_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TinySm))
-                    : cudaFuncSetAttribute(syev_tiny_inline_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(TinySm));
+namespace {
+
+template <int N>
+cudaError_t tiny_launch(const TinyProb* h, const TinyProb* d, int nprob, int* fail, cudaStream_t st) {
+  const int smem = (int)sizeof(TinySm<N>);
+  cudaError_t e = d ? cudaFuncSetAttribute(syev_tiny_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+                    : cudaFuncSetAttribute(syev_tiny_inline_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   if (d) {
-    NRGB_LAUNCH("syev_small", st, syev_tiny_kernel<<<nprob, G * SYEV_TINY, sizeof(TinySm), st>>>(d, fail));
+    NRGB_LAUNCH("syev_small", st, syev_tiny_kernel<N><<<nprob, G * N, smem, st>>>(d, fail));
   } else {
     TinyArgs args;
     for (int i = 0; i < nprob; ++i) args.p[i] = h[i];
-    NRGB_LAUNCH("syev_small", st, syev_tiny_inline_kernel<<<nprob, G * SYEV_TINY, sizeof(TinySm), st>>>(args, fail));
+    NRGB_LAUNCH("syev_small", st, syev_tiny_inline_kernel<N><<<nprob, G * N, smem, st>>>(args, fail));
   }
   return cudaGetLastError();
+}
+
+}  // namespace
+
+// One launch, for the largest block: a CTA for up to 32 rows takes 37 KB of shared
+// memory, so that 6 share an SM, one for up to 8 rows 4 KB and a single warp.
+// Measured (kernel, us; 32 rows for all in brackets; before it a warp a block): 4000
+// blocks of 2 to 4 rows 28 (93; 38), of 8 56 (217; 145), of 16 187 (463 before).
+cudaError_t syev_tiny_launch(const TinyProb* h, const TinyProb* d, int nprob, int* fail, cudaStream_t st) {
+  if (nprob <= 0) return cudaSuccess;
+  int nmax = 0;
+  for (int i = 0; i < nprob; ++i) nmax = std::max(nmax, h[i].n);
+  return nmax <= 8    ? tiny_launch<8>(h, d, nprob, fail, st)
+         : nmax <= 16 ? tiny_launch<16>(h, d, nprob, fail, st)
+                      : tiny_launch<SYEV_TINY>(h, d, nprob, fail, st);
 }
 
 }  // namespace nrgb
