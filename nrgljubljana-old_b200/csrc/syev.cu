@@ -1180,10 +1180,6 @@ SyevBatched::~SyevBatched() {
 }
 
 namespace {
-struct Plan {
-  std::vector<int> small, big;
-};
-
 void plan_tree(int prob, int lo, int hi, std::vector<DcNode>& leaves,
                std::vector<std::pair<int, DcNode>>& merges, int& height) {
   if (hi - lo <= LEAF) {
@@ -1429,8 +1425,7 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       }
     };
     // Larger blocks go to the many-CTA kernel (trd_grid.cu) whole, those
-    // beyond its capacity after panel launches for their leading columns;
-    // without it, panel launches until the trailing block fits a cluster.
+    // beyond its capacity after panel launches for their leading columns.
     std::vector<int> jstop(nbig);
     {
       std::vector<TrdClProb> whole;
@@ -1442,8 +1437,6 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
           via_cluster[b] = 1;
         } else if (glim > 0) {
           jstop[b] = n <= glim ? 0 : ((n - glim + NB - 1) / NB) * NB;
-        } else if (clim > 0) {
-          jstop[b] = ((n - clim + NB - 1) / NB) * NB;
         }
       }
       launch_clusters(whole);
@@ -1621,16 +1614,6 @@ void SyevBatched::run(const std::vector<SyevDesc>& probs, cudaStream_t st) {
       for (int i = 0; i < NAUX; ++i)
         if (aux_[i]) NRGB_CUDA(cudaStreamSynchronize(aux_[i]));
       if (f) throw CudaError("syev: grid barrier timed out");
-    }
-    // without the many-CTA kernel: the trailing blocks in clusters
-    if (glim == 0) {
-      std::vector<TrdClProb> tails;
-      for (int b = 0; b < nbig; ++b) {
-        const int j = jstop[b], n = tp[b].n;
-        if (via_cluster[b] || j >= n) continue;
-        tails.push_back(TrdClProb{tp[b].A + j + (size_t)j * n, tp[b].d + j, tp[b].e + j, tp[b].tau + j, n - j, n});
-      }
-      launch_clusters(tails);
     }
     // WY factors of the blocks that take the slab back-transformation, beside
     // the divide and conquer

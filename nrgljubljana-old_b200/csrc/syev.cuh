@@ -6,16 +6,18 @@
 // is the eigenvector of w[r]; ldz == n).  A is destroyed.
 //
 // Pipeline (all problems of a batch advance together):
-//   n <= 32 : one warp per problem, Householder + implicit QR in shared memory.
-//   n  > 32 : 1) Householder tridiagonalisation, up to n = 640 in one
-//                thread-block cluster with the matrix in its registers
-//                (trd_regs.cu); the leading columns of larger blocks blocked
-//                (panel of 32 columns in a cooperative persistent kernel,
-//                trailing rank-64 update on the DMMA GEMM),
+//   n <= 32 : the whole solution in one CTA per block (dc_base.cu).
+//   n  > 32 : 1) Householder tridiagonalisation with the matrix in registers, up
+//                to n = 640 of one thread-block cluster (trd_regs.cu), up to 1776
+//                of as many SMs as it needs (trd_grid.cu); the leading columns
+//                of larger blocks in panels of 32 (cooperative persistent
+//                kernel, trailing rank-64 update on the DMMA GEMM),
 //             2) divide and conquer on the tridiagonal (Cuppen splitting,
-//                Gu-Eisenstat eigenvectors), merges of equal tree height of all
+//                Gu-Eisenstat eigenvectors), subtrees up to 128 rows in one CTA
+//                (dc_base.cu), above them merges of equal tree height of all
 //                problems in the same launches,
-//             3) back-transformation with blocked (WY) reflectors on the GEMM.
+//             3) back-transformation with blocked (WY) reflectors, up to n = 1616 by
+//                column slabs in one launch (bt_apply.cu), above on the GEMM.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -63,15 +65,17 @@ class SyevBatched : public EigSolver {
   // Launch statistics of the last run().
   int last_launches() const { return launches_; }
   // Largest block the cluster tridiagonalisation holds (0: cluster path off);
-  // larger blocks also take the cooperative panel launches.
+  // larger blocks take the many-CTA kernel, and panels before it.
   int cluster_nmax() const { return cl_use(); }
   // The cluster kernel's capacity, before the schedule's limit.
   int cluster_capacity() const { return cl_nmax_; }
-  // Bound of the grid-barrier waits of the panel launches: 2^poll_log2 polls
-  // (default 23, about a second) before a wait gives up with an error.
+  // Bound of the tridiagonalisations' waits: 2^poll_log2 polls of a grid barrier
+  // (default 23, about a second) before a wait gives up with an error, at most
+  // 2^21 of a word in the many-CTA kernel, 2^12 to 2^20 tries inside a cluster.
   void set_wait_limit(int poll_log2) { wait_log2_ = poll_log2; }
   // Host-side fault injection: while on, every panel launch's barriers
-  // expect one CTA more than is launched (a lost CTA), so each wait must
+  // expect one CTA more than is launched (a lost CTA) and the other
+  // tridiagonalisations a word that nobody sends, so each wait must
   // run out; run() then throws "grid barrier timed out".
   void inject_barrier_shortfall(bool on) { inject_shortfall_ = on; }
 
@@ -82,7 +86,6 @@ class SyevBatched : public EigSolver {
   int launches_ = 0;
   int wait_log2_ = 23;
   bool inject_shortfall_ = false;
-  int coop_ctas_ = 0;
   int sms_ = 0;
   int cl_nmax_ = 0;  // largest block it holds (0: cluster path off)
   // blocks up to this size go to the cluster kernel whole: the capacity, or

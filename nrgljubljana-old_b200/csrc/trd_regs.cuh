@@ -11,7 +11,7 @@ struct TrdClProb {
   double* e;    // n-1
   double* tau;  // n-1
   int n;
-  int ld;       // n for a whole block; the block's size for its trailing part
+  int ld;
 };
 
 // The kernel a block of size n takes: a shape (rows and columns per CTA) and

@@ -276,7 +276,6 @@ struct NrgDriver::Impl {
   };
   // device scratch for descriptors
   DeviceArena desc;
-  size_t desc_off = 0;
 
   // device truncation: splitting map, step workspace, the per-step record
   TruncState tstate;
