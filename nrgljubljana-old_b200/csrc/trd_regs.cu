@@ -35,8 +35,9 @@
 //    ninth warp forms the reflector beside the products.
 //
 // Measured on one B200 (a block alone; before: the shared-memory kernel with
-// one cluster barrier per column): n = 64 0.06 ms, n = 128 0.16, n = 256 0.35,
-// n = 301 0.41 (before 1.35), n = 464 0.73 (2.3), n = 512 0.80, n = 640 1.5 (3.3).
+// one cluster barrier per column): n = 64 0.066 ms, n = 128 0.166, n = 256 0.37,
+// n = 301 0.44 (before 1.35), n = 464 0.75 (2.3), n = 512 0.82, n = 640 1.6 (3.3).
+// The scaling by p and the test for lost squares are 2 to 8 % of that.
 #include <math.h>
 #include <stdint.h>
 
@@ -260,9 +261,7 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
     }
     if (t == n - 1) break;
     __syncthreads();
-    // (nothing is armed or sent after a wait that ran out: the transaction counts
-    // would leave their range)
-    if (!ONE && gave_up) break;
+    const int stop = ONE ? 0 : gave_up;
     if (warp < NW) {
       // ---- matrix: rank-2 update, products of the columns with x ----
       double vj[C], wj[C], acc[C];
@@ -323,6 +322,9 @@ __global__ void __launch_bounds__(trdr::threads(ONE), 1)
       }
     }
     __syncthreads();
+    // (nothing is armed or sent after a wait that ran out: the transaction counts
+    // would leave their range)
+    if (stop) break;
     // ---- S, R of this CTA's columns and P: into the buffer (one CTA), or
     // from every warp to its share of the cluster's CTAs ----
     auto column = [&](int l) {
