@@ -632,8 +632,9 @@ cudaError_t inline_launch(const GemmProb* probs, int nprob, const GemmSeg* segs,
 
 // The 128x128 cp.async variant is used only where the device's schedule
 // (schedule.cuh, set by the autotuner's measurements) says it wins: by
-// default never (measured on B200 at first: 21-25 TF/s against 25-28 TF/s
-// for a register-staged 64x64 kernel on the same shapes).
+// default never (the autotuner's launches on B200: 21-24 TF/s at edges of 256 to
+// 2048 against 28-29 TF/s for the tiles above; 27.8 against 27.6 at 192, which
+// is within its margin).
 
 }  // namespace
 
